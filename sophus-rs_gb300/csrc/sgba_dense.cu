@@ -940,14 +940,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_dense_cluster(DenseArgs a, Ctrl
 // ---------------------------------------------------------------------------
 // Small reduced systems (n <= kSmallMax: local windows of up to 40 cameras):
 // one CTA, the lower triangle of S in float-float in shared memory (packed
-// by rows), LDL^T with the PSD-aware pivot rule and the forward substitution
-// of b fused into it (one barrier per pivot: every thread evaluates the pivot
-// itself; the trailing rows are dealt to the warps, a row's entries to the
-// lanes), then the diagonal and the backward sweep.  Float-float resolves
-// these systems without refinement (their scale gauge is held only by the
-// damping, which an FP32 factor with refinement does not resolve for windows
-// of 26-40 cameras); the cluster kernel's fixed costs (cluster barriers, a
-// large code footprint that starts cold on each SM) dominate at this size.
+// by rows), LDL^T with the PSD-aware pivot rule, the rhs (and the equality
+// columns) carried as rows below the matrix, then the backward sweep.
+// Float-float resolves these systems without refinement (their scale gauge is
+// held only by the damping, which an FP32 factor with refinement does not
+// resolve for windows of 26-40 cameras); the cluster kernel's fixed costs
+// (cluster barriers, a large code footprint that starts cold on each SM)
+// dominate at this size.
+//
+// Bound: the serial pivot chain (rcp, scale, update: ~110 cycles a pivot) for
+// small systems, FP32 issue (n^3 / 6 float-float products of 12 operations on
+// one SM) for large ones.  So the elimination goes by panels of one pose block
+// (6 pivots, the span of the pivot rule's running maximum): one warp factors
+// the 6 x 6 block in registers, a thread per row solves the panel, and the
+// trailing triangle takes all six columns at once in register tiles (RT x RT
+// entries a thread, 4 RT x 8 RT a warp: each entry is read and written once
+// per panel and a loaded operand feeds RT products).  Warp 0 updates and
+// factors the next diagonal block while the others work through the tiles
+// (look-ahead), so a panel costs two barriers and the pivot chain is hidden
+// where the tiles take longer than it.  L is never stored: entries below the
+// diagonal stay unscaled (U = L D) and the products scale by 1/d as they load
+// them, which keeps 40 cameras within one CTA's shared memory.
 // ---------------------------------------------------------------------------
 constexpr int kSmallMax = 234;
 
@@ -967,85 +980,252 @@ __device__ __forceinline__ dd sd_rcp(dd d) {
   return dd_fast_two_sum(r0, __fmul_rn(r0, e));
 }
 
-__device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl, int bid_, int nblk_) {
-  (void)bid_;
-  (void)nblk_;
+// a - (x y): the one operation of the elimination and of the sweeps.  Every
+// entry meets its pivots in order, each as this product and difference, so
+// the panel width and the tiles do not change a result's bits.
+__device__ __forceinline__ dd sd_msub(dd a, dd x, dd y) { return dd_sub(a, dd_mul(x, y)); }
+
+// One warp, every lane the same: LDL^T of the 6 x 6 diagonal block at c0 in
+// registers.  U below the diagonal back to A, 1/d to rdv.  Returns whether a
+// pivot was not finite.
+__device__ __forceinline__ bool sd_diag6(float2* A, float2* rdv, int c0, int lane) {
+  dd d[6][6], r[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int q = 0; q <= i; ++q) d[i][q] = sd_f2dd(A[sd_at(c0 + i, c0 + q)]);
+  float maxp = 1.0f;  // running maximum pivot of the pose block (>= 1)
+  bool bad = false;
+#pragma unroll
+  for (int t = 0; t < 6; ++t) {
+    const float ad = fabsf(d[t][t].hi);
+    const bool fin = ad <= 3.402823466e38f;
+    const bool zero = !fin || !(ad > maxp * kTolRel);
+    bad = bad || !fin;
+    maxp = zero ? maxp : fmaxf(maxp, ad);
+    const dd rc = sd_rcp(d[t][t]);
+    r[t] = zero ? dd_make(0.0f, 0.0f) : rc;
+#pragma unroll
+    for (int i = t + 1; i < 6; ++i) {
+      const dd l = dd_mul(d[i][t], r[t]);
+#pragma unroll
+      for (int q = t + 1; q <= i; ++q) d[i][q] = sd_msub(d[i][q], l, d[q][t]);
+    }
+  }
+  __syncwarp();  // every lane has read the block
+  if (lane == 0) {
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      rdv[c0 + t] = sd_dd2f(r[t]);
+#pragma unroll
+      for (int q = 0; q < t; ++q) A[sd_at(c0 + t, c0 + q)] = sd_dd2f(d[t][q]);
+    }
+  }
+  return bad;
+}
+
+// The triangle is covered by tiles of RH rows and 2 RH columns: row tile x
+// has x / 2 + 1 of them, the first x row tiles sd_tiles(x).
+__device__ __forceinline__ int sd_tiles(int x) {
+  const int h = x >> 1;
+  return (x & 1) ? (h + 1) * (h + 1) : h * (h + 1);
+}
+
+// Trailing update of the entries (i, j), c1 <= j <= i, of one warp tile by the
+// six columns from c0: a_ij -= (U_ik / d_k) U_jk, k in order.  The next
+// diagonal block (rows and columns below c1 + 6) is left to the look-ahead.
+template <int RT>
+__device__ __forceinline__ void sd_tile(float2* A, const float2* rdv, int m, int c0, int n, int lane) {
+  constexpr int RH = 4 * RT, CW = 8 * RT;
+  const int c1 = c0 + 6;
+  int x = static_cast<int>(2.0f * sqrtf(static_cast<float>(n)));
+  while (sd_tiles(x) > n) --x;
+  while (sd_tiles(x + 1) <= n) ++x;
+  const int R0 = c1 + x * RH, C0 = c1 + (n - sd_tiles(x)) * CW;
+  if (C0 >= m) return;
+  const int li = lane >> 3, lj = lane & 7;
+  float2* pr[RT];
+  const float2* pc[RT];
+#pragma unroll
+  for (int q = 0; q < RT; ++q) {
+    pr[q] = A + sd_at(min(R0 + li + 4 * q, m - 1), 0);
+    pc[q] = A + sd_at(min(C0 + lj + 8 * q, m - 1), 0);
+  }
+  dd acc[RT][RT];
+#pragma unroll
+  for (int q = 0; q < RT; ++q)
+#pragma unroll
+    for (int u = 0; u < RT; ++u) {
+      const int i = R0 + li + 4 * q, j = C0 + lj + 8 * u;
+      acc[q][u] = (i < m && j <= i) ? sd_f2dd(pr[q][j]) : dd_make(0.0f, 0.0f);
+    }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const dd rd = sd_f2dd(rdv[c0 + k]);
+    dd l[RT], u[RT];
+#pragma unroll
+    for (int q = 0; q < RT; ++q) {
+      l[q] = dd_mul(sd_f2dd(pr[q][c0 + k]), rd);
+      u[q] = sd_f2dd(pc[q][c0 + k]);
+    }
+#pragma unroll
+    for (int q = 0; q < RT; ++q)
+#pragma unroll
+      for (int v = 0; v < RT; ++v) acc[q][v] = sd_msub(acc[q][v], l[q], u[v]);
+  }
+#pragma unroll
+  for (int q = 0; q < RT; ++q)
+#pragma unroll
+    for (int u = 0; u < RT; ++u) {
+      const int i = R0 + li + 4 * q, j = C0 + lj + 8 * u;
+      if (i < m && j <= i && i >= c1 + 6) pr[q][j] = sd_dd2f(acc[q][u]);
+    }
+}
+
+template <int RT>
+__device__ __forceinline__ void sd_trailing(float2* A, const float2* rdv, int m, int c0, int* next, int lane) {
+  const int ntile = sd_tiles((m - c0 - 6 + 4 * RT - 1) / (4 * RT));
+  for (;;) {
+    int n = 0;
+    if (lane == 0) n = atomicAdd(next, 1);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (n >= ntile) break;
+    sd_tile<RT>(A, rdv, m, c0, n, lane);
+  }
+}
+
+// NT threads; the same results for any NT (an entry's arithmetic does not
+// depend on which warp takes its tile).
+template <int NT>
+__device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl) {
   if (skipping(ctrl)) return;
   extern __shared__ __align__(16) float2 sm[];
-  const int m = a.n;
-  float2* A = sm;                      // lower triangle, packed by rows
-  float2* y = sm + m * (m + 1) / 2;    // rhs -> z -> x
-  float2* rdv = y + m;                 // reciprocal pivots
+  constexpr int NW = NT / 32;
+  const int m = a.n;                   // a multiple of 6
   // equality constraints: columns Y_k = S^-1 G_k^T solved beside the rhs
   // (range-space KKT, schur_ldlt.rs:674-772)
   const int ne = a.n_eq;
-  float2* yg = rdv + m;                // ne x m
-  __shared__ int s_bad;
+  float2* A = sm;                      // lower triangle, packed by rows
+  float2* y = sm + m * (m + 1) / 2;    // rhs -> z -> x
+  float2* yg = y + m;                  // ne x m
+  float2* rdv = yg + ne * m;           // reciprocal pivots
+  __shared__ int s_bad, s_next[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_bad = 0;
-  for (int i = warp; i < m; i += 8)
-    for (int j = lane; j <= i; j += 32) A[sd_at(i, j)] = a.S2[static_cast<int64_t>(i) * m + j];
-  for (int i = tid; i < m; i += 256) y[i] = sd_dd2f(dd_from_double(a.b[i]));
-  for (int e = tid; e < ne * m; e += 256) yg[e] = make_float2(0.0f, 0.0f);
+  if (tid == 0) s_bad = s_next[0] = s_next[1] = 0;
+  for (int i = warp; i < m; i += NW)
+    for (int j = lane; j <= i; j += 32) {
+      const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(A + sd_at(i, j)));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(a.S2 + static_cast<int64_t>(i) * m + j)
+                   : "memory");
+    }
+  for (int i = tid; i < m; i += NT) y[i] = sd_dd2f(dd_from_double(a.b[i]));
+  for (int e = tid; e < ne * m; e += NT) yg[e] = make_float2(0.0f, 0.0f);
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   if (tid < ne && a.eq_fb[tid] >= 0)
     for (int i = 0; i < 3; ++i) yg[tid * m + 6 * a.eq_fb[tid] + 3 + i] = sd_dd2f(dd_from_double(a.eq_jac[3 * tid + i]));
-  __syncthreads();
-  float maxp = 1.0f;
-  for (int t = 0; t < m; ++t) {
-    dd dt = sd_f2dd(A[sd_at(t, t)]);
-    if (t % 6 == 0) maxp = 1.0f;  // a new pose block
-    const float tol = fmaxf(maxp, 1.0f) * 1e-12f;
-    bool bad = false;
-    if (!isfinite(dt.hi)) {
-      bad = true;
-      dt = dd_make(0.0f, 0.0f);
-    } else if (fabsf(dt.hi) <= tol) {
-      dt = dd_make(0.0f, 0.0f);
-    } else {
-      maxp = fmaxf(maxp, fabsf(dt.hi));
+  if (warp == 0 && sd_diag6(A, rdv, 0, lane)) s_bad = 1;
+  for (int c0 = 0; c0 < m; c0 += 6) {
+    const int c1 = c0 + 6, buf = (c0 / 6) & 1;
+    __syncthreads();  // the diagonal block of this panel is factored, the previous panel's tiles are done
+    if (tid == 0) s_next[buf ^ 1] = 0;
+    const float2* dg[6];
+    dd rd[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      dg[k] = A + sd_at(c0 + k, c0);
+      rd[k] = sd_f2dd(rdv[c0 + k]);
     }
-    const dd rd = (dt.hi == 0.0f) ? dd_make(0.0f, 0.0f) : sd_rcp(dt);
-    if (tid == 0) {
-      rdv[t] = sd_dd2f(rd);
-      if (bad) s_bad = 1;
-    }
-    const dd yt = sd_f2dd(y[t]);
-    // trailing rows i > t: a_iq -= (a_it rd) a_qt for t < q <= i; y_i -= (a_it rd) y_t
-    for (int i = t + 1 + warp; i < m; i += 8) {
-      const dd li = dd_mul(sd_f2dd(A[sd_at(i, t)]), rd);
-      const int ri = sd_at(i, 0);
-      for (int q = t + 1 + lane; q <= i; q += 32) {
-        const dd v = dd_sub(sd_f2dd(A[ri + q]), dd_mul(li, sd_f2dd(A[sd_at(q, t)])));
-        A[ri + q] = sd_dd2f(v);
+    // the panel, a thread per row: U_ik = a_ik - sum_{q<k} (U_iq / d_q) U_kq;
+    // threads m .. m + ne: the rhs and the equality columns, z_k = y_k -
+    // sum_{q<k} (U_kq / d_q) z_q
+    for (int i = c1 + tid; i < m + 1 + ne; i += NT) {
+      const bool mat = i < m;
+      float2* r = (mat ? A + sd_at(i, 0) : y + (i - m) * m) + c0;
+      dd u[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) u[k] = sd_f2dd(r[k]);
+#pragma unroll
+      for (int q = 0; q < 5; ++q) {
+        const dd l = dd_mul(u[q], rd[q]);
+#pragma unroll
+        for (int k = q + 1; k < 6; ++k) {
+          const dd v = sd_f2dd(dg[k][q]);
+          u[k] = mat ? sd_msub(u[k], l, v) : sd_msub(u[k], dd_mul(v, rd[q]), u[q]);
+        }
       }
-      if (lane == 0) y[i] = sd_dd2f(dd_sub(sd_f2dd(y[i]), dd_mul(li, yt)));
-      if (lane >= 1 && lane <= ne) {
-        float2* yk = yg + (lane - 1) * m;
-        yk[i] = sd_dd2f(dd_sub(sd_f2dd(yk[i]), dd_mul(li, sd_f2dd(yk[t]))));
-      }
+#pragma unroll
+      for (int k = 1; k < 6; ++k) r[k] = sd_dd2f(u[k]);
     }
     __syncthreads();
+    if (c1 >= m) break;
+    if (warp == 0) {  // look-ahead: the next diagonal block
+      if (lane < 21) {
+        const int i = lane >= 15 ? 5 : lane >= 10 ? 4 : lane >= 6 ? 3 : lane >= 3 ? 2 : lane >= 1 ? 1 : 0;
+        const int q = lane - i * (i + 1) / 2;
+        const float2* ri = A + sd_at(c1 + i, c0);
+        const float2* rq = A + sd_at(c1 + q, c0);
+        dd acc = sd_f2dd(A[sd_at(c1 + i, c1 + q)]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc = sd_msub(acc, dd_mul(sd_f2dd(ri[k]), rd[k]), sd_f2dd(rq[k]));
+        A[sd_at(c1 + i, c1 + q)] = sd_dd2f(acc);
+      }
+      __syncwarp();
+      if (sd_diag6(A, rdv, c1, lane)) s_bad = 1;
+    }
+    // the rhs and the equality columns (the last threads: warp 0 is busy)
+    for (int e = 0; e <= ne; ++e) {
+      float2* w = y + e * m;
+      for (int j = c1 + NT - 1 - tid; j < m; j += NT) {
+        const float2* rj = A + sd_at(j, c0);
+        dd acc = sd_f2dd(w[j]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc = sd_msub(acc, dd_mul(sd_f2dd(rj[k]), rd[k]), sd_f2dd(w[c0 + k]));
+        w[j] = sd_dd2f(acc);
+      }
+    }
+    // tile size by the rows left: the largest that still gives every warp two
+    // tiles, so that the last round is not mostly idle
+    const int left = m - c1;
+    if (NT > 256 && sd_tiles((left + 15) / 16) >= 2 * NW) sd_trailing<4>(A, rdv, m, c0, &s_next[buf], lane);
+    else if (sd_tiles((left + 7) / 8) >= NW) sd_trailing<2>(A, rdv, m, c0, &s_next[buf], lane);
+    else sd_trailing<1>(A, rdv, m, c0, &s_next[buf], lane);
   }
-  // L columns (a_it rd_t), the diagonal solve
-  for (int i = warp; i < m; i += 8)
-    for (int t = lane; t < i; t += 32) {
-      const int e = sd_at(i, t);
-      A[e] = sd_dd2f(dd_mul(sd_f2dd(A[e]), sd_f2dd(rdv[t])));
-    }
-  for (int i = tid; i < m; i += 256) y[i] = sd_dd2f(dd_mul(sd_f2dd(y[i]), sd_f2dd(rdv[i])));
-  for (int e = tid; e < ne * m; e += 256) yg[e] = sd_dd2f(dd_mul(sd_f2dd(yg[e]), sd_f2dd(rdv[e % m])));
+  // backward: x_t = z_t / d_t - sum_{i>t} (U_it / d_t) x_i, i from the last, by
+  // pose blocks.  A warp per column carries the chain (its next block takes
+  // the newest x, then is solved), the other threads fold the newest x into
+  // the earlier entries; one barrier per block.
+  for (int t = tid; t < m * (1 + ne); t += NT) y[t] = sd_dd2f(dd_mul(sd_f2dd(y[t]), sd_f2dd(rdv[t % m])));
   __syncthreads();
-  // backward: x_t final, then x_i -= L_ti x_t for i < t (the rhs and every Y column)
-  for (int t = m - 1; t > 0; --t) {
-    const dd xt = sd_f2dd(y[t]);
-    const int rt = sd_at(t, 0);
-    for (int e = tid; e < (1 + ne) * t; e += 256) {
-      const int col = e / t, i = e - col * t;
-      float2* v = col == 0 ? y : yg + (col - 1) * m;
-      const dd vt = col == 0 ? xt : sd_f2dd(v[t]);
-      v[i] = sd_dd2f(dd_sub(sd_f2dd(v[i]), dd_mul(sd_f2dd(A[rt + i]), vt)));
+  for (int c0 = m - 6; c0 >= 0; c0 -= 6) {
+    const int cn = c0 + 6;  // the block solved last
+    auto fold = [&](float2* w, int j) {
+      const dd rd = sd_f2dd(rdv[j]);
+      dd acc = sd_f2dd(w[j]);
+#pragma unroll
+      for (int k = 5; k >= 0; --k) acc = sd_msub(acc, dd_mul(sd_f2dd(A[sd_at(cn + k, j)]), rd), sd_f2dd(w[cn + k]));
+      w[j] = sd_dd2f(acc);
+    };
+    for (int e = warp; e <= ne; e += NW) {
+      float2* w = y + e * m;
+      if (cn < m && lane < 6) fold(w, c0 + lane);
+      __syncwarp();
+      dd x[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) x[k] = sd_f2dd(w[c0 + k]);
+#pragma unroll
+      for (int k = 5; k >= 1; --k)
+#pragma unroll
+        for (int q = 0; q < k; ++q)
+          x[q] = sd_msub(x[q], dd_mul(sd_f2dd(A[sd_at(c0 + k, c0 + q)]), sd_f2dd(rdv[c0 + q])), x[k]);
+      __syncwarp();
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[c0 + k] = sd_dd2f(x[k]);
     }
+    if (cn < m)
+      for (int e = 0; e <= ne; ++e)
+        for (int j = NT - 1 - tid; j < c0; j += NT) fold(y + e * m, j);
     __syncthreads();
   }
   if (ne > 0) {
@@ -1097,14 +1277,14 @@ __device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl, int bi
       }
     }
     __syncthreads();
-    for (int i = tid; i < m; i += 256) {
+    for (int i = tid; i < m; i += NT) {
       dd v = sd_f2dd(y[i]);
       for (int p = 0; p < ne; ++p) v = dd_sub(v, dd_mul(sd_f2dd(yg[p * m + i]), dd_from_double(s_dlam[p])));
       y[i] = sd_dd2f(v);
     }
     __syncthreads();
   }
-  for (int i = tid; i < m; i += 256) {
+  for (int i = tid; i < m; i += NT) {
     const dd v = sd_f2dd(y[i]);
     a.x[i] = dd_to_double(v);
     a.xdd[2 * i] = v.hi;
@@ -1112,13 +1292,19 @@ __device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl, int bi
   }
   if (tid == 0 && s_bad) ctrl->skip = 2;  // NonFinitePivot -> solve failure -> reject
 }
-__global__ void __launch_bounds__(256, 1) k_small_dense(DenseArgs a, Ctrl* ctrl) {
-  small_dense_body(a, ctrl, blockIdx.x, gridDim.x);
+template <int NT>
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 3) k_small_dense(DenseArgs a, Ctrl* ctrl) {
+  small_dense_body<NT>(a, ctrl);
 }
 
 size_t small_dense_smem(int n, int n_eq = 0) {
   return sizeof(float2) * (static_cast<size_t>(n) * (n + 1) / 2 + (2 + static_cast<size_t>(n_eq)) * n);
 }
+
+// Small windows (up to 56 KiB, 19 cameras) take 256 threads so that several
+// share an SM in the batched launch; larger ones fill an SM with 512.
+constexpr size_t kSmallHalf = 56 * 1024;
+int small_dense_threads(size_t smem) { return smem <= kSmallHalf ? 256 : 512; }
 
 size_t dense_smem_bytes(int P, int C) {
   size_t m = 0;
@@ -1217,21 +1403,17 @@ int dense_cluster_choose(int P, int* cluster, size_t* smem) {
 
 int small_dense_setup_eq(int n, int n_eq) {
   if (n <= 0 || n > kSmallMax || n_eq < 0 || n_eq > kMaxEq) return 0;
-  if (raise_dynamic_smem(reinterpret_cast<const void*>(k_small_dense), small_dense_smem(n, n_eq)) != cudaSuccess) {
+  const size_t bytes = small_dense_smem(n, n_eq);
+  const void* fn = small_dense_threads(bytes) == 256 ? reinterpret_cast<const void*>(k_small_dense<256>)
+                                                     : reinterpret_cast<const void*>(k_small_dense<512>);
+  if (raise_dynamic_smem(fn, bytes) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return 1;
 }
 
-int small_dense_setup(int n) {
-  if (n <= 0 || n > kSmallMax) return 0;
-  if (raise_dynamic_smem(reinterpret_cast<const void*>(k_small_dense), small_dense_smem(n)) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return 1;
-}
+int small_dense_setup(int n) { return small_dense_setup_eq(n, 0); }
 
 namespace {
 
@@ -1273,7 +1455,9 @@ DenseArgs dense_cluster_args(const Sizes& s, const Dev& d) {
 }  // namespace
 
 int launch_small_dense(const Sizes& s, const Dev& d, cudaStream_t st) {
-  k_small_dense<<<1, 256, small_dense_smem(s.n6, s.n_eq), st>>>(small_dense_args(s, d), d.ctrl);
+  const size_t smem = small_dense_smem(s.n6, s.n_eq);
+  if (small_dense_threads(smem) == 256) k_small_dense<256><<<1, 256, smem, st>>>(small_dense_args(s, d), d.ctrl);
+  else k_small_dense<512><<<1, 512, smem, st>>>(small_dense_args(s, d), d.ctrl);
   return 1;
 }
 
@@ -1304,9 +1488,10 @@ int launch_dense_cluster(const Sizes& s, const Dev& d, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 namespace {
 
-__global__ void __launch_bounds__(256, 1) k_small_dense_w(const DenseArgs* args, Ctrl* const* ctrl,
-                                                          const int32_t* win) {
-  small_dense_body(args[blockIdx.x], ctrl[win[blockIdx.x]], 0, 1);
+template <int NT>
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 3) k_small_dense_w(const DenseArgs* args, Ctrl* const* ctrl,
+                                                                        const int32_t* win) {
+  small_dense_body<NT>(args[blockIdx.x], ctrl[win[blockIdx.x]]);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_dense_cluster_w(const DenseArgs* args, Ctrl* const* ctrl,
@@ -1356,7 +1541,7 @@ DenseBatch* dense_batch_create(const std::vector<BatchWin>& wins, Ctrl* const* c
       // by shared memory, so that small windows share an SM: <= 56 KiB,
       // <= 112 KiB, larger (keys 0, -1, -2)
       const size_t b = small_dense_smem(s.n6);
-      const int g = group_of(b <= 56 * 1024 ? 0 : (b <= 112 * 1024 ? -1 : -2));
+      const int g = group_of(b <= kSmallHalf ? 0 : (b <= 112 * 1024 ? -1 : -2));
       args[g].push_back(small_dense_args(s, d));
       win[g].push_back(static_cast<int32_t>(w));
       smem[g] = std::max(smem[g], small_dense_smem(s.n6));
@@ -1394,7 +1579,8 @@ DenseBatch* dense_batch_create(const std::vector<BatchWin>& wins, Ctrl* const* c
     G.args = reinterpret_cast<const DenseArgs*>(static_cast<unsigned char*>(b->dbuf) + a_at[g]);
     G.win = reinterpret_cast<const int32_t*>(static_cast<unsigned char*>(b->dbuf) + w_at[g]);
     const void* fn = G.cluster ? reinterpret_cast<const void*>(k_dense_cluster_w)
-                               : reinterpret_cast<const void*>(k_small_dense_w);
+                               : small_dense_threads(G.smem) == 256 ? reinterpret_cast<const void*>(k_small_dense_w<256>)
+                                                                  : reinterpret_cast<const void*>(k_small_dense_w<512>);
     e = raise_dynamic_smem(fn, G.smem);
     if (e == cudaSuccess && G.cluster > 8)
       e = cudaFuncSetAttribute(k_dense_cluster_w, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -1419,7 +1605,8 @@ int launch_dense_batch(const DenseBatch* b, cudaStream_t st) {
   for (const DenseGroup& G : b->groups) {
     if (G.count == 0) continue;
     if (G.cluster == 0) {
-      k_small_dense_w<<<G.count, 256, G.smem, st>>>(G.args, b->ctrl, G.win);
+      if (small_dense_threads(G.smem) == 256) k_small_dense_w<256><<<G.count, 256, G.smem, st>>>(G.args, b->ctrl, G.win);
+      else k_small_dense_w<512><<<G.count, 512, G.smem, st>>>(G.args, b->ctrl, G.win);
     } else {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(static_cast<unsigned>(G.cluster * G.count));

@@ -843,12 +843,16 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   for (int k = 0; k < 3; ++k) s.gauge_center[k] = P.gauge_center[k];
   int st;
   // host staging of the copies below: alive until the stream is synchronised
-  sgba::RawVec<double2> uv(P.no);
+  sgba::RawVec<float4> uv(P.no);
   std::vector<int32_t> cpt(1, 0);
   std::vector<double> poses(desc->poses, desc->poses + 7 * P.nc);
   std::vector<double> pts(desc->points, desc->points + 3 * P.np);
   par_ranges(P.no, [&](int64_t b, int64_t e) {
-    for (int64_t k = b; k < e; ++k) uv[k] = make_double2(desc->obs_uv[2 * P.ord[k]], desc->obs_uv[2 * P.ord[k] + 1]);
+    for (int64_t k = b; k < e; ++k) {
+      const double u = desc->obs_uv[2 * P.ord[k]], v = desc->obs_uv[2 * P.ord[k] + 1];
+      const float uh = static_cast<float>(u), vh = static_cast<float>(v);
+      uv[k] = make_float4(uh, static_cast<float>(u - uh), vh, static_cast<float>(v - vh));
+    }
   });
   if ((st = dev_upload(p, &d.obs_uv, uv))) return st;
   if ((st = dev_upload(p, &d.obs_pose, P.obs_pose))) return st;
@@ -939,6 +943,9 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   if ((st = dev_alloc(p, &d.res_t, P.no))) return st;
   if ((st = dev_alloc(p, &d.pose_f, 12 * static_cast<size_t>(P.nc)))) return st;
   if ((st = dev_alloc(p, &d.pose_dd, 24 * static_cast<size_t>(P.nc)))) return st;
+  if ((st = dev_alloc(p, &d.points_dd, 3 * static_cast<size_t>(P.np)))) return st;
+  if ((st = dev_alloc(p, &d.pose_v, 3 * static_cast<size_t>(P.nc)))) return st;
+  if ((st = dev_alloc(p, &d.cam_tab, sgba::kCamTabFloats))) return st;
   if ((st = dev_alloc(p, &d.zmat, 20 * static_cast<size_t>(P.ng)))) return st;
   if ((st = dev_alloc(p, &d.cinv, 12 * static_cast<size_t>(P.nm)))) return st;
   if ((st = dev_alloc(p, &d.cvec, 6 * static_cast<size_t>(P.nm)))) return st;

@@ -19,6 +19,7 @@ constexpr int kZddFloats = 40;
 // the S_kk triangle (21), J_k^T r~ (6) and Zk c (6); per marg point Zk (6x3,
 // float-float); per free pose S_kj (6x6).
 constexpr int kIntrMax = 6;
+constexpr int kCamTabFloats = 20;  // camera params split for the kernels (sgba_kernels.cu)
 constexpr int kIntrPart = 33;
 constexpr int kIntrZk = 36;
 constexpr int kIntrScj = 36;
@@ -145,7 +146,7 @@ struct Plan {
 // Device buffers of one problem.
 struct Dev {
   // static structure
-  double2* obs_uv = nullptr;       // sorted
+  float4* obs_uv = nullptr;        // sorted; pixels as (hi, lo) pairs of floats
   int32_t* obs_pose = nullptr;     // sorted
   int32_t* obs_pt = nullptr;       // sorted
   int64_t* g_begin = nullptr;
@@ -226,6 +227,9 @@ struct Dev {
   // per iteration
   float* pose_f = nullptr;         // nc*12: R_cw (row-major) + t_cw, float
   float* pose_dd = nullptr;        // nc*24: R_cw + t_cw as (hi,lo) pairs
+  float2* points_dd = nullptr;     // np*3: the points split into (hi, lo), at the point the pose tables hold
+  float2* pose_v = nullptr;        // nc*3: t_j - gauge center, split
+  float* cam_tab = nullptr;        // split camera params
   float* zmat = nullptr;           // ng*20: Z = W C^-T (6x3 row-major, padded to 20 floats)
   float* cinv = nullptr;           // nm*12: C^-1 lower (00,10,11,20,21,22) as float-float pairs
   float* cvec = nullptr;           // nm*6: C^-1 b_m as float-float pairs
@@ -407,9 +411,6 @@ struct Sizes {
 
 // ---- launchers (sgba_kernels.cu / sgba_solver.cu) -------------------------
 // Each returns the number of kernel launches it enqueued.
-int launch_pose_tables(const Sizes& s, const Dev& d, const double* poses, cudaStream_t st);
-int launch_cost(const Sizes& s, const Dev& d, const double* poses, const double* points,
-                float2* res_out, double* partials, cudaStream_t st);
 int launch_init_merit(const Sizes& s, const Dev& d, cudaStream_t st);
 int launch_iteration_begin(const Sizes& s, const Dev& d, cudaStream_t st);
 int launch_linearize(const Sizes& s, const Dev& d, double nu_override, bool use_override,

@@ -180,6 +180,35 @@ struct CamF {
 struct CamD {
   dd fx, fy, alpha, beta, one_m_alpha;
 };
+// The camera params as the kernels read them: fx fy alpha beta in FP32, then fx
+// fy cx cy alpha beta 1 - alpha as (hi, lo) pairs.  The f64 values are split
+// once per evaluation point (k_pose_tables, k_apply_update): GB300's FP64 pipe
+// takes a warp 16 cycles per operation, and the splits of the camera, of the
+// points and of the pixels, done per observation, held that pipe at 75 % in
+// the trial cost (windows; 149 us per 1.9M observations, ncu).
+constexpr int kCamTab = 4 + 2 * 7;
+static_assert(kCamTab <= kCamTabFloats, "the camera table fits its allocation");
+__device__ __forceinline__ void cam_table(const double* intr, float* tab) {
+  const double f[4] = {intr[0], intr[1], intr[4], intr[5]};
+  const double v[7] = {intr[0], intr[1], intr[2], intr[3], intr[4], intr[5], 1.0 - intr[4]};
+  for (int k = 0; k < 4; ++k) tab[k] = __double2float_rn(f[k]);
+  for (int k = 0; k < 7; ++k) {
+    const dd w = dd_from_double(v[k]);
+    tab[4 + 2 * k] = w.hi;
+    tab[5 + 2 * k] = w.lo;
+  }
+}
+__device__ __forceinline__ dd cam_entry(const float* tab, int k) { return dd_make(tab[4 + 2 * k], tab[5 + 2 * k]); }
+__device__ __forceinline__ CamF cam_f(const float* tab) { return CamF{tab[0], tab[1], tab[2], tab[3]}; }
+__device__ __forceinline__ CamD cam_dd(const float* tab) {
+  return CamD{cam_entry(tab, 0), cam_entry(tab, 1), cam_entry(tab, 4), cam_entry(tab, 5), cam_entry(tab, 6)};
+}
+// coordinate k of point i from the split points
+__device__ __forceinline__ dd pt_dd(const float2* pts, int i, int k) {
+  const float2 v = pts[3 * static_cast<int64_t>(i) + k];
+  return dd_make(v.x, v.y);
+}
+__device__ __forceinline__ float pt_f(const float2* pts, int i, int k) { return pts[3 * static_cast<int64_t>(i) + k].x; }
 __device__ __forceinline__ CamF cam_f(const double* intr) {
   return CamF{__double2float_rn(intr[0]), __double2float_rn(intr[1]), __double2float_rn(intr[4]),
               __double2float_rn(intr[5])};
@@ -363,13 +392,30 @@ __device__ __forceinline__ void pose_table(const double* T, float* pf, float* pd
   }
 }
 
-// Pose tables of every camera.  With `begin` set (the first kernel of an LM
-// iteration) thread 0 also opens the iteration: clears the step flags and
-// maxima and the count of points queued for the float-float redo.
-__device__ __forceinline__ void pose_tables_body(int nc, const double* __restrict__ poses, float* __restrict__ pose_f,
-                              float* __restrict__ pose_dd, const Ctrl* ctrl, int respect_skip, Ctrl* begin,
-                              int32_t* zero_count, int bid_, int nblk_) {
-  if (respect_skip ? skipping(ctrl) : halted(ctrl)) return;
+// What the kernels of one evaluation point read besides the f64 state: the
+// pose tables, the points and the camera params split into (hi, lo) pairs, and
+// the gauge direction of the poses (t - c, for the back-substitution).
+struct TabArgs {
+  int nc, np;
+  const double* poses;
+  const double* points;  // null: pose tables only
+  const double* intr;
+  float* pose_f;
+  float* pose_dd;
+  float2* pts;     // np x 3
+  float* cam;      // kCamTab
+  float2* pose_v;  // nc x 3
+  double cx, cy, cz;
+  int respect_skip;
+  int32_t* zero_count;
+};
+
+// A thread per camera, per point and one for the camera params.  With `begin`
+// set (the first kernel of an LM iteration) thread 0 also opens the iteration:
+// clears the step flags and maxima and the count of points queued for the
+// float-float redo.
+__device__ __forceinline__ void pose_tables_body(const TabArgs& a, const Ctrl* ctrl, Ctrl* begin, int bid_) {
+  if (a.respect_skip ? skipping(ctrl) : halted(ctrl)) return;
   if (begin && bid_ == 0 && threadIdx.x == 0) {
     begin->skip = 0;
     begin->accept = 0;
@@ -377,16 +423,50 @@ __device__ __forceinline__ void pose_tables_body(int nc, const double* __restric
     begin->max_step_bits = 0ull;
     begin->alpha = 0.0;
     begin->pcg_done = 0;
-    if (zero_count) *zero_count = 0;
+    if (a.zero_count) *a.zero_count = 0;
   }
   int j = bid_ * blockDim.x + threadIdx.x;
-  if (j >= nc) return;
-  pose_table(poses + 7 * j, pose_f + 12 * j, pose_dd + 24 * j);
+  if (j < a.nc) {
+    const double* T = a.poses + 7 * j;
+    pose_table(T, a.pose_f + 12 * j, a.pose_dd + 24 * j);
+    if (a.pose_v) {
+      const dd v[3] = {dd_from_double(T[4] - a.cx), dd_from_double(T[5] - a.cy), dd_from_double(T[6] - a.cz)};
+      for (int k = 0; k < 3; ++k) a.pose_v[3 * j + k] = make_float2(v[k].hi, v[k].lo);
+    }
+    return;
+  }
+  if (!a.points) return;
+  j -= a.nc;
+  if (j < a.np) {
+    for (int k = 0; k < 3; ++k) {
+      const dd v = dd_from_double(a.points[3 * static_cast<int64_t>(j) + k]);
+      a.pts[3 * static_cast<int64_t>(j) + k] = make_float2(v.hi, v.lo);
+    }
+  } else if (j == a.np) {
+    cam_table(a.intr, a.cam);
+  }
 }
-__global__ void k_pose_tables(int nc, const double* __restrict__ poses, float* __restrict__ pose_f,
-                              float* __restrict__ pose_dd, const Ctrl* ctrl, int respect_skip, Ctrl* begin,
-                              int32_t* zero_count) {
-  pose_tables_body(nc, poses, pose_f, pose_dd, ctrl, respect_skip, begin, zero_count, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(128) k_pose_tables(TabArgs a, const Ctrl* ctrl, Ctrl* begin) {
+  pose_tables_body(a, ctrl, begin, blockIdx.x);
+}
+int tab_grid(const Sizes& s) { return (s.nc + s.np + 1 + 127) / 128; }
+TabArgs make_tab_args(const Sizes& s, const Dev& d, int32_t* zero_count) {
+  TabArgs a{};
+  a.nc = s.nc;
+  a.np = s.np;
+  a.poses = d.poses;
+  a.points = d.points;
+  a.intr = d.intr;
+  a.pose_f = d.pose_f;
+  a.pose_dd = d.pose_dd;
+  a.pts = d.points_dd;
+  a.cam = d.cam_tab;
+  a.pose_v = s.gauge_kind == 1 ? d.pose_v : nullptr;
+  a.cx = s.gauge_center[0];
+  a.cy = s.gauge_center[1];
+  a.cz = s.gauge_center[2];
+  a.zero_count = zero_count;
+  return a;
 }
 
 // ---------------------------------------------------------------------------
@@ -395,16 +475,15 @@ __global__ void k_pose_tables(int nc, const double* __restrict__ poses, float* _
 // ---------------------------------------------------------------------------
 struct CostArgs {
   int64_t no;
-  const double2* uv;
+  const float4* uv;     // pixels as (hi, lo) pairs
   const int32_t* opose;
   const int32_t* opt;
   const float* pose_dd;
-  const double* points;
+  const float2* pts;
   float2* res_out;
   float2* res_lo_out;  // low parts of the residuals (float-float linearization), or null
   double* partials;
-  dd fx, fy, cx, cy;    // intrinsics when intr is null (the allocation-free entry point)
-  const double* intr;   // device intrinsics fx fy cx cy (current or trial), or null
+  const float* cam;     // split camera params
   float huber;
   dd huber_dd;
   int respect_skip;
@@ -422,10 +501,10 @@ __device__ void decide_body(const double* cost_part, int n_cost, const double* u
 
 template <bool E>
 __device__ __forceinline__ void cost_body(CostArgs a, const Ctrl* ctrl, int bid_, int nblk_) {
-  const dd fx_ = a.intr ? dd_from_double(a.intr[0]) : a.fx, fy_ = a.intr ? dd_from_double(a.intr[1]) : a.fy;
-  const dd cx_ = a.intr ? dd_from_double(a.intr[2]) : a.cx, cy_ = a.intr ? dd_from_double(a.intr[3]) : a.cy;
+  const dd fx_ = cam_entry(a.cam, 0), fy_ = cam_entry(a.cam, 1);
+  const dd cx_ = cam_entry(a.cam, 2), cy_ = cam_entry(a.cam, 3);
   // EUCM camera: the z = 1 projection is divided by norm
-  const CamD camd = E ? cam_dd(a.intr) : CamD{};
+  const CamD camd = E ? cam_dd(a.cam) : CamD{};
   if (a.decide && !halted(ctrl) && skipping(ctrl)) {
     // no trial (gradient tolerance or a failed solve): decide at once
     if (bid_ == 0) decide_body(a.partials, 0, a.upd_part, a.n_upd, a.decide, a.recs, a.last);
@@ -436,8 +515,8 @@ __device__ __forceinline__ void cost_body(CostArgs a, const Ctrl* ctrl, int bid_
   for (int64_t o = bid_ * static_cast<int64_t>(blockDim.x) + threadIdx.x; o < a.no;
        o += static_cast<int64_t>(nblk_) * blockDim.x) {
     const float* P = a.pose_dd + 24 * a.opose[o];
-    const double* pw = a.points + 3 * a.opt[o];
-    dd p0 = dd_from_double(pw[0]), p1 = dd_from_double(pw[1]), p2 = dd_from_double(pw[2]);
+    const int ip = a.opt[o];
+    const dd p0 = pt_dd(a.pts, ip, 0), p1 = pt_dd(a.pts, ip, 1), p2 = pt_dd(a.pts, ip, 2);
     dd xc[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -454,9 +533,9 @@ __device__ __forceinline__ void cost_body(CostArgs a, const Ctrl* ctrl, int bid_
       u = dd_div(u, nrm);
       v = dd_div(v, nrm);
     }
-    double2 z = a.uv[o];
-    dd ru = dd_sub(dd_from_double(z.x), dd_add(dd_mul(u, fx_), cx_));
-    dd rv = dd_sub(dd_from_double(z.y), dd_add(dd_mul(v, fy_), cy_));
+    const float4 z = a.uv[o];
+    dd ru = dd_sub(dd_make(z.x, z.y), dd_add(dd_mul(u, fx_), cx_));
+    dd rv = dd_sub(dd_make(z.z, z.w), dd_add(dd_mul(v, fy_), cy_));
     dd n2 = dd_add(dd_mul(ru, ru), dd_mul(rv, rv));
     dd c = n2;
     if (a.huber > 0.0f) {
@@ -546,9 +625,9 @@ struct LinArgs {
   const double* cnt_m;
   const float* pose_f;
   const float* pose_dd;
-  const double* points;
+  const float2* pts;   // split points
   const float2* res;
-  const double* intr;  // device intrinsics fx fy cx cy
+  const float* cam;    // split camera params
   float huber;
   float* zmat;
   float* cinv;   // 6 float-float per point: C^-1 (00 10 11 20 21 22)
@@ -581,8 +660,8 @@ struct LinArgs {
 
 template <bool E>
 __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, int nblk_) {
-  const CamF cam_ = cam_f(a.intr);
-  const CamD camd_ = cam_dd(a.intr);
+  const CamF cam_ = cam_f(a.cam);
+  const CamD camd_ = cam_dd(a.cam);
   (void)cam_; (void)camd_;
   if (halted(ctrl)) return;
   __shared__ float red[8][9][33];
@@ -600,9 +679,9 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
     const int64_t i = a.list ? static_cast<int64_t>(a.list[item]) : item;
     const int mb = a.pt_mb[i];
     if (mb < 0) continue;  // constant point: no H_mm block
-    const float px = __double2float_rn(a.points[3 * i + 0]);
-    const float py = __double2float_rn(a.points[3 * i + 1]);
-    const float pz = __double2float_rn(a.points[3 * i + 2]);
+    const float px = pt_f(a.pts, i, 0);
+    const float py = pt_f(a.pts, i, 1);
+    const float pz = pt_f(a.pts, i, 2);
     const int64_t g0 = a.pt_g_begin[i], g1 = a.pt_g_begin[i + 1];
     dd Vd[6], b[3];
     bool well = false;
@@ -667,9 +746,9 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
     t22 = V[5] - c20 * c20 - c21 * c21;
     well = !a.list && V[0] > 0.f && t11 > a.well_tol * V[3] && t22 > a.well_tol * V[5];
     }
-    const dd pxd = dd_from_double(a.points[3 * i + 0]);
-    const dd pyd = dd_from_double(a.points[3 * i + 1]);
-    const dd pzd = dd_from_double(a.points[3 * i + 2]);
+    const dd pxd = pt_dd(a.pts, i, 0);
+    const dd pyd = pt_dd(a.pts, i, 1);
+    const dd pzd = pt_dd(a.pts, i, 2);
     if (!well) {
       // The FP32 Jacobians leave a rounding-level component of the gradient and
       // of W along the weakly constrained direction, which 1/(nu n) would
@@ -867,8 +946,8 @@ constexpr int kLmkTerms = 256;
 
 template <bool E>
 __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int bid_, int nblk_) {
-  const CamF cam_ = cam_f(a.intr);
-  const CamD camd_ = cam_dd(a.intr);
+  const CamF cam_ = cam_f(a.cam);
+  const CamD camd_ = cam_dd(a.cam);
   (void)cam_; (void)camd_;
   if (halted(ctrl)) return;
   extern __shared__ float lsm[];        // [cap][9] term contributions
@@ -887,9 +966,9 @@ __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int 
     for (int t = tid; t < nt; t += blockDim.x) {
       const int64_t g = t0 + t;
       const int i = a.g_pt[g];
-      const float px = __double2float_rn(a.points[3 * i + 0]);
-      const float py = __double2float_rn(a.points[3 * i + 1]);
-      const float pz = __double2float_rn(a.points[3 * i + 2]);
+      const float px = pt_f(a.pts, i, 0);
+      const float py = pt_f(a.pts, i, 1);
+      const float pz = pt_f(a.pts, i, 2);
       const float* P = a.pose_f + 12 * a.g_pose[g];
       float v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
       for (int64_t o = a.g_begin[g]; o < a.g_begin[g + 1]; ++o) {
@@ -991,9 +1070,9 @@ __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int 
       if (!sok[q]) continue;
       const int pj = a.g_pose[g];
       if (a.pose_fb[pj] < 0) continue;
-      const float px = __double2float_rn(a.points[3 * i + 0]);
-      const float py = __double2float_rn(a.points[3 * i + 1]);
-      const float pz = __double2float_rn(a.points[3 * i + 2]);
+      const float px = pt_f(a.pts, i, 0);
+      const float py = pt_f(a.pts, i, 1);
+      const float pz = pt_f(a.pts, i, 2);
       const float* P = a.pose_f + 12 * pj;
       float W[18];
 #pragma unroll
@@ -1051,8 +1130,8 @@ constexpr int kLmkDDTermFloats = 18 + 36;  // 9 float-float sums + the Jacobians
 
 template <bool E>
 __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctrl) {
-  const CamF cam_ = cam_f(a.intr);
-  const CamD camd_ = cam_dd(a.intr);
+  const CamF cam_ = cam_f(a.cam);
+  const CamD camd_ = cam_dd(a.cam);
   (void)cam_; (void)camd_;
   if (halted(ctrl)) return;
   extern __shared__ float lsd[];               // [cap][kLmkDDTermFloats]
@@ -1071,9 +1150,9 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
     for (int t = tid; t < nt; t += blockDim.x) {
       const int64_t g = t0 + t;
       const int i = a.g_pt[g];
-      const dd px = dd_from_double(a.points[3 * i + 0]);
-      const dd py = dd_from_double(a.points[3 * i + 1]);
-      const dd pz = dd_from_double(a.points[3 * i + 2]);
+      const dd px = pt_dd(a.pts, i, 0);
+      const dd py = pt_dd(a.pts, i, 1);
+      const dd pz = pt_dd(a.pts, i, 2);
       JacD J;
       jacobians_dd<E>(a.pose_dd + 24 * a.g_pose[g], px, py, pz, camd_, &J);
       float* ts = lsd + static_cast<int64_t>(t) * kLmkDDTermFloats;
@@ -1257,11 +1336,11 @@ struct CamArgs {
   const int32_t* fb_pose;
   const int32_t* pt_mb;
   const float* pose_f;
-  const double* points;
+  const float2* pts;   // split points
   const float2* res;
   const float* zmat;
   const float* cvec;
-  const double* intr;  // device intrinsics fx fy cx cy
+  const float* cam;    // split camera params
   float huber;
   double* tile_part;
   int with_schur;
@@ -1274,8 +1353,8 @@ struct CamArgs {
 
 template <bool E>
 __device__ __forceinline__ void camera_tiles_body(CamArgs a, const Ctrl* ctrl, int bid_, int nblk_) {
-  const CamF cam_ = cam_f(a.intr);
-  const CamD camd_ = cam_dd(a.intr);
+  const CamF cam_ = cam_f(a.cam);
+  const CamD camd_ = cam_dd(a.cam);
   (void)cam_; (void)camd_;
   if (halted(ctrl)) return;
   const int tile = bid_;
@@ -1291,9 +1370,9 @@ __device__ __forceinline__ void camera_tiles_body(CamArgs a, const Ctrl* ctrl, i
   if (e < a.tile_end[tile]) {
     const int64_t g = a.cam_g[e];
     const int pi = a.g_pt[g];
-    const float px = __double2float_rn(a.points[3 * pi + 0]);
-    const float py = __double2float_rn(a.points[3 * pi + 1]);
-    const float pz = __double2float_rn(a.points[3 * pi + 2]);
+    const float px = pt_f(a.pts, pi, 0);
+    const float py = pt_f(a.pts, pi, 1);
+    const float pz = pt_f(a.pts, pi, 2);
     for (int64_t o = a.g_begin[g]; o < a.g_begin[g + 1]; ++o) {
       JacF J;
       jacobians_f<E>(P, px, py, pz, cam_, &J);
@@ -1385,8 +1464,8 @@ __global__ void __launch_bounds__(kTileThreads) k_camera_tiles(CamArgs a, const 
 // k_camera_tiles.
 template <bool E>
 __global__ void __launch_bounds__(kTileThreads, 2) k_camera_tiles_dd(CamArgs a, const Ctrl* ctrl) {
-  const CamF cam_ = cam_f(a.intr);
-  const CamD camd_ = cam_dd(a.intr);
+  const CamF cam_ = cam_f(a.cam);
+  const CamD camd_ = cam_dd(a.cam);
   (void)cam_; (void)camd_;
   if (halted(ctrl)) return;
   const int tile = blockIdx.x;
@@ -1399,9 +1478,9 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_camera_tiles_dd(CamArgs a, 
   if (e < a.tile_end[tile]) {
     const int64_t g = a.cam_g[e];
     const int pi = a.g_pt[g];
-    const dd px = dd_from_double(a.points[3 * pi + 0]);
-    const dd py = dd_from_double(a.points[3 * pi + 1]);
-    const dd pz = dd_from_double(a.points[3 * pi + 2]);
+    const dd px = pt_dd(a.pts, pi, 0);
+    const dd py = pt_dd(a.pts, pi, 1);
+    const dd pz = pt_dd(a.pts, pi, 2);
     for (int64_t o = a.g_begin[g]; o < a.g_begin[g + 1]; ++o) {
       JacD J;
       jacobians_dd<E>(Pd, px, py, pz, camd_, &J);
@@ -1954,8 +2033,7 @@ struct BackArgs {
   // through the same back-substitution, u_m = -C^-T sum Z_g^T v_f (the
   // projection's direction for the points)
   int gauge_kind;
-  const double* poses;
-  double cx, cy, cz;
+  const float2* pose_v;  // nc x 3: t_j - c, split
   double* um;
   // free intrinsics: dx_m also loses C^-T Zk^T dx_k (dx_k at rows 6 nf .. 6 nf + 5)
   const float* zk;  // nm x kIntrZk or null
@@ -2031,8 +2109,7 @@ __device__ __forceinline__ void backsub_body(BackArgs a, const Ctrl* ctrl, int b
         for (int q = 0; q < 3; ++q) t[q] = dd_add(t[q], dd_mul(x, dd_make(zr[6 * r + 2 * q], zr[6 * r + 2 * q + 1])));
       }
       if (gauge) {
-        const double* T = a.poses + 7 * static_cast<int64_t>(pj);
-        const dd v[3] = {dd_from_double(T[4] - a.cx), dd_from_double(T[5] - a.cy), dd_from_double(T[6] - a.cz)};
+        const dd v[3] = {pt_dd(a.pose_v, pj, 0), pt_dd(a.pose_v, pj, 1), pt_dd(a.pose_v, pj, 2)};
 #pragma unroll
         for (int r = 3; r < 6; ++r)
 #pragma unroll
@@ -2129,10 +2206,7 @@ __device__ __forceinline__ void backsub_chunks_body(BackArgs a, const int32_t* c
         const float2* xp = reinterpret_cast<const float2*>(a.xdd) + 6 * fb;
         dd v[3] = {dd_make(0.f, 0.f), dd_make(0.f, 0.f), dd_make(0.f, 0.f)};
         if (gauge) {
-          const double* T = a.poses + 7 * static_cast<int64_t>(pj);
-          v[0] = dd_from_double(T[4] - a.cx);
-          v[1] = dd_from_double(T[5] - a.cy);
-          v[2] = dd_from_double(T[6] - a.cz);
+          for (int k = 0; k < 3; ++k) v[k] = pt_dd(a.pose_v, pj, k);
         }
         bool use_dd = a.zdd != nullptr;
         float Z[20];
@@ -2273,11 +2347,11 @@ struct IntrArgs {
   const int32_t* pose_fb;
   const int32_t* pt_mb;
   const float* pose_dd;
-  const double* points;
+  const float2* pts;
   const float2* res;
   float huber;
   dd huber_dd;
-  const double* intr;
+  const float* cam;
   const float* cinv;
   const float* cvec;
   const float* zmat;
@@ -2339,9 +2413,8 @@ __global__ void __launch_bounds__(128) k_intr_points(IntrArgs a, const Ctrl* ctr
   if (halted(ctrl)) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.np) return;
-  const CamD cam = cam_dd(a.intr);
-  const dd px = dd_from_double(a.points[3 * i]), py = dd_from_double(a.points[3 * i + 1]),
-           pz = dd_from_double(a.points[3 * i + 2]);
+  const CamD cam = cam_dd(a.cam);
+  const dd px = pt_dd(a.pts, i, 0), py = pt_dd(a.pts, i, 1), pz = pt_dd(a.pts, i, 2);
   dd hkk[kKT], gk[kK], Y[3 * kK];
   for (int k = 0; k < kKT; ++k) hkk[k] = dd_make(0.f, 0.f);
   for (int k = 0; k < kK; ++k) gk[k] = dd_make(0.f, 0.f);
@@ -2449,14 +2522,13 @@ __global__ void __launch_bounds__(128) k_intr_cams(IntrArgs a, const Ctrl* ctrl)
   __shared__ float sh_hi[kE][129], sh_lo[kE][129];
   dd acc[kE];
   for (int k = 0; k < kE; ++k) acc[k] = dd_make(0.f, 0.f);
-  const CamD cam = cam_dd(a.intr);
+  const CamD cam = cam_dd(a.cam);
   const int64_t t0 = a.fb_tile_begin[fb], t1 = a.fb_tile_begin[fb + 1];
   const int64_t e0 = (t1 > t0) ? a.tile_begin[t0] : 0, e1 = (t1 > t0) ? a.tile_end[t1 - 1] : 0;
   for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
     const int64_t g = a.cam_g[e];
     const int i = a.g_pt[g];
-    const dd px = dd_from_double(a.points[3 * i]), py = dd_from_double(a.points[3 * i + 1]),
-             pz = dd_from_double(a.points[3 * i + 2]);
+    const dd px = pt_dd(a.pts, i, 0), py = pt_dd(a.pts, i, 1), pz = pt_dd(a.pts, i, 2);
     JacD J;
     dd jk[2 * kK];
     intr_term_jacobians(a.pose_dd + 24 * a.g_pose[g], px, py, pz, cam, a.nk, &J, jk);
@@ -2552,11 +2624,11 @@ IntrArgs intr_args(const Sizes& s, const Dev& d) {
   a.pose_fb = d.pose_fb;
   a.pt_mb = d.pt_mb;
   a.pose_dd = d.pose_dd;
-  a.points = d.points;
+  a.pts = d.points_dd;
   a.res = d.res;
   a.huber = static_cast<float>(s.huber > 0 ? s.huber : 0.0);
   a.huber_dd = dd_make(static_cast<float>(s.huber), static_cast<float>(s.huber - static_cast<float>(s.huber)));
-  a.intr = d.intr;
+  a.cam = d.cam_tab;
   a.cinv = d.cinv;
   a.cvec = d.cvec;
   a.zmat = d.zmat;
@@ -2694,8 +2766,10 @@ struct UpdArgs {
   const double* gauge_part;  // 2 * gauge_blocks partial sums of the gauge projection
   int gauge_blocks;
   const double* um;          // the points' part of the projection direction
-  float* pose_f;   // trial pose tables, written here for the trial cost
+  float* pose_f;   // trial tables, written here for the trial cost
   float* pose_dd;
+  float2* pts;
+  float* cam;
   // free intrinsics: k_t = k + dx_k (dx_k at xf[6 nf .. 6 nf + nk - 1]), neg_grad bk
   int intr_free;
   int intr_nk;
@@ -2740,6 +2814,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
       sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bk[k])));
       mx = fmax(mx, fabs(xk));
     }
+    cam_table(a.intr_t, a.cam);
   }
   const int64_t n = static_cast<int64_t>(a.nc) + a.np;
   for (int64_t t = bid_ * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
@@ -2774,7 +2849,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
       double* O = a.points_t + 3 * i;
       const int mb = a.pt_mb[i];
       if (mb < 0) {
-        O[0] = p[0]; O[1] = p[1]; O[2] = p[2];
+        O[0] = p[0]; O[1] = p[1]; O[2] = p[2];  // its split is the current point's
         continue;
       }
       double d[3] = {a.dm[3 * mb], a.dm[3 * mb + 1], a.dm[3 * mb + 2]};
@@ -2790,6 +2865,8 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
         sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bm[3 * mb + k])));
         mx = fmax(mx, fabs(d[k]));
         O[k] = p[k] + d[k];
+        const dd o = dd_from_double(O[k]);
+        a.pts[3 * static_cast<int64_t>(i) + k] = make_float2(o.hi, o.lo);
       }
     }
   }
@@ -2970,13 +3047,9 @@ int upd_blocks(const Sizes& s) {
 constexpr int kCostPartOff = 4 * kUpdBlocks + 2;
 int cost_partials_needed(const Sizes& s) { return kCostPartOff + cost_grid(s.no) + 2; }
 
-int launch_pose_tables(const Sizes& s, const Dev& d, const double* poses, cudaStream_t st) {
-  k_pose_tables<<<(s.nc + 127) / 128, 128, 0, st>>>(s.nc, poses, d.pose_f, d.pose_dd, d.ctrl, 0, nullptr, nullptr);
-  return 1;
-}
-
-static CostArgs make_cost_args(const Sizes& s, const Dev& d, const double* points, float2* res_out,
-                               double* partials, int respect_skip) {
+// The cost at the point whose tables (poses, split points and camera) are
+// current.
+static CostArgs make_cost_args(const Sizes& s, const Dev& d, float2* res_out, double* partials, int respect_skip) {
   CostArgs a;
   a.res_lo_out = (res_out == d.res) ? d.res_lo : (res_out == d.res_t ? d.res_lo_t : nullptr);
   a.no = s.no;
@@ -2984,11 +3057,10 @@ static CostArgs make_cost_args(const Sizes& s, const Dev& d, const double* point
   a.opose = d.obs_pose;
   a.opt = d.obs_pt;
   a.pose_dd = d.pose_dd;
-  a.points = points;
+  a.pts = d.points_dd;
   a.res_out = res_out;
   a.partials = partials;
-  a.fx = a.fy = a.cx = a.cy = dd_make(0.f, 0.f);
-  a.intr = (points == d.points_t) ? d.intr_t : d.intr;  // the trial point's intrinsics
+  a.cam = d.cam_tab;
   a.huber = static_cast<float>(s.huber > 0 ? s.huber : 0.0);
   a.huber_dd = dd_make(static_cast<float>(s.huber), static_cast<float>(s.huber - static_cast<float>(s.huber)));
   a.respect_skip = respect_skip;
@@ -3001,17 +3073,9 @@ static CostArgs make_cost_args(const Sizes& s, const Dev& d, const double* point
   return a;
 }
 
-int launch_cost(const Sizes& s, const Dev& d, const double* poses, const double* points,
-                float2* res_out, double* partials, cudaStream_t st) {
-  k_pose_tables<<<(s.nc + 127) / 128, 128, 0, st>>>(s.nc, poses, d.pose_f, d.pose_dd, d.ctrl, 1, nullptr, nullptr);
-  CostArgs a = make_cost_args(s, d, points, res_out, partials, 1);
-  (s.eucm ? k_cost<true> : k_cost<false>)<<<cost_grid(s.no), kCostThreads, 0, st>>>(a, d.ctrl);
-  return 2;
-}
-
 int launch_init_merit(const Sizes& s, const Dev& d, cudaStream_t st) {
-  k_pose_tables<<<(s.nc + 127) / 128, 128, 0, st>>>(s.nc, d.poses, d.pose_f, d.pose_dd, d.ctrl, 0, nullptr, nullptr);
-  CostArgs a = make_cost_args(s, d, d.points, d.res, d.part, 0);
+  k_pose_tables<<<tab_grid(s), 128, 0, st>>>(make_tab_args(s, d, nullptr), d.ctrl, nullptr);
+  CostArgs a = make_cost_args(s, d, d.res, d.part, 0);
   const int nb = cost_grid(s.no);
   (s.eucm ? k_cost<true> : k_cost<false>)<<<nb, kCostThreads, 0, st>>>(a, d.ctrl);
   const int np = launch_prior_eval(s, d, d.poses, 0, 0, d.part + nb, st);
@@ -3039,10 +3103,10 @@ static LinArgs make_lin_args(const Sizes& s, const Dev& d, double nu_override, b
   la.pt_mb = d.pt_mb;
   la.cnt_m = d.cnt_m;
   la.pose_f = d.pose_f;
-  la.points = d.points;
+  la.pts = d.points_dd;
   la.pose_dd = d.pose_dd;
   la.res = d.res;
-  la.intr = d.intr;
+  la.cam = d.cam_tab;
   la.huber = static_cast<float>(s.huber > 0 ? s.huber : 0.0);
   la.huber_dd = dd_make(static_cast<float>(s.huber), static_cast<float>(s.huber - static_cast<float>(s.huber)));
   la.zmat = d.zmat;
@@ -3077,11 +3141,11 @@ static CamArgs make_cam_args(const Sizes& s, const Dev& d, int with_schur) {
   ca.fb_pose = d.fb_pose;
   ca.pt_mb = d.pt_mb;
   ca.pose_f = d.pose_f;
-  ca.points = d.points;
+  ca.pts = d.points_dd;
   ca.res = d.res;
   ca.zmat = d.zmat;
   ca.cvec = d.cvec;
-  ca.intr = d.intr;
+  ca.cam = d.cam_tab;
   ca.huber = static_cast<float>(s.huber > 0 ? s.huber : 0.0);
   ca.tile_part = d.tile_part;
   ca.with_schur = with_schur;
@@ -3116,10 +3180,7 @@ static BackArgs make_back_args(const Sizes& s, const Dev& d) {
   b.xdd = d.xdd;
   b.dm = d.dm;
   b.gauge_kind = s.gauge_kind;
-  b.poses = d.poses;
-  b.cx = s.gauge_center[0];
-  b.cy = s.gauge_center[1];
-  b.cz = s.gauge_center[2];
+  b.pose_v = d.pose_v;
   b.um = d.gauge_um;
   b.zk = s.intr_free ? d.intr_zk : nullptr;
   b.k0 = 6 * s.nf;
@@ -3197,9 +3258,8 @@ int launch_linearize(const Sizes& s, const Dev& d, double nu_override, bool use_
                      cudaStream_t st) {
   int n = 0;
   // an LM iteration (not the final linearisation) is opened here
-  k_pose_tables<<<(s.nc + 127) / 128, 128, 0, st>>>(s.nc, d.poses, d.pose_f, d.pose_dd, d.ctrl, 0,
-                                                    use_override ? nullptr : d.ctrl,
-                                                    use_override ? nullptr : d.slow_count);
+  k_pose_tables<<<tab_grid(s), 128, 0, st>>>(make_tab_args(s, d, use_override ? nullptr : d.slow_count), d.ctrl,
+                                             use_override ? nullptr : d.ctrl);
   ++n;
   n += launch_landmark(s, d, make_lin_args(s, d, nu_override, use_override), st, use_override);
   n += launch_intr_linearize(s, d, st);
@@ -3322,6 +3382,8 @@ static UpdArgs make_upd_args(const Sizes& s, const Dev& d) {
   u.bk = d.intr_sum ? d.intr_sum + kIntrPart : nullptr;
   u.pose_f = d.pose_f;
   u.pose_dd = d.pose_dd;
+  u.pts = d.points_dd;
+  u.cam = d.cam_tab;
   return u;
 }
 
@@ -3347,7 +3409,7 @@ int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st) 
     case 3:
       return launch_camera(s, d, 1, st);
     case 4: {
-      CostArgs a = make_cost_args(s, d, d.points_t, d.res_t, d.part + kCostPartOff, 1);
+      CostArgs a = make_cost_args(s, d, d.res_t, d.part + kCostPartOff, 1);
       (s.eucm ? k_cost<true> : k_cost<false>)<<<cost_grid(s.no), kCostThreads, 0, st>>>(a, d.ctrl);
       return 1;
     }
@@ -3364,7 +3426,7 @@ int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st) 
 // were written by k_apply_update); its last block runs the LM decision
 static CostArgs make_decide_args(const Sizes& s, const Dev& d) {
   double* cost_part = d.part + kCostPartOff;
-  CostArgs a = make_cost_args(s, d, d.points_t, d.res_t, cost_part, 1);
+  CostArgs a = make_cost_args(s, d, d.res_t, cost_part, 1);
   a.decide = d.ctrl;
   a.upd_part = d.part + 2 * kUpdBlocks;
   a.n_upd = upd_blocks(s) + (s.n_eq > 0 ? 1 : 0);  // the constraints' slot after the blocks'
@@ -3470,7 +3532,19 @@ unsigned char* g_noalloc_base[kNoAllocMaxDevices] = {};
 // k_cost without the residual output and with index checks: an observation
 // whose pose or point index is out of range contributes NaN (and is never
 // dereferenced), so the returned cost is NaN.
-__global__ void __launch_bounds__(kCostThreads) k_cost_noalloc(CostArgs a, int32_t nc, int32_t np) {
+struct NoAllocArgs {
+  int64_t no;
+  const double2* uv;
+  const int32_t* opose;
+  const int32_t* opt;
+  const float* pose_dd;
+  const double* points;
+  double* partials;
+  dd fx, fy, cx, cy;
+  float huber;
+  dd huber_dd;
+};
+__global__ void __launch_bounds__(kCostThreads) k_cost_noalloc(NoAllocArgs a, int32_t nc, int32_t np) {
   dd acc = dd_make(0.0f, 0.0f);
   bool bad = false;
   for (int64_t o = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; o < a.no;
@@ -3563,28 +3637,27 @@ cudaError_t launch_total_cost_noalloc(int32_t nc, const double* poses, int32_t n
   float* pose_f = reinterpret_cast<float*>(base + kNoAllocPoseFOff);
   float* pose_dd = reinterpret_cast<float*>(base + kNoAllocPoseDDOff);
   double* part = reinterpret_cast<double*>(base + kNoAllocPartOff);
-  k_pose_tables<<<(nc + 127) / 128, 128, 0, st>>>(nc, poses, pose_f, pose_dd, zero_ctrl, 0, nullptr, nullptr);
+  TabArgs t{};
+  t.nc = nc;
+  t.poses = poses;
+  t.pose_f = pose_f;
+  t.pose_dd = pose_dd;
+  k_pose_tables<<<(nc + 127) / 128, 128, 0, st>>>(t, zero_ctrl, nullptr);
   auto split = [](double x) { return dd_make(static_cast<float>(x), static_cast<float>(x - static_cast<float>(x))); };
-  CostArgs a;
+  NoAllocArgs a;
   a.no = no;
   a.uv = reinterpret_cast<const double2*>(obs_uv);
   a.opose = obs_cam;
   a.opt = obs_pt;
   a.pose_dd = pose_dd;
   a.points = points;
-  a.res_out = nullptr;
-  a.res_lo_out = nullptr;
-  a.decide = nullptr;
   a.partials = part;
   a.fx = split(intr[0]);
   a.fy = split(intr[1]);
   a.cx = split(intr[2]);
   a.cy = split(intr[3]);
-  a.intr = nullptr;
   a.huber = static_cast<float>(huber > 0 ? huber : 0.0);
   a.huber_dd = split(huber);
-  a.respect_skip = 0;
-  a.n_extra = 0;
   const int nb = cost_grid(no);
   k_cost_noalloc<<<nb, kCostThreads, 0, st>>>(a, nc, np);
   k_noalloc_finish<<<1, 256, 0, st>>>(part, nb, cost);
@@ -3632,13 +3705,8 @@ __device__ __forceinline__ WinPos win_pos(const WinTab<A>& t) {
 }
 
 struct PoseTabArgs {
-  int nc;
-  const double* poses;
-  float* pose_f;
-  float* pose_dd;
-  int respect_skip;
+  TabArgs t;
   int begin;  // open the iteration (the window's control block)
-  int32_t* zero_count;
 };
 struct FinArgs {
   int nf;
@@ -3676,13 +3744,12 @@ struct CommitArgs {
 
 __global__ void __launch_bounds__(128) k_pose_tables_w(WinTab<PoseTabArgs> t) {
   const WinPos q = win_pos(t);
-  const PoseTabArgs a = t.args[q.w];
+  const PoseTabArgs& a = t.args[q.w];
   Ctrl* c = t.ctrl[q.w];
-  pose_tables_body(a.nc, a.poses, a.pose_f, a.pose_dd, c, a.respect_skip, a.begin ? c : nullptr, a.zero_count, q.b,
-                   q.nb);
+  pose_tables_body(a.t, c, a.begin ? c : nullptr, q.b);
 }
 template <bool E>
-__global__ void __launch_bounds__(kCostThreads) k_cost_w(WinTab<CostArgs> t) {
+__global__ void __launch_bounds__(kCostThreads, 4) k_cost_w(WinTab<CostArgs> t) {
   const WinPos q = win_pos(t);
   cost_body<E>(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }
@@ -3702,7 +3769,7 @@ __global__ void __launch_bounds__(256, 2) k_landmark_w(WinTab<LinArgs> t) {
   landmark_body<E>(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }
 template <bool E>
-__global__ void __launch_bounds__(256) k_landmark_chunks_w(WinTab<LinArgs> t) {
+__global__ void __launch_bounds__(256, 4) k_landmark_chunks_w(WinTab<LinArgs> t) {
   const WinPos q = win_pos(t);
   landmark_chunks_body<E>(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }
@@ -3729,7 +3796,7 @@ __global__ void __launch_bounds__(256) k_schur_reduce_w(WinTab<SchurArgs> t) {
   const WinPos q = win_pos(t);
   schur_reduce_body(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }
-__global__ void __launch_bounds__(256) k_backsub_chunks_w(WinTab<BsubArgs> t) {
+__global__ void __launch_bounds__(256, 4) k_backsub_chunks_w(WinTab<BsubArgs> t) {
   const WinPos q = win_pos(t);
   const BsubArgs& a = t.args[q.w];
   backsub_chunks_body(a.b, a.chunk_pt, a.nchunk, a.g_pt, t.ctrl[q.w], q.b, q.nb);
@@ -3855,11 +3922,11 @@ BatchTables* batch_tables_create(const std::vector<BatchWin>& wins, int skip_fin
     ctrl[w] = d.ctrl;
     recs[w] = d.records;
     rec_cap[w] = d.record_cap;
-    const int pose_grid = (s.nc + 127) / 128;
+    const int pose_grid = tab_grid(s);
     const int lmk_grid = s.nlchunk < 8192 ? s.nlchunk : 8192;
     // iteration (enqueue_iteration: launch_linearize, launch_schur,
     // launch_factor_solve, launch_update, launch_decide)
-    t_pose_it.add(PoseTabArgs{s.nc, d.poses, d.pose_f, d.pose_dd, 0, 1, d.slow_count}, pose_grid);
+    t_pose_it.add(PoseTabArgs{make_tab_args(s, d, d.slow_count), 1}, pose_grid);
     const LinArgs la = make_lin_args(s, d, 0.0, false);
     t_lmk_chunks.add(la, lmk_grid, sizeof(float) * 9 * static_cast<size_t>(s.lmk_cap));
     LinArgs lb = la;
@@ -3881,11 +3948,11 @@ BatchTables* batch_tables_create(const std::vector<BatchWin>& wins, int skip_fin
                             d.res_lo, nullptr, nullptr},
                  commit_grid(s));
     // init (launch_init_merit)
-    t_pose_init.add(PoseTabArgs{s.nc, d.poses, d.pose_f, d.pose_dd, 0, 0, nullptr}, pose_grid);
-    t_cost_init.add(make_cost_args(s, d, d.points, d.res, d.part, 0), cost_grid(s.no));
+    t_pose_init.add(PoseTabArgs{make_tab_args(s, d, nullptr), 0}, pose_grid);
+    t_cost_init.add(make_cost_args(s, d, d.res, d.part, 0), cost_grid(s.no));
     t_merit.add(MeritArgs{d.part, cost_grid(s.no)}, 1);
     // final linearisation (launch_linearize with the damping override)
-    t_pose_fin.add(PoseTabArgs{s.nc, d.poses, d.pose_f, d.pose_dd, 0, 0, nullptr}, pose_grid);
+    t_pose_fin.add(PoseTabArgs{make_tab_args(s, d, nullptr), 0}, pose_grid);
     LinArgs lf = make_lin_args(s, d, 0.0, true);
     lf.nu_ctrl = skip_final_hessian ? 1 : 0;
     t_lmk_fin.add(lf, warp_grid(s.np, 8, 4096));

@@ -1098,6 +1098,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     return set_error(SGBA_ERR_UNSUPPORTED, "internal: no Schur pair lists for a system that needs them");
   if (s.schur_dense) {
     if ((st = dev_alloc(p, &d.zterm, static_cast<size_t>(P.np) * static_cast<size_t>(P.nf)))) return st;
+    if (sgba::schur_dense_setup() != 0) return set_error(SGBA_ERR_CUDA, "shared memory of the tiled Schur pass");
     SGBA_CK(sgba::zterm_fill(s, d, d.zterm, p->stream));
   }
   s.lmk_dd_ok = (s.lin_dd && s.nlchunk > 0 && sgba::landmark_dd_setup(s.lmk_cap) == 0) ? 1 : 0;

@@ -1534,14 +1534,25 @@ DenseBatch* dense_batch_create(const std::vector<BatchWin>& wins, Ctrl* const* c
     smem.push_back(0);
     return static_cast<int>(sizes.size()) - 1;
   };
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    *err = cudaGetLastError();
+    return nullptr;
+  }
+  size_t nsmall = 0;
+  for (const BatchWin& w : wins) nsmall += w.s->small_dense ? 1 : 0;
+  // Up to one window per SM: one launch, every window on an SM of its own (the
+  // launches of a stream follow one another: three size classes of 40 windows
+  // took 0.53 + 0.23 + 0.12 ms in turn).  More: by shared memory, so that
+  // small windows share an SM: <= 56 KiB, <= 112 KiB, larger (keys 0, -1, -2).
+  const bool one_launch = nsmall <= static_cast<size_t>(sms);
   for (size_t w = 0; w < wins.size(); ++w) {
     const Sizes& s = *wins[w].s;
     const Dev& d = *wins[w].d;
     if (s.small_dense) {
-      // by shared memory, so that small windows share an SM: <= 56 KiB,
-      // <= 112 KiB, larger (keys 0, -1, -2)
       const size_t b = small_dense_smem(s.n6);
-      const int g = group_of(b <= kSmallHalf ? 0 : (b <= 112 * 1024 ? -1 : -2));
+      const int g = group_of(one_launch ? -2 : (b <= kSmallHalf ? 0 : (b <= 112 * 1024 ? -1 : -2)));
       args[g].push_back(small_dense_args(s, d));
       win[g].push_back(static_cast<int32_t>(w));
       smem[g] = std::max(smem[g], small_dense_smem(s.n6));

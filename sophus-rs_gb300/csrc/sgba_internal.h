@@ -423,7 +423,8 @@ int launch_decide(const Sizes& s, const Dev& d, cudaStream_t st);
 
 int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st);
 int cost_partials_needed(const Sizes& s);  // reduction partial slots
-int landmark_setup(int cap);  // dynamic shared memory of the chunked landmark pass (0 = ok)
+int landmark_setup(int cap);
+int schur_dense_setup();  // shared memory limits of the tiled Schur pass (0: ok)  // dynamic shared memory of the chunked landmark pass (0 = ok)
 int landmark_dd_setup(int cap);  // the same for its float-float variant (0 = ok)
 int backsub_chunks_setup(int cap);  // the chunked back-substitution (0 = ok)
 int solver_launch_count(const Sizes& s);

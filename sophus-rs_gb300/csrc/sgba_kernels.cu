@@ -1857,23 +1857,30 @@ __global__ void __launch_bounds__(256) k_schur_reduce(SchurArgs a, const Ctrl* c
 // ---------------------------------------------------------------------------
 // Dense reduced systems (local windows: every camera sees most points): S
 // formed by tiles of kSdB x kSdB pose blocks instead of observation pairs.
-// A CTA (kSdThreads threads) owns one tile of the lower triangle and streams
-// every point once, in rounds of kSdPts points: thread (point, slot) fetches
-// the Z records of the point's terms with the slot's row pose and column pose
-// (the term table T; zeros where there is none) into registers one round
-// ahead and stores them into shared memory; every thread then accumulates a
-// 3 x 6 piece of the tile, rows (tid / 8) + 16 i and columns (tid % 8) + 8 j,
-// so that the rows a warp reads are consecutive (no bank conflicts) and each
-// shared-memory load feeds 18 or 9 FMAs (FP32 within a round, float-float
-// across rounds, every entry in point order).  The entries are written as
-// S = U + nu n I - sum Z Z^T (the formula of k_schur_reduce), in f64 and
-// float-float.  Loads per point and tile: 2 kSdB Z records, against two per
-// observation pair.
+// A CTA owns one tile of the lower triangle and streams every point once, in
+// rounds of 16: FP32 products and sums within a round (in point order), the
+// rounds' sums added in float-float in round order, and S = U + nu n I - sum
+// Z Z^T written (the formula of k_schur_reduce) in f64 and float-float.
+//
+// Bound: the shared-memory read path, 128 bytes a clock per SM whatever lanes
+// share an address.  So a thread owns a whole 6 x 6 block (a row pose and a
+// column pose): per point it reads two 72-byte Z records for 108 FMAs (3 x 6
+// pieces read 144 bytes for 54, which held that path at 78 % and the FMA pipe
+// at 29 %).  64 threads make a tile; a CTA holds G such groups, and group g
+// takes the rounds g, g + G, ..: after G rounds the groups' sums meet in shared
+// memory and every thread folds its share of the entries into the float-float
+// sums, round by round, so any G gives the same bits.  The records of four
+// points (a stage) are copied by cp.async two stages ahead, a record per
+// thread; the term indices run a stage further ahead.  Eight groups a CTA
+// (one CTA an SM) where the tiles leave the GPU idle, two (four CTAs an SM)
+// where there are enough of them.
 // ---------------------------------------------------------------------------
 constexpr int kSdB = 8;          // pose blocks per tile side
-constexpr int kSdT = 6 * kSdB;   // 48 rows / columns
-constexpr int kSdPts = 16;       // points per round: 16 points x 8 slots, one per thread
-constexpr int kSdThreads = 128;
+constexpr int kSdGroup = kSdB * kSdB;  // threads of a group
+constexpr int kSdPts = 16;       // points per round
+constexpr int kSdStage = 4;      // points per stage: 4 points x 16 records, one per thread
+constexpr int kSdBufs = 3;
+constexpr int kSdEntries = 36 * kSdGroup;
 
 struct SchurDenseArgs {
   int np, nf, n6;
@@ -1885,131 +1892,139 @@ struct SchurDenseArgs {
   float2* S2;
 };
 
-// the Z record (6 x 3 row-major, 20 floats) of term g, or zeros
-__device__ __forceinline__ void sd_fetch(const float* zmat, int g, float4* v) {
-  if (g >= 0) {
-    const float4* src = reinterpret_cast<const float4*>(zmat + kZS * static_cast<int64_t>(g));
+constexpr size_t schur_dense_smem(int G) {
+  return sizeof(float) * static_cast<size_t>(G) * (kSdBufs * kSdStage * 2 * kSdB * kZS + kSdEntries);
+}
+
+__device__ __forceinline__ void sd_load18(const float* src, float* v) {
 #pragma unroll
-    for (int q = 0; q < 5; ++q) v[q] = __ldg(src + q);
-  } else {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int q = 0; q < 4; ++q) {
+    const float4 w = reinterpret_cast<const float4*>(src)[q];
+    v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
   }
+  const float2 w = reinterpret_cast<const float2*>(src)[8];
+  v[16] = w.x; v[17] = w.y;
 }
 
-// the six rows of a fetched record, padded to float4, into shared memory
-__device__ __forceinline__ void sd_store(float (*dst)[4], const float4* v) {
-  reinterpret_cast<float4*>(dst[0])[0] = make_float4(v[0].x, v[0].y, v[0].z, 0.f);
-  reinterpret_cast<float4*>(dst[1])[0] = make_float4(v[0].w, v[1].x, v[1].y, 0.f);
-  reinterpret_cast<float4*>(dst[2])[0] = make_float4(v[1].z, v[1].w, v[2].x, 0.f);
-  reinterpret_cast<float4*>(dst[3])[0] = make_float4(v[2].y, v[2].z, v[2].w, 0.f);
-  reinterpret_cast<float4*>(dst[4])[0] = make_float4(v[3].x, v[3].y, v[3].z, 0.f);
-  reinterpret_cast<float4*>(dst[5])[0] = make_float4(v[3].w, v[4].x, v[4].y, 0.f);
-}
-
-__device__ __forceinline__ void schur_dense_body(SchurDenseArgs a, const Ctrl* ctrl, int bid_, int nblk_) {
-  (void)nblk_;
+template <int G>
+__device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const Ctrl* ctrl, int bid_) {
   if (skipping(ctrl)) return;
-  __shared__ __align__(16) float zr[kSdPts][kSdT][4];  // Z rows of the tile's row poses (k = 0..2, padded)
-  __shared__ __align__(16) float zc[kSdPts][kSdT][4];  // the same for its column poses
+  extern __shared__ __align__(16) float zs[];  // kSdBufs x G x kSdStage x 16 records, then G x kSdEntries sums
+  constexpr int kStageFloats = kSdStage * 2 * kSdB * kZS;
+  constexpr int kStages = kSdPts / kSdStage;   // stages per round
+  constexpr int kPer = (kSdEntries + kSdGroup * G - 1) / (kSdGroup * G);
+  float* sums = zs + kSdBufs * G * kStageFloats;
   // tile (ti, tj), tj <= ti, of the lower triangle
   int ti = static_cast<int>((sqrtf(8.0f * static_cast<float>(bid_) + 1.0f) - 1.0f) * 0.5f);
   while (ti * (ti + 1) / 2 > bid_) --ti;
   while ((ti + 1) * (ti + 2) / 2 <= bid_) ++ti;
   const int tj = bid_ - ti * (ti + 1) / 2;
   const int I0 = ti * kSdB, J0 = tj * kSdB;
-  const int tid = threadIdx.x;
-  const int rq = tid >> 3, cq = tid & 7;  // rows rq + 16 i, columns cq + 8 j
-  // this thread's staging slot: point pp of each round, row pose I0 + slot and column pose J0 + slot
-  const int pp = tid >> 3, slot = tid & 7;
-  const int fr = I0 + slot, fc = J0 + slot;
-  auto term_of = [&](int p0, int f) {
-    const int i = p0 + pp;
-    return (i < a.np && f < a.nf) ? __ldg(a.zterm + static_cast<int64_t>(i) * a.nf + f) : -1;
+  const int tid = threadIdx.x, grp = tid / kSdGroup, t = tid % kSdGroup;
+  const bool diag = ti == tj;  // one set of records
+  const int nround = (a.np + kSdPts - 1) / kSdPts;
+  const int nsuper = (nround + G - 1) / G;
+  const int nstage = nsuper * kStages;  // of every group (rounds past the end copy zeros)
+  // this thread's record of a stage: point pp, slot (0..7 row poses, 8..15 column poses)
+  const int pp = t >> 4, slot = t & 15;
+  const int f = slot < kSdB ? I0 + slot : J0 + slot - kSdB;
+  const bool mine = (slot < kSdB || !diag) && f < a.nf;
+  auto term_of = [&](int s) {
+    const int i = ((s / kStages) * G + grp) * kSdPts + (s % kStages) * kSdStage + pp;
+    return (mine && s < nstage && i < a.np) ? __ldg(a.zterm + static_cast<int64_t>(i) * a.nf + f) : -1;
   };
-  float acc[3][6];
-  Acc accd[3][6];
+  auto copy = [&](int s, int g) {
+    float* dst = zs + ((s % kSdBufs) * G + grp) * kStageFloats + t * kZS;
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    const float* src = a.zmat + (g >= 0 ? kZS * static_cast<int64_t>(g) : 0);
+    const int bytes = g >= 0 ? 16 : 0;  // 0: zeros
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int q = 0; q < 5; ++q)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa + 16 * q), "l"(src + 4 * q), "r"(bytes)
+                   : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + grp), "r"(kSdGroup) : "memory"); };
+  float acc[36];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      acc[i][j] = 0.0f;
-      accd[i][j] = acc_zero();
+  for (int e = 0; e < 36; ++e) acc[e] = 0.0f;
+  Acc accd[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) accd[u] = acc_zero();
+  copy(0, term_of(0));
+  copy(1, term_of(1));
+  int gnext = term_of(2);
+  const int ra_off = (t >> 3) * kZS, rb_off = ((diag ? 0 : kSdB) + (t & 7)) * kZS;
+  for (int s = 0; s < nstage; ++s) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // stage s landed (this thread's part)
+    group_sync();  // .. and everyone's; everyone is done with stage s - 1
+    copy(s + 2, gnext);
+    gnext = term_of(s + 3);
+    const float* st = zs + ((s % kSdBufs) * G + grp) * kStageFloats;
+#pragma unroll 2
+    for (int q = 0; q < kSdStage; ++q) {
+      float ra[18], rb[18];
+      sd_load18(st + q * (2 * kSdB * kZS) + ra_off, ra);
+      sd_load18(st + q * (2 * kSdB * kZS) + rb_off, rb);
+#pragma unroll
+      for (int r = 0; r < 6; ++r)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          float w = acc[6 * r + c];
+          w = fmaf(ra[3 * r], rb[3 * c], w);
+          w = fmaf(ra[3 * r + 1], rb[3 * c + 1], w);
+          w = fmaf(ra[3 * r + 2], rb[3 * c + 2], w);
+          acc[6 * r + c] = w;
+        }
     }
-  // the term indices run two rounds ahead, the Z records one round ahead
-  float4 vr[5], vc[5];
-  sd_fetch(a.zmat, term_of(0, fr), vr);
-  sd_fetch(a.zmat, term_of(0, fc), vc);
-  int gr_next = term_of(kSdPts, fr), gc_next = term_of(kSdPts, fc);
-  for (int p0 = 0; p0 < a.np; p0 += kSdPts) {
-    __syncthreads();  // the previous round's reads are done
-    sd_store(&zr[pp][6 * slot], vr);
-    sd_store(&zc[pp][6 * slot], vc);
-    __syncthreads();
-    if (p0 + kSdPts < a.np) {  // next round, in flight during the products
-      sd_fetch(a.zmat, gr_next, vr);
-      sd_fetch(a.zmat, gc_next, vc);
-      gr_next = term_of(p0 + 2 * kSdPts, fr);
-      gc_next = term_of(p0 + 2 * kSdPts, fc);
-    }
-    const int npt = a.np - p0 < kSdPts ? a.np - p0 : kSdPts;
-    for (int q = 0; q < npt; ++q) {
-      float4 ra[3];
+    if (s % kStages == kStages - 1) {  // the round is complete
 #pragma unroll
-      for (int i = 0; i < 3; ++i) ra[i] = reinterpret_cast<const float4*>(&zr[q][rq + 16 * i][0])[0];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float4 cb[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) cb[j] = reinterpret_cast<const float4*>(&zc[q][cq + 8 * (3 * h + j)][0])[0];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            float w = acc[i][3 * h + j];
-            w = fmaf(ra[i].x, cb[j].x, w);
-            w = fmaf(ra[i].y, cb[j].y, w);
-            w = fmaf(ra[i].z, cb[j].z, w);
-            acc[i][3 * h + j] = w;
-          }
+      for (int e = 0; e < 36; ++e) {
+        sums[grp * kSdEntries + e * kSdGroup + t] = acc[e];
+        acc[e] = 0.0f;
       }
-    }
+      __syncthreads();
+      const int r0 = (s / kStages) * G, ng = min(G, nround - r0);
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        acc_addf(accd[i][j], acc[i][j]);
-        acc[i][j] = 0.0f;
+      for (int u = 0; u < kPer; ++u) {
+        const int e = tid + u * kSdGroup * G;
+        if (e < kSdEntries)
+          for (int g = 0; g < ng; ++g) acc_addf(accd[u], sums[g * kSdEntries + e]);
       }
+      __syncthreads();
+    }
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   const double nu = ctrl->nu;
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      const int row = 6 * I0 + rq + 16 * i, col = 6 * J0 + cq + 8 * j;
-      if (row >= a.n6 || col >= a.n6 || col > row) continue;
-      const dd t = acc_get(accd[i][j]);
-      const int bj = row / 6, bk = col / 6, r = row % 6, cc = col % 6;
-      dd vd;
-      if (bj == bk) {
-        dd base = dd_from_double(a.ufull[36 * bj + r * 6 + cc]);
-        if (r == cc) base = dd_add(base, dd_from_double(nu * a.cnt_f[bj]));
-        vd = dd_sub(base, t);
-      } else {
-        vd = dd_neg(t);
-      }
-      const double w = dd_to_double(vd);
-      a.S[static_cast<int64_t>(row) * a.n6 + col] = w;
-      a.S[static_cast<int64_t>(col) * a.n6 + row] = w;
-      if (a.S2) {
-        a.S2[static_cast<int64_t>(row) * a.n6 + col] = make_float2(vd.hi, vd.lo);
-        a.S2[static_cast<int64_t>(col) * a.n6 + row] = make_float2(vd.hi, vd.lo);
-      }
+  for (int u = 0; u < kPer; ++u) {
+    const int e = tid + u * kSdGroup * G;
+    if (e >= kSdEntries) continue;
+    const int b = e % kSdGroup, r = (e / kSdGroup) / 6, cc = (e / kSdGroup) % 6;
+    const int bj = I0 + (b >> 3), bk = J0 + (b & 7);
+    const int row = 6 * bj + r, col = 6 * bk + cc;
+    if (row >= a.n6 || col >= a.n6 || col > row) continue;
+    const dd tt = acc_get(accd[u]);
+    dd vd;
+    if (bj == bk) {
+      dd base = dd_from_double(a.ufull[36 * bj + r * 6 + cc]);
+      if (r == cc) base = dd_add(base, dd_from_double(nu * a.cnt_f[bj]));
+      vd = dd_sub(base, tt);
+    } else {
+      vd = dd_neg(tt);
     }
+    const double w = dd_to_double(vd);
+    a.S[static_cast<int64_t>(row) * a.n6 + col] = w;
+    a.S[static_cast<int64_t>(col) * a.n6 + row] = w;
+    if (a.S2) {
+      a.S2[static_cast<int64_t>(row) * a.n6 + col] = make_float2(vd.hi, vd.lo);
+      a.S2[static_cast<int64_t>(col) * a.n6 + row] = make_float2(vd.hi, vd.lo);
+    }
+  }
 }
-__global__ void __launch_bounds__(kSdThreads, 3) k_schur_dense(SchurDenseArgs a, const Ctrl* ctrl) {
-  schur_dense_body(a, ctrl, blockIdx.x, gridDim.x);
+template <int G>
+__global__ void __launch_bounds__(kSdGroup * G, G > 2 ? 1 : 4) k_schur_dense(SchurDenseArgs a, const Ctrl* ctrl) {
+  schur_dense_body<G>(a, ctrl, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -3319,9 +3334,21 @@ static int schur_dense_grid(const Sizes& s) {
   return nb * (nb + 1) / 2;
 }
 
+// Eight groups a CTA up to this many tiles (one CTA an SM), two beyond.
+constexpr int kSdWide = 304;
+
+int schur_dense_setup() {
+  return (raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<8>), schur_dense_smem(8)) == cudaSuccess &&
+          raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<2>), schur_dense_smem(2)) == cudaSuccess)
+             ? 0
+             : -1;
+}
+
 int launch_schur(const Sizes& s, const Dev& d, cudaStream_t st) {
   if (s.schur_dense) {
-    k_schur_dense<<<schur_dense_grid(s), kSdThreads, 0, st>>>(make_schur_dense_args(s, d), d.ctrl);
+    const int grid = schur_dense_grid(s);
+    if (grid <= kSdWide) k_schur_dense<8><<<grid, kSdGroup * 8, schur_dense_smem(8), st>>>(make_schur_dense_args(s, d), d.ctrl);
+    else k_schur_dense<2><<<grid, kSdGroup * 2, schur_dense_smem(2), st>>>(make_schur_dense_args(s, d), d.ctrl);
     return 1 + launch_intr_fill(s, d, st);
   }
   const SchurArgs a = make_schur_args(s, d);
@@ -3784,9 +3811,10 @@ __global__ void __launch_bounds__(64) k_camera_finalize_w(WinTab<FinArgs> t) {
   camera_finalize_body(a.nf, a.fb_tile_begin, a.tile_part, a.ufull, a.bf, a.rb, t.ctrl[q.w], a.with_schur, nullptr,
                        nullptr, nullptr, nullptr, nullptr, q.b, q.nb);
 }
-__global__ void __launch_bounds__(kSdThreads, 3) k_schur_dense_w(WinTab<SchurDenseArgs> t) {
+template <int G>
+__global__ void __launch_bounds__(kSdGroup * G, G > 2 ? 1 : 4) k_schur_dense_w(WinTab<SchurDenseArgs> t) {
   const WinPos q = win_pos(t);
-  schur_dense_body(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
+  schur_dense_body<G>(t.args[q.w], t.ctrl[q.w], q.b);
 }
 __global__ void __launch_bounds__(256, 2) k_schur_w(WinTab<SchurArgs> t) {
   const WinPos q = win_pos(t);
@@ -4019,7 +4047,10 @@ BatchTables* batch_tables_create(const std::vector<BatchWin>& wins, int skip_fin
        raise_dynamic_smem(reinterpret_cast<const void*>(k_landmark_chunks_w<false>), T->lmk_chunks.smem) !=
            cudaSuccess) ||
       (T->bsub.smem > 48 * 1024 &&
-       raise_dynamic_smem(reinterpret_cast<const void*>(k_backsub_chunks_w), T->bsub.smem) != cudaSuccess)) {
+       raise_dynamic_smem(reinterpret_cast<const void*>(k_backsub_chunks_w), T->bsub.smem) != cudaSuccess) ||
+      (T->schur_dense.blocks > 0 &&
+       (raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense_w<8>), schur_dense_smem(8)) != cudaSuccess ||
+        raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense_w<2>), schur_dense_smem(2)) != cudaSuccess))) {
     *err = cudaErrorInvalidValue;
     batch_tables_destroy(T, st);
     return nullptr;
@@ -4080,8 +4111,11 @@ int batch_launch_iteration(const BatchTables* t, cudaStream_t st) {
   if (go(t->fin)) k_camera_finalize_w<<<t->fin.blocks, 64, 0, st>>>(wtab<FinArgs>(t, t->fin));
   if (go(t->schur)) k_schur_w<<<t->schur.blocks, 256, 0, st>>>(wtab<SchurArgs>(t, t->schur));
   if (go(t->schur_red)) k_schur_reduce_w<<<t->schur_red.blocks, 256, 0, st>>>(wtab<SchurArgs>(t, t->schur_red));
-  if (go(t->schur_dense))
-    k_schur_dense_w<<<t->schur_dense.blocks, kSdThreads, 0, st>>>(wtab<SchurDenseArgs>(t, t->schur_dense));
+  if (go(t->schur_dense)) {
+    const int nb = t->schur_dense.blocks;
+    if (nb <= kSdWide) k_schur_dense_w<8><<<nb, kSdGroup * 8, schur_dense_smem(8), st>>>(wtab<SchurDenseArgs>(t, t->schur_dense));
+    else k_schur_dense_w<2><<<nb, kSdGroup * 2, schur_dense_smem(2), st>>>(wtab<SchurDenseArgs>(t, t->schur_dense));
+  }
   n += launch_dense_batch(t->dense, st);
   if (go(t->bsub)) k_backsub_chunks_w<<<t->bsub.blocks, 256, t->bsub.smem, st>>>(wtab<BsubArgs>(t, t->bsub));
   if (go(t->gauge)) k_gauge_partials_w<<<t->gauge.blocks, 256, 0, st>>>(wtab<GaugeArgs>(t, t->gauge));

@@ -123,6 +123,7 @@ struct sgba_problem {
   std::vector<double> cnt_f_base;  // damping counts of the free poses without pose priors
   int gauge_base = -1;             // gauge kind without pose priors (-1: not saved yet)
   int intr_free = 0;  // the camera params are a Free family (sgba_problem_create_ex)
+  int64_t n_cam_g = 0;  // entries of the cameras' term lists
   int camera_model = SGBA_CAMERA_PINHOLE;
   double eucm_ab[2] = {0.0, 0.0};  // EUCM alpha beta
   Sizes sz{};
@@ -868,6 +869,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   if ((st = dev_upload(p, &d.cnt_f, P.cnt_f))) return st;
   if ((st = dev_upload(p, &d.cnt_m, P.cnt_m))) return st;
   if ((st = dev_upload(p, &d.cam_g, P.cam_g))) return st;
+  p->n_cam_g = static_cast<int64_t>(P.cam_g.size());
   if ((st = dev_upload(p, &d.tile_fb, P.tile_fb))) return st;
   if ((st = dev_upload(p, &d.tile_begin, P.tile_begin))) return st;
   if ((st = dev_upload(p, &d.tile_end, P.tile_end))) return st;
@@ -1799,6 +1801,8 @@ int sgba_covariance_prepare(sgba_problem* p, sgba_cov_info* info) {
     if ((st = cov_alloc(p, &c.hcc, 36))) return st;
     if ((st = cov_alloc(p, &c.hcp, 36 * static_cast<size_t>(std::max(s.nf, 1))))) return st;
   }
+  c.ncam_g = p->n_cam_g;
+  if ((st = cov_alloc(p, &c.cam_pt, static_cast<size_t>(c.ncam_g)))) return st;
   if ((st = cov_alloc(p, &c.rec, static_cast<size_t>(sgba::kCovRec) * s.ng))) return st;
   if ((st = cov_alloc(p, &c.y, 18 * static_cast<size_t>(s.ng)))) return st;
   if ((st = cov_alloc(p, &c.vinv, 9 * static_cast<size_t>(s.nm)))) return st;
@@ -1814,7 +1818,6 @@ int sgba_covariance_prepare(sgba_problem* p, sgba_cov_info* info) {
   cudaEvent_t ev[4];
   for (cudaEvent_t& e : ev) SGBA_CK(evs.create(&e));
   SGBA_CK(cudaMemsetAsync(c.status, 0, 2 * sizeof(int), str));
-  SGBA_CK(cudaMemsetAsync(c.y, 0, sizeof(double) * 18 * std::max<int64_t>(s.ng, 1), str));
   if (nn) SGBA_CK(cudaMemsetAsync(c.S, 0, sizeof(double) * nn, str));
   SGBA_CK(cudaEventRecord(ev[0], str));
   int launches = 0;
@@ -1847,7 +1850,7 @@ int sgba_covariance_prepare(sgba_problem* p, sgba_cov_info* info) {
   c.rank = static_cast<int>(J.size());
   if (n > 0) {
     if (c.rank == n) {
-      launches += sgba::launch_cov_inverse(n, c.S, c.ldiag, c.dpiv, c.Z, c.work, str);
+      SGBA_CK(sgba::launch_cov_inverse(n, c.S, c.ldiag, c.dpiv, c.Z, c.work, str, &launches));
     } else {
       int g_ok = 1;
       SGBA_CK(sgba::cov_pinv(n, c.S, c.ldiag, c.dpiv, J, c.Z, p->pool, str, &g_ok));

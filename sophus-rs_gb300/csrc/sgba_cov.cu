@@ -27,32 +27,26 @@
 //                    W = J_pose^T J_point, J_point^T J_point (times the
 //                    term's observation count: its observations share J)
 //   k_cov_points     thread per marginalized point: H_mm = sum over its terms
-//                    (term order), its inverse (cofactors, singular iff the
-//                    determinant is 0, as nalgebra's try_inverse), and
-//                    Y = W H_mm^-1 for its terms with a free pose
-//   k_cov_s          warp per lower block (a, b) of S: the diagonal block
+//                    (term order) and its inverse (cofactors, singular iff
+//                    the determinant is 0, as nalgebra's try_inverse)
+//   k_cov_y          Y = W H_mm^-1 of the terms with a free pose
+//   k_cov_s          CTA per lower block (a, b) of S: the diagonal block
 //                    U_a + priors + edges - sum Y W^T over pose a's terms;
 //                    off-diagonal blocks - sum Y_a W_b^T over the points both
-//                    poses see (the lanes merge slices of the two poses' term
-//                    lists, which are in point order) + J_m^T J_n of edges;
+//                    poses see (32 slices of pose a's term list, in point
+//                    order, searched in pose b's) + J_m^T J_n of edges;
 //                    both triangles written.  No atomics: lane sums by a
 //                    fixed shuffle tree, one writer per entry.
-//   k_cov_panel /    right-looking scalar LDL^T in natural order, one 6-row
-//   k_cov_update     pose block per step: every CTA factors the 6x6 diagonal
-//                    block redundantly with the reference's pivot rule
-//                    (dense_ldlt.rs:164-230: a pivot at most
+//   k_cov_diag /     right-looking scalar LDL^T in natural order, 6-row pose
+//   k_cov_rows /     blocks with the reference's pivot rule
+//   k_cov_update     (dense_ldlt.rs:164-230: a pivot at most
 //                    1e-12 max(1, largest pivot so far in its block) is
-//                    zeroed and zeroes its column of L), solves its rows of
-//                    the column below, then the trailing lower triangle is
-//                    updated in 32 x 32 tiles
-//   k_cov_inv_part / Z = S^-1 by the Takahashi recurrence on the factor,
-//   k_cov_inv_fin /  block rows last to first:
-//   k_cov_inv_diag     Z_rc = delta_rc / d_r - sum_{m > r} L_mr Z_mc  (c >= r);
-//                    the sums over m of the block row's columns beyond the
-//                    block (thread per column, rows m split over CTAs, reading
-//                    rows of Z written by the launches before), their finish
-//                    (the 6-row recurrence, the row and its mirror, the
-//                    diagonal block's sums), then the 6x6 diagonal block
+//                    zeroed and zeroes its column of L), launched by panels
+//                    of eight: the panel's diagonal block, the rows below it,
+//                    the trailing lower triangle in 32 x 32 tiles
+//   k_cov_winv /     S^-1 = W^T D^-1 W, W = L^-1 by doubling blocks, and the
+//   k_cov_wlevel /   product
+//   k_cov_wtw
 //   k_cov_gemm       tiled f64 products of the pseudo-inverse (rank-deficient S)
 //   k_cov_query      CTA per query: covariance or H blocks from Z, Y, H_mm^-1
 #include <cuda_runtime.h>
@@ -72,9 +66,6 @@ namespace {
 constexpr int kCovThreads = 256;
 constexpr double kCovTolRel = 1e-12;  // BlockSparseLdlt's tol_rel
 constexpr int kUT = 32;               // trailing-update tile
-constexpr int kInvRows = 256;         // rows of L staged per round of k_cov_inv_part
-constexpr int kInvSplitMax = 32;      // ranges of rows m of one block row at most
-constexpr int kInvMinRows = 32;       // rows m per range at least
 constexpr int kGT = 64, kGK = 16;     // GEMM tile and depth
 
 // ---------------------------------------------------------------------------
@@ -240,19 +231,19 @@ __device__ bool inverse3(const double* m, double* o) {
   return true;
 }
 
-__global__ void __launch_bounds__(kCovThreads) k_cov_points(int np, const int64_t* __restrict__ pt_g_begin,
-                                                           const int32_t* __restrict__ g_pose,
-                                                           const int32_t* __restrict__ pose_fb,
-                                                           const int32_t* __restrict__ pt_mb,
-                                                           const double* __restrict__ rec, double* __restrict__ vinv,
-                                                           double* __restrict__ y, int* status,
-                                                           const double* __restrict__ crec, double* __restrict__ wc,
-                                                           double* __restrict__ yc) {
+// A thread per point: H_mm over the point's terms in order and its inverse.
+constexpr int kCovPtT = 64;  // small CTAs: a few thousand points spread over the GPU
+__global__ void __launch_bounds__(kCovPtT) k_cov_points(int np, const int64_t* __restrict__ pt_g_begin,
+                                                       const int32_t* __restrict__ pt_mb,
+                                                       const double* __restrict__ rec, double* __restrict__ vinv,
+                                                       int* status, const double* __restrict__ crec,
+                                                       double* __restrict__ wc, double* __restrict__ yc) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= np) return;
   const int mb = pt_mb[q];
   if (mb < 0) return;
   double v[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 4
   for (int64_t g = pt_g_begin[q]; g < pt_g_begin[q + 1]; ++g)
     for (int k = 0; k < 6; ++k) v[k] += rec[kCovRec * g + 39 + k];
   const double V[9] = {v[0], v[1], v[2], v[1], v[3], v[4], v[2], v[4], v[5]};
@@ -264,14 +255,6 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_points(int np, const int64_
     return;
   }
   for (int k = 0; k < 9; ++k) vo[k] = Vi[k];
-  for (int64_t g = pt_g_begin[q]; g < pt_g_begin[q + 1]; ++g) {
-    if (pose_fb[g_pose[g]] < 0) continue;
-    const double* W = rec + kCovRec * g + 21;
-    double* yo = y + 18 * g;
-    for (int a = 0; a < 6; ++a)
-      for (int j = 0; j < 3; ++j)
-        yo[3 * a + j] = W[3 * a] * Vi[j] + W[3 * a + 1] * Vi[3 + j] + W[3 * a + 2] * Vi[6 + j];
-  }
   if (!crec) return;
   // free camera params: W_cq = sum of the point's J_cam^T J_point, Y_cq = W_cq H_mm^-1
   double W[18];
@@ -285,6 +268,31 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_points(int np, const int64_
       wo[3 * a + j] = W[3 * a + j];
       yo[3 * a + j] = W[3 * a] * Vi[j] + W[3 * a + 1] * Vi[3 + j] + W[3 * a + 2] * Vi[6 + j];
     }
+}
+
+// Y = W H_mm^-1 of the terms with a free pose and a marginalized point (zero
+// for the others), a thread per row.  (The thread per point that formed them
+// term by term left most of the GPU idle: 188 us for 5,001 points of 25 terms.)
+__global__ void __launch_bounds__(kCovThreads) k_cov_y(int64_t ng, const int32_t* __restrict__ g_pose,
+                                                      const int32_t* __restrict__ g_pt,
+                                                      const int32_t* __restrict__ pose_fb,
+                                                      const int32_t* __restrict__ pt_mb,
+                                                      const double* __restrict__ rec,
+                                                      const double* __restrict__ vinv, double* __restrict__ y) {
+  const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t g = e / 6;
+  if (g >= ng) return;
+  const int a = static_cast<int>(e - 6 * g);
+  const int mb = pt_mb[g_pt[g]];
+  double* yo = y + 18 * g + 3 * a;
+  if (mb < 0 || pose_fb[g_pose[g]] < 0) {
+    for (int j = 0; j < 3; ++j) yo[j] = 0.0;
+    return;
+  }
+  const double* W = rec + kCovRec * g + 21;
+  const double* Vi = vinv + 9 * static_cast<int64_t>(mb);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) yo[j] = W[3 * a] * Vi[j] + W[3 * a + 1] * Vi[3 + j] + W[3 * a + 2] * Vi[6 + j];
 }
 
 // The camera block of S (free camera params, rows 0..5 of S; rows nk..5 are
@@ -340,7 +348,7 @@ struct CovSArgs {
   const int64_t* tile_begin;
   const int64_t* tile_end;
   const int64_t* cam_g;
-  const int32_t* g_pt;
+  const int32_t* cam_pt;     // point of every entry of cam_g
   const int32_t* pt_mb;
   const double* rec;
   const double* y;
@@ -367,143 +375,177 @@ __device__ __forceinline__ void cam_range(const CovSArgs& a, int fb, int64_t* b,
   *e = t0 < t1 ? a.tile_end[t1 - 1] : 0;
 }
 
-// acc (6x6, row-major) -= Y W^T
+// row r of acc (6x6) -= Y W^T, Y the row's three entries
 __device__ __forceinline__ void sub_ywt(double* acc, const double* Y, const double* W) {
-  for (int r = 0; r < 6; ++r)
-    for (int c = 0; c < 6; ++c)
-      acc[6 * r + c] -= Y[3 * r] * W[3 * c] + Y[3 * r + 1] * W[3 * c + 1] + Y[3 * r + 2] * W[3 * c + 2];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) acc[c] -= Y[0] * W[3 * c] + Y[1] * W[3 * c + 1] + Y[2] * W[3 * c + 2];
 }
 
-// the 36 lane sums of a warp by a fixed shuffle tree (lane 0 holds the totals)
-__device__ __forceinline__ void warp_sum36(double* acc) {
+// the lanes' sums of a warp by a fixed shuffle tree (lane 0 holds the totals)
+__device__ __forceinline__ void warp_sum6(double* acc) {
 #pragma unroll
-  for (int k = 0; k < 36; ++k)
+  for (int k = 0; k < 6; ++k)
     for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], off);
 }
 
-// A warp per lower block (fa, fb) of S.  Diagonal blocks: the lanes take
-// pose fa's terms in turn.  Off-diagonal blocks: lane l merges its slice of
-// pose fa's term list (1/32 of it, in point order) with pose fb's list from
-// the first term at or after the slice's first point (one binary search).
-__global__ void __launch_bounds__(128) k_cov_s(CovSArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t s = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  if (s >= a.nsb) return;  // the whole warp
+// the point of every entry of the cameras' term lists
+__global__ void __launch_bounds__(kCovThreads) k_cov_cam_pt(int64_t n, const int64_t* __restrict__ cam_g,
+                                                           const int32_t* __restrict__ g_pt, int32_t* __restrict__ out) {
+  const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (e < n) out[e] = g_pt[cam_g[e]];
+}
+
+// A CTA per lower block (fa, fb) of S, warp r its row r.  Diagonal blocks: the
+// lanes take pose fa's terms in turn.  Off-diagonal blocks: lane l takes its
+// slice of pose fa's term list (1/32 of it, in point order): for a piece of
+// every slice the CTA first finds the terms of pose fb on the same points (a
+// binary search per term, all of them at once), then the lanes add theirs in
+// order.  (A warp per block that merged the two lists step by step, 36 sums a
+// lane, spent its time on the chain of list loads: 1.5 ms for 741 blocks of
+// 1,250 x 1,250 terms.)
+constexpr int kCovSThreads = 192;
+constexpr int kCovPiece = 32;  // terms of a slice searched at once
+constexpr int kCovStage = 8;   // of which this many have their W (6x3) in shared memory at a time
+__global__ void __launch_bounds__(kCovSThreads) k_cov_s(CovSArgs a) {
+  __shared__ int s_gi[kCovPiece][32], s_gj[kCovPiece][32];
+  // W of the matches, [entry][match]: the lanes' own reads of 18 entries from 32
+  // records would take 32 cache wavefronts each, for every row's warp
+  __shared__ double s_w[18][kCovStage * 32];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int64_t s = blockIdx.x;
   const int fa = a.sb_row[s], fb = a.sb_col[s];
-  double acc[36];
-#pragma unroll
-  for (int k = 0; k < 36; ++k) acc[k] = 0.0;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
   int64_t ib, ie;
   cam_range(a, fa, &ib, &ie);
   if (fa == fb) {
     for (int64_t i = ib + lane; i < ie; i += 32) {
       const double* h = a.rec + kCovRec * a.cam_g[i];
-      for (int r = 0; r < 6; ++r)
-        for (int c = 0; c < 6; ++c) acc[6 * r + c] += h[r <= c ? up_idx(6, r, c) : up_idx(6, c, r)];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) acc[c] += h[r <= c ? up_idx(6, r, c) : up_idx(6, c, r)];
     }
-    warp_sum36(acc);
+    warp_sum6(acc);
     if (lane == 0) {
       if (a.prior_beg)
         for (int q = a.prior_beg[fa]; q < a.prior_beg[fa + 1]; ++q)
-          for (int k = 0; k < 36; ++k) acc[k] += a.prior_out[static_cast<int64_t>(kPriorOut) * q + k];
+          for (int c = 0; c < 6; ++c) acc[c] += a.prior_out[static_cast<int64_t>(kPriorOut) * q + 6 * r + c];
       if (a.e_beg)
         for (int q = a.e_beg[fa]; q < a.e_beg[fa + 1]; ++q)
-          for (int k = 0; k < 36; ++k) acc[k] += a.e_out[static_cast<int64_t>(kPriorOut) * a.e_slot[q] + k];
-      for (int k = 0; k < 36; ++k) a.hdiag[36 * static_cast<int64_t>(fa) + k] = acc[k];
+          for (int c = 0; c < 6; ++c) acc[c] += a.e_out[static_cast<int64_t>(kPriorOut) * a.e_slot[q] + 6 * r + c];
+      for (int c = 0; c < 6; ++c) a.hdiag[36 * static_cast<int64_t>(fa) + 6 * r + c] = acc[c];
     }
     // the Schur part, then lane 0 adds back the H block it stored
+    double h0[6];
 #pragma unroll
-    for (int k = 0; k < 36; ++k) acc[k] = 0.0;
+    for (int c = 0; c < 6; ++c) {
+      h0[c] = acc[c];
+      acc[c] = 0.0;
+    }
     for (int64_t i = ib + lane; i < ie; i += 32) {
       const int64_t g = a.cam_g[i];
-      if (a.pt_mb[a.g_pt[g]] < 0) continue;
-      sub_ywt(acc, a.y + 18 * g, a.rec + kCovRec * g + 21);
+      if (a.pt_mb[a.cam_pt[i]] < 0) continue;
+      sub_ywt(acc, a.y + 18 * g + 3 * r, a.rec + kCovRec * g + 21);
     }
-    warp_sum36(acc);
-    if (lane == 0)
-      for (int k = 0; k < 36; ++k) acc[k] += a.hdiag[36 * static_cast<int64_t>(fa) + k];
+    warp_sum6(acc);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) acc[c] += h0[c];
   } else {
     int64_t jb, je;
     cam_range(a, fb, &jb, &je);
     const int64_t len = ie - ib;
-    int64_t i = ib + len * lane / 32;
-    const int64_t iend = ib + len * (lane + 1) / 32;
-    int64_t j = je;
-    if (i < iend) {
-      // first term of pose fb whose point is >= this slice's first point
-      const int p0 = a.g_pt[a.cam_g[i]];
-      int64_t lo = jb, hi = je;
-      while (lo < hi) {
-        const int64_t mid = lo + (hi - lo) / 2;
-        if (a.g_pt[a.cam_g[mid]] < p0) lo = mid + 1;
-        else hi = mid;
+    const int64_t longest = (len + 31) / 32;
+    for (int64_t p0 = 0; p0 < longest; p0 += kCovPiece) {
+      __syncthreads();
+      for (int e = threadIdx.x; e < 32 * kCovPiece; e += kCovSThreads) {
+        const int l = e & 31, u = e >> 5;
+        const int64_t i = ib + len * l / 32 + p0 + u;
+        int gi = 0, gj = -1;
+        if (i < ib + len * (l + 1) / 32) {
+          const int pt = a.cam_pt[i];
+          if (a.pt_mb[pt] >= 0) {
+            int64_t lo = jb, hi = je;
+            while (lo < hi) {
+              const int64_t mid = lo + (hi - lo) / 2;
+              if (a.cam_pt[mid] < pt) lo = mid + 1;
+              else hi = mid;
+            }
+            if (lo < je && a.cam_pt[lo] == pt) {
+              gi = static_cast<int>(a.cam_g[i]);
+              gj = static_cast<int>(a.cam_g[lo]);
+            }
+          }
+        }
+        s_gi[u][l] = gi;
+        s_gj[u][l] = gj;
       }
-      j = lo;
-    }
-    while (i < iend && j < je) {
-      const int64_t gi = a.cam_g[i], gj = a.cam_g[j];
-      const int pi = a.g_pt[gi], pj = a.g_pt[gj];
-      if (pi < pj) {
-        ++i;
-      } else if (pj < pi) {
-        ++j;
-      } else {
-        if (a.pt_mb[pi] >= 0) sub_ywt(acc, a.y + 18 * gi, a.rec + kCovRec * gj + 21);
-        ++i;
-        ++j;
+      __syncthreads();
+      const int un = static_cast<int>(min(static_cast<int64_t>(kCovPiece), longest - p0));
+      for (int u0 = 0; u0 < un; u0 += kCovStage) {
+        for (int e = threadIdx.x; e < 18 * kCovStage * 32; e += kCovSThreads) {
+          const int m = e / 18, k = e - 18 * m;
+          const int gj = s_gj[u0 + (m >> 5)][m & 31];
+          if (gj >= 0) s_w[k][m] = a.rec[kCovRec * static_cast<int64_t>(gj) + 21 + k];
+        }
+        __syncthreads();
+        for (int u = 0; u < kCovStage; ++u) {
+          if (s_gj[u0 + u][lane] < 0) continue;
+          const double* Y = a.y + 18 * static_cast<int64_t>(s_gi[u0 + u][lane]) + 3 * r;
+          const double y0 = Y[0], y1 = Y[1], y2 = Y[2];
+          const int m = 32 * u + lane;
+#pragma unroll
+          for (int c = 0; c < 6; ++c) acc[c] -= y0 * s_w[3 * c][m] + y1 * s_w[3 * c + 1][m] + y2 * s_w[3 * c + 2][m];
+        }
+        __syncthreads();
       }
     }
-    warp_sum36(acc);
+    warp_sum6(acc);
     if (lane == 0 && a.eblk_begin)
       for (int q = a.eblk_begin[s]; q < a.eblk_begin[s + 1]; ++q) {
         const int32_t tt = a.eblk_term[q];
         const int64_t term = tt & 0x7fffffff;
-        for (int r = 0; r < 6; ++r)
-          for (int c = 0; c < 6; ++c)
-            acc[6 * r + c] += (tt < 0) ? a.e_hmn[36 * term + c * 6 + r] : a.e_hmn[36 * term + r * 6 + c];
+        for (int c = 0; c < 6; ++c)
+          acc[c] += (tt < 0) ? a.e_hmn[36 * term + c * 6 + r] : a.e_hmn[36 * term + r * 6 + c];
       }
   }
   const int64_t n = a.n;
   if (lane == 0)
-    for (int r = 0; r < 6; ++r)
-      for (int c = 0; c < 6; ++c) {
-        // the diagonal block from its lower triangle (exactly symmetric)
-        const double v = (fa == fb && c > r) ? acc[6 * c + r] : acc[6 * r + c];
-        const int64_t row = a.nci + 6 * fa + r, col = a.nci + 6 * fb + c;
-        a.S[row * n + col] = v;
-        a.S[col * n + row] = v;
-      }
+    for (int c = 0; c < 6; ++c) {
+      if (fa == fb && c > r) continue;  // the diagonal block from its lower triangle (exactly symmetric)
+      const int64_t row = a.nci + 6 * fa + r, col = a.nci + 6 * fb + c;
+      a.S[row * n + col] = acc[c];
+      a.S[col * n + row] = acc[c];
+    }
   if (fa != fb || !a.crec) return;
   // free camera params: the pose's camera columns S_ac = H_ac - sum over its
-  // terms with a marginalized point of Y_g W_cq^T (acc[6 r + k]: pose row r, camera column k)
+  // terms with a marginalized point of Y_g W_cq^T (acc[k]: pose row r, camera column k)
 #pragma unroll
-  for (int k = 0; k < 36; ++k) acc[k] = 0.0;
+  for (int k = 0; k < 6; ++k) acc[k] = 0.0;
   for (int64_t i = ib + lane; i < ie; i += 32) {
     const double* hc = a.crec + kCovCamRec * a.cam_g[i] + 21;
-    for (int k = 0; k < 6; ++k)
-      for (int r = 0; r < 6; ++r) acc[6 * r + k] += hc[6 * k + r];
-  }
-  warp_sum36(acc);
-  if (lane == 0)
-    for (int k = 0; k < 6; ++k)
-      for (int r = 0; r < 6; ++r) a.hcp[36 * static_cast<int64_t>(fa) + 6 * k + r] = acc[6 * r + k];
 #pragma unroll
-  for (int k = 0; k < 36; ++k) acc[k] = 0.0;
+    for (int k = 0; k < 6; ++k) acc[k] += hc[6 * k + r];
+  }
+  warp_sum6(acc);
+  double h0[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    h0[k] = acc[k];
+    if (lane == 0) a.hcp[36 * static_cast<int64_t>(fa) + 6 * k + r] = acc[k];
+    acc[k] = 0.0;
+  }
   for (int64_t i = ib + lane; i < ie; i += 32) {
     const int64_t g = a.cam_g[i];
-    const int mb = a.pt_mb[a.g_pt[g]];
+    const int mb = a.pt_mb[a.cam_pt[i]];
     if (mb < 0) continue;
-    sub_ywt(acc, a.y + 18 * g, a.wc + 18 * static_cast<int64_t>(mb));
+    sub_ywt(acc, a.y + 18 * g + 3 * r, a.wc + 18 * static_cast<int64_t>(mb));
   }
-  warp_sum36(acc);
+  warp_sum6(acc);
   if (lane != 0) return;
-  for (int r = 0; r < 6; ++r)
-    for (int k = 0; k < 6; ++k) {
-      const double v = a.hcp[36 * static_cast<int64_t>(fa) + 6 * k + r] + acc[6 * r + k];
-      const int64_t row = a.nci + 6 * fa + r;
-      a.S[row * n + k] = v;
-      a.S[static_cast<int64_t>(k) * n + row] = v;
-    }
+  for (int k = 0; k < 6; ++k) {
+    const double v = h0[k] + acc[k];
+    const int64_t row = a.nci + 6 * fa + r;
+    a.S[row * n + k] = v;
+    a.S[static_cast<int64_t>(k) * n + row] = v;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -545,180 +587,427 @@ __device__ int ldlt6(double* a, double* d) {
   return (neg && cond < 1e-10) ? 2 : 0;
 }
 
-// Step k: the diagonal block's factor (every CTA, in shared memory; CTA 0
-// publishes it) and L of the rows below: L_i = c_i L_kk^-T D^+.
-__global__ void __launch_bounds__(kCovThreads) k_cov_panel(int n, int k, double* S, double* ldiag, double* dpiv,
-                                                          int* status) {
-  __shared__ double L6[36], d6[6];
-  const int c0 = 6 * k;
-  if (threadIdx.x == 0) {
-    double a[36], d[6];
-    for (int r = 0; r < 6; ++r)
-      for (int c = 0; c < 6; ++c) a[6 * r + c] = c <= r ? S[static_cast<int64_t>(c0 + r) * n + c0 + c] : 0.0;
-    const int st = ldlt6(a, d);
-    for (int e = 0; e < 36; ++e) L6[e] = a[e];
-    for (int e = 0; e < 6; ++e) d6[e] = d[e];
-    if (blockIdx.x == 0) {
-      for (int e = 0; e < 36; ++e) ldiag[36 * static_cast<int64_t>(k) + e] = a[e];
-      for (int e = 0; e < 6; ++e) dpiv[c0 + e] = d[e];
-      if (st) atomicMax(status, st);
+// The factor goes by panels of kFP = 48 columns (8 pose blocks), three launches
+// each: the diagonal 48 x 48 block in one CTA, the rows below it (a thread
+// each), the trailing triangle.  Every entry of S meets the 6-column steps in
+// order, each as one difference with a sum over its six columns, so L and the
+// pivots keep the bits of the step-by-step factor (two launches per step, 20 us
+// for a step's 6 x 6 block in one thread).
+constexpr int kFP = 48;
+
+// ldlt6 by lanes 0 .. 5 of a warp, a row each (columns updated as soon as their
+// pivot is known).  The rule compares a pivot with the largest pivot before the
+// row in hand; the lanes compare it when it is formed, so a block in which a
+// kept pivot is below that threshold of a later one is redone by lane 0 alone.
+// a: 6x6 lower in shared memory (row stride ld); L6 (36), d6 (6) out.
+__device__ __forceinline__ int ldlt6_warp(const double* a, int ld, double* L6, double* d6, int lane) {
+  const unsigned all = 0xffffffffu;
+  const int j = lane < 6 ? lane : 5;
+  double v[6], l[6], d[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    v[c] = c <= j ? a[j * ld + c] : 0.0;
+    l[c] = 0.0;
+  }
+  double maxp = 1.0, minp = DBL_MAX;
+  int rank = 0, st = 0;
+  bool neg = false;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double dk = __shfl_sync(all, v[k], k);
+    if (!isfinite(dk) && st == 0) st = 1;
+    const bool zero = fabs(dk) <= fmax(maxp, 1.0) * kCovTolRel;
+    d[k] = zero ? 0.0 : dk;
+    if (!zero) {
+      if (dk < 0.0) neg = true;
+      maxp = fmax(maxp, fabs(dk));
+      minp = fmin(minp, fabs(dk));
+      rank += 1;
+    }
+    l[k] = zero ? 0.0 : v[k] / dk;
+    const double ld_k = l[k] * d[k];
+#pragma unroll
+    for (int c = k + 1; c < 6; ++c) {
+      const double lc = __shfl_sync(all, l[k], c);
+      if (c <= j) v[c] -= ld_k * lc;
     }
   }
-  __syncthreads();
-  const int i = c0 + 6 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double* row = S + static_cast<int64_t>(i) * n + c0;
+  // minp <= tol of the largest pivot: a row may see an earlier pivot as zero
+  if (st == 0 && rank > 0 && minp <= fmax(maxp, 1.0) * kCovTolRel) {
+    if (lane == 0) {
+      double b[36];
+      for (int r = 0; r < 6; ++r)
+        for (int c = 0; c < 6; ++c) b[6 * r + c] = c <= r ? a[r * ld + c] : 0.0;
+      st = ldlt6(b, d);
+      for (int e = 0; e < 36; ++e) L6[e] = b[e];
+      for (int e = 0; e < 6; ++e) d6[e] = d[e];
+    }
+    __syncwarp();
+    return __shfl_sync(all, st, 0);
+  }
+  if (lane < 6) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      L6[6 * j + c] = c < j ? l[c] : (c == j ? 1.0 : 0.0);
+      if (c == j) d6[j] = d[c];
+    }
+  }
+  __syncwarp();
+  if (st) return st;
+  const double cond = rank == 0 ? 0.0 : minp / maxp;
+  return (neg && cond < 1e-10) ? 2 : 0;
+}
+
+// L of a row's six columns from its entries x (L6, d6 of the step): in place
+__device__ __forceinline__ void row_solve6(double* x, const double* L6, const double* d6) {
   double yv[6];
+#pragma unroll
   for (int j = 0; j < 6; ++j) {
-    double v = row[j];
+    double v = x[j];
+#pragma unroll
     for (int t = 0; t < j; ++t) v -= yv[t] * L6[6 * j + t];
     yv[j] = v;
   }
-  for (int j = 0; j < 6; ++j) row[j] = d6[j] == 0.0 ? 0.0 : yv[j] / d6[j];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) x[j] = d6[j] == 0.0 ? 0.0 : yv[j] / d6[j];
 }
 
-// Step k: C_ij -= sum_t L_it d_t L_jt on the lower trailing triangle, 32 x 32
-// tiles (tiles above the diagonal return at once).
-__global__ void __launch_bounds__(kCovThreads) k_cov_update(int n, int k, double* S, const double* dpiv) {
-  const int base = 6 * k + 6;
+// The diagonal block of the panel at c0 (w columns): its 6-column steps in
+// shared memory; L below the 6x6 blocks back to S.
+__global__ void __launch_bounds__(kCovThreads) k_cov_diag(int n, int c0, int w, double* S, double* ldiag, double* dpiv,
+                                                         int* status) {
+  __shared__ double A[kFP][kFP + 1], L6[36], d6[6];
+  const int tid = threadIdx.x;
+  for (int e = tid; e < kFP * kFP; e += kCovThreads) {
+    const int r = e / kFP, c = e % kFP;
+    A[r][c] = (r < w && c <= r) ? S[static_cast<int64_t>(c0 + r) * n + c0 + c] : 0.0;
+  }
+  __syncthreads();
+  for (int k0 = 0; k0 < w; k0 += 6) {
+    if (tid < 32) {
+      const int st = ldlt6_warp(&A[k0][k0], kFP + 1, L6, d6, tid);
+      if (st && tid == 0) atomicMax(status, st);
+      for (int e = tid; e < 36; e += 32) ldiag[6 * static_cast<int64_t>(c0 + k0) + e] = L6[e];
+      if (tid < 6) dpiv[c0 + k0 + tid] = d6[tid];
+    }
+    __syncthreads();
+    const int rows = w - k0 - 6;
+    if (tid < rows) row_solve6(&A[k0 + 6 + tid][k0], L6, d6);
+    __syncthreads();
+    for (int e = tid; e < rows * (rows + 1) / 2; e += kCovThreads) {
+      int i = static_cast<int>((sqrtf(8.0f * static_cast<float>(e) + 1.0f) - 1.0f) * 0.5f);
+      while (i * (i + 1) / 2 > e) --i;
+      while ((i + 1) * (i + 2) / 2 <= e) ++i;
+      const double* li = &A[k0 + 6 + i][k0];
+      const int j = e - i * (i + 1) / 2;
+      const double* lj = &A[k0 + 6 + j][k0];
+      double s = 0.0;
+#pragma unroll
+      for (int t = 0; t < 6; ++t) s += li[t] * (lj[t] * d6[t]);
+      A[k0 + 6 + i][k0 + 6 + j] -= s;
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < kFP * kFP; e += kCovThreads) {
+    const int r = e / kFP, c = e % kFP;
+    if (r < w && c / 6 < r / 6) S[static_cast<int64_t>(c0 + r) * n + c0 + c] = A[r][c];
+  }
+}
+
+// The rows below the panel, a thread per row: per step its six entries of L,
+// then the row's entries in the panel's later columns.
+constexpr int kRowsT = 32;
+__global__ void __launch_bounds__(kRowsT) k_cov_rows(int n, int c0, double* S, const double* __restrict__ ldiag,
+                                                    const double* __restrict__ dpiv) {
+  __shared__ double Ld[kFP][kFP], L6[kFP / 6][36], d[kFP], X[kRowsT][kFP + 1];
+  const int tid = threadIdx.x, r0 = c0 + kFP + blockIdx.x * kRowsT;
+  for (int e = tid; e < kFP * kFP; e += kRowsT) {  // L_jt d_t of the panel's own rows
+    const int r = e / kFP, c = e % kFP;
+    Ld[r][c] = c / 6 < r / 6 ? S[static_cast<int64_t>(c0 + r) * n + c0 + c] * dpiv[c0 + c] : 0.0;
+  }
+  for (int e = tid; e < kFP * 6; e += kRowsT) L6[e / 36][e % 36] = ldiag[6 * static_cast<int64_t>(c0) + e];
+  for (int e = tid; e < kFP; e += kRowsT) d[e] = dpiv[c0 + e];
+  bool any = false;
+  for (int e = tid; e < kRowsT * kFP; e += kRowsT) {
+    const int r = e / kFP, c = e % kFP;
+    const double v = r0 + r < n ? S[static_cast<int64_t>(r0 + r) * n + c0 + c] : 0.0;
+    X[r][c] = v;
+    any = any || v != 0.0;
+  }
+  if (!__syncthreads_or(any)) return;  // rows outside the band: L is zero there
+  double* x = X[tid];
+  for (int k0 = 0; k0 < kFP; k0 += 6) {
+    row_solve6(x + k0, L6[k0 / 6], d + k0);
+    double l[6];
+#pragma unroll
+    for (int t = 0; t < 6; ++t) l[t] = x[k0 + t];
+    for (int j = k0 + 6; j < kFP; j += 6) {  // six columns at a time: independent chains
+      double s[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+      for (int t = 0; t < 6; ++t)
+#pragma unroll
+        for (int u = 0; u < 6; ++u) s[u] += l[t] * Ld[j + u][k0 + t];
+#pragma unroll
+      for (int u = 0; u < 6; ++u) x[j + u] -= s[u];
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < kRowsT * kFP; e += kRowsT) {
+    const int r = e / kFP, c = e % kFP;
+    if (r0 + r < n) S[static_cast<int64_t>(r0 + r) * n + c0 + c] = X[r][c];
+  }
+}
+
+// C_ij -= sum_t L_it (d_t L_jt), step by step of the panel, on the lower
+// trailing triangle in 32 x 32 tiles (tiles above the diagonal, and tiles whose
+// rows or columns are zero in the panel, return at once).
+__global__ void __launch_bounds__(kCovThreads) k_cov_update(int n, int c0, double* S, const double* dpiv) {
+  const int base = c0 + kFP;
   const int ti = blockIdx.y, tj = blockIdx.x;
   if (tj > ti) return;
-  __shared__ double Li[kUT][7], Lj[kUT][7];
+  __shared__ double Li[kUT][kFP + 1], Lj[kUT][kFP + 1];
   const int i0 = base + ti * kUT, j0 = base + tj * kUT;
-  for (int e = threadIdx.x; e < kUT * 6; e += blockDim.x) {
-    const int r = e / 6, t = e % 6;
-    Li[r][t] = (i0 + r < n) ? S[static_cast<int64_t>(i0 + r) * n + 6 * k + t] : 0.0;
-    Lj[r][t] = (j0 + r < n) ? S[static_cast<int64_t>(j0 + r) * n + 6 * k + t] * dpiv[6 * k + t] : 0.0;
+  bool nzi = false, nzj = false;
+  for (int e = threadIdx.x; e < kUT * kFP; e += blockDim.x) {
+    const int r = e / kFP, t = e % kFP;
+    const double vi = (i0 + r < n) ? S[static_cast<int64_t>(i0 + r) * n + c0 + t] : 0.0;
+    const double vj = (j0 + r < n) ? S[static_cast<int64_t>(j0 + r) * n + c0 + t] : 0.0;
+    nzi = nzi || vi != 0.0;
+    nzj = nzj || vj != 0.0;
+    Li[r][t] = vi;
+    Lj[r][t] = vj * dpiv[c0 + t];
   }
-  __syncthreads();
-  const int jj = threadIdx.x & 31;
+  const int some = __syncthreads_or(nzi);
+  if (!__syncthreads_or(nzj) || !some) return;
+  const int jj = threadIdx.x & 31, i1 = threadIdx.x >> 5;
   const int j = j0 + jj;
   if (j >= n) return;
-  for (int ii = threadIdx.x >> 5; ii < kUT; ii += blockDim.x >> 5) {
-    const int i = i0 + ii;
-    if (i >= n || j > i) continue;
-    double s = 0.0;
-    for (int t = 0; t < 6; ++t) s += Li[ii][t] * Lj[jj][t];
-    S[static_cast<int64_t>(i) * n + j] -= s;
+  double c[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = i0 + i1 + 8 * u;
+    c[u] = (i < n && j <= i) ? S[static_cast<int64_t>(i) * n + j] : 0.0;
+  }
+  for (int k0 = 0; k0 < kFP; k0 += 6) {
+    double s[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const double lj = Lj[jj][k0 + t];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] += Li[i1 + 8 * u][k0 + t] * lj;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) c[u] -= s[u];
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = i0 + i1 + 8 * u;
+    if (i < n && j <= i) S[static_cast<int64_t>(i) * n + j] = c[u];
   }
 }
 
 // ---------------------------------------------------------------------------
-// Inverse from the factor (Takahashi), block row i (rows r0 = 6i .. r0 + 5),
-// three launches: the sums over the rows m >= 6i + 6 split over ranges of m
-// (enough CTAs to fill the GPU when few columns remain), the finish (sums in
-// range order, the 6-row recurrence, the row and its mirror, and per CTA the
-// diagonal block's sums over the new row), the diagonal block.
+// Inverse from the factor: S^-1 = W^T D^-1 W with W = L^-1 (unit lower), in
+// blocks of kIB = 48.  The diagonal blocks of W in one launch, then level by
+// level (blocks of 1, 2, 4, .. kIB) W21 = -W22 (L21 W11) for all pairs of
+// neighbouring blocks at once: two launches a level, then one for the product,
+// in place of three for each of the n / 6 block rows of the Takahashi
+// recurrence (28 ms of short, latency-bound launches at n = 1,788).  Tiles of
+// L and of L21 W11 that are zero (outside the band of a loop) are skipped.
+// The recurrence multiplies computed entries of the inverse, this does not:
+// against 80-bit arithmetic its error is a tenth (1e-14 of the norm, 100 loop
+// cameras).  W is kept transposed in the upper triangle of S; L21 W11 lives in
+// Z until the product overwrites it.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kCovThreads) k_cov_inv_part(int n, int i, int kchunk, const double* __restrict__ L,
-                                                             const double* __restrict__ Z, double* __restrict__ part) {
-  const int r0 = 6 * i, cb = r0 + 6, ncols = n - cb;
-  const int c = cb + blockIdx.x * blockDim.x + threadIdx.x;
-  const int mbeg = cb + blockIdx.y * kchunk, mend = min(n, mbeg + kchunk);
-  __shared__ double Ls[kInvRows][6];
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int m0 = mbeg; m0 < mend; m0 += kInvRows) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < kInvRows * 6; e += blockDim.x) {
-      const int mm = e / 6, t = e % 6;
-      Ls[mm][t] = (m0 + mm < mend) ? L[static_cast<int64_t>(m0 + mm) * n + r0 + t] : 0.0;
+constexpr int kIB = 48;
+constexpr int kIBp = kIB + 1;
+constexpr size_t kInvSmem = sizeof(double) * 3 * kIB * kIBp;
+
+// W of the diagonal block b: inverses of its 6x6 blocks (a thread per column),
+// then pairs of 6, 12, 24.  Rows past n: identity.  Also 1/d, and which tiles
+// of block row b of L are not zero.
+__global__ void __launch_bounds__(kCovThreads) k_cov_winv(int n, double* S, const double* __restrict__ ldiag,
+                                                         const double* __restrict__ dpiv, double* __restrict__ dinv,
+                                                         int* __restrict__ lnz, int nb) {
+  extern __shared__ double sh[];
+  double* L = sh;
+  double* W = L + kIB * kIBp;
+  double* T = W + kIB * kIBp;
+  const int b = blockIdx.x, r0 = b * kIB, w = min(kIB, n - r0), tid = threadIdx.x;
+  for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+    const int r = e / kIB, c = e % kIB;
+    double v = r == c ? 1.0 : 0.0;
+    if (r < w && c < r)
+      v = r / 6 == c / 6 ? ldiag[36 * static_cast<int64_t>((r0 + r) / 6) + 6 * (r % 6) + c % 6]
+                         : S[static_cast<int64_t>(r0 + r) * n + r0 + c];
+    L[r * kIBp + c] = v;
+    W[r * kIBp + c] = r == c ? 1.0 : 0.0;
+  }
+  if (tid < w) {
+    const double d = dpiv[r0 + tid];
+    dinv[r0 + tid] = d != 0.0 ? 1.0 / d : 0.0;
+  }
+  __syncthreads();
+  if (tid < kIB) {
+    const int c = tid, q0 = c / 6 * 6;
+    for (int r = c + 1; r < q0 + 6; ++r) {
+      double v = 0.0;
+      for (int k = c; k < r; ++k) v -= L[r * kIBp + k] * W[k * kIBp + c];
+      W[r * kIBp + c] = v;
+    }
+  }
+  __syncthreads();
+  for (int h = 6; h < kIB; h *= 2) {
+    const int per = h * h, pairs = kIB / (2 * h);
+    for (int e = tid; e < pairs * per; e += kCovThreads) {
+      const int q = e / per, l0 = q * 2 * h, i = l0 + h + (e % per) / h, j = l0 + e % h;
+      double v = 0.0;
+      for (int k = j; k < l0 + h; ++k) v += L[i * kIBp + k] * W[k * kIBp + j];
+      T[i * kIBp + j] = v;
     }
     __syncthreads();
-    if (c < n) {
-      const int cnt = min(kInvRows, mend - m0);
-      const double* zc = Z + static_cast<int64_t>(m0) * n + c;
-      for (int mm = 0; mm < cnt; ++mm) {
-        const double z = zc[static_cast<int64_t>(mm) * n];
+    for (int e = tid; e < pairs * per; e += kCovThreads) {
+      const int q = e / per, l0 = q * 2 * h, i = l0 + h + (e % per) / h, j = l0 + e % h;
+      double v = 0.0;
+      for (int k = l0 + h; k <= i; ++k) v -= W[i * kIBp + k] * T[k * kIBp + j];
+      W[i * kIBp + j] = v;
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+    const int c = e / kIB, r = e % kIB;
+    if (c < r && r < w) S[static_cast<int64_t>(r0 + c) * n + r0 + r] = W[r * kIBp + c];
+  }
+  for (int K = 0; K < b; ++K) {
+    bool any = false;
+    for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+      const int r = e / kIB, c = e % kIB;
+      if (r < w) any = any || S[static_cast<int64_t>(r0 + r) * n + K * kIB + c] != 0.0;
+    }
+    const int some = __syncthreads_or(any);
+    if (tid == 0) lnz[b * nb + K] = some;
+  }
+}
+
+// tile (I, K), I >= K, of W as A[row][k]: from the upper triangle of S
+__device__ __forceinline__ void load_w(const double* S, int n, int I, int K, double* dst) {
+  for (int e = threadIdx.x; e < kIB * kIB; e += kCovThreads) {
+    const int c = e / kIB, r = e % kIB;
+    const int row = I * kIB + r, col = K * kIB + c;
+    double v = 0.0;
+    if (row < n && col < n) v = col < row ? S[static_cast<int64_t>(col) * n + row] : (col == row ? 1.0 : 0.0);
+    dst[r * kIBp + c] = v;
+  }
+}
+
+// 48x48 product of two tiles in shared memory, 3x3 entries a thread: rows
+// ty + 16 i of A, columns tx + 16 j of B
+__device__ __forceinline__ void tile_madd(const double* A, const double* B, double (*acc)[3]) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+#pragma unroll 4
+  for (int k = 0; k < kIB; ++k) {
+    double av[3], bv[3];
 #pragma unroll
-        for (int t = 0; t < 6; ++t) acc[t] += Ls[mm][t] * z;
+    for (int i = 0; i < 3; ++i) av[i] = A[(ty + 16 * i) * kIBp + k];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) bv[j] = B[k * kIBp + tx + 16 * j];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[i][j] += av[i] * bv[j];
+  }
+}
+
+// One level (left blocks of h tiles): M = 0: T = L21 W11 into Z, M = 1: W21 =
+// -W22 T.  grid: x the column tile of the left block, y the row tile of the
+// right one, z the pair.
+template <int M>
+__global__ void __launch_bounds__(kCovThreads) k_cov_wlevel(int n, int nb, int h, double* S, double* Z,
+                                                           const int* __restrict__ lnz, int* __restrict__ tnz) {
+  extern __shared__ double sh[];
+  double* A = sh;
+  double* B = A + kIB * kIBp;
+  const int left = blockIdx.z * 2 * h, I = left + h + blockIdx.y, J = left + blockIdx.x;
+  if (I >= nb) return;
+  const int tid = threadIdx.x;
+  double acc[3][3] = {};
+  bool any = false;
+  const int k0 = M == 0 ? J : left + h, k1 = M == 0 ? left + h : I + 1;
+  for (int K = k0; K < k1; ++K) {
+    if (!(M == 0 ? lnz[I * nb + K] : tnz[K * nb + J])) continue;  // uniform over the CTA
+    any = true;
+    __syncthreads();
+    if (M == 0) {
+      for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+        const int r = e / kIB, c = e % kIB, row = I * kIB + r;
+        A[r * kIBp + c] = row < n ? S[static_cast<int64_t>(row) * n + K * kIB + c] : 0.0;
+      }
+      load_w(S, n, K, J, B);
+    } else {
+      load_w(S, n, I, K, A);
+      for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+        const int r = e / kIB, c = e % kIB, row = K * kIB + r;
+        B[r * kIBp + c] = row < n ? Z[static_cast<int64_t>(row) * n + J * kIB + c] : 0.0;
       }
     }
+    __syncthreads();
+    tile_madd(A, B, acc);
   }
-  if (c < n)
-    for (int t = 0; t < 6; ++t) part[(static_cast<int64_t>(blockIdx.y) * 6 + t) * ncols + (c - cb)] = acc[t];
+  const int ty = tid >> 4, tx = tid & 15;
+  if (M == 0) {
+    if (tid == 0) tnz[I * nb + J] = any;
+    if (!any) return;
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int row = I * kIB + ty + 16 * i, col = J * kIB + tx + 16 * j;
+      if (row >= n) continue;
+      if (M == 0) Z[static_cast<int64_t>(row) * n + col] = acc[i][j];
+      else S[static_cast<int64_t>(col) * n + row] = any ? -acc[i][j] : 0.0;
+    }
 }
 
-__global__ void __launch_bounds__(kCovThreads) k_cov_inv_fin(int n, int i, int nk, const double* __restrict__ L,
-                                                            const double* __restrict__ ldiag, double* Z,
-                                                            const double* __restrict__ part,
-                                                            double* __restrict__ dpart) {
-  const int r0 = 6 * i, cb = r0 + 6, ncols = n - cb;
-  const int c = cb + blockIdx.x * blockDim.x + threadIdx.x;
-  double prod[36];
-#pragma unroll
-  for (int k = 0; k < 36; ++k) prod[k] = 0.0;
-  if (c < n) {
-    double acc[6];
-    for (int t = 0; t < 6; ++t) {
-      double s = 0.0;
-      for (int ks = 0; ks < nk; ++ks) s += part[(static_cast<int64_t>(ks) * 6 + t) * ncols + (c - cb)];
-      acc[t] = s;
+// Z_IJ = sum_{K >= I} W_KI^T D_K^-1 W_KJ, tiles I >= J, both triangles written.
+// Tiles in order of I: the longest sums first.
+__global__ void __launch_bounds__(kCovThreads) k_cov_wtw(int n, int nb, const double* __restrict__ S,
+                                                        const double* __restrict__ dinv, double* __restrict__ Z) {
+  extern __shared__ double sh[];
+  double* A = sh;
+  double* B = A + kIB * kIBp;
+  const int q = blockIdx.x;
+  int I = static_cast<int>((sqrtf(8.0f * static_cast<float>(q) + 1.0f) - 1.0f) * 0.5f);
+  while (I * (I + 1) / 2 > q) --I;
+  while ((I + 1) * (I + 2) / 2 <= q) ++I;
+  const int J = q - I * (I + 1) / 2, tid = threadIdx.x;
+  double acc[3][3] = {};
+  for (int K = I; K < nb; ++K) {
+    __syncthreads();
+    for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+      const int r = e / kIB, c = e % kIB;
+      const int m = K * kIB + c, ri = I * kIB + r, rj = J * kIB + r;  // W_m,ri and W_m,rj
+      double vi = 0.0, vj = 0.0;
+      if (m < n) {
+        const double di = dinv[m];
+        if (ri < n) vi = m > ri ? S[static_cast<int64_t>(ri) * n + m] : (m == ri ? 1.0 : 0.0);
+        if (rj < n) vj = m > rj ? S[static_cast<int64_t>(rj) * n + m] * di : (m == rj ? di : 0.0);
+      }
+      A[r * kIBp + c] = vi;
+      B[c * kIBp + r] = vj;
     }
-    const double* Lb = ldiag + 36 * static_cast<int64_t>(i);
-    double z[6];
-    for (int t = 5; t >= 0; --t) {
-      double v = -acc[t];
-      for (int m = t + 1; m < 6; ++m) v -= Lb[6 * m + t] * z[m];
-      z[t] = v;
-    }
-    for (int t = 0; t < 6; ++t) {
-      Z[static_cast<int64_t>(r0 + t) * n + c] = z[t];
-      Z[static_cast<int64_t>(c) * n + r0 + t] = z[t];
-    }
-    // the diagonal block's sums over m >= cb: L_m,r0+t Z_m,r0+u with Z_m,r0+u = z_u of column m = c
-    const double* lc = L + static_cast<int64_t>(c) * n + r0;
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      const double l = lc[t];
-#pragma unroll
-      for (int u = 0; u < 6; ++u) prod[6 * t + u] = l * z[u];
-    }
+    __syncthreads();
+    tile_madd(A, B, acc);
   }
-  // CTA sums in a fixed order: a shuffle tree per warp, then the warps in order
-  __shared__ double ws[kCovThreads / 32][36];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ty = tid >> 4, tx = tid & 15;
 #pragma unroll
-  for (int k = 0; k < 36; ++k) {
-    double v = prod[k];
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) ws[warp][k] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 36) {
-    double s = 0.0;
-    for (int w = 0; w < kCovThreads / 32; ++w) s += ws[w][threadIdx.x];
-    dpart[36 * static_cast<int64_t>(blockIdx.x) + threadIdx.x] = s;
-  }
-}
-
-// The 6x6 diagonal block: the finish CTAs' sums in order, then the recurrence
-// (columns last to first within each row, rows last to first) in one thread.
-__global__ void __launch_bounds__(64) k_cov_inv_diag(int n, int i, int nfin, const double* __restrict__ ldiag,
-                                                    const double* __restrict__ dpiv, const double* __restrict__ dpart,
-                                                    double* Z) {
-  const int r0 = 6 * i;
-  __shared__ double acc[36];
-  if (threadIdx.x < 36) {
-    double s = 0.0;
-    for (int b = 0; b < nfin; ++b) s += dpart[36 * static_cast<int64_t>(b) + threadIdx.x];
-    acc[threadIdx.x] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  const double* Lb = ldiag + 36 * static_cast<int64_t>(i);
-  double Zd[36];
-  for (int t = 5; t >= 0; --t)
-    for (int u = 5; u >= t; --u) {
-      const double dv = dpiv[r0 + t];
-      double v = (u == t && dv != 0.0) ? 1.0 / dv : 0.0;
-      v -= acc[6 * t + u];
-      for (int m = t + 1; m < 6; ++m) v -= Lb[6 * m + t] * (m <= u ? Zd[6 * m + u] : Zd[6 * u + m]);
-      Zd[6 * t + u] = v;
-    }
-  for (int t = 0; t < 6; ++t)
-    for (int u = t; u < 6; ++u) {
-      Z[static_cast<int64_t>(r0 + t) * n + r0 + u] = Zd[6 * t + u];
-      Z[static_cast<int64_t>(r0 + u) * n + r0 + t] = Zd[6 * t + u];
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int row = I * kIB + ty + 16 * i, col = J * kIB + tx + 16 * j;
+      if (row >= n || col > row) continue;
+      Z[static_cast<int64_t>(row) * n + col] = acc[i][j];
+      Z[static_cast<int64_t>(col) * n + row] = acc[i][j];
     }
 }
 
@@ -847,26 +1136,38 @@ __device__ __forceinline__ int64_t cov_zoff(const CovQArgs& a, int kind, int blk
   return kind == 0 ? 0 : a.nci + 6 * static_cast<int64_t>(blk);
 }
 
-// sum over the free blocks f of point pt (its terms with a free pose, then the
-// camera when its params are free) of Z[row, f] Y_f[:, col]
-__device__ double cov_row_times_y(const CovQArgs& a, int64_t row, int pt, int mb, int col) {
-  double v = 0.0;
+// t[c] = sum over the free blocks f of point pt (its terms with a free pose,
+// shared out over the eight lanes of a group, then the camera when its params
+// are free) of Z[row, f] Y_f[:, c]; every lane of the group gets the sums.
+__device__ __forceinline__ void cov_row_times_y(const CovQArgs& a, int64_t row, int pt, int mb, int sub, double* t) {
+  t[0] = t[1] = t[2] = 0.0;
   const double* zr = a.Z + row * a.n;
-  for (int64_t g = a.pt_g_begin[pt]; g < a.pt_g_begin[pt + 1]; ++g) {
+  for (int64_t g = a.pt_g_begin[pt] + sub; g < a.pt_g_begin[pt + 1]; g += 8) {
     const int gb = a.pose_fb[a.g_pose[g]];
     if (gb < 0) continue;
     const double* Y = a.y + 18 * g;
     const double* z = zr + a.nci + 6 * static_cast<int64_t>(gb);
-    for (int k = 0; k < 6; ++k) v += z[k] * Y[3 * k + col];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) t[c] += z[k] * Y[3 * k + c];
   }
-  if (a.nci > 0) {
+  if (a.nci > 0 && sub == 0) {
     const double* Y = a.yc + 18 * static_cast<int64_t>(mb);
-    for (int k = 0; k < a.nk; ++k) v += zr[k] * Y[3 * k + col];
+    for (int k = 0; k < a.nk; ++k)
+      for (int c = 0; c < 3; ++c) t[c] += zr[k] * Y[3 * k + c];
   }
-  return v;
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    for (int off = 4; off > 0; off >>= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], off);
 }
 
-__global__ void __launch_bounds__(64) k_cov_query(CovQArgs a) {
+// One CTA per query.  Blocks of points multiply rows of Z by the points' Y, a
+// group of eight lanes per row: the rows are read together and the chain per
+// lane is an eighth of a row (an entry per thread walked all of them: 0.82 ms
+// for 128 points of 25 terms).
+constexpr int kCovQT = 128;
+__global__ void __launch_bounds__(kCovQT) k_cov_query(CovQArgs a) {
   const int qi = blockIdx.x;
   const int32_t* q = a.q + 4 * qi;
   int rd = 0, cd = 0;
@@ -874,6 +1175,7 @@ __global__ void __launch_bounds__(64) k_cov_query(CovQArgs a) {
   const int e = threadIdx.x;
   double* o = a.out + 36 * static_cast<int64_t>(qi);
   if (e < 36) o[e] = 0.0;
+  __syncthreads();  // entries are written below by other threads
   if (rb < 0 || cb < 0) {
     if (e == 0) a.dims[2 * qi] = a.dims[2 * qi + 1] = 0;  // no block (the reference's None)
     return;
@@ -888,9 +1190,57 @@ __global__ void __launch_bounds__(64) k_cov_query(CovQArgs a) {
     a.dims[2 * qi] = bad ? -1 : rd;
     a.dims[2 * qi + 1] = bad ? -1 : cd;
   }
-  if (bad || e >= rd * cd) return;
-  const int r = e / cd, c = e % cd;
+  if (bad) return;
   const int rp = q[1], cp = q[3];  // the variables' own indices
+  const int grp = e >> 3, sub = e & 7;
+  if (a.mode == 0 && rf != cf) {
+    // -(S^-1[free rows, :] H_fm) H_mm^-1 = -sum over the point's free blocks of Z[rows, block] Y
+    const int fk = rf ? rk : ck, fbk = rf ? rb : cb, pt = rf ? cp : rp, mb = rf ? cb : rb, fd = rf ? rd : cd;
+    const int pr = grp < fd ? grp : fd - 1;
+    double t[3];
+    cov_row_times_y(a, cov_zoff(a, fk, fbk) + pr, pt, mb, sub, t);
+    if (grp < fd && sub < 3) {
+      const double v = sub == 0 ? t[0] : (sub == 1 ? t[1] : t[2]);
+      o[rf ? 3 * pr + sub : fd * sub + pr] = -v;
+    }
+    return;
+  }
+  if (a.mode == 0 && !rf && !cf) {
+    // H_mm[i]^-1 delta_ij + sum over the free blocks g of point i and h of point j of Y_g^T Z[g, h] Y_h
+    double v0 = 0.0, v8 = 0.0;  // entry sub, and entry 8 (lane 0 of the group)
+    auto add = [&](const double* Yrow, const double* t) {
+      v0 += Yrow[sub / 3] * (sub % 3 == 0 ? t[0] : (sub % 3 == 1 ? t[1] : t[2]));
+      if (sub == 0) v8 += Yrow[2] * t[2];
+    };
+    const int64_t g0 = a.pt_g_begin[rp], nrow = 6 * (a.pt_g_begin[rp + 1] - g0);
+    for (int64_t rr = grp; rr - grp < nrow; rr += kCovQT / 8) {  // uniform over the CTA: the sums use whole warps
+      const int64_t g = g0 + (rr < nrow ? rr : 0) / 6;
+      const int k = static_cast<int>((rr < nrow ? rr : 0) % 6);
+      const int gb = a.pose_fb[a.g_pose[g]];
+      double t[3];
+      cov_row_times_y(a, gb < 0 ? 0 : a.nci + 6 * static_cast<int64_t>(gb) + k, cp, cb, sub, t);
+      if (rr < nrow && gb >= 0) add(a.y + 18 * g + 3 * k, t);
+    }
+    if (a.nci > 0) {
+      const int k = grp < a.nk ? grp : 0;
+      double t[3];
+      cov_row_times_y(a, k, cp, cb, sub, t);
+      if (grp < a.nk) add(a.yc + 18 * static_cast<int64_t>(rb) + 3 * k, t);
+    }
+    __shared__ double part[kCovQT / 8][9];
+    part[grp][sub] = v0;
+    if (sub == 0) part[grp][8] = v8;
+    __syncthreads();
+    if (e < 9) {
+      double v = 0.0;
+      for (int w = 0; w < kCovQT / 8; ++w) v += part[w][e];
+      if (rp == cp) v += a.vinv[9 * static_cast<int64_t>(rb) + e];
+      o[e] = v;
+    }
+    return;
+  }
+  if (e >= rd * cd) return;
+  const int r = e / cd, c = e % cd;
   double v = 0.0;
   if (a.mode == 1) {
     // precision: blocks of the undamped H
@@ -918,27 +1268,8 @@ __global__ void __launch_bounds__(64) k_cov_query(CovQArgs a) {
       for (int64_t g = a.pt_g_begin[rp]; g < a.pt_g_begin[rp + 1]; ++g)
         v += a.rec[kCovRec * g + 39 + (r <= c ? up_idx(3, r, c) : up_idx(3, c, r))];
     }
-  } else if (rf && cf) {
-    v = a.Z[(cov_zoff(a, rk, rb) + r) * n + cov_zoff(a, ck, cb) + c];
-  } else if (rf != cf) {
-    // -(S^-1[free rows, :] H_fm) H_mm^-1 = -sum over the point's free blocks of Z[rows, block] Y
-    const int fk = rf ? rk : ck, fbk = rf ? rb : cb, pt = rf ? cp : rp, mb = rf ? cb : rb;
-    const int pr = rf ? r : c, pc = rf ? c : r;
-    v = -cov_row_times_y(a, cov_zoff(a, fk, fbk) + pr, pt, mb, pc);
   } else {
-    // H_mm[i]^-1 delta_ij + sum over the free blocks g of point i and h of point j of Y_g^T Z[g, h] Y_h
-    for (int64_t g = a.pt_g_begin[rp]; g < a.pt_g_begin[rp + 1]; ++g) {
-      const int gb = a.pose_fb[a.g_pose[g]];
-      if (gb < 0) continue;
-      const double* Yg = a.y + 18 * g;
-      for (int k = 0; k < 6; ++k)
-        v += Yg[3 * k + r] * cov_row_times_y(a, a.nci + 6 * static_cast<int64_t>(gb) + k, cp, cb, c);
-    }
-    if (a.nci > 0) {
-      const double* Yc = a.yc + 18 * static_cast<int64_t>(rb);
-      for (int k = 0; k < a.nk; ++k) v += Yc[3 * k + r] * cov_row_times_y(a, k, cp, cb, c);
-    }
-    if (rp == cp) v += a.vinv[9 * static_cast<int64_t>(rb) + 3 * r + c];
+    v = a.Z[(cov_zoff(a, rk, rb) + r) * n + cov_zoff(a, ck, cb) + c];
   }
   o[e] = v;
 }
@@ -961,10 +1292,14 @@ int launch_cov_assemble(const Sizes& s, const Dev& d, const CovBufs& c, cudaStre
     ++nl;
   }
   if (s.np > 0) {
-    k_cov_points<<<blocks_for(s.np, kCovThreads), kCovThreads, 0, st>>>(s.np, d.pt_g_begin, d.g_pose, d.pose_fb,
-                                                                       d.pt_mb, c.rec, c.vinv, c.y, c.status, c.crec,
-                                                                       c.wc, c.yc);
+    k_cov_points<<<blocks_for(s.np, kCovPtT), kCovPtT, 0, st>>>(s.np, d.pt_g_begin, d.pt_mb, c.rec, c.vinv, c.status,
+                                                               c.crec, c.wc, c.yc);
     ++nl;
+    if (s.ng > 0) {
+      k_cov_y<<<blocks_for(6 * s.ng, kCovThreads), kCovThreads, 0, st>>>(s.ng, d.g_pose, d.g_pt, d.pose_fb, d.pt_mb,
+                                                                        c.rec, c.vinv, c.y);
+      ++nl;
+    }
   }
   if (c.crec) {
     k_cov_cam<<<1, kCovThreads, 0, st>>>(s.ng, s.nm, c.nk, c.n, c.crec, c.wc, c.yc, c.S, c.hcc);
@@ -980,7 +1315,7 @@ int launch_cov_assemble(const Sizes& s, const Dev& d, const CovBufs& c, cudaStre
     a.tile_begin = d.tile_begin;
     a.tile_end = d.tile_end;
     a.cam_g = d.cam_g;
-    a.g_pt = d.g_pt;
+    a.cam_pt = c.cam_pt;
     a.pt_mb = d.pt_mb;
     a.rec = c.rec;
     a.y = c.y;
@@ -998,59 +1333,58 @@ int launch_cov_assemble(const Sizes& s, const Dev& d, const CovBufs& c, cudaStre
     a.crec = c.crec;
     a.wc = c.wc;
     a.hcp = c.hcp;
-    k_cov_s<<<blocks_for(32 * s.nsb, 128), 128, 0, st>>>(a);
+    if (c.ncam_g > 0) {
+      k_cov_cam_pt<<<blocks_for(c.ncam_g, kCovThreads), kCovThreads, 0, st>>>(c.ncam_g, d.cam_g, d.g_pt, c.cam_pt);
+      ++nl;
+    }
+    k_cov_s<<<static_cast<unsigned>(s.nsb), kCovSThreads, 0, st>>>(a);
     ++nl;
   }
   return nl;
 }
 
 int launch_cov_factor(int n, double* S, double* ldiag, double* dpiv, int* status, cudaStream_t st) {
-  const int nb = n / 6;
   int nl = 0;
-  for (int k = 0; k < nb; ++k) {
-    const int below = n - 6 * k - 6;
-    k_cov_panel<<<below > 0 ? blocks_for(below, kCovThreads) : 1, kCovThreads, 0, st>>>(n, k, S, ldiag, dpiv,
-                                                                                        status);
+  for (int c0 = 0; c0 < n; c0 += kFP) {
+    const int w = std::min(kFP, n - c0), below = n - c0 - w;
+    k_cov_diag<<<1, kCovThreads, 0, st>>>(n, c0, w, S, ldiag, dpiv, status);
     ++nl;
     if (below > 0) {
+      k_cov_rows<<<blocks_for(below, kRowsT), kRowsT, 0, st>>>(n, c0, S, ldiag, dpiv);
       const unsigned t = blocks_for(below, kUT);
-      k_cov_update<<<dim3(t, t), kCovThreads, 0, st>>>(n, k, S, dpiv);
-      ++nl;
-    }
-  }
-  return nl;
-}
-
-size_t cov_inverse_work(int n) {
-  return static_cast<size_t>(kInvSplitMax) * 6 * n + static_cast<size_t>((n + kCovThreads - 1) / kCovThreads) * 36 + 64;
-}
-
-int launch_cov_inverse(int n, const double* L, const double* ldiag, const double* dpiv, double* Z, double* work,
-                       cudaStream_t st) {
-  const int nb = n / 6;
-  int nl = 0;
-  int num_sms = 152;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-  double* part = work;
-  double* dpart = work + static_cast<size_t>(kInvSplitMax) * 6 * n;
-  for (int i = nb - 1; i >= 0; --i) {
-    const int cols = n - 6 * i - 6;
-    int nfin = 0;
-    if (cols > 0) {
-      nfin = static_cast<int>(blocks_for(cols, kCovThreads));
-      // split the rows m so that about two CTAs per SM run, each range at least kInvMinRows rows
-      int nk = (2 * num_sms + nfin - 1) / nfin;
-      nk = std::max(1, std::min({nk, kInvSplitMax, cols / kInvMinRows}));
-      const int kchunk = (cols + nk - 1) / nk;
-      k_cov_inv_part<<<dim3(nfin, nk), kCovThreads, 0, st>>>(n, i, kchunk, L, Z, part);
-      k_cov_inv_fin<<<nfin, kCovThreads, 0, st>>>(n, i, nk, L, ldiag, Z, part, dpart);
+      k_cov_update<<<dim3(t, t), kCovThreads, 0, st>>>(n, c0, S, dpiv);
       nl += 2;
     }
-    k_cov_inv_diag<<<1, 64, 0, st>>>(n, i, nfin, ldiag, dpiv, dpart, Z);
-    ++nl;
   }
   return nl;
+}
+
+// 1/d, then the nonzero-tile tables of L and of L21 W11
+size_t cov_inverse_work(int n) {
+  const size_t nb = static_cast<size_t>((n + kIB - 1) / kIB);
+  return static_cast<size_t>(n) + nb * nb + 2;
+}
+
+cudaError_t launch_cov_inverse(int n, double* L, const double* ldiag, const double* dpiv, double* Z, double* work,
+                               cudaStream_t st, int* launches) {
+  const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(k_cov_winv), kInvSmem);
+  if (e != cudaSuccess) return e;
+  const int nb = (n + kIB - 1) / kIB;
+  double* dinv = work;
+  int* lnz = reinterpret_cast<int*>(work + n);
+  int* tnz = lnz + static_cast<size_t>(nb) * nb;
+  constexpr size_t two = sizeof(double) * 2 * kIB * kIBp;
+  k_cov_winv<<<nb, kCovThreads, kInvSmem, st>>>(n, L, ldiag, dpiv, dinv, lnz, nb);
+  int nl = 1;
+  for (int h = 1; h < nb; h *= 2) {
+    const dim3 grid(h, h, (nb + h - 1) / (2 * h));  // pairs whose right block exists
+    k_cov_wlevel<0><<<grid, kCovThreads, two, st>>>(n, nb, h, L, Z, lnz, tnz);
+    k_cov_wlevel<1><<<grid, kCovThreads, two, st>>>(n, nb, h, L, Z, lnz, tnz);
+    nl += 2;
+  }
+  k_cov_wtw<<<nb * (nb + 1) / 2, kCovThreads, two, st>>>(n, nb, L, dinv, Z);
+  if (launches) *launches += nl + 1;
+  return cudaGetLastError();
 }
 
 namespace {
@@ -1112,12 +1446,12 @@ cudaError_t cov_pinv(int n, const double* L, const double* ldiag, const double* 
       if (!(hpiv[k] > 0.0)) *g_ok = 0;  // G is positive definite on the positive-pivot subspace
   }
   if (e == cudaSuccess && *g_ok) {
-    launch_cov_inverse(rp, G, gdiag, gpiv, Gi, gwork, st);
+    e = launch_cov_inverse(rp, G, gdiag, gpiv, Gi, gwork, st, nullptr);
     k_cov_recip<<<blocks_for(r, 256), 256, 0, st>>>(r, dJ, dpiv, w);
     gemm(r, r, r, Gi, rp, 1, w, Gi, rp, 1, M, r, st);   // M = G^-1 diag(d_J)^-1 G^-1
     gemm(n, r, r, E, r, 1, nullptr, M, r, 1, F, r, st);  // F = E M
     gemm(n, n, r, F, r, 1, nullptr, E, 1, r, Z, n, st);  // Z = F E^T
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
   }
   const cudaError_t ef = cudaFreeAsync(buf, st);
   return e != cudaSuccess ? e : ef;
@@ -1154,7 +1488,7 @@ cudaError_t launch_cov_query(const Sizes& s, const Dev& d, const CovBufs& c, int
   a.e_hmn = d.edge_hmn;
   a.out = out;
   a.dims = dims;
-  k_cov_query<<<nq, 64, 0, st>>>(a);
+  k_cov_query<<<nq, kCovQT, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -583,6 +583,8 @@ constexpr int kCovRec = 48;
 // per term with free camera params: J_cam^T J_cam (21 upper), J_cam^T J_pose (6 x 6), J_cam^T J_point (6 x 3)
 constexpr int kCovCamRec = 80;
 struct CovBufs {
+  int64_t ncam_g = 0;         // entries of the cameras' term lists
+  int32_t* cam_pt = nullptr;  // ncam_g: their points
   int ready = 0;
   int n = 0;      // rows of S: the camera block (nci rows) and 6 per free pose
   int nci = 0;    // free camera params: 6 rows (their nk params, then identity padding), else 0
@@ -613,10 +615,11 @@ struct CovBufs {
 int launch_cov_assemble(const Sizes& s, const Dev& d, const CovBufs& c, cudaStream_t st);
 // LDL^T of the n x n S in place (the reference's per-block pivot rule).
 int launch_cov_factor(int n, double* S, double* ldiag, double* dpiv, int* status, cudaStream_t st);
-// Z = S^-1 from the factor (full rank); work: cov_inverse_work(n) doubles.
+// Z = S^-1 from the factor (full rank), which the upper triangle beside L is
+// overwritten for; work: cov_inverse_work(n) doubles; *launches += kernels.
 size_t cov_inverse_work(int n);
-int launch_cov_inverse(int n, const double* L, const double* ldiag, const double* dpiv, double* Z, double* work,
-                       cudaStream_t st);
+cudaError_t launch_cov_inverse(int n, double* L, const double* ldiag, const double* dpiv, double* Z, double* work,
+                               cudaStream_t st, int* launches);
 // Z = S+ = E G^-1 diag(d_J)^-1 G^-1 E^T (rank-deficient S; J the positive
 // pivots, host list); temporaries from `pool` on st.  *g_ok = 0 when G has a
 // pivot <= 0 (synchronises st).

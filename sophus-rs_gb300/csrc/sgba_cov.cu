@@ -400,7 +400,9 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_cam_pt(int64_t n, const int
 // slice of pose fa's term list (1/32 of it, in point order): for a piece of
 // every slice the CTA first finds the terms of pose fb on the same points (a
 // binary search per term, all of them at once), then the lanes add theirs in
-// order.  (A warp per block that merged the two lists step by step, 36 sums a
+// order (matches packed to the front of each slice: the FP64 pipe takes a step's
+// time for one lane as for 32, and that pipe bounds this kernel, 77 % busy).  (A
+// warp per block that merged the two lists step by step, 36 sums a
 // lane, spent its time on the chain of list loads: 1.5 ms for 741 blocks of
 // 1,250 x 1,250 terms.)
 constexpr int kCovSThreads = 192;
@@ -411,6 +413,7 @@ __global__ void __launch_bounds__(kCovSThreads) k_cov_s(CovSArgs a) {
   // W of the matches, [entry][match]: the lanes' own reads of 18 entries from 32
   // records would take 32 cache wavefronts each, for every row's warp
   __shared__ double s_w[18][kCovStage * 32];
+  __shared__ int s_most;
   const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int64_t s = blockIdx.x;
   const int fa = a.sb_row[s], fb = a.sb_col[s];
@@ -455,6 +458,7 @@ __global__ void __launch_bounds__(kCovSThreads) k_cov_s(CovSArgs a) {
     const int64_t longest = (len + 31) / 32;
     for (int64_t p0 = 0; p0 < longest; p0 += kCovPiece) {
       __syncthreads();
+#pragma unroll 2
       for (int e = threadIdx.x; e < 32 * kCovPiece; e += kCovSThreads) {
         const int l = e & 31, u = e >> 5;
         const int64_t i = ib + len * l / 32 + p0 + u;
@@ -478,15 +482,30 @@ __global__ void __launch_bounds__(kCovSThreads) k_cov_s(CovSArgs a) {
         s_gj[u][l] = gj;
       }
       __syncthreads();
-      const int un = static_cast<int>(min(static_cast<int64_t>(kCovPiece), longest - p0));
+      if (r == 0) {  // every lane's matches to the front of its slice, in order
+        int m = 0;
+        for (int u = 0; u < kCovPiece; ++u) {
+          const int gi = s_gi[u][lane], gj = s_gj[u][lane];
+          if (gj < 0) continue;
+          s_gi[m][lane] = gi;
+          s_gj[m][lane] = gj;
+          ++m;
+        }
+        for (int u = m; u < kCovPiece; ++u) s_gj[u][lane] = -1;
+        const int most = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) s_most = most;
+      }
+      __syncthreads();
+      const int un = s_most;
       for (int u0 = 0; u0 < un; u0 += kCovStage) {
+#pragma unroll 8
         for (int e = threadIdx.x; e < 18 * kCovStage * 32; e += kCovSThreads) {
           const int m = e / 18, k = e - 18 * m;
           const int gj = s_gj[u0 + (m >> 5)][m & 31];
           if (gj >= 0) s_w[k][m] = a.rec[kCovRec * static_cast<int64_t>(gj) + 21 + k];
         }
         __syncthreads();
-        for (int u = 0; u < kCovStage; ++u) {
+        for (int u = 0; u < kCovStage && u0 + u < un; ++u) {
           if (s_gj[u0 + u][lane] < 0) continue;
           const double* Y = a.y + 18 * static_cast<int64_t>(s_gi[u0 + u][lane]) + 3 * r;
           const double y0 = Y[0], y1 = Y[1], y2 = Y[2];
@@ -593,6 +612,12 @@ __device__ int ldlt6(double* a, double* d) {
 // order, each as one difference with a sum over its six columns, so L and the
 // pivots keep the bits of the step-by-step factor (two launches per step, 20 us
 // for a step's 6 x 6 block in one thread).
+//
+// What shapes these kernels (measured on GB300): an SM sub-partition takes 64
+// cycles for an FP64 instruction of a warp, however many of its lanes are
+// active, and does not overlap two of them; a division is nine such, 566
+// cycles.  So independent FP64 work goes to different lanes first (an entry a
+// thread, the divisions of a row to six threads) and then to four warps.
 constexpr int kFP = 48;
 
 // ldlt6 by lanes 0 .. 5 of a warp, a row each (columns updated as soon as their
@@ -609,31 +634,37 @@ __device__ __forceinline__ int ldlt6_warp(const double* a, int ld, double* L6, d
     v[c] = c <= j ? a[j * ld + c] : 0.0;
     l[c] = 0.0;
   }
-  double maxp = 1.0, minp = DBL_MAX;
+  // magnitudes are compared by their bits (the same order): an FP64 comparison
+  // takes the FP64 pipe's 70 cycles, and the pivots are a serial chain
+  const long long kAbs = 0x7fffffffffffffffll, kInf = 0x7ff0000000000000ll;
+  long long maxb = __double_as_longlong(1.0), minb = kInf;
   int rank = 0, st = 0;
   bool neg = false;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
+    const double tol = __longlong_as_double(maxb) * kCovTolRel;
     const double dk = __shfl_sync(all, v[k], k);
-    if (!isfinite(dk) && st == 0) st = 1;
-    const bool zero = fabs(dk) <= fmax(maxp, 1.0) * kCovTolRel;
+    const long long bits = __double_as_longlong(dk), ab = bits & kAbs;
+    if (ab >= kInf && st == 0) st = 1;
+    const double q = v[k] / dk;
+    const bool zero = ab <= __double_as_longlong(tol);
     d[k] = zero ? 0.0 : dk;
-    if (!zero) {
-      if (dk < 0.0) neg = true;
-      maxp = fmax(maxp, fabs(dk));
-      minp = fmin(minp, fabs(dk));
-      rank += 1;
-    }
-    l[k] = zero ? 0.0 : v[k] / dk;
+    neg = neg || (!zero && bits < 0);
+    maxb = zero ? maxb : max(maxb, ab);
+    minb = zero ? minb : min(minb, ab);
+    rank += zero ? 0 : 1;
+    l[k] = zero ? 0.0 : q;
     const double ld_k = l[k] * d[k];
 #pragma unroll
     for (int c = k + 1; c < 6; ++c) {
       const double lc = __shfl_sync(all, l[k], c);
-      if (c <= j) v[c] -= ld_k * lc;
+      const double nv = v[c] - ld_k * lc;
+      v[c] = c <= j ? nv : v[c];
     }
   }
+  const double maxp = __longlong_as_double(maxb), minp = __longlong_as_double(minb);
   // minp <= tol of the largest pivot: a row may see an earlier pivot as zero
-  if (st == 0 && rank > 0 && minp <= fmax(maxp, 1.0) * kCovTolRel) {
+  if (st == 0 && rank > 0 && minp <= maxp * kCovTolRel) {
     if (lane == 0) {
       double b[36];
       for (int r = 0; r < 6; ++r)
@@ -658,8 +689,9 @@ __device__ __forceinline__ int ldlt6_warp(const double* a, int ld, double* L6, d
   return (neg && cond < 1e-10) ? 2 : 0;
 }
 
-// L of a row's six columns from its entries x (L6, d6 of the step): in place
-__device__ __forceinline__ void row_solve6(double* x, const double* L6, const double* d6) {
+// y of a row's six columns from its entries x (L6 of the step): in place; L is
+// y / d, formed by other threads (div6)
+__device__ __forceinline__ void row_y6(double* x, const double* L6) {
   double yv[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
@@ -669,14 +701,18 @@ __device__ __forceinline__ void row_solve6(double* x, const double* L6, const do
     yv[j] = v;
   }
 #pragma unroll
-  for (int j = 0; j < 6; ++j) x[j] = d6[j] == 0.0 ? 0.0 : yv[j] / d6[j];
+  for (int j = 1; j < 6; ++j) x[j] = yv[j];
+}
+__device__ __forceinline__ double div6(double y, double d) {
+  const double q = y / d;
+  return d == 0.0 ? 0.0 : q;
 }
 
 // The diagonal block of the panel at c0 (w columns): its 6-column steps in
 // shared memory; L below the 6x6 blocks back to S.
 __global__ void __launch_bounds__(kCovThreads) k_cov_diag(int n, int c0, int w, double* S, double* ldiag, double* dpiv,
                                                          int* status) {
-  __shared__ double A[kFP][kFP + 1], L6[36], d6[6];
+  __shared__ double A[kFP][kFP + 1], Ld[kFP][7], L6[36], d6[6];
   const int tid = threadIdx.x;
   for (int e = tid; e < kFP * kFP; e += kCovThreads) {
     const int r = e / kFP, c = e % kFP;
@@ -692,7 +728,14 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_diag(int n, int c0, int w, 
     }
     __syncthreads();
     const int rows = w - k0 - 6;
-    if (tid < rows) row_solve6(&A[k0 + 6 + tid][k0], L6, d6);
+    if (tid < rows) row_y6(&A[k0 + 6 + tid][k0], L6);
+    __syncthreads();
+    if (tid < 6 * rows) {
+      const int r = tid / 6, t = tid - 6 * r;
+      const double l = div6(A[k0 + 6 + r][k0 + t], d6[t]);
+      A[k0 + 6 + r][k0 + t] = l;
+      Ld[r][t] = l * d6[t];
+    }
     __syncthreads();
     for (int e = tid; e < rows * (rows + 1) / 2; e += kCovThreads) {
       int i = static_cast<int>((sqrtf(8.0f * static_cast<float>(e) + 1.0f) - 1.0f) * 0.5f);
@@ -700,10 +743,9 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_diag(int n, int c0, int w, 
       while ((i + 1) * (i + 2) / 2 <= e) ++i;
       const double* li = &A[k0 + 6 + i][k0];
       const int j = e - i * (i + 1) / 2;
-      const double* lj = &A[k0 + 6 + j][k0];
       double s = 0.0;
 #pragma unroll
-      for (int t = 0; t < 6; ++t) s += li[t] * (lj[t] * d6[t]);
+      for (int t = 0; t < 6; ++t) s += li[t] * Ld[j][t];
       A[k0 + 6 + i][k0 + 6 + j] -= s;
     }
     __syncthreads();
@@ -714,49 +756,62 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_diag(int n, int c0, int w, 
   }
 }
 
-// The rows below the panel, a thread per row: per step its six entries of L,
-// then the row's entries in the panel's later columns.
-constexpr int kRowsT = 32;
+// The rows below the panel, 32 to a CTA: per step warp 0 forms y of every row
+// (a thread each), the four warps share out the divisions, then the rows'
+// entries in the panel's later columns.
+constexpr int kRowsT = 128;
 __global__ void __launch_bounds__(kRowsT) k_cov_rows(int n, int c0, double* S, const double* __restrict__ ldiag,
                                                     const double* __restrict__ dpiv) {
-  __shared__ double Ld[kFP][kFP], L6[kFP / 6][36], d[kFP], X[kRowsT][kFP + 1];
-  const int tid = threadIdx.x, r0 = c0 + kFP + blockIdx.x * kRowsT;
-  for (int e = tid; e < kFP * kFP; e += kRowsT) {  // L_jt d_t of the panel's own rows
-    const int r = e / kFP, c = e % kFP;
-    Ld[r][c] = c / 6 < r / 6 ? S[static_cast<int64_t>(c0 + r) * n + c0 + c] * dpiv[c0 + c] : 0.0;
-  }
-  for (int e = tid; e < kFP * 6; e += kRowsT) L6[e / 36][e % 36] = ldiag[6 * static_cast<int64_t>(c0) + e];
-  for (int e = tid; e < kFP; e += kRowsT) d[e] = dpiv[c0 + e];
+  extern __shared__ double sh[];
+  double* Ld = sh;                      // kFP x kFP: L_jt d_t of the panel's own rows
+  double* L6 = Ld + kFP * kFP;          // kFP / 6 x 36
+  double* d = L6 + 6 * kFP;             // kFP
+  double* X = d + kFP;                  // 32 x (kFP + 1)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r0 = c0 + kFP + blockIdx.x * 32;
   bool any = false;
-  for (int e = tid; e < kRowsT * kFP; e += kRowsT) {
+#pragma unroll 12
+  for (int e = tid; e < 32 * kFP; e += kRowsT) {
     const int r = e / kFP, c = e % kFP;
     const double v = r0 + r < n ? S[static_cast<int64_t>(r0 + r) * n + c0 + c] : 0.0;
-    X[r][c] = v;
+    X[r * (kFP + 1) + c] = v;
     any = any || v != 0.0;
   }
   if (!__syncthreads_or(any)) return;  // rows outside the band: L is zero there
-  double* x = X[tid];
+#pragma unroll 6
+  for (int e = tid; e < kFP * kFP; e += kRowsT) {
+    const int r = e / kFP, c = e % kFP;
+    Ld[e] = c / 6 < r / 6 ? S[static_cast<int64_t>(c0 + r) * n + c0 + c] * dpiv[c0 + c] : 0.0;
+  }
+  for (int e = tid; e < kFP * 6; e += kRowsT) L6[e] = ldiag[6 * static_cast<int64_t>(c0) + e];
+  if (tid < kFP) d[tid] = dpiv[c0 + tid];
+  __syncthreads();
+  double* x = X + lane * (kFP + 1);
   for (int k0 = 0; k0 < kFP; k0 += 6) {
-    row_solve6(x + k0, L6[k0 / 6], d + k0);
+    if (warp == 0) row_y6(x + k0, L6 + 6 * k0);
+    __syncthreads();
+    for (int t = warp; t < 6; t += 4) x[k0 + t] = div6(x[k0 + t], d[k0 + t]);
+    __syncthreads();
     double l[6];
 #pragma unroll
     for (int t = 0; t < 6; ++t) l[t] = x[k0 + t];
-    for (int j = k0 + 6; j < kFP; j += 6) {  // six columns at a time: independent chains
+    for (int j = k0 + 6 + 6 * warp; j < kFP; j += 24) {
       double s[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
       for (int t = 0; t < 6; ++t)
 #pragma unroll
-        for (int u = 0; u < 6; ++u) s[u] += l[t] * Ld[j + u][k0 + t];
+        for (int u = 0; u < 6; ++u) s[u] += l[t] * Ld[(j + u) * kFP + k0 + t];
 #pragma unroll
       for (int u = 0; u < 6; ++u) x[j + u] -= s[u];
     }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int e = tid; e < kRowsT * kFP; e += kRowsT) {
+#pragma unroll 12
+  for (int e = tid; e < 32 * kFP; e += kRowsT) {
     const int r = e / kFP, c = e % kFP;
-    if (r0 + r < n) S[static_cast<int64_t>(r0 + r) * n + c0 + c] = X[r][c];
+    if (r0 + r < n) S[static_cast<int64_t>(r0 + r) * n + c0 + c] = X[r * (kFP + 1) + c];
   }
 }
+constexpr size_t kRowsSmem = sizeof(double) * (kFP * kFP + 6 * kFP + kFP + 32 * (kFP + 1));
 
 // C_ij -= sum_t L_it (d_t L_jt), step by step of the panel, on the lower
 // trailing triangle in 32 x 32 tiles (tiles above the diagonal, and tiles whose
@@ -889,28 +944,31 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_winv(int n, double* S, cons
   }
 }
 
-// tile (I, K), I >= K, of W as A[row][k]: from the upper triangle of S
-__device__ __forceinline__ void load_w(const double* S, int n, int I, int K, double* dst) {
-  for (int e = threadIdx.x; e < kIB * kIB; e += kCovThreads) {
+// columns k0 .. k0 + nc - 1 of tile (I, K), I >= K, of W as dst[row][k - k0]:
+// from the upper triangle of S
+__device__ __forceinline__ void load_w(const double* S, int n, int I, int K, int k0, int nc, double* dst) {
+#pragma unroll 6
+  for (int e = threadIdx.x; e < kIB * nc; e += blockDim.x) {
     const int c = e / kIB, r = e % kIB;
-    const int row = I * kIB + r, col = K * kIB + c;
+    const int row = I * kIB + r, col = K * kIB + k0 + c;
     double v = 0.0;
     if (row < n && col < n) v = col < row ? S[static_cast<int64_t>(col) * n + row] : (col == row ? 1.0 : 0.0);
     dst[r * kIBp + c] = v;
   }
 }
 
-// 48x48 product of two tiles in shared memory, 3x3 entries a thread: rows
-// ty + 16 i of A, columns tx + 16 j of B
+// Product of two tiles in shared memory, 3x3 entries a thread: rows ty + 16 i
+// of A, columns tx + TX j of B (48 x 3 TX)
+template <int TX>
 __device__ __forceinline__ void tile_madd(const double* A, const double* B, double (*acc)[3]) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int ty = threadIdx.x / TX, tx = threadIdx.x % TX;
 #pragma unroll 4
   for (int k = 0; k < kIB; ++k) {
     double av[3], bv[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) av[i] = A[(ty + 16 * i) * kIBp + k];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) bv[j] = B[k * kIBp + tx + 16 * j];
+    for (int j = 0; j < 3; ++j) bv[j] = B[k * kIBp + tx + TX * j];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -919,50 +977,63 @@ __device__ __forceinline__ void tile_madd(const double* A, const double* B, doub
 }
 
 // One level (left blocks of h tiles): M = 0: T = L21 W11 into Z, M = 1: W21 =
-// -W22 T.  grid: x the column tile of the left block, y the row tile of the
-// right one, z the pair.
+// -W22 T.  grid: x half a column tile of the left block, y the row tile of the
+// right one, z the pair.  A tile product keeps an SM's FP64 pipe for 28 us, so
+// a CTA takes 24 of the 48 columns (the dense rows of a loop closure are few
+// long sums).
+constexpr int kLvT = 128, kLvC = 24;
 template <int M>
-__global__ void __launch_bounds__(kCovThreads) k_cov_wlevel(int n, int nb, int h, double* S, double* Z,
-                                                           const int* __restrict__ lnz, int* __restrict__ tnz) {
+__global__ void __launch_bounds__(kLvT) k_cov_wlevel(int n, int nb, int h, double* S, double* Z,
+                                                    const int* __restrict__ lnz, int* __restrict__ tnz) {
   extern __shared__ double sh[];
+  __shared__ int s_nz[kLvT];
   double* A = sh;
   double* B = A + kIB * kIBp;
-  const int left = blockIdx.z * 2 * h, I = left + h + blockIdx.y, J = left + blockIdx.x;
+  const int left = blockIdx.z * 2 * h, I = left + h + blockIdx.y, J = left + (blockIdx.x >> 1);
+  const int cc = (blockIdx.x & 1) * kLvC;
   if (I >= nb) return;
   const int tid = threadIdx.x;
   double acc[3][3] = {};
   bool any = false;
   const int k0 = M == 0 ? J : left + h, k1 = M == 0 ? left + h : I + 1;
   for (int K = k0; K < k1; ++K) {
-    if (!(M == 0 ? lnz[I * nb + K] : tnz[K * nb + J])) continue;  // uniform over the CTA
+    const int kk = (K - k0) % kLvT;
+    if (kk == 0) {  // the next flags, all at once
+      __syncthreads();
+      if (K + tid < k1) s_nz[tid] = M == 0 ? lnz[I * nb + K + tid] : tnz[(K + tid) * nb + J];
+      __syncthreads();
+    }
+    if (!s_nz[kk]) continue;  // uniform over the CTA
     any = true;
     __syncthreads();
     if (M == 0) {
-      for (int e = tid; e < kIB * kIB; e += kCovThreads) {
+#pragma unroll 6
+      for (int e = tid; e < kIB * kIB; e += kLvT) {
         const int r = e / kIB, c = e % kIB, row = I * kIB + r;
         A[r * kIBp + c] = row < n ? S[static_cast<int64_t>(row) * n + K * kIB + c] : 0.0;
       }
-      load_w(S, n, K, J, B);
+      load_w(S, n, K, J, cc, kLvC, B);
     } else {
-      load_w(S, n, I, K, A);
-      for (int e = tid; e < kIB * kIB; e += kCovThreads) {
-        const int r = e / kIB, c = e % kIB, row = K * kIB + r;
-        B[r * kIBp + c] = row < n ? Z[static_cast<int64_t>(row) * n + J * kIB + c] : 0.0;
+      load_w(S, n, I, K, 0, kIB, A);
+#pragma unroll 3
+      for (int e = tid; e < kIB * kLvC; e += kLvT) {
+        const int r = e / kLvC, c = e % kLvC, row = K * kIB + r;
+        B[r * kIBp + c] = row < n ? Z[static_cast<int64_t>(row) * n + J * kIB + cc + c] : 0.0;
       }
     }
     __syncthreads();
-    tile_madd(A, B, acc);
+    tile_madd<8>(A, B, acc);
   }
-  const int ty = tid >> 4, tx = tid & 15;
+  const int ty = tid >> 3, tx = tid & 7;
   if (M == 0) {
-    if (tid == 0) tnz[I * nb + J] = any;
+    if (tid == 0) tnz[I * nb + J] = any;  // the same from both halves
     if (!any) return;
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const int row = I * kIB + ty + 16 * i, col = J * kIB + tx + 16 * j;
+      const int row = I * kIB + ty + 16 * i, col = J * kIB + cc + tx + 8 * j;
       if (row >= n) continue;
       if (M == 0) Z[static_cast<int64_t>(row) * n + col] = acc[i][j];
       else S[static_cast<int64_t>(col) * n + row] = any ? -acc[i][j] : 0.0;
@@ -997,7 +1068,7 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_wtw(int n, int nb, const do
       B[c * kIBp + r] = vj;
     }
     __syncthreads();
-    tile_madd(A, B, acc);
+    tile_madd<16>(A, B, acc);
   }
   const int ty = tid >> 4, tx = tid & 15;
 #pragma unroll
@@ -1350,7 +1421,7 @@ int launch_cov_factor(int n, double* S, double* ldiag, double* dpiv, int* status
     k_cov_diag<<<1, kCovThreads, 0, st>>>(n, c0, w, S, ldiag, dpiv, status);
     ++nl;
     if (below > 0) {
-      k_cov_rows<<<blocks_for(below, kRowsT), kRowsT, 0, st>>>(n, c0, S, ldiag, dpiv);
+      k_cov_rows<<<blocks_for(below, 32), kRowsT, kRowsSmem, st>>>(n, c0, S, ldiag, dpiv);
       const unsigned t = blocks_for(below, kUT);
       k_cov_update<<<dim3(t, t), kCovThreads, 0, st>>>(n, c0, S, dpiv);
       nl += 2;
@@ -1377,9 +1448,9 @@ cudaError_t launch_cov_inverse(int n, double* L, const double* ldiag, const doub
   k_cov_winv<<<nb, kCovThreads, kInvSmem, st>>>(n, L, ldiag, dpiv, dinv, lnz, nb);
   int nl = 1;
   for (int h = 1; h < nb; h *= 2) {
-    const dim3 grid(h, h, (nb + h - 1) / (2 * h));  // pairs whose right block exists
-    k_cov_wlevel<0><<<grid, kCovThreads, two, st>>>(n, nb, h, L, Z, lnz, tnz);
-    k_cov_wlevel<1><<<grid, kCovThreads, two, st>>>(n, nb, h, L, Z, lnz, tnz);
+    const dim3 grid(2 * h, h, (nb + h - 1) / (2 * h));  // pairs whose right block exists
+    k_cov_wlevel<0><<<grid, kLvT, two, st>>>(n, nb, h, L, Z, lnz, tnz);
+    k_cov_wlevel<1><<<grid, kLvT, two, st>>>(n, nb, h, L, Z, lnz, tnz);
     nl += 2;
   }
   k_cov_wtw<<<nb * (nb + 1) / 2, kCovThreads, two, st>>>(n, nb, L, dinv, Z);

@@ -40,7 +40,6 @@ using sgba::Plan;
 using sgba::Record;
 using sgba::Sizes;
 using sgba::kIntrMax;
-using sgba::kIntrPart;
 using sgba::kIntrScj;
 using sgba::kIntrSum;
 using sgba::kIntrZk;
@@ -955,9 +954,14 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   if ((st = dev_alloc(p, &d.dm, 3 * static_cast<size_t>(P.nm)))) return st;
   if ((st = dev_alloc(p, &d.gauge_um, 3 * static_cast<size_t>(P.nm)))) return st;
   if (p->intr_free) {
-    if ((st = dev_alloc(p, &d.intr_part, kIntrPart * static_cast<size_t>(std::max(P.np, 1))))) return st;
+    const size_t ng = static_cast<size_t>(std::max<int64_t>(P.ng, 1));
+    if ((st = dev_alloc(p, &d.intr_ty, 18 * ng))) return st;
+    if ((st = dev_alloc(p, &d.intr_tjp, 36 * ng))) return st;
+    if ((st = dev_alloc(p, &d.intr_part, sgba::intr_part_count(s)))) return st;
+    if ((st = dev_alloc(p, &d.intr_ticket, 1))) return st;
+    SGBA_CK(cudaMemsetAsync(d.intr_ticket, 0, sizeof(int), p->stream));
     if ((st = dev_alloc(p, &d.intr_zk, kIntrZk * static_cast<size_t>(std::max(P.nm, 1))))) return st;
-    if ((st = dev_alloc(p, &d.intr_scj, kIntrScj * static_cast<size_t>(std::max(P.nf, 1))))) return st;
+    if ((st = dev_alloc(p, &d.intr_scj, 4 * kIntrScj * static_cast<size_t>(std::max<int64_t>(s.ntiles, 1))))) return st;
     if ((st = dev_alloc(p, &d.intr_sum, kIntrSum))) return st;
     SGBA_CK(cudaMemsetAsync(d.intr_sum, 0, sizeof(double) * kIntrSum, p->stream));
   }

@@ -272,9 +272,12 @@ struct Dev {
   double* dm = nullptr;            // nm*3 point steps
   double* gauge_um = nullptr;      // nm*3 the free poses' gauge direction back-substituted into the points
   // free intrinsics (Sizes::intr_free)
-  double* intr_part = nullptr;     // np*kIntrPart per-point parts of S_kk, J_k^T r~, Zk c
+  float2* intr_ty = nullptr;       // ng*18: J_k^T J_m of each term, split
+  float2* intr_tjp = nullptr;      // ng*36: J_k^T J_p of each term, split
+  float2* intr_part = nullptr;     // intr_part_count: partial sums of S_kk, J_k^T r~, Zk c
+  int* intr_ticket = nullptr;
   float* intr_zk = nullptr;        // nm*kIntrZk Zk = Y C^-T (6x3) as (hi, lo) pairs
-  double* intr_scj = nullptr;      // nf*kIntrScj S_kj (6x6)
+  double* intr_scj = nullptr;      // 4*ntiles*kIntrScj: parts of S_kj (6x6) per quarter camera tile
   double* intr_sum = nullptr;      // kIntrSum: kIntrPart sums + 6 neg_grad of the intrinsics
   double* part = nullptr;          // reduction partials
   int part_cap = 0;
@@ -424,6 +427,7 @@ int launch_decide(const Sizes& s, const Dev& d, cudaStream_t st);
 int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st);
 int cost_partials_needed(const Sizes& s);  // reduction partial slots
 int landmark_setup(int cap);
+size_t intr_part_count(const Sizes& s);  // partial sums of the free intrinsics (float2)
 int schur_dense_setup();  // shared memory limits of the tiled Schur pass (0: ok)  // dynamic shared memory of the chunked landmark pass (0 = ok)
 int landmark_dd_setup(int cap);  // the same for its float-float variant (0 = ok)
 int backsub_chunks_setup(int cap);  // the chunked back-substitution (0 = ok)

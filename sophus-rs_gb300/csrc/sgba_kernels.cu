@@ -2376,10 +2376,15 @@ struct IntrArgs {
   const int64_t* tile_begin;
   const int64_t* tile_end;
   const int64_t* fb_tile_begin;
-  double* ipart;  // np x kIntrPart
-  float* zk;      // nm x kIntrZk: Zk (6x3) as (hi, lo)
-  double* scj;    // nf x kIntrScj: S_kj (6x6)
-  double* isum;   // kIntrPart sums, then -sum J_k^T r~ (6)
+  // per term Y_g = J_k^T J_m (6x3) and J_k^T J_p (6x6), split (k_intr_terms)
+  float2* ty;
+  float2* tjp;
+  float2* ipart;   // partial sums: J_k^T J_k, J_k^T r~ per warp of terms, then - Zk Zk^T, Zk c per CTA of points
+  int* ticket;     // CTAs of k_intr_points done
+  int nterm_part;  // warps of terms
+  float* zk;       // nm x kIntrZk: Zk (6x3) as (hi, lo)
+  double* scj;     // per quarter tile kIntrScj: its part of S_kj (6x6)
+  double* isum;    // kIntrPart sums, then -sum J_k^T r~ (6)
   double* S;
   float2* S2;
   double* rb;
@@ -2421,168 +2426,262 @@ __device__ void intr_term_jacobians(const float* Pd, dd px, dd py, dd pz, const 
   else jacobians_dd<false>(Pd, px, py, pz, c, J);
 }
 
-// One thread per point: its terms' J_k^T J_k, J_k^T r~, Y = J_k^T J_m, then
-// with the point's C^-1 (landmark pass) Zk = Y C^-T and its parts of S_kk and
-// rhs_k.
-__global__ void __launch_bounds__(128) k_intr_points(IntrArgs a, const Ctrl* ctrl) {
-  if (halted(ctrl)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.np) return;
-  const CamD cam = cam_dd(a.cam);
-  const dd px = pt_dd(a.pts, i, 0), py = pt_dd(a.pts, i, 1), pz = pt_dd(a.pts, i, 2);
-  dd hkk[kKT], gk[kK], Y[3 * kK];
-  for (int k = 0; k < kKT; ++k) hkk[k] = dd_make(0.f, 0.f);
-  for (int k = 0; k < kK; ++k) gk[k] = dd_make(0.f, 0.f);
-  for (int k = 0; k < 3 * kK; ++k) Y[k] = dd_make(0.f, 0.f);
-  for (int64_t g = a.pt_g_begin[i]; g < a.pt_g_begin[i + 1]; ++g) {
-    JacD J;
-    dd jk[2 * kK];
-    intr_term_jacobians(a.pose_dd + 24 * a.g_pose[g], px, py, pz, cam, a.nk, &J, jk);
-    for (int64_t o = a.g_begin[g]; o < a.g_begin[g + 1]; ++o) {
-      const float2 r = a.res[o];
-      dd r0, r1;
-      huber_weighted_dd(a.huber, a.huber_dd, dd_from_float(r.x), dd_from_float(r.y), &r0, &r1);
-      int k = 0;
-      for (int p = 0; p < kK; ++p) {
-        for (int q = p; q < kK; ++q) {
-          hkk[k] = dd_add(hkk[k], dd_add(dd_mul(jk[p], jk[q]), dd_mul(jk[kK + p], jk[kK + q])));
-          ++k;
-        }
-        gk[p] = dd_add(gk[p], dd_add(dd_mul(jk[p], r0), dd_mul(jk[kK + p], r1)));
-        for (int s2 = 0; s2 < 3; ++s2)
-          Y[p * 3 + s2] = dd_add(Y[p * 3 + s2], dd_add(dd_mul(jk[p], J.jm[s2]), dd_mul(jk[kK + p], J.jm[3 + s2])));
-      }
-    }
-  }
-  double* out = a.ipart + static_cast<int64_t>(i) * kIntrPart;
-  const int mb = a.pt_mb[i];
-  dd zz[kKT], zc[kK];
-  for (int k = 0; k < kKT; ++k) zz[k] = dd_make(0.f, 0.f);
-  for (int k = 0; k < kK; ++k) zc[k] = dd_make(0.f, 0.f);
-  if (mb >= 0 && a.pt_g_begin[i + 1] > a.pt_g_begin[i]) {
-    const float* cp = a.cinv + 12 * mb;
-    dd I[6];
-    for (int k = 0; k < 6; ++k) I[k] = dd_make(cp[2 * k], cp[2 * k + 1]);
-    const float* cv = a.cvec + 6 * mb;
-    const dd c[3] = {dd_make(cv[0], cv[1]), dd_make(cv[2], cv[3]), dd_make(cv[4], cv[5])};
-    dd Zk[3 * kK];
-    for (int r = 0; r < kK; ++r) {
-      Zk[r * 3 + 0] = dd_mul(I[0], Y[r * 3 + 0]);
-      Zk[r * 3 + 1] = dd_add(dd_mul(I[1], Y[r * 3 + 0]), dd_mul(I[2], Y[r * 3 + 1]));
-      Zk[r * 3 + 2] = dd_add(dd_add(dd_mul(I[3], Y[r * 3 + 0]), dd_mul(I[4], Y[r * 3 + 1])), dd_mul(I[5], Y[r * 3 + 2]));
-    }
-    int k = 0;
-    for (int p = 0; p < kK; ++p) {
-      for (int q = p; q < kK; ++q) {
-        dd t = dd_make(0.f, 0.f);
-        for (int s2 = 0; s2 < 3; ++s2) t = dd_add(t, dd_mul(Zk[p * 3 + s2], Zk[q * 3 + s2]));
-        zz[k++] = t;
-      }
-      dd t = dd_make(0.f, 0.f);
-      for (int s2 = 0; s2 < 3; ++s2) t = dd_add(t, dd_mul(Zk[p * 3 + s2], c[s2]));
-      zc[p] = t;
-    }
-    float* zo = a.zk + kIntrZk * static_cast<int64_t>(mb);
-    for (int k2 = 0; k2 < 3 * kK; ++k2) {
-      zo[2 * k2] = Zk[k2].hi;
-      zo[2 * k2 + 1] = Zk[k2].lo;
-    }
-  }
-  for (int k = 0; k < kKT; ++k) out[k] = dd_to_double(dd_sub(hkk[k], zz[k]));
-  for (int k = 0; k < kK; ++k) out[kIntrG + k] = dd_to_double(gk[k]);
-  for (int k = 0; k < kK; ++k) out[kIntrZc + k] = dd_to_double(zc[k]);
+// These problems are small (the dense solvers), so the kernels below are bound
+// by the chains of one thread.  The terms' Jacobians are formed once, a thread
+// per term, and their products by 32 lanes a point and 64 threads a quarter
+// tile.  (A thread per point over its terms, one CTA for the sums and one per
+// pose, each forming the Jacobians again, took 78 + 62 + 57 us an iteration of
+// the 10-camera, 5,000-term problem.)
+
+// Lanes' values v[0 .. NV - 1] summed over a warp in float-float: lane k gets
+// the sum of value k (hi parts in lane order, then lo parts).
+template <int NV>
+__device__ __forceinline__ dd intr_warp_sum(const dd* v, float (*red)[33]) {
+  const int lane = threadIdx.x & 31;
+  Acc t = acc_zero();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) red[k][lane] = v[k].hi;
+  __syncwarp();
+  if (lane < NV)
+    for (int l = 0; l < 32; ++l) acc_addf(t, red[lane][l]);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) red[k][lane] = v[k].lo;
+  __syncwarp();
+  if (lane < NV)
+    for (int l = 0; l < 32; ++l) acc_addf(t, red[lane][l]);
+  __syncwarp();
+  return acc_get(t);
 }
 
-// One CTA: the per-point parts summed in a fixed order; the intrinsics'
-// neg_grad -sum J_k^T r~ joins the gradient-tolerance maximum.
-__global__ void __launch_bounds__(256) k_intr_reduce(IntrArgs a, Ctrl* ctrl) {
+// A thread per term: Y_g and J_k^T J_p stored, J_k^T J_k and J_k^T r~ summed per warp.
+constexpr int kIntrTermT = 64;
+constexpr int kIntrOwn = kKT + kK;  // 27 sums
+__global__ void __launch_bounds__(kIntrTermT) k_intr_terms(IntrArgs a, const Ctrl* ctrl) {
   if (halted(ctrl)) return;
-  __shared__ float sh_hi[256], sh_lo[256];
-  for (int k = 0; k < kIntrPart; ++k) {
-    dd acc = dd_make(0.f, 0.f);
-    for (int i = threadIdx.x; i < a.np; i += blockDim.x)
-      acc = dd_add(acc, dd_from_double(a.ipart[static_cast<int64_t>(i) * kIntrPart + k]));
-    sh_hi[threadIdx.x] = acc.hi;
-    sh_lo[threadIdx.x] = acc.lo;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-      if (threadIdx.x < h) {
-        const dd t = dd_add(dd_make(sh_hi[threadIdx.x], sh_lo[threadIdx.x]),
-                            dd_make(sh_hi[threadIdx.x + h], sh_lo[threadIdx.x + h]));
-        sh_hi[threadIdx.x] = t.hi;
-        sh_lo[threadIdx.x] = t.lo;
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) a.isum[k] = dd_to_double(dd_make(sh_hi[0], sh_lo[0]));
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double mg = 0.0;
-    for (int k = 0; k < kK; ++k) {
-      const double bk = -a.isum[kIntrG + k];
-      a.isum[kIntrPart + k] = bk;
-      mg = fmax(mg, fabs(bk));
-    }
-    atomic_max_nonneg(&ctrl->max_grad_bits, mg);
-  }
-}
-
-// One CTA per free pose: S_kj = sum over its terms of J_k^T J_p - Zk_i Z_g^T.
-// Thread t < nk * 6 of the final sum owns entry t (row t / 6 of S_kj).
-__global__ void __launch_bounds__(128) k_intr_cams(IntrArgs a, const Ctrl* ctrl) {
-  if (halted(ctrl)) return;
-  const int fb = blockIdx.x;
-  constexpr int kE = kK * 6;
-  __shared__ float sh_hi[kE][129], sh_lo[kE][129];
-  dd acc[kE];
-  for (int k = 0; k < kE; ++k) acc[k] = dd_make(0.f, 0.f);
-  const CamD cam = cam_dd(a.cam);
-  const int64_t t0 = a.fb_tile_begin[fb], t1 = a.fb_tile_begin[fb + 1];
-  const int64_t e0 = (t1 > t0) ? a.tile_begin[t0] : 0, e1 = (t1 > t0) ? a.tile_end[t1 - 1] : 0;
-  for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const int64_t g = a.cam_g[e];
+  __shared__ float red[kIntrTermT / 32][kIntrOwn][33];
+  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const dd zero = dd_make(0.f, 0.f);
+  dd own[kIntrOwn];
+#pragma unroll
+  for (int k = 0; k < kIntrOwn; ++k) own[k] = zero;
+  if (g < a.ng) {
+    const CamD cam = cam_dd(a.cam);
     const int i = a.g_pt[g];
-    const dd px = pt_dd(a.pts, i, 0), py = pt_dd(a.pts, i, 1), pz = pt_dd(a.pts, i, 2);
     JacD J;
     dd jk[2 * kK];
-    intr_term_jacobians(a.pose_dd + 24 * a.g_pose[g], px, py, pz, cam, a.nk, &J, jk);
-    for (int64_t o = a.g_begin[g]; o < a.g_begin[g + 1]; ++o)
-      for (int p = 0; p < kK; ++p)
-        for (int q = 0; q < 6; ++q)
-          acc[p * 6 + q] = dd_add(acc[p * 6 + q], dd_add(dd_mul(jk[p], J.jp[q]), dd_mul(jk[kK + p], J.jp[6 + q])));
+    intr_term_jacobians(a.pose_dd + 24 * static_cast<int64_t>(a.g_pose[g]), pt_dd(a.pts, i, 0), pt_dd(a.pts, i, 1),
+                        pt_dd(a.pts, i, 2), cam, a.nk, &J, jk);
+    const int64_t o0 = a.g_begin[g], o1 = a.g_begin[g + 1];
+    // the term's observations share J: their products are n times one product
+    const float cnt = static_cast<float>(o1 - o0);
+    dd r0 = zero, r1 = zero;
+    for (int64_t o = o0; o < o1; ++o) {
+      const float2 r = a.res[o];
+      dd w0, w1;
+      huber_weighted_dd(a.huber, a.huber_dd, dd_from_float(r.x), dd_from_float(r.y), &w0, &w1);
+      r0 = dd_add(r0, w0);
+      r1 = dd_add(r1, w1);
+    }
+    float2* ty = a.ty + 18 * g;
+    float2* tj = a.tjp + 36 * g;
+    int k = 0;
+#pragma unroll
+    for (int p = 0; p < kK; ++p) {
+      const dd u = dd_mul_f(jk[p], cnt), v = dd_mul_f(jk[kK + p], cnt);
+#pragma unroll
+      for (int q = p; q < kK; ++q) own[k++] = dd_add(dd_mul(u, jk[q]), dd_mul(v, jk[kK + q]));
+      own[kKT + p] = dd_add(dd_mul(jk[p], r0), dd_mul(jk[kK + p], r1));
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const dd t = dd_add(dd_mul(u, J.jm[q]), dd_mul(v, J.jm[3 + q]));
+        ty[3 * p + q] = make_float2(t.hi, t.lo);
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const dd t = dd_add(dd_mul(u, J.jp[q]), dd_mul(v, J.jp[6 + q]));
+        tj[6 * p + q] = make_float2(t.hi, t.lo);
+      }
+    }
+  }
+  const dd t = intr_warp_sum<kIntrOwn>(own, red[wib]);
+  if (lane < kIntrOwn)
+    a.ipart[kIntrOwn * (static_cast<int64_t>(blockIdx.x) * (kIntrTermT / 32) + wib) + lane] = make_float2(t.hi, t.lo);
+}
+
+// A warp per point: Y over its terms, with the point's C^-1 (landmark pass)
+// Zk = Y C^-T and its parts of S_kk (subtracted) and of rhs_k; the last CTA to
+// finish sums every partial in order and forms the intrinsics' neg_grad
+// -sum J_k^T r~, which joins the gradient-tolerance maximum.
+constexpr int kIntrPtWarps = 8;
+__global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, Ctrl* ctrl) {
+  if (halted(ctrl)) return;
+  __shared__ float2 sy[kIntrPtWarps][3 * kK], sz[kIntrPtWarps][3 * kK], sp[kIntrPtWarps][kIntrOwn];
+  __shared__ double s_tot[2][kIntrOwn];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const dd zero = dd_make(0.f, 0.f);
+  // this lane's value: entry (p, q) of Zk Zk^T (lanes 0 .. 20), then Zk c
+  int p = 0, q = lane;
+  if (lane < kKT) {
+    while (q >= kK - p) {
+      q -= kK - p;
+      ++p;
+    }
+    q += p;
+  } else {
+    p = lane - kKT;
+  }
+  dd acc = zero;
+  for (int i = blockIdx.x * kIntrPtWarps + wib; i < a.np; i += gridDim.x * kIntrPtWarps) {
     const int mb = a.pt_mb[i];
+    const int64_t g0 = a.pt_g_begin[i], g1 = a.pt_g_begin[i + 1];
+    if (mb < 0 || g1 == g0) continue;  // the whole warp
+    if (lane < 3 * kK) {
+      dd y = zero;
+      for (int64_t g = g0; g < g1; ++g) {
+        const float2 v = a.ty[18 * g + lane];
+        y = dd_add(y, dd_make(v.x, v.y));
+      }
+      sy[wib][lane] = make_float2(y.hi, y.lo);
+    }
+    __syncwarp();
+    if (lane < 3 * kK) {
+      const int r = lane / 3, c = lane % 3;
+      const float2* ci = reinterpret_cast<const float2*>(a.cinv + 12 * static_cast<int64_t>(mb)) + (c == 0 ? 0 : (c == 1 ? 1 : 3));
+      dd z = zero;
+      for (int t = 0; t <= c; ++t) {
+        const float2 w = ci[t], y = sy[wib][3 * r + t];
+        z = dd_add(z, dd_mul(dd_make(w.x, w.y), dd_make(y.x, y.y)));
+      }
+      sz[wib][lane] = make_float2(z.hi, z.lo);
+      reinterpret_cast<float2*>(a.zk + kIntrZk * static_cast<int64_t>(mb))[lane] = make_float2(z.hi, z.lo);
+    }
+    __syncwarp();
+    if (lane < kIntrOwn) {
+      const float2* o = lane < kKT ? sz[wib] + 3 * q : reinterpret_cast<const float2*>(a.cvec + 6 * static_cast<int64_t>(mb));
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const float2 z = sz[wib][3 * p + t], w = o[t];
+        acc = dd_add(acc, dd_mul(dd_make(z.x, z.y), dd_make(w.x, w.y)));
+      }
+    }
+    __syncwarp();
+  }
+  if (lane < kIntrOwn) sp[wib][lane] = make_float2(acc.hi, acc.lo);
+  __syncthreads();
+  float2* pts = a.ipart + static_cast<int64_t>(kIntrOwn) * a.nterm_part;
+  if (threadIdx.x < kIntrOwn) {
+    dd t = zero;
+    for (int w = 0; w < kIntrPtWarps; ++w) t = dd_add(t, dd_make(sp[w][threadIdx.x].x, sp[w][threadIdx.x].y));
+    pts[static_cast<int64_t>(kIntrOwn) * blockIdx.x + threadIdx.x] = make_float2(t.hi, t.lo);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(a.ticket, 1) == static_cast<int>(gridDim.x) - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // the partials: those of the terms, then those of the points; eight warps take
+  // ranges of them, a lane per value, and the ranges are added in order
+  for (int part = 0; part < 2; ++part) {
+    const float2* src = part == 0 ? a.ipart : pts;
+    const int n = part == 0 ? a.nterm_part : static_cast<int>(gridDim.x);
+    dd t = zero;
+    if (lane < kIntrOwn)
+      for (int k = n * wib / kIntrPtWarps; k < n * (wib + 1) / kIntrPtWarps; ++k) {
+        const float2 v = __ldcg(src + static_cast<int64_t>(kIntrOwn) * k + lane);
+        t = dd_add(t, dd_make(v.x, v.y));
+      }
+    __syncthreads();
+    if (lane < kIntrOwn) sp[wib][lane] = make_float2(t.hi, t.lo);
+    __syncthreads();
+    if (threadIdx.x < kIntrOwn) {
+      dd u = zero;
+      for (int w = 0; w < kIntrPtWarps; ++w) u = dd_add(u, dd_make(sp[w][threadIdx.x].x, sp[w][threadIdx.x].y));
+      s_tot[part][threadIdx.x] = dd_to_double(u);
+    }
+  }
+  __syncthreads();
+  const int k = threadIdx.x;
+  if (k < kKT) a.isum[k] = s_tot[0][k] - s_tot[1][k];
+  if (k < kK) {
+    const double gk = s_tot[0][kKT + k];
+    a.isum[kIntrG + k] = gk;
+    a.isum[kIntrZc + k] = s_tot[1][kKT + k];
+    a.isum[kIntrPart + k] = -gk;
+  }
+  if (k == 0) {
+    double mg = 0.0;
+    for (int t = 0; t < kK; ++t) mg = fmax(mg, fabs(s_tot[0][kKT + t]));
+    atomic_max_nonneg(&ctrl->max_grad_bits, mg);
+    *a.ticket = 0;
+  }
+}
+
+// S_kj = sum over pose j's terms of J_k^T J_p - Zk_i Z_g^T: a CTA per quarter of
+// a camera tile, a thread per term; k_intr_fill adds a pose's parts.
+constexpr int kIntrCamT = 64;
+__global__ void __launch_bounds__(kIntrCamT) k_intr_cams(IntrArgs a, const Ctrl* ctrl) {
+  if (halted(ctrl)) return;
+  constexpr int kE = kK * 6;
+  __shared__ float sh_hi[kE][kIntrCamT + 1], sh_lo[kE][kIntrCamT + 1];
+  __shared__ float2 half[2][kE];
+  const int tile = blockIdx.x >> 2;
+  const int64_t e = a.tile_begin[tile] + (blockIdx.x & 3) * kIntrCamT + threadIdx.x;
+  const dd zero = dd_make(0.f, 0.f);
+  const bool on = e < a.tile_end[tile];
+  int64_t g = 0;
+  int mb = -1;
+  dd Z[18], zk[18];
+  if (on) {
+    g = a.cam_g[e];
+    mb = a.pt_mb[a.g_pt[g]];
     if (mb >= 0) {
       // Z_g (6x3): float-float where the landmark pass kept it so, else FP32
-      dd Z[18];
-      const float4* z4 = reinterpret_cast<const float4*>(a.zmat + 20 * g);
-      float zf[20];
-      for (int k = 0; k < 5; ++k) {
-        const float4 w4 = z4[k];
-        zf[4 * k] = w4.x; zf[4 * k + 1] = w4.y; zf[4 * k + 2] = w4.z; zf[4 * k + 3] = w4.w;
+      const float* zf = a.zmat + 20 * g;
+      const float* zd = a.zdd ? a.zdd + kZddFloats * g
+                              : ((zf[18] != 0.f && a.zdd_flagged) ? a.zdd_flagged + kZddFloats * g : nullptr);
+      const float2* zs = reinterpret_cast<const float2*>(a.zk + kIntrZk * static_cast<int64_t>(mb));
+#pragma unroll
+      for (int k = 0; k < 18; ++k) {
+        Z[k] = zd ? dd_make(zd[2 * k], zd[2 * k + 1]) : dd_from_float(zf[k]);
+        zk[k] = dd_make(zs[k].x, zs[k].y);
       }
-      const float* zd = a.zdd ? a.zdd + kZddFloats * g : ((zf[18] != 0.f && a.zdd_flagged) ? a.zdd_flagged + kZddFloats * g : nullptr);
-      for (int k = 0; k < 18; ++k) Z[k] = zd ? dd_make(zd[2 * k], zd[2 * k + 1]) : dd_from_float(zf[k]);
-      const float* zk = a.zk + kIntrZk * static_cast<int64_t>(mb);
-      for (int p = 0; p < kK; ++p)
-        for (int q = 0; q < 6; ++q) {
-          dd t = dd_make(0.f, 0.f);
-          for (int s2 = 0; s2 < 3; ++s2)
-            t = dd_add(t, dd_mul(dd_make(zk[2 * (p * 3 + s2)], zk[2 * (p * 3 + s2) + 1]), Z[q * 3 + s2]));
-          acc[p * 6 + q] = dd_sub(acc[p * 6 + q], t);
-        }
     }
   }
-  for (int k = 0; k < kE; ++k) {
-    sh_hi[k][threadIdx.x] = acc[k].hi;
-    sh_lo[k][threadIdx.x] = acc[k].lo;
+#pragma unroll
+  for (int p = 0; p < kK; ++p)
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      dd v = zero;
+      if (on) {
+        const float2 j = a.tjp[36 * g + 6 * p + q];
+        v = dd_make(j.x, j.y);
+        if (mb >= 0) {
+          dd t = zero;
+#pragma unroll
+          for (int u = 0; u < 3; ++u) t = dd_add(t, dd_mul(zk[3 * p + u], Z[3 * q + u]));
+          v = dd_sub(v, t);
+        }
+      }
+      sh_hi[6 * p + q][threadIdx.x] = v.hi;
+      sh_lo[6 * p + q][threadIdx.x] = v.lo;
+    }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, h = threadIdx.x >> 5;
+  for (int k = lane; k < kE; k += 32) {
+    Acc t = acc_zero();
+    for (int l = 0; l < 32; ++l) acc_addf(t, sh_hi[k][32 * h + l]);
+    for (int l = 0; l < 32; ++l) acc_addf(t, sh_lo[k][32 * h + l]);
+    const dd v = acc_get(t);
+    half[h][k] = make_float2(v.hi, v.lo);
   }
   __syncthreads();
   if (threadIdx.x < kE) {
-    const int k = threadIdx.x;
-    dd t = dd_make(0.f, 0.f);
-    for (int q = 0; q < static_cast<int>(blockDim.x); ++q) t = dd_add(t, dd_make(sh_hi[k][q], sh_lo[k][q]));
-    a.scj[kIntrScj * static_cast<int64_t>(fb) + k] = dd_to_double(t);
+    const float2 u = half[0][threadIdx.x], v = half[1][threadIdx.x];
+    a.scj[kIntrScj * static_cast<int64_t>(blockIdx.x) + threadIdx.x] = dd_to_double(dd_add(dd_make(u.x, u.y), dd_make(v.x, v.y)));
   }
 }
 
@@ -2596,7 +2695,11 @@ __global__ void __launch_bounds__(64) k_intr_fill(IntrArgs a, const Ctrl* ctrl) 
   if (e >= 36) return;
   const int r = e / 6, c = e % 6;
   if (b < a.nf) {
-    const double v = (r < a.nk) ? a.scj[kIntrScj * static_cast<int64_t>(b) + r * 6 + c] : 0.0;
+    dd t = dd_make(0.f, 0.f);
+    if (r < a.nk)
+      for (int64_t k = 4 * a.fb_tile_begin[b]; k < 4 * a.fb_tile_begin[b + 1]; ++k)
+        t = dd_add(t, dd_from_double(a.scj[kIntrScj * k + e]));
+    const double v = dd_to_double(t);
     const int64_t row = k0 + r, col = 6 * b + c;
     a.S[row * a.n6 + col] = v;
     a.S[col * a.n6 + row] = v;
@@ -2624,6 +2727,12 @@ __global__ void __launch_bounds__(64) k_intr_fill(IntrArgs a, const Ctrl* ctrl) 
     if (c == 0) a.rb[k0 + r] = (r < a.nk) ? a.isum[kIntrPart + r] - a.isum[kIntrZc + r] : 0.0;
   }
 }
+
+// partial sums of the terms (a warp each, whole CTAs) and CTAs of the points
+int intr_term_parts(int64_t ng) {
+  return static_cast<int>((ng + kIntrTermT - 1) / kIntrTermT) * (kIntrTermT / 32);
+}
+int intr_point_blocks(int np) { return np > 0 ? std::min((np + kIntrPtWarps - 1) / kIntrPtWarps, 608) : 1; }
 
 IntrArgs intr_args(const Sizes& s, const Dev& d) {
   IntrArgs a;
@@ -2653,7 +2762,11 @@ IntrArgs intr_args(const Sizes& s, const Dev& d) {
   a.tile_begin = d.tile_begin;
   a.tile_end = d.tile_end;
   a.fb_tile_begin = d.fb_tile_begin;
+  a.ty = d.intr_ty;
+  a.tjp = d.intr_tjp;
   a.ipart = d.intr_part;
+  a.ticket = d.intr_ticket;
+  a.nterm_part = intr_term_parts(s.ng);
   a.zk = d.intr_zk;
   a.scj = d.intr_scj;
   a.isum = d.intr_sum;
@@ -2667,10 +2780,10 @@ IntrArgs intr_args(const Sizes& s, const Dev& d) {
 int launch_intr_linearize(const Sizes& s, const Dev& d, cudaStream_t st) {
   if (!s.intr_free) return 0;
   const IntrArgs a = intr_args(s, d);
-  k_intr_points<<<(s.np + 127) / 128 > 0 ? (s.np + 127) / 128 : 1, 128, 0, st>>>(a, d.ctrl);
-  k_intr_reduce<<<1, 256, 0, st>>>(a, d.ctrl);
-  if (s.nf > 0) k_intr_cams<<<s.nf, 128, 0, st>>>(a, d.ctrl);
-  return s.nf > 0 ? 3 : 2;
+  if (s.ng > 0) k_intr_terms<<<a.nterm_part / (kIntrTermT / 32), kIntrTermT, 0, st>>>(a, d.ctrl);
+  k_intr_points<<<intr_point_blocks(s.np), 32 * kIntrPtWarps, 0, st>>>(a, d.ctrl);
+  if (s.ntiles > 0) k_intr_cams<<<static_cast<unsigned>(4 * s.ntiles), kIntrCamT, 0, st>>>(a, d.ctrl);
+  return 1 + (s.ng > 0 ? 1 : 0) + (s.ntiles > 0 ? 1 : 0);
 }
 
 int launch_intr_fill(const Sizes& s, const Dev& d, cudaStream_t st) {
@@ -4140,6 +4253,10 @@ int batch_launch_collect(const BatchTables* t, Ctrl* ctrl_out, Record* rec_out, 
   if (t->n == 0) return 0;
   k_collect_w<<<t->n, 128, 0, st>>>(t->ctrl, t->recs, t->rec_cap, t->n, ctrl_out, rec_out, cap);
   return 1;
+}
+
+size_t intr_part_count(const Sizes& s) {
+  return static_cast<size_t>(kIntrOwn) * (static_cast<size_t>(intr_term_parts(s.ng)) + intr_point_blocks(s.np));
 }
 
 }  // namespace sgba

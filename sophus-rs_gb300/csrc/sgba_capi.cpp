@@ -1125,6 +1125,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     if ((st = dev_alloc(p, &d.wpanel, n6 * 48))) return st;
   }
   if ((st = dev_alloc(p, &d.x, n6))) return st;
+  if ((st = dev_alloc(p, &d.x0, n6))) return st;
   if ((st = dev_alloc(p, &d.xdd, 2 * n6))) return st;
   if ((st = dev_alloc(p, &d.r, n6))) return st;
   SGBA_CK(cudaMemsetAsync(d.x, 0, sizeof(double) * std::max<size_t>(n6, 1), p->stream));

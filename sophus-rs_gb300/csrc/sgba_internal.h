@@ -267,6 +267,7 @@ struct Dev {
   float* dpiv = nullptr;           // n6 pivots
   float* wpanel = nullptr;         // n6*64 panel scratch (A_ip L^-T)
   double* x = nullptr;             // n6 solution / refinement
+  double* x0 = nullptr;            // 6 nf: x before the gauge projection
   float* xdd = nullptr;            // n6*2: solution as float-float pairs
   double* r = nullptr;             // n6 residual
   double* dm = nullptr;            // nm*3 point steps

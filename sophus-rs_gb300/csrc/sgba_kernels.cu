@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "sgba_dd.cuh"
+#include "sgba_pose.cuh"
 #include "sgba_internal.h"
 
 namespace sgba {
@@ -26,7 +27,6 @@ namespace {
 
 constexpr int kCostThreads = 256;
 constexpr int kCostMaxBlocks = 1216;  // 8 x 152 SMs
-constexpr double kEps = 1e-6;         // EPS_F64 (crates/sophus_autodiff/src/linalg.rs:75)
 
 __device__ __forceinline__ bool halted(const Ctrl* c) { return c->done != 0; }
 __device__ __forceinline__ bool skipping(const Ctrl* c) { return c->done != 0 || c->skip != 0; }
@@ -35,75 +35,6 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, doub
   // Non-negative doubles order like their bit patterns.
   if (!(v >= 0.0)) v = (v != v) ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
   atomicMax(addr, static_cast<unsigned long long>(__double_as_longlong(v)));
-}
-
-// --- SE(3) in f64 (restated from sophus_lie, see the oracle for citations) --
-// Rotation3Impl::matrix (crates/sophus_lie/src/groups/rotation3.rs:449-492)
-__device__ void rot_matrix(const double* q, double* m) {
-  double r = q[0], x = q[1], y = q[2], z = q[3];
-  double tx = 2.0 * x, ty = 2.0 * y, tz = 2.0 * z, tr = 2.0 * r;
-  double txx = tx * x, tyy = ty * y, tzz = tz * z;
-  double txy = tx * y, txz = tx * z, tyz = ty * z;
-  double trx = tr * x, try_ = tr * y, trz = tr * z;
-  m[0] = 1.0 - (tyy + tzz); m[1] = txy - trz; m[2] = txz + try_;
-  m[3] = txy + trz; m[4] = 1.0 - (txx + tzz); m[5] = tyz - trx;
-  m[6] = txz - try_; m[7] = tyz + trx; m[8] = 1.0 - (txx + tyy);
-}
-
-// Left-perturbation update T <- exp(xi) * T
-// (crates/sophus_lie/src/lie_group/lie_group_manifold.rs:33-35,57-64;
-//  exp: crates/sophus_lie/src/groups/affine_group_template.rs:354-360,
-//       crates/sophus_lie/src/groups/rotation3.rs:363-387 and mat_v :761-778;
-//  group_mul: affine_group_template.rs:387-396, quaternion.rs:212-225;
-//  disambiguate: rotation3.rs:176-182).
-__device__ void se3_left_update(const double* xi, const double* T, double* out) {
-  const double w0 = xi[0], w1 = xi[1], w2 = xi[2];
-  double th2 = w0 * w0 + w1 * w1 + w2 * w2;
-  double eq[4];
-  if (th2 <= kEps * kEps) {
-    double th4 = th2 * th2;
-    double im = 0.5 - (1.0 / 48.0) * th2 + (1.0 / 3840.0) * th4;
-    eq[0] = 1.0 - (1.0 / 8.0) * th2 + (1.0 / 384.0) * th4;
-    eq[1] = im * w0; eq[2] = im * w1; eq[3] = im * w2;
-  } else {
-    double th = sqrt(th2);
-    double s, c;
-    sincos(0.5 * th, &s, &c);
-    double im = s / th;
-    eq[0] = c; eq[1] = im * w0; eq[2] = im * w1; eq[3] = im * w2;
-  }
-  // mat_v * nu
-  double h[9] = {0.0, -w2, w1, w2, 0.0, -w0, -w1, w0, 0.0};
-  double v[9];
-  if (th2 <= kEps) {
-    for (int i = 0; i < 9; ++i) v[i] = 0.5 * h[i];
-  } else {
-    double h2[9];
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j)
-        h2[i * 3 + j] = h[i * 3 + 0] * h[0 * 3 + j] + h[i * 3 + 1] * h[1 * 3 + j] + h[i * 3 + 2] * h[2 * 3 + j];
-    double th = sqrt(th2);
-    double a = (1.0 - cos(th)) / th2;
-    double b = (th - sin(th)) / (th2 * th);
-    for (int i = 0; i < 9; ++i) v[i] = a * h[i] + b * h2[i];
-  }
-  v[0] += 1.0; v[4] += 1.0; v[8] += 1.0;
-  double et[3];
-  for (int i = 0; i < 3; ++i) et[i] = v[i * 3 + 0] * xi[3] + v[i * 3 + 1] * xi[4] + v[i * 3 + 2] * xi[5];
-  if (!(0.0 <= eq[0])) { for (int i = 0; i < 4; ++i) eq[i] = -eq[i]; }
-  // exp(xi) * T
-  const double* b = T;
-  double q[4];
-  q[0] = eq[0] * b[0] - (eq[1] * b[1] + eq[2] * b[2] + eq[3] * b[3]);
-  q[1] = b[1] * eq[0] + eq[1] * b[0] + (eq[2] * b[3] - eq[3] * b[2]);
-  q[2] = b[2] * eq[0] + eq[2] * b[0] + (eq[3] * b[1] - eq[1] * b[3]);
-  q[3] = b[3] * eq[0] + eq[3] * b[0] + (eq[1] * b[2] - eq[2] * b[1]);
-  double r[9];
-  rot_matrix(eq, r);
-  for (int i = 0; i < 3; ++i)
-    out[4 + i] = (r[i * 3 + 0] * b[4] + r[i * 3 + 1] * b[5] + r[i * 3 + 2] * b[6]) + et[i];
-  if (!(0.0 <= q[0])) { for (int i = 0; i < 4; ++i) q[i] = -q[i]; }
-  for (int i = 0; i < 4; ++i) out[i] = q[i];
 }
 
 // HuberKernel (crates/sophus_opt/src/robust_kernel.rs:13-35): weight applied to
@@ -370,28 +301,8 @@ __device__ void jacobians_dd(const float* Pd /*R_cw 9 + t_cw 3, (hi, lo) pairs*/
 }
 
 // ---------------------------------------------------------------------------
-// Pose tables: T_cw = T_wc^-1 in f64, published as float and float-float.
+// Pose tables (sgba_pose.cuh).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pose_table(const double* T, float* pf, float* pd) {
-  double qc[4] = {T[0], -T[1], -T[2], -T[3]};
-  double R[9];
-  rot_matrix(qc, R);
-  double t[3];
-  for (int i = 0; i < 3; ++i) t[i] = -(R[i * 3 + 0] * T[4] + R[i * 3 + 1] * T[5] + R[i * 3 + 2] * T[6]);
-  for (int i = 0; i < 9; ++i) {
-    pf[i] = __double2float_rn(R[i]);
-    dd v = dd_from_double(R[i]);
-    pd[2 * i] = v.hi;
-    pd[2 * i + 1] = v.lo;
-  }
-  for (int i = 0; i < 3; ++i) {
-    pf[9 + i] = __double2float_rn(t[i]);
-    dd v = dd_from_double(t[i]);
-    pd[18 + 2 * i] = v.hi;
-    pd[18 + 2 * i + 1] = v.lo;
-  }
-}
-
 // What the kernels of one evaluation point read besides the f64 state: the
 // pose tables, the points and the camera params split into (hi, lo) pairs, and
 // the gauge direction of the poses (t - c, for the back-substitution).
@@ -2820,6 +2731,7 @@ struct GaugeArgs {
   const double* um;  // back-substituted gauge direction of the points
   double cx, cy, cz;
   double* part;  // 2 * gridDim
+  double* x0;    // copy of xf, which k_apply_update projects in place
 };
 
 __device__ __forceinline__ void gauge_partials_body(GaugeArgs a, const Ctrl* ctrl, int bid_, int nblk_) {
@@ -2834,6 +2746,7 @@ __device__ __forceinline__ void gauge_partials_body(GaugeArgs a, const Ctrl* ctr
       v[0] = T[4] - a.cx; v[1] = T[5] - a.cy; v[2] = T[6] - a.cz;
       u[0] = v[0]; u[1] = v[1]; u[2] = v[2];
       d[0] = a.xf[6 * t + 3]; d[1] = a.xf[6 * t + 4]; d[2] = a.xf[6 * t + 5];
+      for (int k = 0; k < 6; ++k) a.x0[6 * t + k] = a.xf[6 * t + k];
       w = a.cnt_f[t];
     } else {
       const int mb = static_cast<int>(t - a.nf);
@@ -2875,6 +2788,11 @@ __global__ void __launch_bounds__(256) k_gauge_partials(GaugeArgs a, const Ctrl*
 // Apply the (projected) step: trial poses exp(delta) * T, trial points p + d
 // (VarFamilies::update, crates/sophus_opt/src/variables/var_families.rs:203-209);
 // partial sums of delta.delta and delta.neg_grad for the gain ratio and max |delta|.
+//
+// The first sum_blocks CTAs take a thread per pose and per point: the sums, the
+// maximum, the projected step and the trial points.  Bound by the FP64 chain of
+// a trial pose, those have CTAs of their own, sixteen lanes a pose
+// (pose_update16): 24 -> 12 us (10 poses).
 // ---------------------------------------------------------------------------
 struct UpdArgs {
   int nc, np, nf, nm;
@@ -2885,6 +2803,8 @@ struct UpdArgs {
   double* poses_t;
   double* points_t;
   double* xf;   // projected in place
+  const double* x0;  // the step before the projection
+  int sum_blocks;
   double* dm;   // projected in place
   const double* bf;
   const double* bm;
@@ -2906,6 +2826,7 @@ struct UpdArgs {
   const double* bk;
 };
 
+constexpr int kUpdPoses = 16;  // trial poses of a CTA
 __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid_, int nblk_) {
   if (skipping(ctrl)) return;
   // gauge coefficient alpha = sum num / sum den over the k_gauge_partials
@@ -2930,8 +2851,24 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
     alpha = s_alpha;
     if (bid_ == 0 && threadIdx.x == 0) ctrl->alpha = alpha;
   }
+  if (bid_ >= a.sum_blocks) {
+    const int l = threadIdx.x & 15, p = (bid_ - a.sum_blocks) * kUpdPoses + (threadIdx.x >> 4);
+    const bool off = p >= a.nc;
+    const int j = off ? a.nc - 1 : p, fb = a.pose_fb[j];
+    const double Tl = l < 7 ? a.poses[7 * j + l] : 0.0;
+    const double Tt = __shfl_sync(0xffffffffu, Tl, l >= 3 ? min(l + 1, 6) : 4, 16);
+    double x = (fb >= 0 && l < 6) ? a.x0[6 * fb + l] : 0.0;
+    if (l >= 3) x -= alpha * (Tt - (l == 3 ? a.cx : (l == 4 ? a.cy : a.cz)));
+    pose_update16(x, Tl, fb < 0, off, a.poses_t + 7 * j, a.pose_f + 12 * j, a.pose_dd + 24 * j);
+    return;
+  }
   dd sdd = dd_make(0.f, 0.f), sdg = dd_make(0.f, 0.f);
-  double mx = 0.0;
+  // max |step| by bit patterns: non-negative doubles order like them (NaN left out)
+  unsigned long long mx = 0ull;
+  auto step_max = [&](double v) {
+    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+    if (u <= 0x7ff0000000000000ull && u > mx) mx = u;
+  };
   if (a.intr_free && bid_ == 0 && threadIdx.x == 0) {
     // the intrinsics are a vector space: k + dx_k (no gauge component)
     for (int k = 0; k < a.intr_nk; ++k) {
@@ -2940,37 +2877,30 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
       const dd x = dd_from_double(xk);
       sdd = dd_add(sdd, dd_mul(x, x));
       sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bk[k])));
-      mx = fmax(mx, fabs(xk));
+      step_max(xk);
     }
     cam_table(a.intr_t, a.cam);
   }
   const int64_t n = static_cast<int64_t>(a.nc) + a.np;
   for (int64_t t = bid_ * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
-       t += static_cast<int64_t>(nblk_) * blockDim.x) {
+       t += static_cast<int64_t>(a.sum_blocks) * blockDim.x) {
     if (t < a.nc) {
       const int j = static_cast<int>(t);
       const double* T = a.poses + 7 * j;
-      double* O = a.poses_t + 7 * j;
       const int fb = a.pose_fb[j];
-      if (fb < 0) {
-        for (int k = 0; k < 7; ++k) O[k] = T[k];
-        pose_table(O, a.pose_f + 12 * j, a.pose_dd + 24 * j);
-        continue;
-      }
+      if (fb < 0) continue;
       double xi[6];
-      for (int k = 0; k < 6; ++k) xi[k] = a.xf[6 * fb + k];
+      for (int k = 0; k < 6; ++k) xi[k] = a.x0[6 * fb + k];
       xi[3] -= alpha * (T[4] - a.cx);
       xi[4] -= alpha * (T[5] - a.cy);
       xi[5] -= alpha * (T[6] - a.cz);
       for (int k = 0; k < 6; ++k) {
-        a.xf[6 * fb + k] = xi[k];
+        if (a.gauge_kind == 1) a.xf[6 * fb + k] = xi[k];
         dd x = dd_from_double(xi[k]);
         sdd = dd_add(sdd, dd_mul(x, x));
         sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bf[6 * fb + k])));
-        mx = fmax(mx, fabs(xi[k]));
+        step_max(xi[k]);
       }
-      se3_left_update(xi, T, O);
-      pose_table(O, a.pose_f + 12 * j, a.pose_dd + 24 * j);
     } else {
       const int i = static_cast<int>(t - a.nc);
       const double* p = a.points + 3 * i;
@@ -2991,7 +2921,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
         dd x = dd_from_double(d[k]);
         sdd = dd_add(sdd, dd_mul(x, x));
         sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bm[3 * mb + k])));
-        mx = fmax(mx, fabs(d[k]));
+        step_max(d[k]);
         O[k] = p[k] + d[k];
         const dd o = dd_from_double(O[k]);
         a.pts[3 * static_cast<int64_t>(i) + k] = make_float2(o.hi, o.lo);
@@ -2999,11 +2929,11 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
     }
   }
   __shared__ float sh[4][8];
-  __shared__ double shm[8];
+  __shared__ unsigned long long shm[8];
   sdd = dd_warp_sum(sdd);
   sdg = dd_warp_sum(sdg);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     sh[0][w] = sdd.hi; sh[1][w] = sdd.lo; sh[2][w] = sdg.hi; sh[3][w] = sdg.lo;
@@ -3012,15 +2942,15 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
   __syncthreads();
   if (threadIdx.x == 0) {
     dd s0 = dd_make(0.f, 0.f), s1 = dd_make(0.f, 0.f);
-    double m = 0.0;
+    unsigned long long m = 0ull;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
       s0 = dd_add(s0, dd_make(sh[0][q], sh[1][q]));
       s1 = dd_add(s1, dd_make(sh[2][q], sh[3][q]));
-      m = fmax(m, shm[q]);
+      m = max(m, shm[q]);
     }
     a.part[2 * bid_] = dd_to_double(s0);
     a.part[2 * bid_ + 1] = dd_to_double(s1);
-    atomic_max_nonneg(&ctrl->max_step_bits, m);
+    atomicMax(&ctrl->max_step_bits, m);
   }
 }
 __global__ void __launch_bounds__(256) k_apply_update(UpdArgs a, Ctrl* ctrl) {
@@ -3157,6 +3087,7 @@ int warp_grid(int64_t items, int warps_per_block, int cap) {
 }
 
 constexpr int kUpdBlocks = 152;
+int upd_pose_blocks(const Sizes& s) { return (s.nc + kUpdPoses - 1) / kUpdPoses; }
 
 // CTAs of the update and gauge kernels: kUpdBlocks, or one per 256 poses and
 // points for small problems (local windows), whose update is a few thousand
@@ -3482,6 +3413,7 @@ static GaugeArgs make_gauge_args(const Sizes& s, const Dev& d) {
   g.cnt_f = d.cnt_f;
   g.cnt_m = d.cnt_m;
   g.xf = d.x;
+  g.x0 = d.x0;
   g.dm = d.dm;
   g.um = d.gauge_um;
   g.cx = s.gauge_center[0];
@@ -3504,6 +3436,8 @@ static UpdArgs make_upd_args(const Sizes& s, const Dev& d) {
   u.poses_t = d.poses_t;
   u.points_t = d.points_t;
   u.xf = d.x;
+  u.x0 = s.gauge_kind == 1 ? d.x0 : d.x;
+  u.sum_blocks = upd_blocks(s);
   u.dm = d.dm;
   u.bf = d.bf;
   u.bm = d.bm;
@@ -3534,7 +3468,7 @@ int launch_update(const Sizes& s, const Dev& d, cudaStream_t st) {
     k_gauge_partials<<<upd_blocks(s), 256, 0, st>>>(make_gauge_args(s, d), d.ctrl);
     n += 1;
   }
-  k_apply_update<<<upd_blocks(s), 256, 0, st>>>(make_upd_args(s, d), d.ctrl);
+  k_apply_update<<<upd_blocks(s) + upd_pose_blocks(s), 256, 0, st>>>(make_upd_args(s, d), d.ctrl);
   ++n;
   n += launch_eq_post(s, d, d.part + 2 * kUpdBlocks + 2 * upd_blocks(s), st);
   return n;
@@ -4083,7 +4017,7 @@ BatchTables* batch_tables_create(const std::vector<BatchWin>& wins, int skip_fin
     t_bsub.add(BsubArgs{make_back_args(s, d), d.lmk_chunk_pt, s.nlchunk, d.g_pt}, lmk_grid,
                sizeof(float) * 12 * static_cast<size_t>(s.lmk_cap));
     t_gauge.add(make_gauge_args(s, d), s.gauge_kind == 1 ? upd_blocks(s) : 0);
-    t_upd.add(make_upd_args(s, d), upd_blocks(s));
+    t_upd.add(make_upd_args(s, d), upd_blocks(s) + upd_pose_blocks(s));
     t_cost.add(make_decide_args(s, d), cost_grid(s.no));
     t_commit.add(CommitArgs{s.nc, s.np, s.no, d.poses_t, d.poses, d.points_t, d.points, d.res_t, d.res, d.res_lo_t,
                             d.res_lo, nullptr, nullptr},

@@ -42,9 +42,10 @@ __device__ __forceinline__ void pose_table(const double* T, float* pf, float* pd
 // number of active lanes, so one pose in one thread is bound by the count of
 // its FP64 operations (~170 of them, and two sincos, two square roots, three
 // divisions).  Here the entries of each small matrix, the two angles and the
-// three divisions lie in lanes.  Each entry is formed by the operations, and the
-// fused multiply-adds, of the plain expressions: rot_matrix and pose_table
-// above give the same bits.
+// three divisions lie in lanes.  Which product of a sum is fused and which is
+// rounded first is spelled out as the compiler chose it for the plain
+// expressions of rot_matrix and of the update in one thread, so the trial poses
+// kept their bits (a last-place change of a pose flips FP32 roundings later on).
 __device__ __forceinline__ double pose_neg(double x, bool n) {
   return n ? __longlong_as_double(__double_as_longlong(x) ^ (1ll << 63)) : x;
 }
@@ -96,9 +97,9 @@ __device__ __forceinline__ void pose_update16(double xil, double Tl, bool still,
   w[3] = 0.0;
   for (int k = 0; k < 7; ++k) T[k] = pose_shfl(Tl, k);
   const double th2 = fma(w[2], w[2], fma(w[0], w[0], w[1] * w[1]));
-  double eq[4], va = 0.0, vb = 0.0;
+  double eq[4];
   const bool small_q = th2 <= kPoseEps * kPoseEps, small_v = th2 <= kPoseEps;
-  double th = sqrt(th2);
+  const double th = sqrt(th2);
   // lane 0: sin, cos of th / 2; lane 1: of th
   double s, co;
   sincos((l & 1) ? th : 0.5 * th, &s, &co);
@@ -108,8 +109,7 @@ __device__ __forceinline__ void pose_update16(double xil, double Tl, bool still,
   const double den = l == 0 ? th : (l == 1 ? th2 : th2 * th);
   const double quo = num / den;
   double im = pose_shfl(quo, 0);
-  va = pose_shfl(quo, 1);
-  vb = pose_shfl(quo, 2);
+  const double va = pose_shfl(quo, 1), vb = pose_shfl(quo, 2);
   eq[0] = c0;
   if (small_q) {
     const double th4 = th2 * th2;
@@ -128,27 +128,15 @@ __device__ __forceinline__ void pose_update16(double xil, double Tl, bool still,
     double v = 0.5 * h;
     if (!small_v) {
       double h2 = fma(W(r, 2), W(2, c), fma(W(r, 0), W(0, c), W(r, 1) * W(1, c)));
-#ifdef A0
-      if (l == 0) h2 = A0 == 1 ? fma(W(0, 1), W(1, 0), W(0, 2) * W(2, 0)) : A0 == 2 ? __dadd_rn(__dmul_rn(W(0, 1), W(1, 0)), __dmul_rn(W(0, 2), W(2, 0))) : h2;
-      if (l == 8) h2 = A8 == 1 ? fma(W(2, 1), W(1, 2), W(0, 2) * W(2, 0)) : A8 == 2 ? __dadd_rn(__dmul_rn(W(2, 1), W(1, 2)), __dmul_rn(W(0, 2), W(2, 0))) : h2;
-#endif
-#ifdef V1
+      if (l == 0) h2 = __dadd_rn(__dmul_rn(w[2], -w[2]), __dmul_rn(w[1], -w[1]));  // both products rounded
+      if (l == 8) h2 = fma(w[0], -w[0], w[1] * -w[1]);
       v = fma(vb, h2, va * h);
-#else
-      v = fma(va, h, vb * h2);
-#endif
     }
     if (r == c) v += 1.0;
     const int base = 3 * (l % 3);
     const double v0 = pose_shfl(v, base), v1 = pose_shfl(v, base + 1), v2 = pose_shfl(v, base + 2);
     // lanes 0 .. 2; v0 is the constant 1 in row 0 for small angles
-#ifdef E1
-    et = fma(v2, tr[2], fma(v1, tr[1], v0 * tr[0]));
-#elif defined(E2)
     et = fma(v2, tr[2], (small_v && l == 0) ? fma(v1, tr[1], tr[0]) : fma(v0, tr[0], v1 * tr[1]));
-#else
-    et = fma(v2, tr[2], fma(v0, tr[0], v1 * tr[1]));
-#endif
   }
   if (!(0.0 <= eq[0]))
     for (int i = 0; i < 4; ++i) eq[i] = pose_neg(eq[i], true);
@@ -170,11 +158,7 @@ __device__ __forceinline__ void pose_update16(double xil, double Tl, bool still,
   double ot;
   {
     const double r0 = pose_shfl(R, base), r1 = pose_shfl(R, base + 1), r2 = pose_shfl(R, base + 2);
-#ifdef O1
-    ot = fma(r2, T[6], fma(r1, T[5], r0 * T[4])) + et;  // lanes 0 .. 2: the translation
-#else
     ot = fma(r2, T[6], fma(r0, T[4], r1 * T[5])) + et;  // lanes 0 .. 2: the translation
-#endif
   }
   if (!(0.0 <= q[0]))
     for (int i = 0; i < 4; ++i) q[i] = pose_neg(q[i], true);

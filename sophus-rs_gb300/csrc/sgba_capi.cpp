@@ -1827,8 +1827,7 @@ int sgba_covariance_prepare(sgba_problem* p, sgba_cov_info* info) {
   SGBA_CK(cudaEventRecord(ev[0], str));
   int launches = 0;
   // the pose-only cost functions' blocks at the current poses
-  launches += sgba::launch_prior_eval(s, d, d.poses, 1, 0, nullptr, str);
-  launches += sgba::launch_edge_eval(s, d, d.poses, 1, 0, nullptr, str);
+  launches += sgba::launch_pose_terms(s, d, d.poses, 1, 0, nullptr, str);
   launches += sgba::launch_cov_assemble(s, d, c, str);
   SGBA_CK(cudaGetLastError());
   SGBA_CK(cudaEventRecord(ev[1], str));

@@ -76,7 +76,7 @@ constexpr int kGT = 64, kGK = 16;     // GEMM tile and depth
 template <bool E>
 __device__ void cov_jacobians(const double* T, const double* p, const double* intr, double* jp, double* jm) {
   double Rwc[9];
-  lie::quat_matrix<double>(T, Rwc);
+  lie::quat_matrix(T, Rwc);
   double R[9], t[3];
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) R[3 * i + j] = Rwc[3 * j + i];
@@ -139,7 +139,7 @@ __device__ __forceinline__ int up_idx(int k, int a, int b) { return a * k - a * 
 template <bool E>
 __device__ void cov_cam_jacobian(const double* T, const double* p, const double* intr, double* jc) {
   double Rwc[9];
-  lie::quat_matrix<double>(T, Rwc);
+  lie::quat_matrix(T, Rwc);
   double R[9], t[3];
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) R[3 * i + j] = Rwc[3 * j + i];

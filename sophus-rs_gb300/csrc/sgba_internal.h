@@ -509,17 +509,16 @@ struct PriorArgs {
   const double* W;
   double* out;
 };
-// The priors at `poses`: with lin, their blocks into Dev::prior_out (priors
-// on free poses); their total cost into *cost_sum (float-float sum in prior
-// order).  gate: 0 always, 1 unless the LM loop is done, 2 unless done or the
-// step is skipped.  Returns the launches (0 without priors).
-int launch_prior_eval(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost_sum,
+// The pose-graph edges (PoseGraph3CostTerm) and the priors at `poses`: with
+// lin, per reduced edge term its records into Dev::edge_out and Dev::edge_hmn
+// and the blocks of the priors on free poses into Dev::prior_out; with cost,
+// one partial of their total cost per CTA (pose_term_blocks of them,
+// float-float sums).  gate: 0 always, 1 unless the LM loop is done, 2 unless
+// done or the step is skipped.  Returns the launches (0 without either).
+int launch_pose_terms(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost,
                       cudaStream_t st);
-// The pose-graph edges at `poses` (PoseGraph3CostTerm): with lin, per reduced
-// term the records of both sides into Dev::edge_out and J_m^T J_n into
-// Dev::edge_hmn; their total cost into *cost_sum.  The same gates.
-int launch_edge_eval(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost_sum,
-                     cudaStream_t st);
+int pose_term_blocks(const Sizes& s);
+constexpr int kPoseTermMaxBlocks = 256;  // of the edges, and of the priors
 // Equality constraints (TranslationNormConstraint) at the current poses: c and
 // G, and G^T lambda added to the free gradient and the reduced rhs (after the
 // camera finalisation, before the solve).  Returns the launches.

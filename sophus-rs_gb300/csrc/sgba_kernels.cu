@@ -3104,7 +3104,7 @@ int upd_blocks(const Sizes& s) {
 // partials: gauge (2 per block), update (2 per block, then the constraints'
 // slot), cost (one per block, then the priors' and the edges')
 constexpr int kCostPartOff = 4 * kUpdBlocks + 2;
-int cost_partials_needed(const Sizes& s) { return kCostPartOff + cost_grid(s.no) + 2; }
+int cost_partials_needed(const Sizes& s) { return kCostPartOff + cost_grid(s.no) + 2 * kPoseTermMaxBlocks; }
 
 // The cost at the point whose tables (poses, split points and camera) are
 // current.
@@ -3137,10 +3137,9 @@ int launch_init_merit(const Sizes& s, const Dev& d, cudaStream_t st) {
   CostArgs a = make_cost_args(s, d, d.res, d.part, 0);
   const int nb = cost_grid(s.no);
   (s.eucm ? k_cost<true> : k_cost<false>)<<<nb, kCostThreads, 0, st>>>(a, d.ctrl);
-  const int np = launch_prior_eval(s, d, d.poses, 0, 0, d.part + nb, st);
-  const int ne = launch_edge_eval(s, d, d.poses, 0, 0, d.part + nb + np, st);
-  k_init_merit<<<1, 256, 0, st>>>(d.part, nb + np + ne, d.ctrl);
-  return 3 + np + ne;
+  const int nt = launch_pose_terms(s, d, d.poses, 0, 0, d.part + nb, st);
+  k_init_merit<<<1, 256, 0, st>>>(d.part, nb + pose_term_blocks(s), d.ctrl);
+  return 3 + nt;
 }
 
 int launch_iteration_begin(const Sizes& s, const Dev& d, cudaStream_t st) {
@@ -3323,8 +3322,7 @@ int launch_linearize(const Sizes& s, const Dev& d, double nu_override, bool use_
   n += launch_landmark(s, d, make_lin_args(s, d, nu_override, use_override), st, use_override);
   n += launch_intr_linearize(s, d, st);
   n += launch_camera(s, d, use_override ? 0 : 1, st);
-  n += launch_prior_eval(s, d, d.poses, 1, 1, nullptr, st);
-  n += launch_edge_eval(s, d, d.poses, 1, 1, nullptr, st);
+  n += launch_pose_terms(s, d, d.poses, 1, 1, nullptr, st);
   // the last block of the finalisation runs the gradient check of an LM iteration
   k_camera_finalize<<<s.nf, 64, 0, st>>>(s.nf, d.fb_tile_begin, d.tile_part, d.ufull, d.bf, d.rb, d.ctrl,
                                          use_override ? 0 : 1, s.n_prior > 0 ? d.prior_fb_begin : nullptr,
@@ -3521,15 +3519,15 @@ static int commit_grid(const Sizes& s) {
 int launch_decide(const Sizes& s, const Dev& d, cudaStream_t st) {
   const int nb = cost_grid(s.no);
   CostArgs a = make_decide_args(s, d);
-  // the priors' trial cost first: one more partial for the decision
-  a.n_extra = launch_prior_eval(s, d, d.poses_t, 0, 2, a.partials + nb, st);
-  a.n_extra += launch_edge_eval(s, d, d.poses_t, 0, 2, a.partials + nb + a.n_extra, st);
+  // the pose-only terms' trial cost first: more partials for the decision
+  const int nt = launch_pose_terms(s, d, d.poses_t, 0, 2, a.partials + nb, st);
+  a.n_extra = pose_term_blocks(s);
   (s.eucm ? k_cost<true> : k_cost<false>)<<<nb, kCostThreads, 0, st>>>(a, d.ctrl);
   const int cb = commit_grid(s);
   k_commit<<<cb, 256, 0, st>>>(s.nc, s.np, s.no, d.poses_t, d.poses, d.points_t, d.points, d.res_t, d.res,
                                d.res_lo_t, d.res_lo, s.intr_free ? d.intr_t : nullptr,
                                s.intr_free ? d.intr : nullptr, d.ctrl);
-  return 2 + a.n_extra;
+  return 2 + nt;
 }
 
 // ---------------------------------------------------------------------------

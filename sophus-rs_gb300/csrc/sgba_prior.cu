@@ -6,14 +6,14 @@
 // Each prior k on pose j has a mean E_k and a 6x6 precision W_k; its residual
 // is g = log(T_j E_k^-1) and its Jacobian J the derivative of
 // log(exp(x) T_j E_k^-1) at x = 0, taken here by forward-mode derivatives in
-// f64 (sgba_lie.cuh).  EvaluatedCostTerm::make
+// f64 (sgba_lie.cuh: a direction per lane).  EvaluatedCostTerm::make
 // (crates/sophus_opt/src/nlls/cost/evaluated_term.rs:286-327) then gives the
 // Hessian block J^T W J, the gradient J^T W g and the cost g^T W g.  The
-// priors are few (at most one group per pose) and run in f64 in one CTA; the
+// priors are few (at most one group per pose) and run in f64; the
 // blocks go to the pose's diagonal block in k_camera_finalize (damping once
 // per pose with a prior: one reduced term of the prior cost function,
-// cost_system.rs:229-236), the costs into one extra partial of the merit and
-// of the trial cost.
+// cost_system.rs:229-236), the costs into extra partials of the merit and of
+// the trial cost.
 //
 // Each edge on poses (m, n) with the measured pose_m_from_pose_n M has the
 // residual g = log(T_m^-1 T_n M^-1), no precision and no robust kernel: cost
@@ -34,8 +34,6 @@ namespace sgba {
 
 namespace {
 
-constexpr int kPriorThreads = 256;
-
 struct EdgeArgs {
   int nt;              // reduced terms
   const int32_t* tbeg; // nt + 1: edge ranges
@@ -49,158 +47,174 @@ struct EdgeArgs {
 __device__ __forceinline__ bool prior_halted(const Ctrl* c) { return c->done != 0; }
 __device__ __forceinline__ bool prior_skipping(const Ctrl* c) { return c->done != 0 || c->skip != 0; }
 
-// Priors (sorted by pose) at the given poses.  lin: also J^T W J and J^T W g
-// for the priors on free poses (out, kPriorOut doubles per prior).  The
-// costs g^T W g are summed in prior order in float-float and written to
-// *cost_sum.  gate: 0 none, 1 the control block's done flag, 2 done or a
-// skipped step.
-__global__ void __launch_bounds__(kPriorThreads) k_prior_eval(PriorArgs a, const double* __restrict__ poses, int lin,
-                                                             int gate, double* cost_sum, const Ctrl* ctrl) {
-  if ((gate == 1 && prior_halted(ctrl)) || (gate == 2 && prior_skipping(ctrl))) return;
-  dd acc = dd_make(0.0f, 0.0f);
-  for (int k = threadIdx.x; k < a.n; k += kPriorThreads) {
-    const double* T = poses + 7 * a.pose[k];
-    const double* W = a.W + 36 * k;
-    double einv[7], te[7], g[6];
-    lie::se3_inverse(a.mean + 7 * k, einv);
-    lie::se3_mul(T, einv, te);
-    lie::se3_log(te, g);
-    double wg[6];
-    for (int r = 0; r < 6; ++r) {
-      double s = 0.0;
-      for (int c = 0; c < 6; ++c) s += W[6 * r + c] * g[c];
-      wg[r] = s;
+// Eight lanes per term, one of the six tangent directions in each (two idle),
+// and two warps per CTA, so that the terms lie on as many FP64 pipes as there
+// are: a term's ~300 f64 operations, 64 cycles each whatever the lanes, bound
+// the kernel.  (A thread per term with all six directions, in one CTA: 135 +
+// 86 us an iteration of 151 poses, 150 edges and two priors; now 35 for both.)
+constexpr int kTermLanes = 8;
+constexpr int kTermThreads = 64;
+constexpr int kTermsPerBlock = kTermThreads / kTermLanes;
+
+__device__ __forceinline__ double term_shfl(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane, kTermLanes); }
+
+__device__ __forceinline__ double pick3(const double* v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); }
+
+// Residual g = log(q), its derivative d along this lane's direction k of x in
+// A exp(x) B = (q, t), with A's rotation qa (identity: null) and B = b.
+// `turned`: the signs of the product quaternion were turned.
+__device__ __forceinline__ void term_log(const double* qa, const double* b, const double* ab, bool turned, int k,
+                                         double* g, double* d) {
+  // exp(x) B: the quaternion moves by (0, e_k / 2) b, the translation by e_k x t_b or e_k
+  const int j = k % 3;
+  double h[4] = {0.0, 0.0, 0.0, 0.0}, u[3], dq[4], dt[3];
+  if (k < 3) {
+    h[0] = -0.5 * pick3(b + 1, j);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int o = 3 - i - j;  // the third axis
+      const bool next = i == j + 1 || (j == 2 && i == 0);  // e_j x v: -v_o at j + 1, +v_o at j + 2
+      const double bq = pick3(b + 1, o), bt = pick3(b + 4, o);
+      h[1 + i] = 0.5 * (i == j ? b[0] : (next ? -bq : bq));
+      u[i] = i == j ? 0.0 : (next ? -bt : bt);
     }
-    double cst = 0.0;
-    for (int r = 0; r < 6; ++r) cst += g[r] * wg[r];
-    acc = dd_add(acc, dd_from_double(cst));
-    if (lin && a.fb[k] >= 0) {
-      lie::D6 e[7], td[7], ed[7], p1[7], p2[7], gd[6];
-      lie::se3_exp_at_zero(e);
-      for (int i = 0; i < 7; ++i) {
-        td[i] = lie::dc(T[i]);
-        ed[i] = lie::dc(einv[i]);
-      }
-      lie::se3_mul(e, td, p1);
-      lie::se3_mul(p1, ed, p2);
-      lie::se3_log(p2, gd);
-      double J[36], WJ[36];
-      for (int r = 0; r < 6; ++r)
-        for (int c = 0; c < 6; ++c) J[6 * r + c] = gd[r].d[c];
-      for (int r = 0; r < 6; ++r)
-        for (int c = 0; c < 6; ++c) {
-          double s = 0.0;
-          for (int q = 0; q < 6; ++q) s += W[6 * r + q] * J[6 * q + c];
-          WJ[6 * r + c] = s;
-        }
-      double* o = a.out + static_cast<int64_t>(kPriorOut) * k;
-      for (int r = 0; r < 6; ++r) {
-        double s = 0.0;
-        for (int q = 0; q < 6; ++q) s += J[6 * q + r] * wg[q];
-        o[36 + r] = s;  // J^T W g
-        for (int c = 0; c < 6; ++c) {
-          double h = 0.0;
-          for (int q = 0; q < 6; ++q) h += J[6 * q + r] * WJ[6 * q + c];
-          o[6 * r + c] = h;  // J^T W J
-        }
-      }
-    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) u[i] = i == j ? 1.0 : 0.0;
   }
-  if (!cost_sum) return;
-  // fixed tree over the CTA: thread t holds priors t, t + 256, ...
-  __shared__ float sh_hi[kPriorThreads], sh_lo[kPriorThreads];
-  sh_hi[threadIdx.x] = acc.hi;
-  sh_lo[threadIdx.x] = acc.lo;
-  __syncthreads();
-  for (int h = kPriorThreads / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) {
-      const dd v = dd_add(dd_make(sh_hi[threadIdx.x], sh_lo[threadIdx.x]),
-                          dd_make(sh_hi[threadIdx.x + h], sh_lo[threadIdx.x + h]));
-      sh_hi[threadIdx.x] = v.hi;
-      sh_lo[threadIdx.x] = v.lo;
-    }
-    __syncthreads();
+  if (qa) {
+    lie::quat_mul(qa, h, dq);
+    lie::rotate(qa, u, dt);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dq[i] = h[i];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dt[i] = u[i];
   }
-  if (threadIdx.x == 0) *cost_sum = dd_to_double(dd_make(sh_hi[0], sh_lo[0]));
+  if (turned)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dq[i] = -dq[i];
+  lie::se3_log(ab, dq, dt, g, d);
 }
 
-// Reduced edge terms at the given poses (one CTA; a thread per term, its
-// edges in order).  lin: the records of both sides and J_m^T J_n.  Costs
-// summed as in k_prior_eval.
-__global__ void __launch_bounds__(kPriorThreads) k_edge_eval(EdgeArgs a, const double* __restrict__ poses, int lin,
-                                                            int gate, double* cost_sum, const Ctrl* ctrl) {
+// CTAs [0, edge_blocks): reduced edge terms (the edges of a term in order); the
+// others: priors (sorted by pose).  At `poses`; lin: the records of both sides
+// and J_m^T J_n of a term, J^T W J and J^T W g of the priors on free poses
+// (kPriorOut doubles each).  cost: a CTA's sum of g^T g and g^T W g in
+// float-float to cost[blockIdx.x].  gate: 0 none, 1 the control block's done
+// flag, 2 done or a skipped step.
+__global__ void __launch_bounds__(kTermThreads) k_pose_terms(EdgeArgs ea, PriorArgs pa, int edge_blocks,
+                                                             const double* __restrict__ poses, int lin, int gate,
+                                                             double* cost, const Ctrl* ctrl) {
   if ((gate == 1 && prior_halted(ctrl)) || (gate == 2 && prior_skipping(ctrl))) return;
+  const int k = threadIdx.x % kTermLanes, slot = threadIdx.x / kTermLanes;
+  const int c = k < 6 ? k : 5;  // this lane's direction and column
   dd acc = dd_make(0.0f, 0.0f);
-  for (int t = threadIdx.x; t < a.nt; t += kPriorThreads) {
-    double hmm[36], hnn[36], hmn[36], gm[6], gn[6];
-    for (int i = 0; i < 36; ++i) hmm[i] = hnn[i] = hmn[i] = 0.0;
-    for (int i = 0; i < 6; ++i) gm[i] = gn[i] = 0.0;
-    for (int e = a.tbeg[t]; e < a.tbeg[t + 1]; ++e) {
-      const double* Tm = poses + 7 * a.m[e];
-      const double* Tn = poses + 7 * a.n[e];
-      double ai[7], mninv[7], b[7], ab[7], g[6];
-      lie::se3_inverse(Tm, ai);
-      lie::se3_inverse(a.mn + 7 * e, mninv);
-      lie::se3_mul(Tn, mninv, b);
-      lie::se3_mul(ai, b, ab);
-      lie::se3_log(ab, g);
-      double cst = 0.0;
-      for (int r = 0; r < 6; ++r) cst += g[r] * g[r];
-      acc = dd_add(acc, dd_from_double(cst));
-      if (!lin) continue;
-      lie::D6 ex[7], ad[7], bd[7], t1[7], t2[7], gd[6];
-      lie::se3_exp_at_zero(ex);
-      for (int i = 0; i < 7; ++i) {
-        ad[i] = lie::dc(ai[i]);
-        bd[i] = lie::dc(b[i]);
-      }
-      lie::se3_mul(ad, ex, t1);
-      lie::se3_mul(t1, bd, t2);
-      lie::se3_log(t2, gd);
-      // J_n = D, J_m = -D
-      for (int r = 0; r < 6; ++r) {
+  if (static_cast<int>(blockIdx.x) < edge_blocks) {
+    const int stride = edge_blocks * kTermsPerBlock;
+    // whole warps loop together; a slot past the end repeats the last term and stores nothing
+    for (int t0 = blockIdx.x * kTermsPerBlock; t0 < ea.nt; t0 += stride) {
+      const bool on = t0 + slot < ea.nt;
+      const int t = on ? t0 + slot : ea.nt - 1;
+      double hcol[6], gc = 0.0;  // column c of D^T D, (D^T g)_c
+#pragma unroll
+      for (int i = 0; i < 6; ++i) hcol[i] = 0.0;
+      const int e1 = ea.tbeg[t + 1];
+      for (int e = ea.tbeg[t]; __any_sync(0xffffffffu, e < e1); ++e) {
+        const bool live = e < e1;
+        const int ei = live ? e : e1 - 1;
+        double ai[7], mi[7], b[7], ab[7], g[6], d[6];
+        lie::se3_inverse(poses + 7 * ea.m[ei], ai);
+        lie::se3_inverse(ea.mn + 7 * ei, mi);
+        lie::se3_mul(poses + 7 * ea.n[ei], mi, b);
+        const bool turned = lie::se3_mul(ai, b, ab);
+        term_log(ai, b, ab, turned, c, g, d);
+        double cst = 0.0;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) cst += g[r] * g[r];
+        if (on && live && k == 0) acc = dd_add(acc, dd_from_double(cst));
+        if (!lin) continue;
+        // J_n = D, J_m = -D
         double sg = 0.0;
-        for (int q = 0; q < 6; ++q) sg += gd[q].d[r] * g[q];
-        gn[r] += sg;
-        gm[r] -= sg;
-        for (int c = 0; c < 6; ++c) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sg += d[q] * g[q];
+        if (live) gc += sg;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
           double s2 = 0.0;
-          for (int q = 0; q < 6; ++q) s2 += gd[q].d[r] * gd[q].d[c];
-          hnn[6 * r + c] += s2;
-          hmm[6 * r + c] += s2;
-          hmn[6 * r + c] -= s2;
+#pragma unroll
+          for (int q = 0; q < 6; ++q) s2 += term_shfl(d[q], r) * d[q];
+          if (live) hcol[r] += s2;
         }
       }
+      if (lin && on && k < 6) {
+        double* o0 = ea.out + static_cast<int64_t>(kPriorOut) * (2 * t);
+        double* o1 = o0 + kPriorOut;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+          o0[6 * r + c] = hcol[r];
+          o1[6 * r + c] = hcol[r];
+          ea.hmn[36 * static_cast<int64_t>(t) + 6 * r + c] = -hcol[r];
+        }
+        o0[36 + c] = -gc;
+        o1[36 + c] = gc;
+      }
     }
-    if (lin) {
-      double* o0 = a.out + static_cast<int64_t>(kPriorOut) * (2 * t);
-      double* o1 = o0 + kPriorOut;
-      for (int i = 0; i < 36; ++i) {
-        o0[i] = hmm[i];
-        o1[i] = hnn[i];
-        a.hmn[36 * static_cast<int64_t>(t) + i] = hmn[i];
+  } else {
+    const int stride = (gridDim.x - edge_blocks) * kTermsPerBlock;
+    for (int p0 = (blockIdx.x - edge_blocks) * kTermsPerBlock; p0 < pa.n; p0 += stride) {
+      const bool on = p0 + slot < pa.n;
+      const int p = on ? p0 + slot : pa.n - 1;
+      const double* W = pa.W + 36 * static_cast<int64_t>(p);
+      double einv[7], te[7], g[6], d[6];
+      lie::se3_inverse(pa.mean + 7 * p, einv);
+      lie::se3_mul(poses + 7 * pa.pose[p], einv, te);
+      term_log(nullptr, te, te, false, c, g, d);
+      // lane r: (W g)_r
+      double wr = 0.0;
+#pragma unroll
+      for (int q = 0; q < 6; ++q) wr += W[6 * c + q] * g[q];
+      double wg[6];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) wg[r] = term_shfl(wr, r);
+      double cst = 0.0;
+#pragma unroll
+      for (int r = 0; r < 6; ++r) cst += g[r] * wg[r];
+      if (on && k == 0) acc = dd_add(acc, dd_from_double(cst));
+      if (!lin) continue;
+      double wj[6], s = 0.0;  // column c of W J, (J^T W g)_c
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v += W[6 * r + q] * d[q];
+        wj[r] = v;
+        s += d[r] * wg[r];
       }
-      for (int i = 0; i < 6; ++i) {
-        o0[36 + i] = gm[i];
-        o1[36 + i] = gn[i];
+      double* o = pa.out + static_cast<int64_t>(kPriorOut) * p;
+      const bool store = on && k < 6 && pa.fb[p] >= 0;
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        double h = 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) h += term_shfl(d[q], r) * wj[q];
+        if (store) o[6 * r + c] = h;  // J^T W J
       }
+      if (store) o[36 + c] = s;
     }
   }
-  if (!cost_sum) return;
-  __shared__ float sh_hi[kPriorThreads], sh_lo[kPriorThreads];
-  sh_hi[threadIdx.x] = acc.hi;
-  sh_lo[threadIdx.x] = acc.lo;
+  if (!cost) return;
+  __shared__ float2 part[kTermThreads / 32];
+  acc = dd_warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_float2(acc.hi, acc.lo);
   __syncthreads();
-  for (int h = kPriorThreads / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) {
-      const dd v = dd_add(dd_make(sh_hi[threadIdx.x], sh_lo[threadIdx.x]),
-                          dd_make(sh_hi[threadIdx.x + h], sh_lo[threadIdx.x + h]));
-      sh_hi[threadIdx.x] = v.hi;
-      sh_lo[threadIdx.x] = v.lo;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *cost_sum = dd_to_double(dd_make(sh_hi[0], sh_lo[0]));
+  if (threadIdx.x == 0)
+    cost[blockIdx.x] = dd_to_double(dd_add(dd_make(part[0].x, part[0].y), dd_make(part[1].x, part[1].y)));
+}
+
+int term_blocks(int n) {
+  const int b = (n + kTermsPerBlock - 1) / kTermsPerBlock;
+  return b < kPoseTermMaxBlocks ? b : kPoseTermMaxBlocks;
 }
 
 // Equality constraints c_k = |t(T_k)| - r_k (TranslationNormConstraint,
@@ -261,19 +275,18 @@ int launch_eq_post(const Sizes& s, const Dev& d, double* upd_slot, cudaStream_t 
   return 1;
 }
 
-int launch_edge_eval(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost_sum,
-                     cudaStream_t st) {
-  if (s.n_edge <= 0) return 0;
-  EdgeArgs a{s.n_eterm, d.eterm_begin, d.edge_m, d.edge_n, d.edge_mn, d.edge_out, d.edge_hmn};
-  k_edge_eval<<<1, kPriorThreads, 0, st>>>(a, poses, lin, gate, cost_sum, d.ctrl);
-  return 1;
+int pose_term_blocks(const Sizes& s) {
+  return (s.n_edge > 0 ? term_blocks(s.n_eterm) : 0) + (s.n_prior > 0 ? term_blocks(s.n_prior) : 0);
 }
 
-int launch_prior_eval(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost_sum,
+int launch_pose_terms(const Sizes& s, const Dev& d, const double* poses, int lin, int gate, double* cost,
                       cudaStream_t st) {
-  if (s.n_prior <= 0) return 0;
-  PriorArgs a{s.n_prior, d.prior_pose, d.prior_fb, d.prior_mean, d.prior_W, d.prior_out};
-  k_prior_eval<<<1, kPriorThreads, 0, st>>>(a, poses, lin, gate, cost_sum, d.ctrl);
+  const int blocks = pose_term_blocks(s);
+  if (blocks == 0) return 0;
+  EdgeArgs ea{s.n_eterm, d.eterm_begin, d.edge_m, d.edge_n, d.edge_mn, d.edge_out, d.edge_hmn};
+  PriorArgs pa{s.n_prior, d.prior_pose, d.prior_fb, d.prior_mean, d.prior_W, d.prior_out};
+  k_pose_terms<<<blocks, kTermThreads, 0, st>>>(ea, pa, s.n_edge > 0 ? term_blocks(s.n_eterm) : 0, poses, lin, gate,
+                                                cost, d.ctrl);
   return 1;
 }
 

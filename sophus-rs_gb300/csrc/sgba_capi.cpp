@@ -2127,6 +2127,12 @@ void pcg_structure(const Plan& P, std::vector<int32_t>* rowptr, std::vector<int3
   }
 }
 
+int pcg_longest_row(const std::vector<int32_t>& rowptr) {
+  int m = 0;
+  for (size_t j = 0; j + 1 < rowptr.size(); ++j) m = std::max(m, rowptr[j + 1] - rowptr[j]);
+  return m;
+}
+
 int pcg_alloc(sgba_problem* p) {
   Dev& d = p->d;
   if (d.pcg_rowptr) return SGBA_OK;
@@ -2155,6 +2161,8 @@ int pcg_alloc(sgba_problem* p) {
   if ((st = dev_alloc(p, &d.pcg_msg, nf * sgba::kPcgHidden))) return st;
   if ((st = dev_alloc(p, &d.pcg_L, nf * sgba::kPcgOut))) return st;
   s.pcg_nnzb = static_cast<int64_t>(cols.size());
+  const int longest = pcg_longest_row(rowptr);
+  s.pcg_row_max = sgba::pcg_rows_setup(s.nf, longest) ? longest : 0;
   SGBA_CK(cudaStreamSynchronize(p->stream));  // the host vectors above go out of scope
   return SGBA_OK;
 }
@@ -2353,6 +2361,7 @@ int trainset_append(sgba_pcg_trainset* h, const Plan* plan, int nf, const std::v
   for (int j = 0; j < nf; ++j)
     if (diag[j] < 0) return set_error(SGBA_ERR_INVALID_ARGUMENT, "block row %d has no diagonal block", j);
   s.nnzb = static_cast<int64_t>(cols.size());
+  s.row_max = pcg_longest_row(rowptr);
   const size_t n6 = 6 * static_cast<size_t>(nf), nb = 36 * static_cast<size_t>(s.nsb);
   auto fail = [&](cudaError_t e) {
     cudaFree(s.rowptr); cudaFree(s.cols); cudaFree(s.blks); cudaFree(s.diag);

@@ -325,6 +325,7 @@ struct PcgModel {
 struct PcgSystem {
   int nf = 0;
   int64_t nsb = 0, nnzb = 0;
+  int row_max = 0;
   int32_t* rowptr = nullptr;
   int32_t* cols = nullptr;
   int32_t* blks = nullptr;
@@ -408,6 +409,7 @@ struct Sizes {
   int pcg_max_iters;
   double pcg_tol;      // relative residual of the Jacobi-scaled system
   int pcg_grid;        // CTAs of the cooperative PCG kernel
+  int pcg_row_max;     // longest block row, 0: the rows do not fit k_pcg_rows
   int64_t pcg_nnzb;    // entries of the full block rows
   float lmk_well_tol;  // point blocks: FP32 Cholesky kept while every pivot keeps this fraction
   int lmk_list_grid;   // CTAs of the float-float redo of the other points
@@ -478,6 +480,7 @@ cudaError_t zterm_fill(const Sizes& s, const Dev& d, int32_t* T, cudaStream_t st
 // converged (Ctrl::pcg_done).
 constexpr int kPcgMaxGrid = 2048;  // CTAs of the cooperative PCG kernel at most (partial-sum slots)
 int pcg_setup(int nf, int* grid);
+bool pcg_rows_setup(int nf, int row_max);
 int launch_pcg(const Sizes& s, const Dev& d, cudaStream_t st);
 // The same after the scaled blocks exist (pcg_S, pcg_S2; d.rb already scaled
 // when d.pcg_scl is null): network, preconditioner, solve.

@@ -690,6 +690,7 @@ cudaError_t pcg_evaluate(const PcgModel* m, PcgTrainSet& t, int idx, int mode, i
   z.pcg_max_iters = max_iters;
   z.pcg_tol = tol;
   z.pcg_grid = grid;
+  z.pcg_row_max = pcg_rows_setup(s.nf, s.row_max) ? s.row_max : 0;
   z.pcg_nnzb = s.nnzb;
   Dev d;
   d.pcg_rowptr = s.rowptr;

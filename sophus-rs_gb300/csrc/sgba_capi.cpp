@@ -1107,6 +1107,8 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     if (sgba::schur_dense_setup() != 0) return set_error(SGBA_ERR_CUDA, "shared memory of the tiled Schur pass");
     SGBA_CK(sgba::zterm_fill(s, d, d.zterm, p->stream));
   }
+  if (s.lin_dd && sgba::schur_dd_setup() != 0)
+    return set_error(SGBA_ERR_CUDA, "shared memory of the float-float Schur pass");
   s.lmk_dd_ok = (s.lin_dd && s.nlchunk > 0 && sgba::landmark_dd_setup(s.lmk_cap) == 0) ? 1 : 0;
   s.bsub_chunks_ok = (s.nlchunk > 0 && sgba::backsub_chunks_setup(s.lmk_cap) == 0) ? 1 : 0;
   if (s.lin_dd) {

@@ -431,6 +431,7 @@ int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st);
 int cost_partials_needed(const Sizes& s);  // reduction partial slots
 int landmark_setup(int cap);
 size_t intr_part_count(const Sizes& s);  // partial sums of the free intrinsics (float2)
+int schur_dd_setup();     // of the float-float Schur pass
 int schur_dense_setup();  // shared memory limits of the tiled Schur pass (0: ok)  // dynamic shared memory of the chunked landmark pass (0 = ok)
 int landmark_dd_setup(int cap);  // the same for its float-float variant (0 = ok)
 int backsub_chunks_setup(int cap);  // the chunked back-substitution (0 = ok)

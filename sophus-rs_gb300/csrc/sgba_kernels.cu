@@ -221,7 +221,19 @@ __device__ __forceinline__ void jacobians_f(const float* pt /*R_cw 9 + t_cw 3*/,
 
 
 constexpr int kZS = 20;  // floats per Z row block (18 used; padded for float4 loads)
-constexpr int kZD = kZddFloats;  // floats per float-float Z (36 used; padded for float4 loads)
+// Floats per float-float Z (6x3): column by column, entry (r, q) as (hi, lo) at
+// zd_at(r, q), so that 16-byte accesses take pairs of rows of one column (36
+// used; padded to a multiple of 32 bytes).
+constexpr int kZD = kZddFloats;
+__host__ __device__ constexpr int zd_at(int r, int q) { return 2 * (6 * q + r); }
+__device__ __forceinline__ void load_zdd(const float* zd, float* z) {  // all 36
+  const float4* p = reinterpret_cast<const float4*>(zd);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const float4 v = __ldg(p + k);
+    z[4 * k] = v.x; z[4 * k + 1] = v.y; z[4 * k + 2] = v.z; z[4 * k + 3] = v.w;
+  }
+}
 
 // Sum over the 32 lanes of a warp of `nv` float values per lane, in
 // float-float: values are transposed through shared memory (red[nv][33]) and
@@ -817,9 +829,9 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
           Z[r * 3 + 1] = z1.hi + z1.lo;
           Z[r * 3 + 2] = z2.hi + z2.lo;
           if (zd) {
-            zd[6 * r + 0] = z0.hi; zd[6 * r + 1] = z0.lo;
-            zd[6 * r + 2] = z1.hi; zd[6 * r + 3] = z1.lo;
-            zd[6 * r + 4] = z2.hi; zd[6 * r + 5] = z2.lo;
+            zd[zd_at(r, 0)] = z0.hi; zd[zd_at(r, 0) + 1] = z0.lo;
+            zd[zd_at(r, 1)] = z1.hi; zd[zd_at(r, 1) + 1] = z1.lo;
+            zd[zd_at(r, 2)] = z2.hi; zd[zd_at(r, 2) + 1] = z2.lo;
           }
         }
       }
@@ -1037,7 +1049,7 @@ __global__ void __launch_bounds__(256) k_landmark_chunks(LinArgs a, Ctrl* ctrl) 
 // over the term's observations and Z = W C^-T in float-float.  The same
 // arithmetic as k_landmark's float-float path; only the order of the sums
 // over a point's terms differs (sequential here, a lane tree there).
-constexpr int kLmkDDTermFloats = 18 + 36;  // 9 float-float sums + the Jacobians (18 float-float)
+constexpr int kLmkDDTermFloats = 18 + 36 + 1;  // 9 float-float sums + the Jacobians (18 float-float); odd: no bank conflicts
 
 template <bool E>
 __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctrl) {
@@ -1196,8 +1208,7 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
       dd I[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) I[k] = dd_make(sci[q][2 * k], sci[q][2 * k + 1]);
-      float Z[20];
-      float* zd = a.zdd + kZD * g;
+      float Z[20], zo[36];
 #pragma unroll
       for (int r = 0; r < 6; ++r) {
         const dd z0 = dd_mul(I[0], Wd[r * 3 + 0]);
@@ -1206,10 +1217,13 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
         Z[r * 3 + 0] = z0.hi + z0.lo;
         Z[r * 3 + 1] = z1.hi + z1.lo;
         Z[r * 3 + 2] = z2.hi + z2.lo;
-        zd[6 * r + 0] = z0.hi; zd[6 * r + 1] = z0.lo;
-        zd[6 * r + 2] = z1.hi; zd[6 * r + 3] = z1.lo;
-        zd[6 * r + 4] = z2.hi; zd[6 * r + 5] = z2.lo;
+        zo[zd_at(r, 0)] = z0.hi; zo[zd_at(r, 0) + 1] = z0.lo;
+        zo[zd_at(r, 1)] = z1.hi; zo[zd_at(r, 1) + 1] = z1.lo;
+        zo[zd_at(r, 2)] = z2.hi; zo[zd_at(r, 2) + 1] = z2.lo;
       }
+      float4* zd = reinterpret_cast<float4*>(a.zdd + kZD * g);
+#pragma unroll
+      for (int u = 0; u < 9; ++u) zd[u] = make_float4(zo[4 * u], zo[4 * u + 1], zo[4 * u + 2], zo[4 * u + 3]);
       Z[18] = 1.f;  // float-float Z in zdd
       Z[19] = 0.f;
       float4* dst = reinterpret_cast<float4*>(a.zmat + kZS * g);
@@ -1314,9 +1328,9 @@ __device__ __forceinline__ void camera_tiles_body(CamArgs a, const Ctrl* ctrl, i
         const float* zd = a.zdd + kZD * g;
 #pragma unroll
         for (int r = 0; r < 6; ++r) {
-          dd t = dd_add(dd_add(dd_mul(c0, dd_make(zd[6 * r + 0], zd[6 * r + 1])),
-                               dd_mul(c1, dd_make(zd[6 * r + 2], zd[6 * r + 3]))),
-                        dd_mul(c2, dd_make(zd[6 * r + 4], zd[6 * r + 5])));
+          dd t = dd_add(dd_add(dd_mul(c0, dd_make(zd[zd_at(r, 0)], zd[zd_at(r, 0) + 1])),
+                               dd_mul(c1, dd_make(zd[zd_at(r, 1)], zd[zd_at(r, 1) + 1]))),
+                        dd_mul(c2, dd_make(zd[zd_at(r, 2)], zd[zd_at(r, 2) + 1])));
           zc[2 * r] = t.hi;
           zc[2 * r + 1] = t.lo;
         }
@@ -1413,14 +1427,17 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_camera_tiles_dd(CamArgs a, 
     }
     const int mb = a.pt_mb[pi];
     if (a.with_schur && mb >= 0) {
-      const float* zd = a.zdd + kZD * g;
-      const float* cv = a.cvec + 6 * mb;
-      const dd c0 = dd_make(cv[0], cv[1]), c1 = dd_make(cv[2], cv[3]), c2 = dd_make(cv[4], cv[5]);
+      const float4* zd = reinterpret_cast<const float4*>(a.zdd + kZD * g);
+      const float2* cv = reinterpret_cast<const float2*>(a.cvec + 6 * mb);
 #pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        acc_madd(u[27 + r], dd_make(zd[6 * r + 0], zd[6 * r + 1]), c0);
-        acc_madd(u[27 + r], dd_make(zd[6 * r + 2], zd[6 * r + 3]), c1);
-        acc_madd(u[27 + r], dd_make(zd[6 * r + 4], zd[6 * r + 5]), c2);
+      for (int q = 0; q < 3; ++q) {
+        const float2 c = __ldg(cv + q);
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+          const float4 z = __ldg(zd + 3 * q + h);  // rows 2 h, 2 h + 1 of column q
+          acc_madd(u[27 + 2 * h], dd_make(z.x, z.y), dd_make(c.x, c.y));
+          acc_madd(u[28 + 2 * h], dd_make(z.z, z.w), dd_make(c.x, c.y));
+        }
       }
     }
   }
@@ -1659,52 +1676,90 @@ __global__ void __launch_bounds__(256, 2) k_schur(SchurArgs a, const Ctrl* ctrl)
 // a pair go by the inner index t (column t of both Z, 24 floats live instead
 // of 72), which keeps two CTAs per SM; every accumulator still receives its
 // t = 0, 1, 2 terms in that order.
+//
+// A round takes 32 pairs, one per lane.  Their 64 Z are copied to shared memory
+// by the warp together (consecutive lanes copy consecutive 16-byte parts of a Z;
+// a lane reading its own Z from global memory touched a line per load, and those
+// wavefronts held the pass: 84 % of the L1's; 1.52 -> 1.31 ms with the 1,500-camera loop),
+// nine 16-byte parts per Z, an odd count, so that the lanes' reads meet no bank
+// conflict.  Sixteen warps an SM hide the copies of one under the products of
+// the others; the buffer then serves the sum over the lanes.
+constexpr int kSddZ = 9;                       // 16-byte parts of a Z
+constexpr int kSddWarp = 2 * 32 * kSddZ;       // float4 per warp
+constexpr size_t kSddSmem = 8 * kSddWarp * sizeof(float4);
+static_assert(kSddWarp * 4 >= 36 * 33, "the lane sums fit in the pairs' buffer");
 __global__ void __launch_bounds__(256, 2) k_schur_dd(SchurArgs a, const Ctrl* ctrl) {
   if (skipping(ctrl)) return;
-  __shared__ float red[8][36][33];
+  extern __shared__ float4 sdd_sm[];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
+  float4* zs = sdd_sm + kSddWarp * wib;
+  float (*red)[33] = reinterpret_cast<float (*)[33]>(zs);
+  const unsigned zs_addr = static_cast<unsigned>(__cvta_generic_to_shared(zs));
   for (int64_t ch = static_cast<int64_t>(blockIdx.x) * wpb + wib; ch < a.nchunk;
        ch += static_cast<int64_t>(gridDim.x) * wpb) {
     Acc acc[36];
 #pragma unroll
     for (int e = 0; e < 36; ++e) acc[e] = acc_zero();
-    const int64_t q1 = a.chunk_begin[ch + 1];
-    for (int64_t q = a.chunk_begin[ch] + lane; q < q1; q += 32) {
-      const int2 pr = a.pairs[q];
-      const float2* pa = reinterpret_cast<const float2*>(a.zdd + kZD * static_cast<int64_t>(pr.x));
-      const float2* pb = reinterpret_cast<const float2*>(a.zdd + kZD * static_cast<int64_t>(pr.y));
+    const int64_t q0 = a.chunk_begin[ch], q1 = a.chunk_begin[ch + 1];
+    int2 next = q0 + lane < q1 ? a.pairs[q0 + lane] : make_int2(0, 0);
+    for (int64_t q = q0; q < q1; q += 32) {
+      const int2 pr = next;
+      const int n = static_cast<int>(min(static_cast<int64_t>(32), q1 - q));
+      if (q + 32 + lane < q1) next = a.pairs[q + 32 + lane];
+      // side s of pair p: parts (32 s + p) kSddZ + 0 .. 8
 #pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        float2 za[6], zb[6];  // column t of each Z: (hi, lo) of rows 0..5
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-          za[r] = __ldg(pa + 3 * r + t);
-          zb[r] = __ldg(pb + 3 * r + t);
+      for (int k = 0; k < 2 * kSddZ; ++k) {
+        const int z = 32 * k + lane, side = k / kSddZ;  // 288 parts a side, nine rounds of lanes
+        const int p = (z - 32 * kSddZ * side) / kSddZ, part = (z - 32 * kSddZ * side) % kSddZ;
+        const int g = __shfl_sync(0xffffffffu, side ? pr.y : pr.x, p);
+        if (p < n) {
+          const float4* src = reinterpret_cast<const float4*>(a.zdd + kZD * static_cast<int64_t>(g)) + part;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(zs_addr + 16u * z), "l"(src) : "memory");
         }
-#pragma unroll
-        for (int r = 0; r < 6; ++r)
-#pragma unroll
-          for (int c = 0; c < 6; ++c)
-            acc_madd(acc[r * 6 + c], dd_make(za[r].x, za[r].y), dd_make(zb[c].x, zb[c].y));
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      if (lane < n) {
+        const float4* pa = zs + kSddZ * lane;
+        const float4* pb = zs + kSddZ * (32 + lane);
+#pragma unroll 1
+        for (int t = 0; t < 3; ++t) {
+          float2 za[6], zb[6];  // column t of each Z: (hi, lo) of rows 0..5
+#pragma unroll
+          for (int h = 0; h < 3; ++h) {
+            const float4 x = pa[3 * t + h], y = pb[3 * t + h];
+            za[2 * h] = make_float2(x.x, x.y);
+            za[2 * h + 1] = make_float2(x.z, x.w);
+            zb[2 * h] = make_float2(y.x, y.y);
+            zb[2 * h + 1] = make_float2(y.z, y.w);
+          }
+#pragma unroll
+          for (int r = 0; r < 6; ++r)
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+              acc_madd(acc[r * 6 + c], dd_make(za[r].x, za[r].y), dd_make(zb[c].x, zb[c].y));
+        }
+      }
+      __syncwarp();
     }
     // lanes' accumulators summed in float-float: hi parts, then lo parts
     Acc t0 = acc_zero(), t1 = acc_zero();  // entries lane and lane + 32
 #pragma unroll
-    for (int e = 0; e < 36; ++e) red[wib][e][lane] = acc[e].hi;
+    for (int e = 0; e < 36; ++e) red[e][lane] = acc[e].hi;
     __syncwarp();
-    for (int l = 0; l < 32; ++l) acc_addf(t0, red[wib][lane][l]);
+    for (int l = 0; l < 32; ++l) acc_addf(t0, red[lane][l]);
     if (lane < 4)
-      for (int l = 0; l < 32; ++l) acc_addf(t1, red[wib][lane + 32][l]);
+      for (int l = 0; l < 32; ++l) acc_addf(t1, red[lane + 32][l]);
     __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 36; ++e) red[wib][e][lane] = acc[e].lo;
+    for (int e = 0; e < 36; ++e) red[e][lane] = acc[e].lo;
     __syncwarp();
-    for (int l = 0; l < 32; ++l) acc_addf(t0, red[wib][lane][l]);
+    for (int l = 0; l < 32; ++l) acc_addf(t0, red[lane][l]);
     if (lane < 4)
-      for (int l = 0; l < 32; ++l) acc_addf(t1, red[wib][lane + 32][l]);
+      for (int l = 0; l < 32; ++l) acc_addf(t1, red[lane + 32][l]);
     const dd v0 = acc_get(t0);
     a.part[36 * ch + lane] = make_float2(v0.hi, v0.lo);
     if (lane < 4) {
@@ -2012,27 +2067,19 @@ __device__ __forceinline__ void backsub_body(BackArgs a, const Ctrl* ctrl, int b
         if (!use_dd) {
 #pragma unroll
           for (int k = 0; k < 18; ++k) {
-            zr[2 * k] = Z[k];
-            zr[2 * k + 1] = 0.f;
+            zr[zd_at(k / 3, k % 3)] = Z[k];
+            zr[zd_at(k / 3, k % 3) + 1] = 0.f;
           }
         }
       }
-      if (use_dd) {
-        const float4* zp = reinterpret_cast<const float4*>((a.zdd ? a.zdd : a.zdd_flagged) + kZD * g);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          const float4 v = __ldg(zp + k);
-          zr[4 * k] = v.x; zr[4 * k + 1] = v.y; zr[4 * k + 2] = v.z; zr[4 * k + 3] = v.w;
-        }
-      }
-      // entry (r, q) of Z: (zr[6 r + 2 q], zr[6 r + 2 q + 1]) as (hi, lo)
+      if (use_dd) load_zdd((a.zdd ? a.zdd : a.zdd_flagged) + kZD * g, zr);
       const float2* xp = reinterpret_cast<const float2*>(a.xdd) + 6 * fb;
 #pragma unroll
       for (int r = 0; r < 6; ++r) {
         const float2 xv = xp[r];
         const dd x = dd_make(xv.x, xv.y);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) t[q] = dd_add(t[q], dd_mul(x, dd_make(zr[6 * r + 2 * q], zr[6 * r + 2 * q + 1])));
+        for (int q = 0; q < 3; ++q) t[q] = dd_add(t[q], dd_mul(x, dd_make(zr[zd_at(r, q)], zr[zd_at(r, q) + 1])));
       }
       if (gauge) {
         const dd v[3] = {pt_dd(a.pose_v, pj, 0), pt_dd(a.pose_v, pj, 1), pt_dd(a.pose_v, pj, 2)};
@@ -2040,7 +2087,7 @@ __device__ __forceinline__ void backsub_body(BackArgs a, const Ctrl* ctrl, int b
         for (int r = 3; r < 6; ++r)
 #pragma unroll
           for (int q = 0; q < 3; ++q)
-            tg[q] = dd_add(tg[q], dd_mul(v[r - 3], dd_make(zr[6 * r + 2 * q], zr[6 * r + 2 * q + 1])));
+            tg[q] = dd_add(tg[q], dd_mul(v[r - 3], dd_make(zr[zd_at(r, q)], zr[zd_at(r, q) + 1])));
       }
     }
     // float-float sum over the lanes: fixed tree through shared memory
@@ -2141,20 +2188,15 @@ __device__ __forceinline__ void backsub_chunks_body(BackArgs a, const int32_t* c
           use_dd = Z[18] != 0.f && a.zdd_flagged;
         }
         if (use_dd) {
-          const float4* zp = reinterpret_cast<const float4*>((a.zdd ? a.zdd : a.zdd_flagged) + kZD * g);
           float zr[36];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) {
-            const float4 w4 = __ldg(zp + k);
-            zr[4 * k] = w4.x; zr[4 * k + 1] = w4.y; zr[4 * k + 2] = w4.z; zr[4 * k + 3] = w4.w;
-          }
+          load_zdd((a.zdd ? a.zdd : a.zdd_flagged) + kZD * g, zr);
 #pragma unroll
           for (int r = 0; r < 6; ++r) {
             const float2 xv = xp[r];
             const dd x = dd_make(xv.x, xv.y);
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-              const dd z = dd_make(zr[6 * r + 2 * q], zr[6 * r + 2 * q + 1]);
+              const dd z = dd_make(zr[zd_at(r, q)], zr[zd_at(r, q) + 1]);
               tt[q] = dd_add(tt[q], dd_mul(x, z));
               if (gauge && r >= 3) tg[q] = dd_add(tg[q], dd_mul(v[r - 3], z));
             }
@@ -2557,7 +2599,7 @@ __global__ void __launch_bounds__(kIntrCamT) k_intr_cams(IntrArgs a, const Ctrl*
       const float2* zs = reinterpret_cast<const float2*>(a.zk + kIntrZk * static_cast<int64_t>(mb));
 #pragma unroll
       for (int k = 0; k < 18; ++k) {
-        Z[k] = zd ? dd_make(zd[2 * k], zd[2 * k + 1]) : dd_from_float(zf[k]);
+        Z[k] = zd ? dd_make(zd[zd_at(k / 3, k % 3)], zd[zd_at(k / 3, k % 3) + 1]) : dd_from_float(zf[k]);
         zk[k] = dd_make(zs[k].x, zs[k].y);
       }
     }
@@ -3379,6 +3421,10 @@ static int schur_dense_grid(const Sizes& s) {
 // Eight groups a CTA up to this many tiles (one CTA an SM), two beyond.
 constexpr int kSdWide = 304;
 
+int schur_dd_setup() {
+  return raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dd), kSddSmem) == cudaSuccess ? 0 : -1;
+}
+
 int schur_dense_setup() {
   return (raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<8>), schur_dense_smem(8)) == cudaSuccess &&
           raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<2>), schur_dense_smem(2)) == cudaSuccess)
@@ -3394,7 +3440,7 @@ int launch_schur(const Sizes& s, const Dev& d, cudaStream_t st) {
     return 1 + launch_intr_fill(s, d, st);
   }
   const SchurArgs a = make_schur_args(s, d);
-  if (s.lin_dd) k_schur_dd<<<warp_grid(s.nchunk, 8, 65536), 256, 0, st>>>(a, d.ctrl);
+  if (s.lin_dd) k_schur_dd<<<warp_grid(s.nchunk, 8, 65536), 256, kSddSmem, st>>>(a, d.ctrl);
   else k_schur<<<warp_grid(s.nchunk, 8, 65536), 256, 0, st>>>(a, d.ctrl);
   k_schur_reduce<<<warp_grid(s.nsb, 8, 8192), 256, 0, st>>>(a, d.ctrl);
   return 2 + launch_intr_fill(s, d, st);

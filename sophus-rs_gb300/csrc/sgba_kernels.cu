@@ -172,9 +172,23 @@ struct JacF {
   float jp[12];  // row-major 2x6
   float jm[6];   // row-major 2x3
 };
+// A pose's table (16-byte aligned) by 16-byte loads: the lanes of a warp read
+// tables of different poses, a wavefront per lane and load.
+template <int N>
+__device__ __forceinline__ void load16(const float* src, float* v) {
+  const float4* p = reinterpret_cast<const float4*>(src);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const float4 q = p[k];
+    v[4 * k] = q.x; v[4 * k + 1] = q.y; v[4 * k + 2] = q.z; v[4 * k + 3] = q.w;
+  }
+}
+
 template <bool E>  // E: the EUCM camera, else the pinhole
-__device__ __forceinline__ void jacobians_f(const float* pt /*R_cw 9 + t_cw 3*/, float px, float py,
+__device__ __forceinline__ void jacobians_f(const float* pose /*R_cw 9 + t_cw 3*/, float px, float py,
                                             float pz, const CamF& c, JacF* J) {
+  float pt[12];
+  load16<3>(pose, pt);
   float xc = pt[0] * px + pt[1] * py + pt[2] * pz + pt[9];
   float yc = pt[3] * px + pt[4] * py + pt[5] * pz + pt[10];
   float zc = pt[6] * px + pt[7] * py + pt[8] * pz + pt[11];
@@ -262,9 +276,11 @@ struct JacD {
 template <bool E>
 __device__ void jacobians_dd(const float* Pd /*R_cw 9 + t_cw 3, (hi, lo) pairs*/, dd px, dd py, dd pz, const CamD& c,
                              JacD* J) {
+  float P[24];
+  load16<6>(Pd, P);
   dd R[9], t[3];
-  for (int i = 0; i < 9; ++i) R[i] = dd_make(Pd[2 * i], Pd[2 * i + 1]);
-  for (int i = 0; i < 3; ++i) t[i] = dd_make(Pd[18 + 2 * i], Pd[18 + 2 * i + 1]);
+  for (int i = 0; i < 9; ++i) R[i] = dd_make(P[2 * i], P[2 * i + 1]);
+  for (int i = 0; i < 3; ++i) t[i] = dd_make(P[18 + 2 * i], P[18 + 2 * i + 1]);
   dd xc = dd_add(dd_add(dd_add(dd_mul(R[0], px), dd_mul(R[1], py)), dd_mul(R[2], pz)), t[0]);
   dd yc = dd_add(dd_add(dd_add(dd_mul(R[3], px), dd_mul(R[4], py)), dd_mul(R[5], pz)), t[1]);
   dd zc = dd_add(dd_add(dd_add(dd_mul(R[6], px), dd_mul(R[7], py)), dd_mul(R[8], pz)), t[2]);
@@ -437,7 +453,8 @@ __device__ __forceinline__ void cost_body(CostArgs a, const Ctrl* ctrl, int bid_
   dd acc = dd_make(0.0f, 0.0f);
   for (int64_t o = bid_ * static_cast<int64_t>(blockDim.x) + threadIdx.x; o < a.no;
        o += static_cast<int64_t>(nblk_) * blockDim.x) {
-    const float* P = a.pose_dd + 24 * a.opose[o];
+    float P[24];
+    load16<6>(a.pose_dd + 24 * a.opose[o], P);
     const int ip = a.opt[o];
     const dd p0 = pt_dd(a.pts, ip, 0), p1 = pt_dd(a.pts, ip, 1), p2 = pt_dd(a.pts, ip, 2);
     dd xc[3];
@@ -2347,9 +2364,11 @@ struct IntrArgs {
 // The observation's projection Jacobians: J_p, J_m as jacobians_dd and J_k
 // (2x6 row-major, columns nk..5 zero).
 __device__ void intr_term_jacobians(const float* Pd, dd px, dd py, dd pz, const CamD& c, int nk, JacD* J, dd* jk) {
+  float P[24];
+  load16<6>(Pd, P);
   dd R[9], t[3];
-  for (int i = 0; i < 9; ++i) R[i] = dd_make(Pd[2 * i], Pd[2 * i + 1]);
-  for (int i = 0; i < 3; ++i) t[i] = dd_make(Pd[18 + 2 * i], Pd[18 + 2 * i + 1]);
+  for (int i = 0; i < 9; ++i) R[i] = dd_make(P[2 * i], P[2 * i + 1]);
+  for (int i = 0; i < 3; ++i) t[i] = dd_make(P[18 + 2 * i], P[18 + 2 * i + 1]);
   const dd xc = dd_add(dd_add(dd_add(dd_mul(R[0], px), dd_mul(R[1], py)), dd_mul(R[2], pz)), t[0]);
   const dd yc = dd_add(dd_add(dd_add(dd_mul(R[3], px), dd_mul(R[4], py)), dd_mul(R[5], pz)), t[1]);
   const dd zc = dd_add(dd_add(dd_add(dd_mul(R[6], px), dd_mul(R[7], py)), dd_mul(R[8], pz)), t[2]);
@@ -3589,7 +3608,7 @@ __global__ void k_debug_jacobians(int64_t n, const int32_t* __restrict__ cam, co
                                   double* __restrict__ jm) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  float pf[12], pd[24];
+  __align__(16) float pf[12], pd[24];
   pose_table(poses + 7 * static_cast<int64_t>(cam[i]), pf, pd);
   const double* pw = points + 3 * static_cast<int64_t>(pt[i]);
   if (precision == 0) {

@@ -31,11 +31,22 @@ constexpr int kCostMaxBlocks = 1216;  // 8 x 152 SMs
 __device__ __forceinline__ bool halted(const Ctrl* c) { return c->done != 0; }
 __device__ __forceinline__ bool skipping(const Ctrl* c) { return c->done != 0 || c->skip != 0; }
 
-__device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, double v) {
-  // Non-negative doubles order like their bit patterns.
-  if (!(v >= 0.0)) v = (v != v) ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
-  atomicMax(addr, static_cast<unsigned long long>(__double_as_longlong(v)));
-}
+// max |v| by bit patterns: non-negative doubles order like them (a NaN is left
+// out, as fmax does).  An FP64 maximum takes a warp over 200 cycles.
+struct MaxAbs {
+  unsigned long long u = 0ull;
+  __device__ __forceinline__ void add(double v) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+    if (b <= 0x7ff0000000000000ull && b > u) u = b;
+  }
+  __device__ __forceinline__ void warp() {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) u = max(u, __shfl_xor_sync(0xffffffffu, u, off));
+  }
+  __device__ __forceinline__ void to(unsigned long long* addr) const {
+    if (u > *static_cast<volatile unsigned long long*>(addr)) atomicMax(addr, u);
+  }
+};
 
 // HuberKernel (crates/sophus_opt/src/robust_kernel.rs:13-35): weight applied to
 // the residual; H stays J^T J.
@@ -612,7 +623,7 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
   const int wib = threadIdx.x >> 5;
   const int warps_per_block = blockDim.x >> 5;
   const double nu = (a.use_override && !a.nu_ctrl) ? a.nu_override : ctrl->nu;
-  double warp_max = 0.0;  // max |neg_grad| of this warp's points
+  MaxAbs warp_max;  // max |neg_grad| of this warp's points
   const int64_t nitems = a.list ? static_cast<int64_t>(*a.list_count) : static_cast<int64_t>(a.np);
   for (int64_t item = static_cast<int64_t>(bid_) * warps_per_block + wib; item < nitems;
        item += static_cast<int64_t>(nblk_) * warps_per_block) {
@@ -668,7 +679,7 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
       bp[0] = dd_to_double(b[0]);
       bp[1] = dd_to_double(b[1]);
       bp[2] = dd_to_double(b[2]);
-      warp_max = fmax(warp_max, fmax(fabs(bp[0]), fmax(fabs(bp[1]), fabs(bp[2]))));
+      for (int k = 0; k < 3; ++k) warp_max.add(bp[k]);
     }
     // Cholesky V' = C C^T (V layout: 00 01 02 11 12 22).  FP32 when the point
     // block is well conditioned; float-float when a pivot lost more than three
@@ -741,7 +752,8 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
         bp[0] = dd_to_double(b[0]);
         bp[1] = dd_to_double(b[1]);
         bp[2] = dd_to_double(b[2]);
-        if (a.force_dd) warp_max = fmax(warp_max, fmax(fabs(bp[0]), fmax(fabs(bp[1]), fabs(bp[2]))));
+        if (a.force_dd)
+          for (int k = 0; k < 3; ++k) warp_max.add(bp[k]);
       }
     }
     dd I[6];  // C^-1 (00 10 11 20 21 22)
@@ -861,13 +873,13 @@ __device__ __forceinline__ void landmark_body(LinArgs a, Ctrl* ctrl, int bid_, i
       for (int q = 0; q < 5; ++q) dst[q] = make_float4(Z[4 * q], Z[4 * q + 1], Z[4 * q + 2], Z[4 * q + 3]);
     }
   }
-  __shared__ double s_max[8];
-  if (lane == 0) s_max[wib] = warp_max;
+  __shared__ unsigned long long s_max[8];
+  if (lane == 0) s_max[wib] = warp_max.u;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int q = 0; q < warps_per_block; ++q) m = fmax(m, s_max[q]);
-    atomic_max_nonneg(&ctrl->max_grad_bits, m);
+    MaxAbs m;
+    for (int q = 0; q < warps_per_block; ++q) m.u = max(m.u, s_max[q]);
+    m.to(&ctrl->max_grad_bits);
   }
 }
 template <bool E>
@@ -894,10 +906,10 @@ __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int 
   __shared__ float sci[kLmkTerms][6];   // C^-1 per point of the chunk (FP32)
   __shared__ float2 ssum[kLmkTerms][9]; // per point: the 9 sums over its terms (float-float)
   __shared__ unsigned char sok[kLmkTerms];
-  __shared__ double smax[8];
+  __shared__ unsigned long long smax[8];
   const int tid = threadIdx.x;
   const double nu = ctrl->nu;
-  double tmax = 0.0;
+  MaxAbs tmax;
   for (int c = bid_; c < a.nchunk; c += nblk_) {
     const int p0 = a.chunk_pt[c], p1 = a.chunk_pt[c + 1];
     const int64_t t0 = a.pt_g_begin[p0];
@@ -963,7 +975,7 @@ __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int 
       bp[0] = dd_to_double(b[0]);
       bp[1] = dd_to_double(b[1]);
       bp[2] = dd_to_double(b[2]);
-      tmax = fmax(tmax, fmax(fabs(bp[0]), fmax(fabs(bp[1]), fabs(bp[2]))));
+      for (int k = 0; k < 3; ++k) tmax.add(bp[k]);
       float V[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) V[k] = acc[k].hi + acc[k].lo;
@@ -1042,13 +1054,13 @@ __device__ __forceinline__ void landmark_chunks_body(LinArgs a, Ctrl* ctrl, int 
     __syncthreads();
   }
   // max |neg_grad| over the block
-  for (int off = 16; off > 0; off >>= 1) tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
-  if ((tid & 31) == 0) smax[tid >> 5] = tmax;
+  tmax.warp();
+  if ((tid & 31) == 0) smax[tid >> 5] = tmax.u;
   __syncthreads();
   if (tid == 0) {
-    double m = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) m = fmax(m, smax[q]);
-    atomic_max_nonneg(&ctrl->max_grad_bits, m);
+    MaxAbs m;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) m.u = max(m.u, smax[q]);
+    m.to(&ctrl->max_grad_bits);
   }
 }
 template <bool E>
@@ -1078,10 +1090,10 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
   __shared__ float sci[kLmkTerms][12];         // C^-1 of each point of the chunk (float-float)
   __shared__ float2 ssum[kLmkTerms][9];        // per point: the 9 sums over its terms
   __shared__ unsigned char sok[kLmkTerms];
-  __shared__ double smax[8];
+  __shared__ unsigned long long smax[8];
   const int tid = threadIdx.x;
   const double nu = ctrl->nu;
-  double tmax = 0.0;
+  MaxAbs tmax;
   for (int c = blockIdx.x; c < a.nchunk; c += gridDim.x) {
     const int p0 = a.chunk_pt[c], p1 = a.chunk_pt[c + 1];
     const int64_t t0 = a.pt_g_begin[p0];
@@ -1157,7 +1169,7 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
       bp[0] = dd_to_double(b[0]);
       bp[1] = dd_to_double(b[1]);
       bp[2] = dd_to_double(b[2]);
-      tmax = fmax(tmax, fmax(fabs(bp[0]), fmax(fabs(bp[1]), fabs(bp[2]))));
+      for (int k = 0; k < 3; ++k) tmax.add(bp[k]);
       bool ok = Vd[0].hi > 0.0f;
       const dd e00 = dd_sqrt(Vd[0]);
       const dd e10 = dd_div(Vd[1], e00), e20 = dd_div(Vd[2], e00);
@@ -1249,13 +1261,13 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
     }
     __syncthreads();
   }
-  for (int off = 16; off > 0; off >>= 1) tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
-  if ((tid & 31) == 0) smax[tid >> 5] = tmax;
+  tmax.warp();
+  if ((tid & 31) == 0) smax[tid >> 5] = tmax.u;
   __syncthreads();
   if (tid == 0) {
-    double m = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) m = fmax(m, smax[q]);
-    atomic_max_nonneg(&ctrl->max_grad_bits, m);
+    MaxAbs m;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) m.u = max(m.u, smax[q]);
+    m.to(&ctrl->max_grad_bits);
   }
 }
 
@@ -1558,9 +1570,9 @@ __device__ __forceinline__ void camera_finalize_body(int nf, const int64_t* fb_t
     if (with_schur) rb[6 * fb + k] = vals[27 + k];
   }
   if (k == 0) {
-    double mg = 0.0;
-    for (int p = 0; p < 6; ++p) mg = fmax(mg, fabs(vals[21 + p]));
-    atomic_max_nonneg(&ctrl->max_grad_bits, mg);
+    MaxAbs mg;
+    for (int p = 0; p < 6; ++p) mg.add(vals[21 + p]);
+    mg.to(&ctrl->max_grad_bits);
   }
   if (with_schur) {
     // the last block to finish: gradient-tolerance check before the solve
@@ -2585,9 +2597,9 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
     a.isum[kIntrPart + k] = -gk;
   }
   if (k == 0) {
-    double mg = 0.0;
-    for (int t = 0; t < kK; ++t) mg = fmax(mg, fabs(s_tot[0][kKT + t]));
-    atomic_max_nonneg(&ctrl->max_grad_bits, mg);
+    MaxAbs mg;
+    for (int t = 0; t < kK; ++t) mg.add(s_tot[0][kKT + t]);
+    mg.to(&ctrl->max_grad_bits);
     *a.ticket = 0;
   }
 }
@@ -2924,12 +2936,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
     return;
   }
   dd sdd = dd_make(0.f, 0.f), sdg = dd_make(0.f, 0.f);
-  // max |step| by bit patterns: non-negative doubles order like them (NaN left out)
-  unsigned long long mx = 0ull;
-  auto step_max = [&](double v) {
-    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
-    if (u <= 0x7ff0000000000000ull && u > mx) mx = u;
-  };
+  MaxAbs mx;
   if (a.intr_free && bid_ == 0 && threadIdx.x == 0) {
     // the intrinsics are a vector space: k + dx_k (no gauge component)
     for (int k = 0; k < a.intr_nk; ++k) {
@@ -2938,7 +2945,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
       const dd x = dd_from_double(xk);
       sdd = dd_add(sdd, dd_mul(x, x));
       sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bk[k])));
-      step_max(xk);
+      mx.add(xk);
     }
     cam_table(a.intr_t, a.cam);
   }
@@ -2960,7 +2967,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
         dd x = dd_from_double(xi[k]);
         sdd = dd_add(sdd, dd_mul(x, x));
         sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bf[6 * fb + k])));
-        step_max(xi[k]);
+        mx.add(xi[k]);
       }
     } else {
       const int i = static_cast<int>(t - a.nc);
@@ -2982,7 +2989,7 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
         dd x = dd_from_double(d[k]);
         sdd = dd_add(sdd, dd_mul(x, x));
         sdg = dd_add(sdg, dd_mul(x, dd_from_double(a.bm[3 * mb + k])));
-        step_max(d[k]);
+        mx.add(d[k]);
         O[k] = p[k] + d[k];
         const dd o = dd_from_double(O[k]);
         a.pts[3 * static_cast<int64_t>(i) + k] = make_float2(o.hi, o.lo);
@@ -2993,25 +3000,24 @@ __device__ __forceinline__ void apply_update_body(UpdArgs a, Ctrl* ctrl, int bid
   __shared__ unsigned long long shm[8];
   sdd = dd_warp_sum(sdd);
   sdg = dd_warp_sum(sdg);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  mx.warp();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) {
     sh[0][w] = sdd.hi; sh[1][w] = sdd.lo; sh[2][w] = sdg.hi; sh[3][w] = sdg.lo;
-    shm[w] = mx;
+    shm[w] = mx.u;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     dd s0 = dd_make(0.f, 0.f), s1 = dd_make(0.f, 0.f);
-    unsigned long long m = 0ull;
+    MaxAbs m;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
       s0 = dd_add(s0, dd_make(sh[0][q], sh[1][q]));
       s1 = dd_add(s1, dd_make(sh[2][q], sh[3][q]));
-      m = max(m, shm[q]);
+      m.u = max(m.u, shm[q]);
     }
     a.part[2 * bid_] = dd_to_double(s0);
     a.part[2 * bid_ + 1] = dd_to_double(s1);
-    atomicMax(&ctrl->max_step_bits, m);
+    m.to(&ctrl->max_step_bits);
   }
 }
 __global__ void __launch_bounds__(256) k_apply_update(UpdArgs a, Ctrl* ctrl) {

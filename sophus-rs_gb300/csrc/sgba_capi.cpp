@@ -1176,6 +1176,10 @@ int enqueue_iteration(sgba_problem* p, cudaStream_t st) {
 
 int ensure_graph(sgba_problem* p) {
   if (p->graph_exec) return SGBA_OK;
+  if (const size_t rounds = p->d.sd_rounds ? 0 : sgba::schur_split_floats(p->sz)) {
+    // without it the tiled Schur pass is not split (the same S, slower)
+    if (dev_alloc(p, &p->d.sd_rounds, rounds) != SGBA_OK) p->d.sd_rounds = nullptr;
+  }
   SGBA_CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
   int n = enqueue_iteration(p, p->stream);
   cudaGraph_t g = nullptr;

@@ -266,6 +266,7 @@ struct Dev {
   float* A = nullptr;              // n6*n6 FP32 factor (lower: unit L)
   float* dpiv = nullptr;           // n6 pivots
   float* wpanel = nullptr;         // n6*64 panel scratch (A_ip L^-T)
+  float* sd_rounds = nullptr;      // sums of the tiled Schur pass per round (schur_split_floats), single problems
   double* x = nullptr;             // n6 solution / refinement
   double* x0 = nullptr;            // 6 nf: x before the gauge projection
   float* xdd = nullptr;            // n6*2: solution as float-float pairs
@@ -431,6 +432,7 @@ int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st);
 int cost_partials_needed(const Sizes& s);  // reduction partial slots
 int landmark_setup(int cap);
 size_t intr_part_count(const Sizes& s);  // partial sums of the free intrinsics (float2)
+size_t schur_split_floats(const Sizes& s);  // Dev::sd_rounds of the tiled Schur pass of few tiles (0: not split)
 int schur_dd_setup();     // of the float-float Schur pass
 int schur_dense_setup();  // shared memory limits of the tiled Schur pass (0: ok)  // dynamic shared memory of the chunked landmark pass (0 = ok)
 int landmark_dd_setup(int cap);  // the same for its float-float variant (0 = ok)

@@ -1922,6 +1922,8 @@ struct SchurDenseArgs {
   const double* cnt_f;
   double* S;
   float2* S2;
+  float* rounds;  // split pass: the sums of every round of every tile
+  int nsplit;     // split pass: CTAs of a tile
 };
 
 constexpr size_t schur_dense_smem(int G) {
@@ -1938,7 +1940,44 @@ __device__ __forceinline__ void sd_load18(const float* src, float* v) {
   v[16] = w.x; v[17] = w.y;
 }
 
-template <int G>
+// The tile (ti, tj), tj <= ti, of the lower triangle.
+__device__ __forceinline__ void schur_dense_tile(int tile, int* ti, int* tj) {
+  int i = static_cast<int>((sqrtf(8.0f * static_cast<float>(tile) + 1.0f) - 1.0f) * 0.5f);
+  while (i * (i + 1) / 2 > tile) --i;
+  while ((i + 1) * (i + 2) / 2 <= tile) ++i;
+  *ti = i;
+  *tj = tile - i * (i + 1) / 2;
+}
+
+// Entry e of the tile's sums (36 entries of 64 blocks) into S.
+__device__ __forceinline__ void schur_dense_store(const SchurDenseArgs& a, double nu, int I0, int J0, int e,
+                                                  const Acc& sum) {
+  const int b = e % kSdGroup, r = (e / kSdGroup) / 6, cc = (e / kSdGroup) % 6;
+  const int bj = I0 + (b >> 3), bk = J0 + (b & 7);
+  const int row = 6 * bj + r, col = 6 * bk + cc;
+  if (row >= a.n6 || col >= a.n6 || col > row) return;
+  const dd tt = acc_get(sum);
+  dd vd;
+  if (bj == bk) {
+    dd base = dd_from_double(a.ufull[36 * bj + r * 6 + cc]);
+    if (r == cc) base = dd_add(base, dd_from_double(nu * a.cnt_f[bj]));
+    vd = dd_sub(base, tt);
+  } else {
+    vd = dd_neg(tt);
+  }
+  const double w = dd_to_double(vd);
+  a.S[static_cast<int64_t>(row) * a.n6 + col] = w;
+  a.S[static_cast<int64_t>(col) * a.n6 + row] = w;
+  if (a.S2) {
+    a.S2[static_cast<int64_t>(row) * a.n6 + col] = make_float2(vd.hi, vd.lo);
+    a.S2[static_cast<int64_t>(col) * a.n6 + row] = make_float2(vd.hi, vd.lo);
+  }
+}
+
+// SPLIT: a.nsplit CTAs of a tile take ranges of its rounds and leave each
+// round's sums in a.rounds; k_schur_dense_sum adds them in the order of the
+// rounds, so S keeps its bits.
+template <int G, bool SPLIT = false>
 __device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const Ctrl* ctrl, int bid_) {
   if (skipping(ctrl)) return;
   extern __shared__ __align__(16) float zs[];  // kSdBufs x G x kSdStage x 16 records, then G x kSdEntries sums
@@ -1946,23 +1985,23 @@ __device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const 
   constexpr int kStages = kSdPts / kSdStage;   // stages per round
   constexpr int kPer = (kSdEntries + kSdGroup * G - 1) / (kSdGroup * G);
   float* sums = zs + kSdBufs * G * kStageFloats;
-  // tile (ti, tj), tj <= ti, of the lower triangle
-  int ti = static_cast<int>((sqrtf(8.0f * static_cast<float>(bid_) + 1.0f) - 1.0f) * 0.5f);
-  while (ti * (ti + 1) / 2 > bid_) --ti;
-  while ((ti + 1) * (ti + 2) / 2 <= bid_) ++ti;
-  const int tj = bid_ - ti * (ti + 1) / 2;
+  const int tile = SPLIT ? bid_ / a.nsplit : bid_, part = SPLIT ? bid_ % a.nsplit : 0;
+  int ti, tj;
+  schur_dense_tile(tile, &ti, &tj);
   const int I0 = ti * kSdB, J0 = tj * kSdB;
   const int tid = threadIdx.x, grp = tid / kSdGroup, t = tid % kSdGroup;
   const bool diag = ti == tj;  // one set of records
   const int nround = (a.np + kSdPts - 1) / kSdPts;
   const int nsuper = (nround + G - 1) / G;
-  const int nstage = nsuper * kStages;  // of every group (rounds past the end copy zeros)
+  const int super0 = SPLIT ? static_cast<int>(static_cast<int64_t>(nsuper) * part / a.nsplit) : 0;
+  const int super1 = SPLIT ? static_cast<int>(static_cast<int64_t>(nsuper) * (part + 1) / a.nsplit) : nsuper;
+  const int nstage = (super1 - super0) * kStages;  // of every group (rounds past the end copy zeros)
   // this thread's record of a stage: point pp, slot (0..7 row poses, 8..15 column poses)
   const int pp = t >> 4, slot = t & 15;
   const int f = slot < kSdB ? I0 + slot : J0 + slot - kSdB;
   const bool mine = (slot < kSdB || !diag) && f < a.nf;
   auto term_of = [&](int s) {
-    const int i = ((s / kStages) * G + grp) * kSdPts + (s % kStages) * kSdStage + pp;
+    const int i = ((super0 + s / kStages) * G + grp) * kSdPts + (s % kStages) * kSdStage + pp;
     return (mine && s < nstage && i < a.np) ? __ldg(a.zterm + static_cast<int64_t>(i) * a.nf + f) : -1;
   };
   auto copy = [&](int s, int g) {
@@ -2009,7 +2048,15 @@ __device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const 
           acc[6 * r + c] = w;
         }
     }
-    if (s % kStages == kStages - 1) {  // the round is complete
+    if (SPLIT && s % kStages == kStages - 1) {
+      const int round = (super0 + s / kStages) * G + grp;
+      float* out = a.rounds + (static_cast<int64_t>(tile) * nround + round) * kSdEntries + t;
+#pragma unroll
+      for (int e = 0; e < 36; ++e) {
+        if (round < nround) out[e * kSdGroup] = acc[e];
+        acc[e] = 0.0f;
+      }
+    } else if (!SPLIT && s % kStages == kStages - 1) {  // the round is complete
 #pragma unroll
       for (int e = 0; e < 36; ++e) {
         sums[grp * kSdEntries + e * kSdGroup + t] = acc[e];
@@ -2027,36 +2074,36 @@ __device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const 
     }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (SPLIT) return;
   const double nu = ctrl->nu;
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int e = tid + u * kSdGroup * G;
-    if (e >= kSdEntries) continue;
-    const int b = e % kSdGroup, r = (e / kSdGroup) / 6, cc = (e / kSdGroup) % 6;
-    const int bj = I0 + (b >> 3), bk = J0 + (b & 7);
-    const int row = 6 * bj + r, col = 6 * bk + cc;
-    if (row >= a.n6 || col >= a.n6 || col > row) continue;
-    const dd tt = acc_get(accd[u]);
-    dd vd;
-    if (bj == bk) {
-      dd base = dd_from_double(a.ufull[36 * bj + r * 6 + cc]);
-      if (r == cc) base = dd_add(base, dd_from_double(nu * a.cnt_f[bj]));
-      vd = dd_sub(base, tt);
-    } else {
-      vd = dd_neg(tt);
-    }
-    const double w = dd_to_double(vd);
-    a.S[static_cast<int64_t>(row) * a.n6 + col] = w;
-    a.S[static_cast<int64_t>(col) * a.n6 + row] = w;
-    if (a.S2) {
-      a.S2[static_cast<int64_t>(row) * a.n6 + col] = make_float2(vd.hi, vd.lo);
-      a.S2[static_cast<int64_t>(col) * a.n6 + row] = make_float2(vd.hi, vd.lo);
-    }
+    if (e < kSdEntries) schur_dense_store(a, nu, I0, J0, e, accd[u]);
   }
 }
 template <int G>
 __global__ void __launch_bounds__(kSdGroup * G, G > 2 ? 1 : 4) k_schur_dense(SchurDenseArgs a, const Ctrl* ctrl) {
   schur_dense_body<G>(a, ctrl, blockIdx.x);
+}
+__global__ void __launch_bounds__(kSdGroup * 2, 4) k_schur_dense_split(SchurDenseArgs a, const Ctrl* ctrl) {
+  schur_dense_body<2, true>(a, ctrl, blockIdx.x);
+}
+// The rounds of a tile added in order, a thread per entry.
+constexpr int kSdSumT = 128;
+static_assert(kSdEntries % kSdSumT == 0, "whole CTAs");
+__global__ void __launch_bounds__(kSdSumT) k_schur_dense_sum(SchurDenseArgs a, const Ctrl* ctrl) {
+  if (skipping(ctrl)) return;
+  constexpr int kPerTile = kSdEntries / kSdSumT;
+  const int tile = blockIdx.x / kPerTile, e = (blockIdx.x % kPerTile) * kSdSumT + threadIdx.x;
+  int ti, tj;
+  schur_dense_tile(tile, &ti, &tj);
+  const int nround = (a.np + kSdPts - 1) / kSdPts;
+  const float* src = a.rounds + static_cast<int64_t>(tile) * nround * kSdEntries + e;
+  Acc sum = acc_zero();
+#pragma unroll 16
+  for (int r = 0; r < nround; ++r) acc_addf(sum, src[static_cast<int64_t>(r) * kSdEntries]);
+  schur_dense_store(a, ctrl->nu, ti * kSdB, tj * kSdB, e, sum);
 }
 
 // ---------------------------------------------------------------------------
@@ -3472,12 +3519,24 @@ static SchurDenseArgs make_schur_dense_args(const Sizes& s, const Dev& d) {
   a.cnt_f = d.cnt_f;
   a.S = d.S;
   a.S2 = d.S2;
+  a.rounds = d.sd_rounds;
+  a.nsplit = 1;
   return a;
 }
 
 static int schur_dense_grid(const Sizes& s) {
   const int nb = (s.nf + kSdB - 1) / kSdB;
   return nb * (nb + 1) / 2;
+}
+
+// Few tiles leave most SMs idle (a tile's rounds are 0.5 us each, eight at a
+// time): up to half an SM count of tiles the rounds are spread over ~608 CTAs
+// and summed by a second launch, where their sums fit in 64 MB (10 cameras and
+// 1,000 points: 35 -> 8 us).  0 floats: not split.
+size_t schur_split_floats(const Sizes& s) {
+  if (!s.schur_dense || schur_dense_grid(s) > 76) return 0;
+  const size_t f = static_cast<size_t>(schur_dense_grid(s)) * ((s.np + kSdPts - 1) / kSdPts) * kSdEntries;
+  return f * sizeof(float) <= (64u << 20) ? f : 0;
 }
 
 // Eight groups a CTA up to this many tiles (one CTA an SM), two beyond.
@@ -3489,7 +3548,8 @@ int schur_dd_setup() {
 
 int schur_dense_setup() {
   return (raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<8>), schur_dense_smem(8)) == cudaSuccess &&
-          raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<2>), schur_dense_smem(2)) == cudaSuccess)
+          raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense<2>), schur_dense_smem(2)) == cudaSuccess &&
+          raise_dynamic_smem(reinterpret_cast<const void*>(k_schur_dense_split), schur_dense_smem(2)) == cudaSuccess)
              ? 0
              : -1;
 }
@@ -3497,6 +3557,14 @@ int schur_dense_setup() {
 int launch_schur(const Sizes& s, const Dev& d, cudaStream_t st) {
   if (s.schur_dense) {
     const int grid = schur_dense_grid(s);
+    if (d.sd_rounds) {
+      SchurDenseArgs a = make_schur_dense_args(s, d);
+      const int nsuper = (s.np + 2 * kSdPts - 1) / (2 * kSdPts);
+      a.nsplit = std::max(1, std::min(nsuper, 608 / grid));
+      k_schur_dense_split<<<grid * a.nsplit, kSdGroup * 2, schur_dense_smem(2), st>>>(a, d.ctrl);
+      k_schur_dense_sum<<<grid * (kSdEntries / kSdSumT), kSdSumT, 0, st>>>(a, d.ctrl);
+      return 2 + launch_intr_fill(s, d, st);
+    }
     if (grid <= kSdWide) k_schur_dense<8><<<grid, kSdGroup * 8, schur_dense_smem(8), st>>>(make_schur_dense_args(s, d), d.ctrl);
     else k_schur_dense<2><<<grid, kSdGroup * 2, schur_dense_smem(2), st>>>(make_schur_dense_args(s, d), d.ctrl);
     return 1 + launch_intr_fill(s, d, st);

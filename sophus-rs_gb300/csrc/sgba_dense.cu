@@ -985,42 +985,41 @@ __device__ __forceinline__ dd sd_rcp(dd d) {
 // the panel width and the tiles do not change a result's bits.
 __device__ __forceinline__ dd sd_msub(dd a, dd x, dd y) { return dd_sub(a, dd_mul(x, y)); }
 
-// One warp, every lane the same: LDL^T of the 6 x 6 diagonal block at c0 in
-// registers.  U below the diagonal back to A, 1/d to rdv.  Returns whether a
-// pivot was not finite.
-__device__ __forceinline__ bool sd_diag6(float2* A, float2* rdv, int c0, int lane) {
-  dd d[6][6], r[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int q = 0; q <= i; ++q) d[i][q] = sd_f2dd(A[sd_at(c0 + i, c0 + q)]);
+// One warp: LDL^T of the 6 x 6 diagonal block at c0, lane i (i + 1) / 2 + q with
+// entry (i, q) = v (lanes 0 .. 20), the pivot's column by shuffles.  (Every lane
+// with the whole block is a thousand instructions a block, cold in a CTA that
+// runs them nine times: 43 -> 34 us a 54-row solve.)  U below the diagonal to A,
+// 1/d to rdv.  Returns whether a pivot was not finite.
+__device__ __forceinline__ void sd_entry(int lane, int* i, int* q) {
+  *i = lane >= 15 ? 5 : lane >= 10 ? 4 : lane >= 6 ? 3 : lane >= 3 ? 2 : lane >= 1 ? 1 : 0;
+  *q = lane - *i * (*i + 1) / 2;
+}
+__device__ __forceinline__ dd sd_shfl(dd v, int lane) {
+  return dd_make(__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane));
+}
+__device__ __forceinline__ bool sd_diag6(float2* A, float2* rdv, int c0, int lane, dd v) {
+  int i, q;
+  sd_entry(min(lane, 20), &i, &q);
   float maxp = 1.0f;  // running maximum pivot of the pose block (>= 1)
   bool bad = false;
-#pragma unroll
+  dd mine = dd_make(0.0f, 0.0f);  // lane t: 1/d_t
+#pragma unroll 1
   for (int t = 0; t < 6; ++t) {
-    const float ad = fabsf(d[t][t].hi);
+    const dd p = sd_shfl(v, t * (t + 1) / 2 + t);
+    const dd it = sd_shfl(v, i * (i + 1) / 2 + min(t, i)), qt = sd_shfl(v, q * (q + 1) / 2 + min(t, q));
+    const float ad = fabsf(p.hi);
     const bool fin = ad <= 3.402823466e38f;
     const bool zero = !fin || !(ad > maxp * kTolRel);
     bad = bad || !fin;
     maxp = zero ? maxp : fmaxf(maxp, ad);
-    const dd rc = sd_rcp(d[t][t]);
-    r[t] = zero ? dd_make(0.0f, 0.0f) : rc;
-#pragma unroll
-    for (int i = t + 1; i < 6; ++i) {
-      const dd l = dd_mul(d[i][t], r[t]);
-#pragma unroll
-      for (int q = t + 1; q <= i; ++q) d[i][q] = sd_msub(d[i][q], l, d[q][t]);
-    }
+    const dd rc = sd_rcp(p);
+    const dd r = zero ? dd_make(0.0f, 0.0f) : rc;
+    if (lane == t) mine = r;
+    const dd nv = sd_msub(v, dd_mul(it, r), qt);
+    if (q > t) v = nv;  // then i >= q > t too
   }
-  __syncwarp();  // every lane has read the block
-  if (lane == 0) {
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      rdv[c0 + t] = sd_dd2f(r[t]);
-#pragma unroll
-      for (int q = 0; q < t; ++q) A[sd_at(c0 + t, c0 + q)] = sd_dd2f(d[t][q]);
-    }
-  }
+  if (lane < 21 && q < i) A[sd_at(c0 + i, c0 + q)] = sd_dd2f(v);
+  if (lane < 6) rdv[c0 + lane] = sd_dd2f(mine);
   return bad;
 }
 
@@ -1124,7 +1123,11 @@ __device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl) {
   __syncthreads();
   if (tid < ne && a.eq_fb[tid] >= 0)
     for (int i = 0; i < 3; ++i) yg[tid * m + 6 * a.eq_fb[tid] + 3 + i] = sd_dd2f(dd_from_double(a.eq_jac[3 * tid + i]));
-  if (warp == 0 && sd_diag6(A, rdv, 0, lane)) s_bad = 1;
+  if (warp == 0) {
+    int i, q;
+    sd_entry(min(lane, 20), &i, &q);
+    if (sd_diag6(A, rdv, 0, lane, sd_f2dd(A[sd_at(i, q)]))) s_bad = 1;
+  }
   for (int c0 = 0; c0 < m; c0 += 6) {
     const int c1 = c0 + 6, buf = (c0 / 6) & 1;
     __syncthreads();  // the diagonal block of this panel is factored, the previous panel's tiles are done
@@ -1160,18 +1163,14 @@ __device__ __forceinline__ void small_dense_body(DenseArgs a, Ctrl* ctrl) {
     __syncthreads();
     if (c1 >= m) break;
     if (warp == 0) {  // look-ahead: the next diagonal block
-      if (lane < 21) {
-        const int i = lane >= 15 ? 5 : lane >= 10 ? 4 : lane >= 6 ? 3 : lane >= 3 ? 2 : lane >= 1 ? 1 : 0;
-        const int q = lane - i * (i + 1) / 2;
-        const float2* ri = A + sd_at(c1 + i, c0);
-        const float2* rq = A + sd_at(c1 + q, c0);
-        dd acc = sd_f2dd(A[sd_at(c1 + i, c1 + q)]);
+      int i, q;
+      sd_entry(min(lane, 20), &i, &q);
+      const float2* ri = A + sd_at(c1 + i, c0);
+      const float2* rq = A + sd_at(c1 + q, c0);
+      dd acc = sd_f2dd(A[sd_at(c1 + i, c1 + q)]);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) acc = sd_msub(acc, dd_mul(sd_f2dd(ri[k]), rd[k]), sd_f2dd(rq[k]));
-        A[sd_at(c1 + i, c1 + q)] = sd_dd2f(acc);
-      }
-      __syncwarp();
-      if (sd_diag6(A, rdv, c1, lane)) s_bad = 1;
+      for (int k = 0; k < 6; ++k) acc = sd_msub(acc, dd_mul(sd_f2dd(ri[k]), rd[k]), sd_f2dd(rq[k]));
+      if (sd_diag6(A, rdv, c1, lane, acc)) s_bad = 1;
     }
     // the rhs and the equality columns (the last threads: warp 0 is busy)
     for (int e = 0; e <= ne; ++e) {

@@ -112,7 +112,8 @@ struct EventSet {
 };
 
 constexpr int kTile = 256;           // terms per camera tile (one CTA)
-constexpr int64_t kSchurChunk = 256;  // observation pairs per warp in the Schur assembly
+constexpr int64_t kSchurChunk = 256;  // observation pairs per warp in the Schur assembly (at most)
+constexpr int64_t kSchurWarps = 152 * 16;  // warps of the assembly that run at once
 constexpr int32_t kMaxDenseFree = 4096;  // reduced-camera-system limit (6 * 4096 rows, stored dense in f64)
 
 }  // namespace
@@ -782,14 +783,22 @@ int build_schur_pattern(sgba_problem* p) {
   if (tiled) return dev_alloc(p, &d.pairs, 0);
   if (npairs >= (int64_t(1) << 31))
     return set_error(SGBA_ERR_UNSUPPORTED, "%lld observation pairs exceed the 2^31 limit", (long long)npairs);
-  // chunks of at most kSchurChunk pairs within one block (at least one per block)
+  // Chunks of at most kSchurChunk pairs within one block (at least one per
+  // block).  The EUCM camera and pose-graph edges, which come with float-float
+  // sums, take shorter ones where 256 would leave warps idle (a warp's 256
+  // pairs are eight rounds in series: 27 us of 27,000 pairs, 7 with 32 a
+  // warp); FP32 partial sums keep their partition, and so their rounding.
+  const int64_t chunk =
+      p->camera_model == SGBA_CAMERA_PINHOLE && P.eterm_fm.empty()
+          ? kSchurChunk
+          : std::min(kSchurChunk, std::max<int64_t>(32, (npairs / kSchurWarps + 31) / 32 * 32));
   P.block_chunk_begin.assign(nb + 1, 0);
   for (int64_t b = 0; b < nb; ++b) {
     P.block_chunk_begin[b] = static_cast<int32_t>(P.chunk_begin.size());
     int64_t q = P.sb_pair_begin[b];
     do {
       P.chunk_begin.push_back(q);
-      q += kSchurChunk;
+      q += chunk;
     } while (q < P.sb_pair_begin[b + 1]);
   }
   P.block_chunk_begin[nb] = static_cast<int32_t>(P.chunk_begin.size());

@@ -604,26 +604,6 @@ __device__ void gather_x(const Ctx& X, cg::cluster_group& cl) {
   __syncthreads();
 }
 
-// Sum over one warp through shared memory (fixed tree, no shuffles).
-__device__ dd warp_sum_dd(dd v, float* wred, int lane) {
-  wred[2 * lane] = v.hi;
-  wred[2 * lane + 1] = v.lo;
-  __syncwarp();
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    if (lane < s) {
-      const dd u = dd_add(dd_make(wred[2 * lane], wred[2 * lane + 1]),
-                          dd_make(wred[2 * (lane + s)], wred[2 * (lane + s) + 1]));
-      wred[2 * lane] = u.hi;
-      wred[2 * lane + 1] = u.lo;
-    }
-    __syncwarp();
-  }
-  const dd r = dd_make(wred[0], wred[1]);
-  __syncwarp();
-  return r;
-}
-
 // Sum over the CTA through shared memory (fixed tree); every thread gets it.
 __device__ dd block_sum_dd(dd v, float* red) {
   const int tid = threadIdx.x;
@@ -652,7 +632,6 @@ __device__ void residual(const Ctx& X, const DenseArgs& a, float alpha) {
   const float* vd = X.sm + X.cv->vdef;
   const float* ud = X.sm + X.cv->udef;
   float* bl = X.sm + X.cv->bl;
-  float* wred = X.sm + X.cv->red + 64 * warp;
   // deflated operator (retry after a breakdown): subtract alpha u (u . x~), x~ = D^1/2 x
   dd g = dd_make(0.f, 0.f);
   if (alpha != 0.0f) {
@@ -660,34 +639,54 @@ __device__ void residual(const Ctx& X, const DenseArgs& a, float alpha) {
     g = block_sum_dd(g, X.sm + X.cv->red);
   }
   const dd ag = dd_mul_f(g, alpha);
+  // kResRows rows of a warp at a time, so that their loads and their float-float
+  // chains (a lane's entries of a row in order) run beside one another: a row at
+  // a time took 36,000 cycles a residual of 594 rows on 16 CTAs; 412 -> 401 us a
+  // solve so.
+  constexpr int kResRows = kNB / kWarps;
+  static_assert(kNB % kWarps == 0, "whole rows per warp");
   for (int jr = 0; jr < X.cv->nown; ++jr) {
-    const int r = X.rank + jr * X.C;
-    for (int i = warp; i < kNB; i += kWarps) {
-      const int row = kNB * r + i;
+    const int row0 = kNB * (X.rank + jr * X.C) + warp;
+    dd acc[kResRows];
+#pragma unroll
+    for (int t = 0; t < kResRows; ++t) acc[t] = dd_make(0.f, 0.f);
+    for (int k0 = lane; k0 < a.n; k0 += 32 * 4) {
+      float2 sv[kResRows][4];
+#pragma unroll
+      for (int t = 0; t < kResRows; ++t) {
+        const int row = row0 + kWarps * t;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = k0 + 32 * u;
+          sv[t][u] = (row < a.n && k < a.n) ? a.S2[static_cast<int64_t>(row) * a.n + k] : make_float2(0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = k0 + 32 * u;
+        if (k >= a.n) break;
+        const dd x = dd_make(xh[k], xl[k]);
+#pragma unroll
+        for (int t = 0; t < kResRows; ++t) acc[t] = dd_add(acc[t], dd_mul(dd_make(sv[t][u].x, sv[t][u].y), x));
+      }
+    }
+    // lane l takes lane l + off: lane 0 ends with the sum of a fixed tree
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int t = 0; t < kResRows; ++t)
+        acc[t] = dd_add(acc[t], dd_make(__shfl_down_sync(0xffffffffu, acc[t].hi, off), __shfl_down_sync(0xffffffffu, acc[t].lo, off)));
+#pragma unroll
+    for (int t = 0; t < kResRows; ++t) {
+      const int row = row0 + kWarps * t;
+      const dd sum = acc[t];
+      if (lane != 0) continue;
       if (row >= a.n) {
-        if (lane == 0) bl[row] = 0.f;
+        bl[row] = 0.f;
         continue;
       }
-      const float2* srow = a.S2 + static_cast<int64_t>(row) * a.n;
-      dd acc = dd_make(0.f, 0.f);
-      for (int k0 = lane; k0 < a.n; k0 += 32 * 8) {
-        float2 sv[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = k0 + 32 * u;
-          sv[u] = (k < a.n) ? srow[k] : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = k0 + 32 * u;
-          if (k < a.n) acc = dd_add(acc, dd_mul(dd_make(sv[u].x, sv[u].y), dd_make(xh[k], xl[k])));
-        }
-      }
-      acc = warp_sum_dd(acc, wred, lane);
-      if (lane == 0) {
-        const dd rr = dd_sub(dd_from_double(a.b[row]), acc);
-        bl[row] = (rr.hi + rr.lo) * vd[row] - (ag.hi + ag.lo) * ud[row];
-      }
+      const dd rr = dd_sub(dd_from_double(a.b[row]), sum);
+      bl[row] = (rr.hi + rr.lo) * vd[row] - (ag.hi + ag.lo) * ud[row];
     }
   }
 }

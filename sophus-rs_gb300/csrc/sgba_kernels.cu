@@ -1519,10 +1519,23 @@ __device__ __forceinline__ void camera_finalize_body(int nf, const int64_t* fb_t
   const int fb = bid_;
   const int k = threadIdx.x;
   __shared__ double vals[kTileVals];
+  __shared__ float2 grad[6];  // sum J^T r~, which the reduced rhs takes too
+  dd acc = dd_make(0.f, 0.f);
   if (k < kTileVals) {
-    dd acc = dd_make(0.f, 0.f);
-    for (int64_t t = fb_tile_begin[fb]; t < fb_tile_begin[fb + 1]; ++t)
-      acc = dd_add(acc, dd_from_double(tile_part[t * kTileVals + k]));
+    // the tiles in order, eight loads ahead of the additions
+    const int64_t t1 = fb_tile_begin[fb + 1];
+    for (int64_t t = fb_tile_begin[fb]; t < t1; t += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = t + u < t1 ? tile_part[(t + u) * kTileVals + k] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (t + u < t1) acc = dd_add(acc, dd_from_double(v[u]));
+    }
+    if (k >= 21 && k < 27) grad[k - 21] = make_float2(acc.hi, acc.lo);
+  }
+  __syncthreads();
+  if (k < kTileVals) {
     // cost functions on the poses alone (sgba_prior.cu): the priors on this
     // pose in prior order, then its pose-graph records in term order; J^T W J
     // into the 21 upper entries, J^T W g with the gradient sums
@@ -1549,10 +1562,7 @@ __device__ __forceinline__ void camera_finalize_body(int nf, const int64_t* fb_t
       acc = dd_neg(dd_add(acc, pr));  // neg_grad = -sum J^T r~ - sum J^T W g
     } else {
       // reduced rhs: b_f - sum Z c  (b_f = -g)
-      dd g = dd_make(0.f, 0.f);
-      for (int64_t t = fb_tile_begin[fb]; t < fb_tile_begin[fb + 1]; ++t)
-        g = dd_add(g, dd_from_double(tile_part[t * kTileVals + k - 6]));
-      g = dd_add(g, pr);
+      const dd g = dd_add(dd_make(grad[k - 27].x, grad[k - 27].y), pr);
       acc = dd_sub(dd_neg(g), acc);
     }
     vals[k] = dd_to_double(acc);
@@ -1851,9 +1861,13 @@ __device__ __forceinline__ void schur_reduce_body(SchurArgs a, const Ctrl* ctrl,
     const int c0 = a.block_chunk_begin[blk], c1 = a.block_chunk_begin[blk + 1];
     for (int e = lane; e < 36; e += 32) {
       dd t = dd_make(0.f, 0.f);
-      for (int c = c0; c < c1; ++c) {
-        const float2 v = a.part[36 * static_cast<int64_t>(c) + e];
-        t = dd_add(t, dd_make(v.x, v.y));
+      for (int c = c0; c < c1; c += 4) {  // in order, four loads ahead of the additions
+        float2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = c + u < c1 ? a.part[36 * static_cast<int64_t>(c + u) + e] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (c + u < c1) t = dd_add(t, dd_make(v[u].x, v[u].y));
       }
       const int r = e / 6, cc = e % 6;
       dd vd;

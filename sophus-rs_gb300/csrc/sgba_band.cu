@@ -64,6 +64,7 @@ constexpr int kMaxBorder = 6 * kMaxBorderBlocks;
 // threads 32 .. W + 30 of a CTA, so W <= kFT - 32 (288 rows, 48 pose blocks).
 constexpr int kMaxCornerBlocks = 48;
 constexpr int kMaxW = 6 * kMaxCornerBlocks;  // widest band the factor kernel takes (the corner's)
+static_assert(kMaxW == kBandMaxW, "Dev::band_P");
 constexpr int kMaxOwnRows = (kMaxW - 1 + 7) / 8;  // rows of one CTA in a window (cluster >= 8)
 constexpr float kTolRel = 1e-12f;
 constexpr size_t kSmemLimit = 227 * 1024;
@@ -142,7 +143,7 @@ struct BandArgs {
   float2* Mb;       // npan x 24 x W: X_p^T L^T (rows c1 .. c1 + W - 2 below the panel), backward sweep
   float2* dpiv;     // n: pivots
   float2* rdpiv;    // n: 1 / pivot (0 for a zero pivot)
-  float2* Pbuf;     // (W - 1) x 24: L D of the current panel, rows below it
+  float2* Pbuf;     // per segment kMaxW x 24: L D of the current panel, rows below it
   float2* Zc;       // (nbd + 1) x nband: border rows of C and the scaled right-hand side, then L_A^-1 of them
   float2* Zd;       // (nbd + 1) x nband: D_A^-1 Zc
   float2* Cn;       // (nbd + 1) x (nbd + 1): E and the border part of the right-hand side, then the corner
@@ -179,6 +180,7 @@ __device__ __forceinline__ BandArgs seg_view(const BandArgs& a, int sg) {
   b.Mb = a.Mb + static_cast<int64_t>(a.seg_pan0[sg]) * kBP * a.W;
   b.dpiv = a.dpiv + a.seg_row0[sg];
   b.rdpiv = a.rdpiv + a.seg_row0[sg];
+  b.Pbuf = a.Pbuf + static_cast<int64_t>(sg) * kMaxW * kBP;
   return b;
 }
 
@@ -252,7 +254,6 @@ struct FactorShared {
   float2 xs[kBP][kBP];       // xs[t][q]: row t of X once final (q < t)
   float2 arow[kMaxOwnRows][kBP];
   const float2* dsrc[kBP];   // diagonal-block rows: their slots in the owners' shared memory
-  const float4* psrc[kMaxW]; // L D rows of the panel in their owners' shared memory
   int rofs[kMaxOwnRows];     // own window rows: offset of column 0 in `rows`
   int pre[kMaxOwnRows + 1];  // update work prefix over the own rows
   int bad;
@@ -268,7 +269,7 @@ struct FactorShared {
 // Per panel: every CTA gathers the 24x24 diagonal block from the owners
 // (DSMEM) and factors it redundantly; each CTA solves its own rows of the
 // panel and publishes L D of them; after a cluster barrier every CTA gathers
-// the panel's L D (DSMEM) and updates its own rows in place.
+// the panel's L D (through L2) and updates its own rows in place.
 template <int C>
 __global__ void __launch_bounds__(kFT, 1) k_band_factor(BandArgs a0, Ctrl* ctrl) {
   // Every CTA reads the control block before the first cluster barrier and
@@ -284,8 +285,7 @@ __global__ void __launch_bounds__(kFT, 1) k_band_factor(BandArgs a0, Ctrl* ctrl)
   const int tid = threadIdx.x;
   const int W = a.W, rmask = a.ring - 1;
   float2* rows = dyn;                  // ring x W
-  float2* pld = rows + a.ring * W;     // ring x kBP: L D of the own rows of the current panel
-  float2* pb = pld + a.ring * kBP;     // (W - 1) x (kBP + 1): L D of the panel, all rows below it
+  float2* pb = rows + a.ring * W;      // (W - 1) x (kBP + 1): L D of the panel, all rows below it
   auto slot = [&](int r) { return (r / C) & rmask; };
   // element (r, c) of an own row r: rows[rbase(r) + c]
   auto rbase = [&](int r) { return slot(r) * W + (W - 1 - r); };
@@ -330,10 +330,6 @@ __global__ void __launch_bounds__(kFT, 1) k_band_factor(BandArgs a0, Ctrl* ctrl)
     if (tid < w) {
       const int r = c0 + tid;
       sh.dsrc[tid] = cl.map_shared_rank(rows + slot(r) * W, r % C);  // slot base; column c at c - r + W - 1
-    }
-    if (tid >= 32 && tid - 32 < rend - c1) {
-      const int r = c1 + tid - 32;
-      sh.psrc[tid - 32] = reinterpret_cast<const float4*>(cl.map_shared_rank(pld + slot(r) * kBP, r % C));
     }
     if (tid == 64) {
       int acc = 0;
@@ -459,11 +455,14 @@ __global__ void __launch_bounds__(kFT, 1) k_band_factor(BandArgs a0, Ctrl* ctrl)
         l = dd_mul(acc_get(acc), f2dd(sh.srd[k]));
         if (c0 + k >= r - W + 1) rows[sh.rofs[ri] + c0 + k] = dd2f(l);
       }
-      pld[slot(r) * kBP + k] = dd2f(k < w ? dd_mul(l, f2dd(sh.sd[k])) : l);
+      a.Pbuf[(r - c1) * kBP + k] = dd2f(k < w ? dd_mul(l, f2dd(sh.sd[k])) : l);
     }
     cl.sync();  // L D of every row of the panel is published
-    // (5) the panel's L D, all rows below it, from their owners: 16-byte
-    // loads (a row is 12 float4), eight in flight per thread
+    // (5) the panel's L D, all rows below it, through L2: 16-byte loads (a row
+    // is 12 float4), eight in flight per thread.  (From the owners' shared
+    // memory, 16 CTAs reading all of it at once: 4,300 of a panel's 22,600
+    // cycles at W = 150; the 1,500-camera loop's factor 2.29 -> 2.17 ms.)  The next
+    // panel writes it after the cluster barrier at its top.
     const int nrows = rend - c1;
     {
       constexpr int kQ = kBP / 2;
@@ -473,7 +472,7 @@ __global__ void __launch_bounds__(kFT, 1) k_band_factor(BandArgs a0, Ctrl* ctrl)
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int e = e0 + u * kFT;
-          if (e < nq) v4[u] = sh.psrc[e / kQ][e % kQ];
+          if (e < nq) v4[u] = __ldcg(reinterpret_cast<const float4*>(a.Pbuf) + e);
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -1082,8 +1081,7 @@ int band_ring(int W, int C) {
 
 size_t factor_dyn_smem(int W, int C) {
   const int ring = band_ring(W, C);
-  return sizeof(float2) * (static_cast<size_t>(ring) * W + static_cast<size_t>(ring) * kBP +
-                           static_cast<size_t>(W - 1) * (kBP + 1));
+  return sizeof(float2) * (static_cast<size_t>(ring) * W + static_cast<size_t>(W - 1) * (kBP + 1));
 }
 
 // Three panel buffers in the sweeps where they fit in shared memory, else two.

@@ -1144,7 +1144,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
       if ((st = dev_alloc(p, &d.band_Mb, npan * 24 * static_cast<size_t>(w)))) return st;
       if ((st = dev_alloc(p, &d.band_d, n6))) return st;
       if ((st = dev_alloc(p, &d.band_rd, n6))) return st;
-      if ((st = dev_alloc(p, &d.band_P, static_cast<size_t>(w) * 24))) return st;
+      if ((st = dev_alloc(p, &d.band_P, 2 * static_cast<size_t>(sgba::kBandMaxW) * 24))) return st;
       if ((st = dev_alloc(p, &d.band_Z, nbd1 * rows))) return st;
       if ((st = dev_alloc(p, &d.band_Zd, nbd1 * rows))) return st;
       if ((st = dev_alloc(p, &d.band_E, nbd1 * nbd1))) return st;

@@ -13,6 +13,7 @@
 namespace sgba {
 
 // floats per term of the float-float Z (6x3 as (hi, lo) pairs, padded to float4)
+constexpr int kBandMaxW = 288;  // widest band the banded solver factors (a dissected loop's corner)
 constexpr int kZddFloats = 40;
 // Camera params on the device: fx fy cx cy alpha beta (the enhanced unified
 // camera model; alpha = beta = 0 is the pinhole).  Free intrinsics: per point
@@ -248,7 +249,7 @@ struct Dev {
   float2* band_Mb = nullptr;       // panels x 24 x band_w: X_p^T L^T of the rows below (backward sweep)
   float2* band_d = nullptr;        // n6 pivots
   float2* band_rd = nullptr;       // n6 reciprocal pivots
-  float2* band_P = nullptr;        // band_w x 24 panel exchange
+  float2* band_P = nullptr;        // 2 x kBandMaxW x 24: panel exchange of each segment
   float2* band_Z = nullptr;        // (border + 1) x band_rows
   float2* band_Zd = nullptr;       // (border + 1) x band_rows
   float2* band_E = nullptr;        // (border + 1)^2

@@ -1408,7 +1408,7 @@ __device__ __forceinline__ void camera_tiles_body(CamArgs a, const Ctrl* ctrl, i
   }
 }
 template <bool E>
-__global__ void __launch_bounds__(kTileThreads) k_camera_tiles(CamArgs a, const Ctrl* ctrl) {
+__global__ void __launch_bounds__(kTileThreads, 3) k_camera_tiles(CamArgs a, const Ctrl* ctrl) {
   camera_tiles_body<E>(a, ctrl, blockIdx.x, gridDim.x);
 }
 
@@ -4036,7 +4036,7 @@ __global__ void __launch_bounds__(256, 4) k_landmark_chunks_w(WinTab<LinArgs> t)
   landmark_chunks_body<E>(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }
 template <bool E>
-__global__ void __launch_bounds__(kTileThreads) k_camera_tiles_w(WinTab<CamArgs> t) {
+__global__ void __launch_bounds__(kTileThreads, 3) k_camera_tiles_w(WinTab<CamArgs> t) {
   const WinPos q = win_pos(t);
   camera_tiles_body<E>(t.args[q.w], t.ctrl[q.w], q.b, q.nb);
 }

@@ -30,7 +30,7 @@
 //                     diagonal block (and the inverse of its unit lower factor) redundantly, solves
 //                     its own rows of the panel, then updates its own rows of the trailing band
 //   k_band_sweepmat   per panel, the sweep matrices X_p L_p and X_p^T L_b^T (one CTA per panel)
-//   k_band_fwd        one CTA per border row and one for the right-hand side: z = L_A^-1 c
+//   k_band_fwd        border rows and the right-hand side, one or two a CTA: z = L_A^-1 c
 //   k_band_corner     E - Z D_A^-1 Z^T (one warp per entry; the right-hand side row gives y_C)
 //   k_band_corner_solve  LDL^T of the corner and its solve
 //   k_band_tvec       t = D_A^-1 y_A - L_C^T x_C
@@ -133,7 +133,7 @@ struct BandArgs {
   int nbd;    // border rows (n - nband)
   int ring;   // row slots per CTA in the factor kernel
   int nbuf;   // panel buffers of the backward sweep (2 or 3)
-  int nbuf_f; // panel buffers of the forward sweep (2 where two CTAs per SM keep its many rows in one wave)
+  int nbuf_f; // panel buffers of the forward sweep (fwd_nbuf)
   const double* S;  // n x n, both triangles
   const double* b;  // reduced right-hand side
   float* scl;       // n: D^-1/2
@@ -601,21 +601,44 @@ __global__ void __launch_bounds__(kBT) k_band_sweepmat(BandArgs a0, const Ctrl* 
 // a group of kSweepG threads per row (warps 0..5).  The panel's inputs c come
 // from the unchanged Zc row (staged with the panel), so the outputs can go
 // straight into the vector; one barrier per panel.
+//
+// Every row of a segment reads the same matrices, 33 KB a panel through L2: with
+// a row per CTA and the whole row in shared memory, 578 CTAs at two an SM took
+// two waves and 3.6 GB on the arcs of the 1,500-camera loop.  So a
+// CTA takes R neighbouring rows, whose solved entries leave for global memory
+// panel by panel and stay in shared memory only as far back as the band reaches:
+// one wave, half the traffic, an M entry read once for both rows (486 -> 432 us).
+constexpr int kFwdRing = 512;  // >= kMaxW + kBP, a power of two
+static_assert(kFwdRing >= kMaxW + kBP, "the ring holds the band's reach");
+__host__ __device__ inline size_t fwd_smem_floats2(int W, int nbuf, int R) {
+  return static_cast<size_t>(R) * kFwdRing +
+         static_cast<size_t>(nbuf) * (static_cast<size_t>(kBP) * W + kBP * kBP + kBP * (R + 1));
+}
+
+template <int R>
 __global__ void __launch_bounds__(kBT) k_band_fwd(BandArgs a0, const Ctrl* ctrl) {
   if (skipping(ctrl)) return;
   extern __shared__ __align__(16) float2 sw[];
-  // CTA (row, segment): the row's part in one segment of the band
+  // CTA (rows, segment): the rows' parts in one segment of the band
   const int sg = static_cast<int>(blockIdx.x) % a0.nseg;
-  const int row = static_cast<int>(blockIdx.x) / a0.nseg;
+  const int row0 = R * (static_cast<int>(blockIdx.x) / a0.nseg);
   const BandArgs a = seg_view(a0, sg);
   const int W = a.W;
   const int nb = a.nbuf_f;
-  float2* v = sw;
-  float2* mbuf = v + ((a.nband + 1) & ~1);  // nb x kBP x W (16-byte aligned: W is even)
-  float2* xb = mbuf + nb * kBP * W;         // nb x kBP x kBP
-  float2* cb = xb + nb * kBP * kBP;         // nb x kBP
+  const int nr = min(R, a0.nbd + 1 - row0);
+  float2* v = sw;                              // R x kFwdRing: column c at c mod kFwdRing
+  float2* mbuf = v + R * kFwdRing;             // nb x kBP x W (16-byte aligned: W is even)
+  float2* xb = mbuf + nb * kBP * W;            // nb x kBP x kBP
+  float2* cb = xb + nb * kBP * kBP;            // nb x R x kBP: the rows' inputs
+  float2* rb = cb + nb * R * kBP;              // nb x kBP: reciprocal pivots
   const int tid = threadIdx.x;
-  float2* zrow = a0.Zc + static_cast<int64_t>(row) * a0.nband + a0.seg_row0[sg];
+  float2 *zrow[R], *drow[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const int64_t o = static_cast<int64_t>(min(row0 + u, a0.nbd)) * a0.nband + a0.seg_row0[sg];
+    zrow[u] = a0.Zc + o;
+    drow[u] = a0.Zd + o;
+  }
   const int h = W / 2;
   const int i0 = tid / h, q0 = tid % h, di = kBT / h, dq = kBT % h;
   auto stage = [&](int p) {
@@ -633,23 +656,37 @@ __global__ void __launch_bounds__(kBT) k_band_fwd(BandArgs a0, const Ctrl* ctrl)
     }
     for (int e = tid; e < kBP * kBP / 2; e += kBT)
       cp_async16(xb + buf * kBP * kBP + 2 * e, a.Xinv + static_cast<int64_t>(p) * kBP * kBP + 2 * e);
-    if (tid < w / 2) cp_async16(cb + buf * kBP + 2 * tid, zrow + c0 + 2 * tid);
+    if (tid < w / 2) {
+#pragma unroll
+      for (int u = 0; u < R; ++u) cp_async16(cb + (buf * R + u) * kBP + 2 * tid, zrow[u] + c0 + 2 * tid);
+    }
+    if (tid >= 32 && tid - 32 < w) cp_async8(rb + buf * kBP + tid - 32, a.rdpiv + c0 + tid - 32);
     cp_async_commit();
   };
-  // the row's first nonzero in the segment: the panels before it stay zero
-  __shared__ int s_first;
-  if (tid == 0) s_first = a.nband;
+  // the rows' first nonzeros in the segment: the panels before them stay zero
+  __shared__ int s_first[R];
+  if (tid < R) s_first[tid] = a.nband;
   __syncthreads();
-  int myfirst = a.nband;
-  for (int c = tid; c < a.nband; c += kBT) {
-    const float2 z = zrow[c];
-    v[c] = z;
-    if ((z.x != 0.0f || z.y != 0.0f) && c < myfirst) myfirst = c;
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    int myfirst = a.nband;
+    for (int c = tid; c < a.nband && myfirst == a.nband; c += kBT) {
+      const float2 z = zrow[u][c];
+      if (z.x != 0.0f || z.y != 0.0f) myfirst = c;
+    }
+    atomicMin(&s_first[u], myfirst);
   }
-  atomicMin(&s_first, myfirst);
+  for (int e = tid; e < R * kFwdRing; e += kBT) v[e] = make_float2(0.0f, 0.0f);
   __syncthreads();
-  const int pstart = s_first / kBP;
-  if (tid == 0 && a0.zlo) a0.zlo[row * a0.nseg + sg] = s_first;
+  int pstart = a.npan, pfirst[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    pfirst[u] = s_first[u] / kBP;
+    pstart = min(pstart, pfirst[u]);
+    if (u < nr && tid == 0 && a0.zlo) a0.zlo[(row0 + u) * a0.nseg + sg] = s_first[u];
+    if (u < nr)  // D^-1 z of the zero entries
+      for (int c = tid; c < min(kBP * pfirst[u], a.nband); c += kBT) drow[u][c] = make_float2(0.0f, 0.0f);
+  }
   for (int s0 = 0; s0 < nb - 1; ++s0) {
     if (pstart + s0 < a.npan) stage(pstart + s0);
     else cp_async_commit();
@@ -665,39 +702,59 @@ __global__ void __launch_bounds__(kBT) k_band_fwd(BandArgs a0, const Ctrl* ctrl)
     if (p + nb - 1 < a.npan) stage(p + nb - 1);
     else cp_async_commit();
     if (tid < kBP * kSweepG) {
-      Acc a0 = acc_init(dd_make(0.0f, 0.0f)), a1 = a0, a2 = a0, a3 = a0;
+      Acc s0[R], s1[R], s2[R], s3[R];
+#pragma unroll
+      for (int u = 0; u < R; ++u) s0[u] = s1[u] = s2[u] = s3[u] = acc_init(dd_make(0.0f, 0.0f));
       if (k < w) {
         const float2* xr = xb + buf * kBP * kBP + k * kBP;
-        const float2* cp = cb + buf * kBP;
-        for (int kk = g; kk <= k; kk += kSweepG) acc_madd(a0, f2dd(xr[kk]), f2dd(cp[kk]));
+        for (int kk = g; kk <= k; kk += kSweepG) {
+          const dd x = f2dd(xr[kk]);
+#pragma unroll
+          for (int u = 0; u < R; ++u) acc_madd(s0[u], x, f2dd(cb[(buf * R + u) * kBP + kk]));
+        }
         const float2* mrow = mbuf + (buf * kBP + k) * W;
         const int vb = c0 - W + 1;  // column of slot 0
-        int s2 = max(0, -vb) + g;
-        for (; s2 + 3 * kSweepG < W - 1; s2 += 4 * kSweepG) {
-          const float2 m0 = mrow[s2], m1 = mrow[s2 + kSweepG], m2 = mrow[s2 + 2 * kSweepG], m3 = mrow[s2 + 3 * kSweepG];
-          const float2 v0 = v[vb + s2], v1 = v[vb + s2 + kSweepG], v2 = v[vb + s2 + 2 * kSweepG],
-                       v3 = v[vb + s2 + 3 * kSweepG];
-          acc_madd(a1, dd_neg(f2dd(m0)), f2dd(v0));
-          acc_madd(a2, dd_neg(f2dd(m1)), f2dd(v1));
-          acc_madd(a3, dd_neg(f2dd(m2)), f2dd(v2));
-          acc_madd(a0, dd_neg(f2dd(m3)), f2dd(v3));
+        auto at = [&](int u, int c) { return f2dd(v[u * kFwdRing + (c & (kFwdRing - 1))]); };
+        int s = max(0, -vb) + g;
+        for (; s + 3 * kSweepG < W - 1; s += 4 * kSweepG) {
+          const dd m0 = dd_neg(f2dd(mrow[s])), m1 = dd_neg(f2dd(mrow[s + kSweepG])),
+                   m2 = dd_neg(f2dd(mrow[s + 2 * kSweepG])), m3 = dd_neg(f2dd(mrow[s + 3 * kSweepG]));
+#pragma unroll
+          for (int u = 0; u < R; ++u) {
+            acc_madd(s1[u], m0, at(u, vb + s));
+            acc_madd(s2[u], m1, at(u, vb + s + kSweepG));
+            acc_madd(s3[u], m2, at(u, vb + s + 2 * kSweepG));
+            acc_madd(s0[u], m3, at(u, vb + s + 3 * kSweepG));
+          }
         }
-        for (; s2 < W - 1; s2 += kSweepG) acc_madd(a1, dd_neg(f2dd(mrow[s2])), f2dd(v[vb + s2]));
+        for (; s < W - 1; s += kSweepG) {
+          const dd m = dd_neg(f2dd(mrow[s]));
+#pragma unroll
+          for (int u = 0; u < R; ++u) acc_madd(s1[u], m, at(u, vb + s));
+        }
       }
-      acc_add(a0, acc_get(a1));
-      acc_add(a2, acc_get(a3));
-      acc_add(a0, acc_get(a2));
-      const dd sm = group_sum(acc_get(a0));
-      if (g == 0 && k < w) v[c0 + k] = dd2f(sm);
+      dd sm[R];
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        acc_add(s0[u], acc_get(s1[u]));
+        acc_add(s2[u], acc_get(s3[u]));
+        acc_add(s0[u], acc_get(s2[u]));
+        sm[u] = group_sum(acc_get(s0[u]));
+      }
+      if (g == 0 && k < w) {
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          if (p < pfirst[u]) continue;  // still zero
+          v[u * kFwdRing + ((c0 + k) & (kFwdRing - 1))] = dd2f(sm[u]);
+          if (u < nr) {
+            zrow[u][c0 + k] = dd2f(sm[u]);
+            drow[u][c0 + k] = dd2f(dd_mul(f2dd(dd2f(sm[u])), f2dd(rb[buf * kBP + k])));
+          }
+        }
+      }
     }
   }
   cp_async_wait_all();
-  __syncthreads();
-  float2* drow = a0.Zd + static_cast<int64_t>(row) * a0.nband + a0.seg_row0[sg];
-  for (int c = tid; c < a.nband; c += kBT) {
-    zrow[c] = v[c];
-    drow[c] = dd2f(dd_mul(f2dd(v[c]), f2dd(a.rdpiv[c])));
-  }
 }
 
 // ----------------------------------------------------------- corner -------
@@ -997,7 +1054,8 @@ __global__ void __launch_bounds__(kBT) k_band_bwd(BandArgs a0, const Ctrl* ctrl)
 }
 
 int sweep_nbuf(int nband, int W);
-int fwd_nbuf(int nband, int W, int nctas);
+int fwd_rows(int nrows, int nseg);
+int fwd_nbuf(int W, int R);
 
 BandArgs band_args(const Sizes& s, const Dev& d) {
   BandArgs a{};
@@ -1034,7 +1092,7 @@ BandArgs band_args(const Sizes& s, const Dev& d) {
   a.npan = a.seg_pan0[1] + (a.nseg > 1 ? (a.seg_rows[1] + kBP - 1) / kBP : 0);
   const int segmax = a.seg_rows[0] > a.seg_rows[1] ? a.seg_rows[0] : a.seg_rows[1];
   a.nbuf = sweep_nbuf(segmax, a.W);
-  a.nbuf_f = fwd_nbuf(segmax, a.W, (a.nbd + 1) * a.nseg);
+  a.nbuf_f = fwd_nbuf(a.W, fwd_rows(a.nbd + 1, a.nseg));
   a.zlo = d.band_zlo;
   a.out_scaled = nullptr;
   return a;
@@ -1051,7 +1109,7 @@ BandArgs corner_args(const Sizes& s, const Dev& d, const BandArgs& a) {
   c.nbd = 0;
   c.ring = s.band_ring_c;
   c.nbuf = sweep_nbuf(m, m);
-  c.nbuf_f = c.nbuf;
+  c.nbuf_f = fwd_nbuf(m, 1);
   c.Lb = d.band_Lc;
   c.Xinv = d.band_Xc;
   c.Mf = d.band_Mfc;
@@ -1097,17 +1155,13 @@ size_t band_sweep_smem(int nband, int W) {
   return sizeof(float2) * sweep_smem_floats2(nband, W, sweep_nbuf(nband, W));
 }
 
-// The forward sweep runs one CTA per border row and segment: with more CTAs
-// than SMs, two buffers (two CTAs per SM where they fit) keep the rows in one
-// wave; otherwise the deeper prefetch of sweep_nbuf.
-int fwd_nbuf(int nband, int W, int nctas) {
-  if (nctas > 132 && 2 * (sizeof(float2) * sweep_smem_floats2(nband, W, 2) + 1024) <= kSmemLimit) return 2;
-  return sweep_nbuf(nband, W);
+// Rows of a CTA of the forward sweep: two where one each would not fit the SMs
+// in one wave; three panel buffers where two CTAs of them fit an SM, else two.
+int fwd_rows(int nrows, int nseg) { return nrows * nseg > 152 ? 2 : 1; }
+int fwd_nbuf(int W, int R) {
+  return sizeof(float2) * fwd_smem_floats2(W, 3, R) <= (R == 1 ? kSmemLimit - 4096 : (kSmemLimit - 4096) / 2) ? 3 : 2;
 }
-
-size_t fwd_sweep_smem(int nband, int W, int nctas) {
-  return sizeof(float2) * sweep_smem_floats2(nband, W, fwd_nbuf(nband, W, nctas));
-}
+size_t fwd_smem(int W, int R) { return sizeof(float2) * fwd_smem_floats2(W, fwd_nbuf(W, R), R); }
 
 }  // namespace
 
@@ -1167,7 +1221,9 @@ int band_setup(int n, int nband, int W, int nseg, int seg_rows_max, int* cluster
     corner = sizeof(float2) * static_cast<size_t>(m) * (m + 2);
     if (corner > kSmemLimit - 4096) return 0;
   }
-  if (raise_dynamic_smem(reinterpret_cast<const void*>(k_band_fwd), sweep) != cudaSuccess ||
+  if (raise_dynamic_smem(reinterpret_cast<const void*>(k_band_fwd<1>),
+                         std::max(fwd_smem(W, 1), nseg > 1 ? fwd_smem(m, 1) : 0)) != cudaSuccess ||
+      raise_dynamic_smem(reinterpret_cast<const void*>(k_band_fwd<2>), fwd_smem(W, 2)) != cudaSuccess ||
       raise_dynamic_smem(reinterpret_cast<const void*>(k_band_sweepmat), smat) != cudaSuccess ||
       raise_dynamic_smem(reinterpret_cast<const void*>(k_band_bwd), sweep) != cudaSuccess ||
       raise_dynamic_smem(reinterpret_cast<const void*>(k_band_corner_solve), std::max<size_t>(corner, 16)) !=
@@ -1255,7 +1311,10 @@ int launch_band(const Sizes& s, const Dev& d, cudaStream_t st) {
   k_band_sweepmat<<<a.npan, kBT, sweepmat_smem(a.W), st>>>(a, d.ctrl);
   ++launches;
   const int segmax = std::max(a.seg_rows[0], a.seg_rows[1]);
-  k_band_fwd<<<(a.nbd + 1) * a.nseg, kBT, fwd_sweep_smem(segmax, a.W, (a.nbd + 1) * a.nseg), st>>>(a, d.ctrl);
+  if (fwd_rows(a.nbd + 1, a.nseg) == 2)
+    k_band_fwd<2><<<(a.nbd + 2) / 2 * a.nseg, kBT, fwd_smem(a.W, 2), st>>>(a, d.ctrl);
+  else
+    k_band_fwd<1><<<(a.nbd + 1) * a.nseg, kBT, fwd_smem(a.W, 1), st>>>(a, d.ctrl);
   ++launches;
   {
     const int64_t nt = (a.nbd + 1 + kCornerTile - 1) / kCornerTile;
@@ -1272,7 +1331,7 @@ int launch_band(const Sizes& s, const Dev& d, cudaStream_t st) {
                                                                                                    d.ctrl);
     launch_factor(c, s.band_c, 1, st, d.ctrl);
     k_band_sweepmat<<<c.npan, kBT, sweepmat_smem(c.W), st>>>(c, d.ctrl);
-    k_band_fwd<<<1, kBT, band_sweep_smem(c.nband, c.W), st>>>(c, d.ctrl);
+    k_band_fwd<1><<<1, kBT, fwd_smem(c.W, 1), st>>>(c, d.ctrl);
     k_band_bwd<<<1, kBT, band_sweep_smem(c.nband, c.W), st>>>(c, d.ctrl);
     launches += 5;
   } else {

@@ -667,7 +667,7 @@ def main():
                                     "length" % ((nb + 23) // 24))
         elif lay.solver == 3:
             roofline["note"] = ("latency-bound dependency chain: float-float LDL^T of the %d-row reduced system "
-                                "in one CTA, one barrier per pivot" % (n6 + lay.intrinsics_rows))
+                                "in one CTA, by pose-block panels" % (n6 + lay.intrinsics_rows))
         else:
             roofline["note"] = ("latency-bound dependency chain (one cluster of 16 CTAs: %d panel steps, then a "
                                 "forward and a backward sweep per solve, one solve plus one or two refinement "

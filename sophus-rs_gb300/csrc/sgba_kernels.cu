@@ -3546,7 +3546,7 @@ static int schur_dense_grid(const Sizes& s) {
 // Few tiles leave most SMs idle (a tile's rounds are 0.5 us each, eight at a
 // time): up to half an SM count of tiles the rounds are spread over ~608 CTAs
 // and summed by a second launch, where their sums fit in 64 MB (10 cameras and
-// 1,000 points: 35 -> 8 us).  0 floats: not split.
+// 500 points: 35 -> 8 us).  0 floats: not split.
 size_t schur_split_floats(const Sizes& s) {
   if (!s.schur_dense || schur_dense_grid(s) > 76) return 0;
   const size_t f = static_cast<size_t>(schur_dense_grid(s)) * ((s.np + kSdPts - 1) / kSdPts) * kSdEntries;

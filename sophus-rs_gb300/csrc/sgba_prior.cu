@@ -5,7 +5,7 @@
 //
 // Each prior k on pose j has a mean E_k and a 6x6 precision W_k; its residual
 // is g = log(T_j E_k^-1) and its Jacobian J the derivative of
-// log(exp(x) T_j E_k^-1) at x = 0, taken here by forward-mode derivatives in
+// log(exp(x) T_j E_k^-1) at x = 0, taken here in closed form, in
 // f64 (sgba_lie.cuh: a direction per lane).  EvaluatedCostTerm::make
 // (crates/sophus_opt/src/nlls/cost/evaluated_term.rs:286-327) then gives the
 // Hessian block J^T W J, the gradient J^T W g and the cost g^T W g.  The

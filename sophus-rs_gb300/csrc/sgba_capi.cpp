@@ -1590,10 +1590,15 @@ int sgba_set_pose_priors(sgba_problem* p, int32_t n, const int32_t* pose, const 
   SGBA_CK(cudaStreamSynchronize(p->stream));
   Dev& d = p->d;
   Sizes& s = p->sz;
-  // CostFn::sort order: by pose, stable
+  // CostFn::sort order (by pose, stable), the priors on constant poses after the
+  // others: they have only a cost, and a free pose's priors are read by their
+  // range of positions (prior_fb_begin)
   std::vector<int32_t> ord(n);
   for (int32_t k = 0; k < n; ++k) ord[k] = k;
-  std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t b) { return pose[a] < pose[b]; });
+  std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t b) {
+    const bool ca = P.pose_fb[pose[a]] < 0, cb = P.pose_fb[pose[b]] < 0;
+    return ca != cb ? cb : pose[a] < pose[b];
+  });
   std::vector<int32_t> hp(n), hfb(n), beg(P.nf + 1, 0);
   std::vector<double> hm(7 * static_cast<size_t>(n)), hw(36 * static_cast<size_t>(n));
   for (int32_t k = 0; k < n; ++k) {

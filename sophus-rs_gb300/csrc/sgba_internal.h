@@ -174,7 +174,7 @@ struct Dev {
   float2* schur_part = nullptr;    // 36 float-float partials per chunk
   int32_t* lmk_chunk_pt = nullptr; // landmark pass: point chunks (<= 256 terms), nlchunk + 1
   int32_t* zterm = nullptr;        // np x nf: term of each (point, free block) or -1 (tiled Schur pass)
-  // pose priors (sgba_prior.cu), sorted by pose: pose, its free block (-1:
+  // pose priors (sgba_prior.cu), sorted by pose, constant poses last: pose, its free block (-1:
   // constant pose), mean (7), precision (36), and per prior J^T W J (36) and
   // J^T W g (6); per free block the range of its priors (nf + 1)
   int32_t* prior_pose = nullptr;

@@ -98,7 +98,7 @@ __device__ __forceinline__ void term_log(const double* qa, const double* b, cons
 }
 
 // CTAs [0, edge_blocks): reduced edge terms (the edges of a term in order); the
-// others: priors (sorted by pose).  At `poses`; lin: the records of both sides
+// others: priors (sorted by pose, constant poses last).  At `poses`; lin: the records of both sides
 // and J_m^T J_n of a term, J^T W J and J^T W g of the priors on free poses
 // (kPriorOut doubles each).  cost: a CTA's sum of g^T g and g^T W g in
 // float-float to cost[blockIdx.x].  gate: 0 none, 1 the control block's done

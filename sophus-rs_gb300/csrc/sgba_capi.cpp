@@ -879,26 +879,6 @@ int build_schur_pattern(sgba_problem* p) {
   if (tiled) return dev_alloc(p, &d.pairs, 0);
   if (npairs >= (int64_t(1) << 31))
     return set_error(SGBA_ERR_UNSUPPORTED, "%lld observation pairs exceed the 2^31 limit", (long long)npairs);
-  // Chunks of at most kSchurChunk pairs within one block (at least one per
-  // block).  The EUCM camera and pose-graph edges, which come with float-float
-  // sums, take shorter ones where 256 would leave warps idle (a warp's 256
-  // pairs are eight rounds in series: 27 us of 27,000 pairs, 7 with 32 a
-  // warp); FP32 partial sums keep their partition, and so their rounding.
-  const int64_t chunk =
-      p->camera_model == SGBA_CAMERA_PINHOLE && P.eterm_fm.empty()
-          ? kSchurChunk
-          : std::min(kSchurChunk, std::max<int64_t>(32, (npairs / kSchurWarps + 31) / 32 * 32));
-  P.block_chunk_begin.assign(nb + 1, 0);
-  for (int64_t b = 0; b < nb; ++b) {
-    P.block_chunk_begin[b] = static_cast<int32_t>(P.chunk_begin.size());
-    int64_t q = P.sb_pair_begin[b];
-    do {
-      P.chunk_begin.push_back(q);
-      q += chunk;
-    } while (q < P.sb_pair_begin[b + 1]);
-  }
-  P.block_chunk_begin[nb] = static_cast<int32_t>(P.chunk_begin.size());
-  P.chunk_begin.push_back(npairs);
   if ((st = dev_alloc(p, &d.pairs, static_cast<size_t>(npairs)))) return st;
   if (npairs == 0) return SGBA_OK;
   // point chunks: as many as keep the (chunk x block) table near 64 Mi entries
@@ -920,6 +900,44 @@ int build_schur_pattern(sgba_problem* p) {
   if (e != cudaSuccess)
     return set_error(e == cudaErrorMemoryAllocation ? SGBA_ERR_OUT_OF_MEMORY : SGBA_ERR_CUDA, "Schur pattern (pairs): %s",
                      cudaGetErrorString(e));
+  return SGBA_OK;
+}
+
+// Chunks of the pair lists within one block (at least one per block): at most
+// kSchurChunk pairs.  Float-float sums of the EUCM camera and of problems with
+// pose-graph edges take shorter ones where 256 would leave warps idle (a warp's
+// 256 pairs are eight rounds in series: 27 us of 27,000 pairs, 7 with 32 a
+// warp).  FP32 partial sums (an EUCM camera with fixed params on more than 39
+// poses among them) keep their partition, and so their rounding; those of
+// pinhole loops, float-float too, were not measured with shorter chunks.
+int build_pair_chunks(sgba_problem* p) {
+  Plan& P = p->plan;
+  Sizes& s = p->sz;
+  s.nchunk = 0;
+  if (!p->pairs_built || P.sb_pair_begin.empty()) return SGBA_OK;
+  const int64_t nb = static_cast<int64_t>(P.sb_row.size()), npairs = P.sb_pair_begin[nb];
+  const int64_t chunk =
+      s.lin_dd && (s.eucm || s.n_edge > 0)
+          ? std::min(kSchurChunk, std::max<int64_t>(32, (npairs / kSchurWarps + 31) / 32 * 32))
+          : kSchurChunk;
+  P.block_chunk_begin.assign(nb + 1, 0);
+  for (int64_t b = 0; b < nb; ++b) {
+    P.block_chunk_begin[b] = static_cast<int32_t>(P.chunk_begin.size());
+    int64_t q = P.sb_pair_begin[b];
+    do {
+      P.chunk_begin.push_back(q);
+      q += chunk;
+    } while (q < P.sb_pair_begin[b + 1]);
+  }
+  P.block_chunk_begin[nb] = static_cast<int32_t>(P.chunk_begin.size());
+  P.chunk_begin.push_back(npairs);
+  s.nchunk = static_cast<int64_t>(P.chunk_begin.size()) - 1;
+  int st;
+  if (s.nchunk > 0) {
+    if ((st = dev_upload(p, &p->d.chunk_begin, P.chunk_begin))) return st;
+    if ((st = dev_upload(p, &p->d.block_chunk_begin, P.block_chunk_begin))) return st;
+    if ((st = dev_alloc(p, &p->d.schur_part, 36 * static_cast<size_t>(s.nchunk)))) return st;
+  }
   return SGBA_OK;
 }
 
@@ -1028,15 +1046,9 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     if ((st = dev_upload(p, &d.eblk_term, P.eblk_term))) return st;
   }
   s.nsb = static_cast<int64_t>(P.sb_row.size());
-  s.nchunk = P.chunk_begin.empty() ? 0 : static_cast<int64_t>(P.chunk_begin.size()) - 1;
   if ((st = dev_upload(p, &d.sb_row, P.sb_row))) return st;
   if ((st = dev_upload(p, &d.sb_col, P.sb_col))) return st;
   if ((st = dev_upload(p, &d.sb_pair_begin, P.sb_pair_begin))) return st;
-  if (s.nchunk > 0) {
-    if ((st = dev_upload(p, &d.chunk_begin, P.chunk_begin))) return st;
-    if ((st = dev_upload(p, &d.block_chunk_begin, P.block_chunk_begin))) return st;
-    if ((st = dev_alloc(p, &d.schur_part, 36 * static_cast<size_t>(s.nchunk)))) return st;
-  }
   // state (quaternions disambiguated to w >= 0 as from_params does)
   for (int j = 0; j < P.nc; ++j)
     if (!(0.0 <= poses[7 * j]))
@@ -1205,6 +1217,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   // moved the step along that direction by ~10 % (measured on an 8-camera
   // circle with odometry edges).
   s.lin_dd = (loop_shaped || (s.eucm && (p->intr_free || s.small_dense)) || s.n_edge > 0) ? 1 : 0;
+  if ((st = build_pair_chunks(p))) return st;
   // S by tiles of pose blocks when nearly every block of S is present and a
   // point is seen by at least half the free poses on average (local windows):
   // each point's Z is then streamed once per tile instead of once per pair

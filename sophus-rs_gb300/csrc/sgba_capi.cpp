@@ -116,67 +116,20 @@ constexpr int64_t kSchurChunk = 256;  // observation pairs per warp in the Schur
 constexpr int64_t kSchurWarps = 152 * 16;  // warps of the assembly that run at once
 constexpr int32_t kMaxDenseFree = 4096;  // reduced-camera-system limit (6 * 4096 rows, stored dense in f64)
 
-// Page-locked staging blocks for the copies of small problems: kStageBytes
-// each, at most kStageBlocks in the process, handed out to one holder at a time
-// and taken back when its copies are complete.  A copy from pageable memory goes
-// through the driver's own staging, and every call through its lock: 24 windows
-// created by 16 threads spent 10 ms, most of it in 620 copies; gathered in a
-// block and copied together, 7.5 ms.
-// Without a block (all out, or no page-locked memory) the copies are pageable.
+// The small arrays of a problem being set up gather in a block of host memory
+// and go to the device in one copy: every copy takes the driver's lock, and 24
+// windows created by 16 threads spent most of 10 ms in 620 of them (7.5 ms so;
+// a page-locked block gave the same).  At most kStageBytes; the holder waits
+// for the copies before the object goes.
 constexpr size_t kStageBytes = size_t(4) << 20;
-constexpr size_t kStageBlocks = 16;
-class StagePool {
- public:
-  static StagePool& get() {
-    static StagePool* pool = new StagePool();  // never destroyed: the driver may be gone before it
-    return *pool;
-  }
-  char* take() {
-    std::lock_guard<std::mutex> lk(mu_);
-    if (!free_.empty()) {
-      char* b = free_.back();
-      free_.pop_back();
-      return b;
-    }
-    if (made_ >= kStageBlocks) return nullptr;
-    void* v = nullptr;
-    if (cudaHostAlloc(&v, kStageBytes, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    ++made_;
-    return static_cast<char*>(v);
-  }
-  void give(char* b) {
-    std::lock_guard<std::mutex> lk(mu_);
-    free_.push_back(b);
-  }
-
- private:
-  std::mutex mu_;
-  std::vector<char*> free_;
-  size_t made_ = 0;
-};
-
-// A staging block for the life of the object.  Whoever holds one waits for the
-// copies from or to it before the object goes.
 struct Stage {
-  char* base;
-  size_t used = 0;
-  // set-up: the device block that mirrors the first `cap` bytes, copied up to `sent`
-  char* dev = nullptr;
-  size_t cap = 0, sent = 0;
-  Stage() : base(StagePool::get().take()) {}
-  ~Stage() {
-    if (base) StagePool::get().give(base);
-  }
-  Stage(const Stage&) = delete;
-  Stage& operator=(const Stage&) = delete;
-  // room for `bytes`, or null
+  std::unique_ptr<char[]> base;
+  char* dev = nullptr;  // the device block that mirrors it, copied up to `sent`
+  size_t used = 0, cap = 0, sent = 0;
+  // room for `bytes` (at most cap - used)
   char* room(size_t bytes) {
-    if (!base || bytes > kStageBytes - used) return nullptr;
-    char* r = base + used;
-    used += std::min((bytes + 255) & ~size_t(255), kStageBytes - used);
+    char* r = base.get() + used;
+    used += std::min((bytes + 255) & ~size_t(255), cap - used);
     return r;
   }
 };
@@ -215,7 +168,7 @@ struct sgba_problem {
   size_t chunk_size = size_t(1) << 20;
   // covariance of the solution (sgba_covariance_prepare)
   sgba::CovBufs cov;
-  Stage* stage = nullptr;  // page-locked staging while the problem is being set up
+  Stage* stage = nullptr;  // gathers the small uploads while the problem is being set up
   bool pairs_built = true;  // the Schur pair lists exist (not for the tiled pass of nearly dense systems)
 };
 
@@ -285,10 +238,10 @@ int dev_alloc(sgba_problem* p, T** ptr, size_t count) {
 template <class T, class A>
 int dev_upload(sgba_problem* p, T** ptr, const std::vector<T, A>& h) {
   const size_t bytes = sizeof(T) * h.size();
-  if (Stage* s = p->stage; s && s->dev && bytes > 0 && bytes <= s->cap - std::min(s->used, s->cap)) {
+  if (Stage* s = p->stage; s && bytes > 0 && bytes <= s->cap - s->used) {
     char* room = s->room(bytes);
     std::memcpy(room, h.data(), bytes);
-    *ptr = reinterpret_cast<T*>(s->dev + (room - s->base));
+    *ptr = reinterpret_cast<T*>(s->dev + (room - s->base.get()));
     return SGBA_OK;
   }
   int st = dev_alloc(p, ptr, h.size());
@@ -300,9 +253,9 @@ int dev_upload(sgba_problem* p, T** ptr, const std::vector<T, A>& h) {
 // The gathered arrays to the device: before a kernel reads them.
 int upload_flush(sgba_problem* p) {
   Stage* s = p->stage;
-  const size_t end = s ? std::min(s->used, s->cap) : 0;
-  if (!s || !s->dev || end <= s->sent) return SGBA_OK;
-  SGBA_CK(cudaMemcpyAsync(s->dev + s->sent, s->base + s->sent, end - s->sent, cudaMemcpyHostToDevice, p->stream));
+  if (!s || s->used <= s->sent) return SGBA_OK;
+  const size_t end = s->used;
+  SGBA_CK(cudaMemcpyAsync(s->dev + s->sent, s->base.get() + s->sent, end - s->sent, cudaMemcpyHostToDevice, p->stream));
   s->sent = end;
   return SGBA_OK;
 }
@@ -980,12 +933,16 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   s.gauge_kind = P.gauge_kind;
   for (int k = 0; k < 3; ++k) s.gauge_center[k] = P.gauge_center[k];
   int st;
-  if (p->stage && p->stage->base) {
+  {
     // about what the arrays below take; those that do not fit are copied one by one
     const size_t want = 24 * static_cast<size_t>(P.no) + 28 * static_cast<size_t>(P.ng) + 64 * static_cast<size_t>(P.np) +
                         128 * static_cast<size_t>(P.nc) + (size_t(64) << 10);
-    p->stage->cap = std::min(want & ~size_t(255), kStageBytes);
-    if ((st = dev_alloc(p, &p->stage->dev, p->stage->cap))) return st;
+    const size_t cap = std::min(want & ~size_t(255), kStageBytes);
+    p->stage->base.reset(new (std::nothrow) char[cap]);
+    if (p->stage->base) {
+      if ((st = dev_alloc(p, &p->stage->dev, cap))) return st;
+      p->stage->cap = cap;
+    }
   }
   // host staging of the copies below: alive until the stream is synchronised
   sgba::RawVec<float4> uv(P.no);
@@ -1579,24 +1536,9 @@ int sgba_get_variables(sgba_problem* p, double* poses, double* points) {
   if (!p) return set_error(SGBA_ERR_INVALID_ARGUMENT, "NULL problem");
   SGBA_CK(cudaSetDevice(p->device));
   SGBA_CK(cudaStreamSynchronize(p->stream));
-  const size_t nb = poses ? sizeof(double) * 7 * p->plan.nc : 0;
-  const size_t pb = points ? sizeof(double) * 3 * p->plan.np : 0;
-  Stage stage;
-  char* const sp = stage.room(nb);
-  char* const st = stage.room(pb);
-  if (sp && st) {  // both queued, one wait
-    cudaError_t e = cudaSuccess;
-    if (nb) e = cudaMemcpyAsync(sp, p->d.poses, nb, cudaMemcpyDeviceToHost, p->stream);
-    if (e == cudaSuccess && pb) e = cudaMemcpyAsync(st, p->d.points, pb, cudaMemcpyDeviceToHost, p->stream);
-    const cudaError_t w = cudaStreamSynchronize(p->stream);
-    SGBA_CK(e);
-    SGBA_CK(w);
-    if (nb) std::memcpy(poses, sp, nb);
-    if (pb) std::memcpy(points, st, pb);
-    return SGBA_OK;
-  }
-  if (nb) SGBA_CK(cudaMemcpy(poses, p->d.poses, nb, cudaMemcpyDeviceToHost));
-  if (pb) SGBA_CK(cudaMemcpy(points, p->d.points, pb, cudaMemcpyDeviceToHost));
+  if (poses) SGBA_CK(cudaMemcpy(poses, p->d.poses, sizeof(double) * 7 * p->plan.nc, cudaMemcpyDeviceToHost));
+  if (points && p->plan.np > 0)
+    SGBA_CK(cudaMemcpy(points, p->d.points, sizeof(double) * 3 * p->plan.np, cudaMemcpyDeviceToHost));
   return SGBA_OK;
 }
 

@@ -1062,7 +1062,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     SGBA_CK(cudaMemsetAsync(d.intr_sum, 0, sizeof(double) * kIntrSum, p->stream));
   }
   if ((st = dev_alloc(p, &d.bf, 6 * static_cast<size_t>(P.nf)))) return st;
-  if ((st = dev_alloc(p, &d.rb, 6 * static_cast<size_t>(P.nf)))) return st;
+  if ((st = dev_alloc(p, &d.rb, static_cast<size_t>(s.n6)))) return st;  // the camera params' rows too
   if ((st = dev_alloc(p, &d.ufull, 36 * static_cast<size_t>(P.nf)))) return st;
   if ((st = dev_alloc(p, &d.tile_part, 33 * static_cast<size_t>(s.ntiles)))) return st;
   const size_t n6 = static_cast<size_t>(s.n6);

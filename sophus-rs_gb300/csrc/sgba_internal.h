@@ -237,7 +237,7 @@ struct Dev {
   double* bm = nullptr;            // nm*3: neg_grad of points
   double* bf = nullptr;            // nf*6: neg_grad of poses
   double* ufull = nullptr;         // nf*36: U_j (undamped J^T J) full 6x6
-  double* rb = nullptr;            // nf*6: reduced rhs
+  double* rb = nullptr;            // n6: reduced rhs
   double* tile_part = nullptr;     // ntiles*33 partial sums
   double* S = nullptr;             // n6*n6 FP64 (lower valid)
   float2* S2 = nullptr;            // n6*n6 float-float copy of S (cluster solver only)

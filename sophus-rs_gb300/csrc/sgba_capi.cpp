@@ -142,6 +142,8 @@ struct sgba_problem {
   int gauge_base = -1;             // gauge kind without pose priors (-1: not saved yet)
   int intr_free = 0;  // the camera params are a Free family (sgba_problem_create_ex)
   int64_t n_cam_g = 0;  // entries of the cameras' term lists
+  std::vector<int64_t> intr_chunk_g;   // free camera params: bounds of the chunks, in terms
+  std::vector<int32_t> intr_chunk_pt;  // and in points
   int camera_model = SGBA_CAMERA_PINHOLE;
   double eucm_ab[2] = {0.0, 0.0};  // EUCM alpha beta
   Sizes sz{};
@@ -1050,9 +1052,24 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   if ((st = dev_alloc(p, &d.dm, 3 * static_cast<size_t>(P.nm)))) return st;
   if ((st = dev_alloc(p, &d.gauge_um, 3 * static_cast<size_t>(P.nm)))) return st;
   if (p->intr_free) {
-    const size_t ng = static_cast<size_t>(std::max<int64_t>(P.ng, 1));
-    if ((st = dev_alloc(p, &d.intr_ty, 18 * ng))) return st;
-    if ((st = dev_alloc(p, &d.intr_tjp, 36 * ng))) return st;
+    std::vector<int64_t>& cg = p->intr_chunk_g;
+    std::vector<int32_t>& cp = p->intr_chunk_pt;
+    cg.assign(1, 0);
+    cp.assign(1, 0);
+    for (int i = 0; i < P.np; ++i)
+      if (P.pt_g_begin[i + 1] - cg.back() > sgba::kIntrChunk && i > cp.back()) {
+        cg.push_back(P.pt_g_begin[i]);
+        cp.push_back(i);
+      }
+    cg.push_back(P.ng);
+    cp.push_back(P.np);
+    s.intr_nchunk = static_cast<int>(cp.size()) - 1;
+    s.intr_chunk_g = cg.data();
+    s.intr_chunk_pt = cp.data();
+    int64_t most = 0;
+    for (size_t k = 1; k < cg.size(); ++k) most = std::max(most, cg[k] - cg[k - 1]);
+    if ((st = dev_alloc(p, &d.intr_ty, 18 * static_cast<size_t>(most)))) return st;
+    if (s.intr_nchunk == 1 && (st = dev_alloc(p, &d.intr_tjp, 36 * static_cast<size_t>(most)))) return st;
     if ((st = dev_alloc(p, &d.intr_part, sgba::intr_part_count(s)))) return st;
     if ((st = dev_alloc(p, &d.intr_ticket, 1))) return st;
     SGBA_CK(cudaMemsetAsync(d.intr_ticket, 0, sizeof(int), p->stream));

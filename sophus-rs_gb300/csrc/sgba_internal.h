@@ -24,6 +24,12 @@ constexpr int kCamTabFloats = 20;  // camera params split for the kernels (sgba_
 constexpr int kIntrPart = 33;
 constexpr int kIntrZk = 36;
 constexpr int kIntrScj = 36;
+// Terms whose J_k^T J_m and J_k^T J_p are kept (432 bytes a term, 113 MB): a
+// larger problem goes by chunks of them and forms J_k^T J_p again for its camera
+// tiles, which costs less than reading it (an iteration of 400,000 terms 1,040
+// us, 1,249 with all of them kept; 1.5M terms 3.3 and 3.9 ms).  Below, one chunk:
+// two launches fewer and the small problems' chains shorter.
+constexpr int64_t kIntrChunk = int64_t(1) << 18;
 constexpr int kIntrSum = kIntrPart + kIntrMax;
 
 // Device-resident LM control block (one per problem).  Written only by the
@@ -275,8 +281,8 @@ struct Dev {
   double* dm = nullptr;            // nm*3 point steps
   double* gauge_um = nullptr;      // nm*3 the free poses' gauge direction back-substituted into the points
   // free intrinsics (Sizes::intr_free)
-  float2* intr_ty = nullptr;       // ng*18: J_k^T J_m of each term, split
-  float2* intr_tjp = nullptr;      // ng*36: J_k^T J_p of each term, split
+  float2* intr_ty = nullptr;       // 18 a term of the largest chunk: J_k^T J_m, split
+  float2* intr_tjp = nullptr;      // ng*36: J_k^T J_p of each term, split; null with several chunks
   float2* intr_part = nullptr;     // intr_part_count: partial sums of S_kk, J_k^T r~, Zk c
   int* intr_ticket = nullptr;
   float* intr_zk = nullptr;        // nm*kIntrZk Zk = Y C^-T (6x3) as (hi, lo) pairs
@@ -404,6 +410,11 @@ struct Sizes {
   int n_eterm;         // their reduced terms (distinct (m, n))
   int intr_free;       // the camera params are Free: one more 6-row block, last in S
   int intr_nk;         // free params: 4 (pinhole, padded to 6 rows) or 6 (EUCM)
+  // chunks of whole points of at most kIntrChunk terms (nchunk + 1 bounds each,
+  // in host memory of the problem): the per-term buffers hold one
+  int intr_nchunk;
+  const int64_t* intr_chunk_g;
+  const int32_t* intr_chunk_pt;
   int eucm;            // the camera is the enhanced unified camera model (else the pinhole)
   int lmk_dd_ok;       // the chunked float-float landmark pass fits (else the warp-per-point kernel)
   int bsub_chunks_ok;  // the chunked back-substitution fits (else the warp-per-point kernel)

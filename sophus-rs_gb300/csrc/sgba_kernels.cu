@@ -2456,12 +2456,18 @@ struct IntrArgs {
   const int64_t* tile_begin;
   const int64_t* tile_end;
   const int64_t* fb_tile_begin;
-  // per term Y_g = J_k^T J_m (6x3) and J_k^T J_p (6x6), split (k_intr_terms)
+  // per term Y_g = J_k^T J_m (6x3) and J_k^T J_p (6x6), split (k_intr_terms);
+  // in several chunks: Y_g of the chunk's terms, tjp null
   float2* ty;
   float2* tjp;
+  int64_t g0, g1;  // this chunk's terms
+  int p0, p1;      // and points
   float2* ipart;   // partial sums: J_k^T J_k, J_k^T r~ per warp of terms, then - Zk Zk^T, Zk c per CTA of points
-  int* ticket;     // CTAs of k_intr_points done
+  float2* ipart_g; // this chunk's, of its terms
+  float2* ipart_p; // and of its points
+  int* ticket;     // CTAs of the last chunk's k_intr_points done; null before it
   int nterm_part;  // warps of terms
+  int npoint_part; // CTAs of points
   float* zk;       // nm x kIntrZk: Zk (6x3) as (hi, lo)
   double* scj;     // per quarter tile kIntrScj: its part of S_kj (6x6)
   double* isum;    // kIntrPart sums, then -sum J_k^T r~ (6)
@@ -2542,13 +2548,13 @@ constexpr int kIntrOwn = kKT + kK;  // 27 sums
 __global__ void __launch_bounds__(kIntrTermT) k_intr_terms(IntrArgs a, const Ctrl* ctrl) {
   if (halted(ctrl)) return;
   __shared__ float red[kIntrTermT / 32][kIntrOwn][33];
-  const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t g = a.g0 + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const dd zero = dd_make(0.f, 0.f);
   dd own[kIntrOwn];
 #pragma unroll
   for (int k = 0; k < kIntrOwn; ++k) own[k] = zero;
-  if (g < a.ng) {
+  if (g < a.g1) {
     const CamD cam = cam_dd(a.cam);
     const int i = a.g_pt[g];
     JacD J;
@@ -2566,8 +2572,8 @@ __global__ void __launch_bounds__(kIntrTermT) k_intr_terms(IntrArgs a, const Ctr
       r0 = dd_add(r0, w0);
       r1 = dd_add(r1, w1);
     }
-    float2* ty = a.ty + 18 * g;
-    float2* tj = a.tjp + 36 * g;
+    float2* ty = a.ty + 18 * (g - a.g0);
+    float2* tj = a.tjp ? a.tjp + 36 * g : nullptr;
     int k = 0;
 #pragma unroll
     for (int p = 0; p < kK; ++p) {
@@ -2580,21 +2586,22 @@ __global__ void __launch_bounds__(kIntrTermT) k_intr_terms(IntrArgs a, const Ctr
         const dd t = dd_add(dd_mul(u, J.jm[q]), dd_mul(v, J.jm[3 + q]));
         ty[3 * p + q] = make_float2(t.hi, t.lo);
       }
+      if (tj)
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        const dd t = dd_add(dd_mul(u, J.jp[q]), dd_mul(v, J.jp[6 + q]));
-        tj[6 * p + q] = make_float2(t.hi, t.lo);
-      }
+        for (int q = 0; q < 6; ++q) {
+          const dd t = dd_add(dd_mul(u, J.jp[q]), dd_mul(v, J.jp[6 + q]));
+          tj[6 * p + q] = make_float2(t.hi, t.lo);
+        }
     }
   }
   const dd t = intr_warp_sum<kIntrOwn>(own, red[wib]);
   if (lane < kIntrOwn)
-    a.ipart[kIntrOwn * (static_cast<int64_t>(blockIdx.x) * (kIntrTermT / 32) + wib) + lane] = make_float2(t.hi, t.lo);
+    a.ipart_g[kIntrOwn * (static_cast<int64_t>(blockIdx.x) * (kIntrTermT / 32) + wib) + lane] = make_float2(t.hi, t.lo);
 }
 
 // A warp per point: Y over its terms, with the point's C^-1 (landmark pass)
-// Zk = Y C^-T and its parts of S_kk (subtracted) and of rhs_k; the last CTA to
-// finish sums every partial in order and forms the intrinsics' neg_grad
+// Zk = Y C^-T and its parts of S_kk (subtracted) and of rhs_k; the last CTA of the
+// last chunk to finish sums every partial in order and forms the intrinsics' neg_grad
 // -sum J_k^T r~, which joins the gradient-tolerance maximum.
 constexpr int kIntrPtWarps = 8;
 __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, Ctrl* ctrl) {
@@ -2616,14 +2623,14 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
     p = lane - kKT;
   }
   dd acc = zero;
-  for (int i = blockIdx.x * kIntrPtWarps + wib; i < a.np; i += gridDim.x * kIntrPtWarps) {
+  for (int i = a.p0 + blockIdx.x * kIntrPtWarps + wib; i < a.p1; i += gridDim.x * kIntrPtWarps) {
     const int mb = a.pt_mb[i];
     const int64_t g0 = a.pt_g_begin[i], g1 = a.pt_g_begin[i + 1];
     if (mb < 0 || g1 == g0) continue;  // the whole warp
     if (lane < 3 * kK) {
       dd y = zero;
       for (int64_t g = g0; g < g1; ++g) {
-        const float2 v = a.ty[18 * g + lane];
+        const float2 v = a.ty[18 * (g - a.g0) + lane];
         y = dd_add(y, dd_make(v.x, v.y));
       }
       sy[wib][lane] = make_float2(y.hi, y.lo);
@@ -2653,12 +2660,12 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
   }
   if (lane < kIntrOwn) sp[wib][lane] = make_float2(acc.hi, acc.lo);
   __syncthreads();
-  float2* pts = a.ipart + static_cast<int64_t>(kIntrOwn) * a.nterm_part;
   if (threadIdx.x < kIntrOwn) {
     dd t = zero;
     for (int w = 0; w < kIntrPtWarps; ++w) t = dd_add(t, dd_make(sp[w][threadIdx.x].x, sp[w][threadIdx.x].y));
-    pts[static_cast<int64_t>(kIntrOwn) * blockIdx.x + threadIdx.x] = make_float2(t.hi, t.lo);
+    a.ipart_p[static_cast<int64_t>(kIntrOwn) * blockIdx.x + threadIdx.x] = make_float2(t.hi, t.lo);
   }
+  if (!a.ticket) return;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = atomicAdd(a.ticket, 1) == static_cast<int>(gridDim.x) - 1;
@@ -2668,8 +2675,8 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
   // the partials: those of the terms, then those of the points; eight warps take
   // ranges of them, a lane per value, and the ranges are added in order
   for (int part = 0; part < 2; ++part) {
-    const float2* src = part == 0 ? a.ipart : pts;
-    const int n = part == 0 ? a.nterm_part : static_cast<int>(gridDim.x);
+    const float2* src = part == 0 ? a.ipart : a.ipart + static_cast<int64_t>(kIntrOwn) * a.nterm_part;
+    const int n = part == 0 ? a.nterm_part : a.npoint_part;
     dd t = zero;
     if (lane < kIntrOwn)
       for (int k = n * wib / kIntrPtWarps; k < n * (wib + 1) / kIntrPtWarps; ++k) {
@@ -2704,7 +2711,9 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
 
 // S_kj = sum over pose j's terms of J_k^T J_p - Zk_i Z_g^T: a CTA per quarter of
 // a camera tile, a thread per term; k_intr_fill adds a pose's parts.
+// STORED: J_k^T J_p from k_intr_terms; else formed here again.
 constexpr int kIntrCamT = 64;
+template <bool STORED>
 __global__ void __launch_bounds__(kIntrCamT) k_intr_cams(IntrArgs a, const Ctrl* ctrl) {
   if (halted(ctrl)) return;
   constexpr int kE = kK * 6;
@@ -2733,14 +2742,30 @@ __global__ void __launch_bounds__(kIntrCamT) k_intr_cams(IntrArgs a, const Ctrl*
       }
     }
   }
+  [[maybe_unused]] JacD J;
+  [[maybe_unused]] dd jk[2 * kK];
+  if constexpr (!STORED) {
+    if (on) {
+      const int i = a.g_pt[g];
+      intr_term_jacobians(a.pose_dd + 24 * static_cast<int64_t>(a.g_pose[g]), pt_dd(a.pts, i, 0), pt_dd(a.pts, i, 1),
+                          pt_dd(a.pts, i, 2), cam_dd(a.cam), a.nk, &J, jk);
+      const float cnt = static_cast<float>(a.g_begin[g + 1] - a.g_begin[g]);
+#pragma unroll
+      for (int k = 0; k < 2 * kK; ++k) jk[k] = dd_mul_f(jk[k], cnt);
+    }
+  }
 #pragma unroll
   for (int p = 0; p < kK; ++p)
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
       dd v = zero;
       if (on) {
-        const float2 j = a.tjp[36 * g + 6 * p + q];
-        v = dd_make(j.x, j.y);
+        if constexpr (STORED) {
+          const float2 j = a.tjp[36 * g + 6 * p + q];
+          v = dd_make(j.x, j.y);
+        } else {
+          v = dd_add(dd_mul(jk[p], J.jp[q]), dd_mul(jk[kK + p], J.jp[6 + q]));
+        }
         if (mb >= 0) {
           dd t = zero;
 #pragma unroll
@@ -2817,7 +2842,7 @@ int intr_term_parts(int64_t ng) {
 int intr_point_blocks(int np) { return np > 0 ? std::min((np + kIntrPtWarps - 1) / kIntrPtWarps, 608) : 1; }
 
 IntrArgs intr_args(const Sizes& s, const Dev& d) {
-  IntrArgs a;
+  IntrArgs a{};
   a.np = s.np;
   a.nf = s.nf;
   a.n6 = s.n6;
@@ -2847,8 +2872,6 @@ IntrArgs intr_args(const Sizes& s, const Dev& d) {
   a.ty = d.intr_ty;
   a.tjp = d.intr_tjp;
   a.ipart = d.intr_part;
-  a.ticket = d.intr_ticket;
-  a.nterm_part = intr_term_parts(s.ng);
   a.zk = d.intr_zk;
   a.scj = d.intr_scj;
   a.isum = d.intr_sum;
@@ -2861,11 +2884,37 @@ IntrArgs intr_args(const Sizes& s, const Dev& d) {
 
 int launch_intr_linearize(const Sizes& s, const Dev& d, cudaStream_t st) {
   if (!s.intr_free) return 0;
-  const IntrArgs a = intr_args(s, d);
-  if (s.ng > 0) k_intr_terms<<<a.nterm_part / (kIntrTermT / 32), kIntrTermT, 0, st>>>(a, d.ctrl);
-  k_intr_points<<<intr_point_blocks(s.np), 32 * kIntrPtWarps, 0, st>>>(a, d.ctrl);
-  if (s.ntiles > 0) k_intr_cams<<<static_cast<unsigned>(4 * s.ntiles), kIntrCamT, 0, st>>>(a, d.ctrl);
-  return 1 + (s.ng > 0 ? 1 : 0) + (s.ntiles > 0 ? 1 : 0);
+  IntrArgs a = intr_args(s, d);
+  for (int c = 0; c < s.intr_nchunk; ++c) {
+    a.nterm_part += intr_term_parts(s.intr_chunk_g[c + 1] - s.intr_chunk_g[c]);
+    a.npoint_part += intr_point_blocks(s.intr_chunk_pt[c + 1] - s.intr_chunk_pt[c]);
+  }
+  a.ipart_g = a.ipart;
+  a.ipart_p = a.ipart + static_cast<int64_t>(kIntrOwn) * a.nterm_part;
+  int n = 0;
+  for (int c = 0; c < s.intr_nchunk; ++c) {
+    a.g0 = s.intr_chunk_g[c];
+    a.g1 = s.intr_chunk_g[c + 1];
+    a.p0 = s.intr_chunk_pt[c];
+    a.p1 = s.intr_chunk_pt[c + 1];
+    a.ticket = c + 1 == s.intr_nchunk ? d.intr_ticket : nullptr;
+    const int tp = intr_term_parts(a.g1 - a.g0), pb = intr_point_blocks(a.p1 - a.p0);
+    if (tp > 0) {
+      k_intr_terms<<<tp / (kIntrTermT / 32), kIntrTermT, 0, st>>>(a, d.ctrl);
+      ++n;
+    }
+    k_intr_points<<<pb, 32 * kIntrPtWarps, 0, st>>>(a, d.ctrl);
+    ++n;
+    a.ipart_g += static_cast<int64_t>(kIntrOwn) * tp;
+    a.ipart_p += static_cast<int64_t>(kIntrOwn) * pb;
+  }
+  if (s.ntiles > 0) {
+    const unsigned grid = static_cast<unsigned>(4 * s.ntiles);
+    if (a.tjp) k_intr_cams<true><<<grid, kIntrCamT, 0, st>>>(a, d.ctrl);
+    else k_intr_cams<false><<<grid, kIntrCamT, 0, st>>>(a, d.ctrl);
+    ++n;
+  }
+  return n;
 }
 
 int launch_intr_fill(const Sizes& s, const Dev& d, cudaStream_t st) {
@@ -4378,7 +4427,11 @@ int batch_launch_collect(const BatchTables* t, Ctrl* ctrl_out, Record* rec_out, 
 }
 
 size_t intr_part_count(const Sizes& s) {
-  return static_cast<size_t>(kIntrOwn) * (static_cast<size_t>(intr_term_parts(s.ng)) + intr_point_blocks(s.np));
+  size_t n = 0;
+  for (int c = 0; c < s.intr_nchunk; ++c)
+    n += static_cast<size_t>(intr_term_parts(s.intr_chunk_g[c + 1] - s.intr_chunk_g[c])) +
+         static_cast<size_t>(intr_point_blocks(s.intr_chunk_pt[c + 1] - s.intr_chunk_pt[c]));
+  return static_cast<size_t>(kIntrOwn) * n;
 }
 
 }  // namespace sgba

@@ -1936,8 +1936,10 @@ struct SchurDenseArgs {
   const double* cnt_f;
   double* S;
   float2* S2;
-  float* rounds;  // split pass: the sums of every round of every tile
-  int nsplit;     // split pass: CTAs of a tile
+  float* rounds;  // split pass: the sums of its rounds of every tile
+  float2* carry;  // the tiles' sums so far, between passes
+  int nsplit;     // CTAs of a tile
+  int round0, nrounds;  // the rounds of this pass
 };
 
 constexpr size_t schur_dense_smem(int G) {
@@ -1988,7 +1990,7 @@ __device__ __forceinline__ void schur_dense_store(const SchurDenseArgs& a, doubl
   }
 }
 
-// SPLIT: a.nsplit CTAs of a tile take ranges of its rounds and leave each
+// SPLIT: a.nsplit CTAs of a tile take ranges of the pass's rounds and leave each
 // round's sums in a.rounds; k_schur_dense_sum adds them in the order of the
 // rounds, so S keeps its bits.
 template <int G, bool SPLIT = false>
@@ -2005,17 +2007,18 @@ __device__ __forceinline__ void schur_dense_body(const SchurDenseArgs& a, const 
   const int I0 = ti * kSdB, J0 = tj * kSdB;
   const int tid = threadIdx.x, grp = tid / kSdGroup, t = tid % kSdGroup;
   const bool diag = ti == tj;  // one set of records
-  const int nround = (a.np + kSdPts - 1) / kSdPts;
+  const int nround = SPLIT ? a.nrounds : (a.np + kSdPts - 1) / kSdPts;
   const int nsuper = (nround + G - 1) / G;
   const int super0 = SPLIT ? static_cast<int>(static_cast<int64_t>(nsuper) * part / a.nsplit) : 0;
   const int super1 = SPLIT ? static_cast<int>(static_cast<int64_t>(nsuper) * (part + 1) / a.nsplit) : nsuper;
+  const int point0 = SPLIT ? a.round0 * kSdPts : 0;
   const int nstage = (super1 - super0) * kStages;  // of every group (rounds past the end copy zeros)
   // this thread's record of a stage: point pp, slot (0..7 row poses, 8..15 column poses)
   const int pp = t >> 4, slot = t & 15;
   const int f = slot < kSdB ? I0 + slot : J0 + slot - kSdB;
   const bool mine = (slot < kSdB || !diag) && f < a.nf;
   auto term_of = [&](int s) {
-    const int i = ((super0 + s / kStages) * G + grp) * kSdPts + (s % kStages) * kSdStage + pp;
+    const int i = point0 + ((super0 + s / kStages) * G + grp) * kSdPts + (s % kStages) * kSdStage + pp;
     return (mine && s < nstage && i < a.np) ? __ldg(a.zterm + static_cast<int64_t>(i) * a.nf + f) : -1;
   };
   auto copy = [&](int s, int g) {
@@ -2103,21 +2106,27 @@ __global__ void __launch_bounds__(kSdGroup * G, G > 2 ? 1 : 4) k_schur_dense(Sch
 __global__ void __launch_bounds__(kSdGroup * 2, 4) k_schur_dense_split(SchurDenseArgs a, const Ctrl* ctrl) {
   schur_dense_body<2, true>(a, ctrl, blockIdx.x);
 }
-// The rounds of a tile added in order, a thread per entry.
+// The pass's rounds of a tile added in order to those before, a thread per entry;
+// `last`: the sums into S.
 constexpr int kSdSumT = 128;
 static_assert(kSdEntries % kSdSumT == 0, "whole CTAs");
-__global__ void __launch_bounds__(kSdSumT) k_schur_dense_sum(SchurDenseArgs a, const Ctrl* ctrl) {
+__global__ void __launch_bounds__(kSdSumT) k_schur_dense_sum(SchurDenseArgs a, int last, const Ctrl* ctrl) {
   if (skipping(ctrl)) return;
   constexpr int kPerTile = kSdEntries / kSdSumT;
   const int tile = blockIdx.x / kPerTile, e = (blockIdx.x % kPerTile) * kSdSumT + threadIdx.x;
   int ti, tj;
   schur_dense_tile(tile, &ti, &tj);
-  const int nround = (a.np + kSdPts - 1) / kSdPts;
-  const float* src = a.rounds + static_cast<int64_t>(tile) * nround * kSdEntries + e;
+  const float* src = a.rounds + static_cast<int64_t>(tile) * a.nrounds * kSdEntries + e;
+  float2* carry = a.carry + static_cast<int64_t>(tile) * kSdEntries + e;
   Acc sum = acc_zero();
+  if (a.round0 > 0) {
+    const float2 c = *carry;
+    sum = Acc{c.x, c.y};
+  }
 #pragma unroll 16
-  for (int r = 0; r < nround; ++r) acc_addf(sum, src[static_cast<int64_t>(r) * kSdEntries]);
-  schur_dense_store(a, ctrl->nu, ti * kSdB, tj * kSdB, e, sum);
+  for (int r = 0; r < a.nrounds; ++r) acc_addf(sum, src[static_cast<int64_t>(r) * kSdEntries]);
+  if (last) schur_dense_store(a, ctrl->nu, ti * kSdB, tj * kSdB, e, sum);
+  else *carry = make_float2(sum.hi, sum.lo);
 }
 
 // ---------------------------------------------------------------------------
@@ -3594,12 +3603,25 @@ static int schur_dense_grid(const Sizes& s) {
 
 // Few tiles leave most SMs idle (a tile's rounds are 0.5 us each, eight at a
 // time): up to half an SM count of tiles the rounds are spread over ~608 CTAs
-// and summed by a second launch, where their sums fit in 64 MB (10 cameras and
-// 500 points: 35 -> 8 us).  0 floats: not split.
-size_t schur_split_floats(const Sizes& s) {
+// and summed by a second launch (10 cameras and 500 points: 35 -> 8 us).  Where
+// their sums take more than kSdRoundBytes, which the problem keeps, by passes of
+// that many; beyond kSdSplitBytes in all not split.  The bound holds one pass of
+// the largest local maps (40 cameras, 4,000 points: 35 MB); with 16 MB, three
+// passes, an iteration of theirs took 686 us in place of 669.
+constexpr size_t kSdRoundBytes = size_t(36) << 20, kSdSplitBytes = size_t(64) << 20;
+
+// rounds of a pass (a multiple of the split kernel's two groups); 0: not split
+static int schur_split_rounds(const Sizes& s) {
   if (!s.schur_dense || schur_dense_grid(s) > 76) return 0;
-  const size_t f = static_cast<size_t>(schur_dense_grid(s)) * ((s.np + kSdPts - 1) / kSdPts) * kSdEntries;
-  return f * sizeof(float) <= (64u << 20) ? f : 0;
+  const int nround = (s.np + kSdPts - 1) / kSdPts;
+  const size_t per = sizeof(float) * kSdEntries * static_cast<size_t>(schur_dense_grid(s));
+  if (per * static_cast<size_t>(nround) > kSdSplitBytes) return 0;
+  return std::min(static_cast<int>(kSdRoundBytes / per) & ~1, (nround + 1) & ~1);
+}
+
+// Dev::sd_rounds: the rounds of a pass and the sums between passes (0: not split)
+size_t schur_split_floats(const Sizes& s) {
+  return static_cast<size_t>(schur_dense_grid(s)) * kSdEntries * (schur_split_rounds(s) > 0 ? schur_split_rounds(s) + 2 : 0);
 }
 
 // Eight groups a CTA up to this many tiles (one CTA an SM), two beyond.
@@ -3622,11 +3644,18 @@ int launch_schur(const Sizes& s, const Dev& d, cudaStream_t st) {
     const int grid = schur_dense_grid(s);
     if (d.sd_rounds) {
       SchurDenseArgs a = make_schur_dense_args(s, d);
-      const int nsuper = (s.np + 2 * kSdPts - 1) / (2 * kSdPts);
-      a.nsplit = std::max(1, std::min(nsuper, 608 / grid));
-      k_schur_dense_split<<<grid * a.nsplit, kSdGroup * 2, schur_dense_smem(2), st>>>(a, d.ctrl);
-      k_schur_dense_sum<<<grid * (kSdEntries / kSdSumT), kSdSumT, 0, st>>>(a, d.ctrl);
-      return 2 + launch_intr_fill(s, d, st);
+      const int nround = (s.np + kSdPts - 1) / kSdPts, per = schur_split_rounds(s);
+      a.carry = reinterpret_cast<float2*>(d.sd_rounds + static_cast<size_t>(grid) * kSdEntries * per);
+      int n = 0;
+      for (int r = 0; r < nround; r += per) {
+        a.round0 = r;
+        a.nrounds = std::min(per, nround - r);
+        a.nsplit = std::max(1, std::min((a.nrounds + 1) / 2, 608 / grid));
+        k_schur_dense_split<<<grid * a.nsplit, kSdGroup * 2, schur_dense_smem(2), st>>>(a, d.ctrl);
+        k_schur_dense_sum<<<grid * (kSdEntries / kSdSumT), kSdSumT, 0, st>>>(a, r + per >= nround, d.ctrl);
+        n += 2;
+      }
+      return n + launch_intr_fill(s, d, st);
     }
     if (grid <= kSdWide) k_schur_dense<8><<<grid, kSdGroup * 8, schur_dense_smem(8), st>>>(make_schur_dense_args(s, d), d.ctrl);
     else k_schur_dense<2><<<grid, kSdGroup * 2, schur_dense_smem(2), st>>>(make_schur_dense_args(s, d), d.ctrl);

@@ -272,7 +272,7 @@ struct Dev {
   int32_t* band_zloc = nullptr;    // 1
   float* A = nullptr;              // n6*n6 FP32 factor (lower: unit L)
   float* dpiv = nullptr;           // n6 pivots
-  float* wpanel = nullptr;         // n6*64 panel scratch (A_ip L^-T)
+  float* wpanel = nullptr;         // n6*48 panel scratch (the diagonal block's factor, A_ip L^-T below it)
   float* sd_rounds = nullptr;      // sums of the tiled Schur pass per round of a pass (schur_split_floats), single problems
   double* x = nullptr;             // n6 solution / refinement
   double* x0 = nullptr;            // 6 nf: x before the gauge projection

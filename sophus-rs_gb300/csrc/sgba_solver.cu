@@ -40,8 +40,10 @@ __global__ void k_s_to_f32(int n, const double* __restrict__ S, float* __restric
 
 // Panel step: factor the w x w diagonal block at (c0, c0) and solve the rows
 // below it.  Every CTA factors the diagonal block redundantly in shared memory
-// (no grid-wide dependency); CTA 0 writes it back.  Then each thread owns one
-// row i >= c0 + w:  y = a_i L_pp^-T (= L_i d), L_i = y / d.
+// (no grid-wide dependency); CTA 0 leaves the factor in rows c0 .. c0 + w - 1 of
+// wpanel, from where k_ldlt_update moves it to A: a CTA that starts late still
+// finds the unfactored block there.  Then each thread owns one row i >= c0 + w:
+// y = a_i L_pp^-T (= L_i d), L_i = y / d.
 constexpr int kPanelThreads = 256;
 constexpr int kLowerPairs = kPW * (kPW - 1) / 2;
 
@@ -101,8 +103,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_ldlt_panel(int n, int c0, int
   if (blockIdx.x == 0) {
     for (int e = tid; e < w * w; e += blockDim.x) {
       const int i = e / w, k = e % w;
-      if (k < i) A[static_cast<int64_t>(c0 + i) * n + c0 + k] = a[i][k];
-      else if (k == i) A[static_cast<int64_t>(c0 + i) * n + c0 + k] = 1.0f;
+      if (k <= i) wpanel[static_cast<int64_t>(c0 + i) * kPW + k] = k < i ? a[i][k] : 1.0f;
     }
     for (int t = tid; t < w; t += blockDim.x) dpiv[c0 + t] = dsh[t];
     if (tid == 0 && s_bad) ctrl->skip = 2;  // NonFinitePivot -> solve failure -> reject
@@ -133,11 +134,16 @@ __global__ void __launch_bounds__(kPanelThreads) k_ldlt_panel(int n, int c0, int
 }
 
 // Trailing update A[i][k] -= sum_t W[i][t] L[k][t] for c1 <= k <= i < n,
-// 32x32 lower tiles.
+// 32x32 lower tiles; CTA 0 also stores the factored diagonal block.
 __global__ void __launch_bounds__(256) k_ldlt_update(int n, int c0, int w, float* __restrict__ A,
                                                      const float* __restrict__ wpanel, const Ctrl* ctrl) {
   if (skipping(ctrl)) return;
   const int c1 = c0 + w;
+  if (blockIdx.x == 0)
+    for (int q = threadIdx.x; q < w * w; q += blockDim.x) {
+      const int i = q / w, t = q % w;
+      if (t <= i) A[static_cast<int64_t>(c0 + i) * n + c0 + t] = wpanel[static_cast<int64_t>(c0 + i) * kPW + t];
+    }
   // decode the lower tile (I, K), I >= K
   const int e = blockIdx.x;
   int I = static_cast<int>((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
@@ -306,7 +312,7 @@ int launch_exact_solve(const Sizes& s, const Dev& d, cudaStream_t st) {
       const int nt = (rows + 31) / 32;
       k_ldlt_update<<<nt * (nt + 1) / 2, 256, 0, st>>>(n, c0, w, d.A, d.wpanel, d.ctrl);
     } else {
-      k_ldlt_update<<<1, 256, 0, st>>>(n, n, 0, d.A, d.wpanel, d.ctrl);  // fixed graph shape
+      k_ldlt_update<<<1, 256, 0, st>>>(n, c0, w, d.A, d.wpanel, d.ctrl);  // the diagonal block alone
     }
     launches += 2;
   }

@@ -170,6 +170,7 @@ struct sgba_problem {
   size_t chunk_size = size_t(1) << 20;
   // covariance of the solution (sgba_covariance_prepare)
   sgba::CovBufs cov;
+  int64_t points_at = 0;   // doubles from the poses to the points in one gathered block (0: apart)
   Stage* stage = nullptr;  // gathers the small uploads while the problem is being set up
   bool pairs_built = true;  // the Schur pair lists exist (not for the tiled pass of nearly dense systems)
 };
@@ -1036,6 +1037,14 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   }
   if ((st = dev_upload(p, &d.poses, poses))) return st;
   if ((st = dev_upload(p, &d.points, pts))) return st;
+  {
+    const Stage* g = p->stage;
+    auto gathered = [&](const double* v) {
+      const char* c = reinterpret_cast<const char*>(v);
+      return g->cap > 0 && c >= g->dev && c < g->dev + g->cap;
+    };
+    if (gathered(d.poses) && gathered(d.points)) p->points_at = d.points - d.poses;
+  }
   if ((st = dev_alloc(p, &d.poses_t, 7 * static_cast<size_t>(P.nc)))) return st;
   if ((st = dev_alloc(p, &d.points_t, 3 * static_cast<size_t>(P.np)))) return st;
   if ((st = dev_alloc(p, &d.res, P.no))) return st;
@@ -1553,6 +1562,15 @@ int sgba_get_variables(sgba_problem* p, double* poses, double* points) {
   if (!p) return set_error(SGBA_ERR_INVALID_ARGUMENT, "NULL problem");
   SGBA_CK(cudaSetDevice(p->device));
   SGBA_CK(cudaStreamSynchronize(p->stream));
+  if (poses && points && p->points_at > 0) {  // a small problem: one copy for both
+    const size_t n = static_cast<size_t>(p->points_at) + 3 * static_cast<size_t>(p->plan.np);
+    std::unique_ptr<double[]> h(new (std::nothrow) double[n]);
+    if (!h) return set_error(SGBA_ERR_OUT_OF_MEMORY, "host allocation failed");
+    SGBA_CK(cudaMemcpy(h.get(), p->d.poses, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    std::memcpy(poses, h.get(), sizeof(double) * 7 * p->plan.nc);
+    std::memcpy(points, h.get() + p->points_at, sizeof(double) * 3 * p->plan.np);
+    return SGBA_OK;
+  }
   if (poses) SGBA_CK(cudaMemcpy(poses, p->d.poses, sizeof(double) * 7 * p->plan.nc, cudaMemcpyDeviceToHost));
   if (points && p->plan.np > 0)
     SGBA_CK(cudaMemcpy(points, p->d.points, sizeof(double) * 3 * p->plan.np, cudaMemcpyDeviceToHost));

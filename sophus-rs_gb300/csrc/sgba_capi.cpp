@@ -111,7 +111,7 @@ struct EventSet {
   }
 };
 
-constexpr int kTile = 256;           // terms per camera tile (one CTA)
+constexpr int kTile = sgba::kCamTile;
 constexpr int64_t kSchurChunk = 256;  // observation pairs per warp in the Schur assembly (at most)
 constexpr int64_t kSchurWarps = 152 * 16;  // warps of the assembly that run at once
 constexpr int32_t kMaxDenseFree = 4096;  // reduced-camera-system limit (6 * 4096 rows, stored dense in f64)

@@ -947,9 +947,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_dense_cluster(DenseArgs a, Ctrl
 // (cluster barriers, a large code footprint that starts cold on each SM)
 // dominate at this size.
 //
-// Bound: the serial pivot chain (rcp, scale, update: ~110 cycles a pivot) for
-// small systems, FP32 issue (n^3 / 6 float-float products of 12 operations on
-// one SM) for large ones.  So the elimination goes by panels of one pose block
+// Bound: FP32 issue (n^3 / 6 float-float products of 12 operations on one SM) for
+// large systems.  Small ones are latency: 31 us for 54 rows, of which the serial
+// pivot chain (rcp, scale, update: ~110 cycles a pivot) is 3; the rest is
+// barriers, the panel and backward phases' short loops and their instructions,
+// fetched cold by the one CTA.  The elimination goes by panels of one pose block
 // (6 pivots, the span of the pivot rule's running maximum): one warp factors
 // the 6 x 6 block in registers, a thread per row solves the panel, and the
 // trailing triangle takes all six columns at once in register tiles (RT x RT

@@ -12,13 +12,14 @@
 
 namespace sgba {
 
-// floats per term of the float-float Z (6x3 as (hi, lo) pairs, padded to float4)
+constexpr int kCamTile = 256;   // terms of a camera tile (one CTA)
 constexpr int kBandMaxW = 288;  // widest band the banded solver factors (a dissected loop's corner)
+// floats per term of the float-float Z (6x3 as (hi, lo) pairs, padded to float4)
 constexpr int kZddFloats = 40;
 // Camera params on the device: fx fy cx cy alpha beta (the enhanced unified
-// camera model; alpha = beta = 0 is the pinhole).  Free intrinsics: per point
-// the S_kk triangle (21), J_k^T r~ (6) and Zk c (6); per marg point Zk (6x3,
-// float-float); per free pose S_kj (6x6).
+// camera model; alpha = beta = 0 is the pinhole).  Free intrinsics: the sums
+// (kIntrPart) are the S_kk triangle (21), J_k^T r~ (6) and Zk c (6); per marg
+// point Zk (6x3, float-float); per quarter of a camera tile its part of S_kj (6x6).
 constexpr int kIntrMax = 6;
 constexpr int kCamTabFloats = 20;  // camera params split for the kernels (sgba_kernels.cu)
 constexpr int kIntrPart = 33;
@@ -442,12 +443,13 @@ int launch_decide(const Sizes& s, const Dev& d, cudaStream_t st);
 
 int launch_single(const Sizes& s, const Dev& d, int kernel_id, cudaStream_t st);
 int cost_partials_needed(const Sizes& s);  // reduction partial slots
-int landmark_setup(int cap);
 size_t intr_part_count(const Sizes& s);  // partial sums of the free intrinsics (float2)
 size_t schur_split_floats(const Sizes& s);  // Dev::sd_rounds of the tiled Schur pass of few tiles (0: not split)
-int schur_dd_setup();     // of the float-float Schur pass
-int schur_dense_setup();  // shared memory limits of the tiled Schur pass (0: ok)  // dynamic shared memory of the chunked landmark pass (0 = ok)
-int landmark_dd_setup(int cap);  // the same for its float-float variant (0 = ok)
+// dynamic shared memory (0 = ok)
+int schur_dense_setup();         // of the tiled Schur pass
+int schur_dd_setup();            // of the float-float Schur pass
+int landmark_setup(int cap);     // of the chunked landmark pass
+int landmark_dd_setup(int cap);  // of its float-float variant
 int backsub_chunks_setup(int cap);  // the chunked back-substitution (0 = ok)
 int solver_launch_count(const Sizes& s);
 

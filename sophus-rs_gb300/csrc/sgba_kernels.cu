@@ -124,10 +124,10 @@ struct CamD {
 };
 // The camera params as the kernels read them: fx fy alpha beta in FP32, then fx
 // fy cx cy alpha beta 1 - alpha as (hi, lo) pairs.  The f64 values are split
-// once per evaluation point (k_pose_tables, k_apply_update): GB300's FP64 pipe
-// takes a warp 16 cycles per operation, and the splits of the camera, of the
-// points and of the pixels, done per observation, held that pipe at 75 % in
-// the trial cost (windows; 149 us per 1.9M observations, ncu).
+// once per evaluation point (k_pose_tables, k_apply_update): the FP64 pipe of an
+// SM sub-partition takes a warp's instruction 64 cycles, and the splits of the
+// camera, of the points and of the pixels, done per observation, held that pipe
+// at 75 % in the trial cost (windows; 149 us per 1.9M observations, ncu).
 constexpr int kCamTab = 4 + 2 * 7;
 static_assert(kCamTab <= kCamTabFloats, "the camera table fits its allocation");
 __device__ __forceinline__ void cam_table(const double* intr, float* tab) {
@@ -1277,7 +1277,7 @@ __global__ void __launch_bounds__(256) k_landmark_chunks_dd(LinArgs a, Ctrl* ctr
 // reduced-rhs term sum Z_g (C^-1 b_m).  FP32 warp sums, float-float across
 // warps; the Z c products in float-float.
 // ---------------------------------------------------------------------------
-constexpr int kTileThreads = 256;
+constexpr int kTileThreads = kCamTile;
 constexpr int kTileVals = 33;
 
 struct CamArgs {
@@ -2436,9 +2436,9 @@ __global__ void __launch_bounds__(256) k_backsub_chunks(BackArgs a, const int32_
 // ---------------------------------------------------------------------------
 constexpr int kK = kIntrMax;           // 6 params per J_k row
 constexpr int kKT = kK * (kK + 1) / 2;  // 21 entries of the S_kk triangle
-constexpr int kIntrG = kKT;             // offset of J_k^T r~ in a point's part
+constexpr int kIntrG = kKT;             // offset of J_k^T r~ in the sums
 constexpr int kIntrZc = kKT + kK;       // offset of Zk c
-static_assert(kIntrZc + kK == kIntrPart, "per-point intrinsics part layout");
+static_assert(kIntrZc + kK == kIntrPart, "layout of the intrinsics' sums");
 
 struct IntrArgs {
   int np, nf, n6;
@@ -2722,6 +2722,7 @@ __global__ void __launch_bounds__(32 * kIntrPtWarps) k_intr_points(IntrArgs a, C
 // a camera tile, a thread per term; k_intr_fill adds a pose's parts.
 // STORED: J_k^T J_p from k_intr_terms; else formed here again.
 constexpr int kIntrCamT = 64;
+static_assert(4 * kIntrCamT == kCamTile, "four CTAs a camera tile");
 template <bool STORED>
 __global__ void __launch_bounds__(kIntrCamT) k_intr_cams(IntrArgs a, const Ctrl* ctrl) {
   if (halted(ctrl)) return;

@@ -43,9 +43,10 @@ __device__ __forceinline__ void pose_table(const double* T, float* pf, float* pd
 // its FP64 operations (~170 of them, and two sincos, two square roots, three
 // divisions).  Here the entries of each small matrix, the two angles and the
 // three divisions lie in lanes.  Which product of a sum is fused and which is
-// rounded first is spelled out as the compiler chose it for the plain
-// expressions of rot_matrix and of the update in one thread, so the trial poses
-// kept their bits (a last-place change of a pose flips FP32 roundings later on).
+// rounded first is spelled out, and is this function's own definition; it was
+// settled by comparing outputs with one thread's plain expressions, which the
+// tables have to match: pose_table forms them from the same pose at the next
+// linearisation, and a last-place change of a pose flips FP32 roundings there.
 __device__ __forceinline__ double pose_neg(double x, bool n) {
   return n ? __longlong_as_double(__double_as_longlong(x) ^ (1ll << 63)) : x;
 }

@@ -116,16 +116,18 @@ constexpr int64_t kSchurChunk = 256;  // observation pairs per warp in the Schur
 constexpr int64_t kSchurWarps = 152 * 16;  // warps of the assembly that run at once
 constexpr int32_t kMaxDenseFree = 4096;  // reduced-camera-system limit (6 * 4096 rows, stored dense in f64)
 
-// The small arrays of a problem being set up gather in a block of host memory
-// and go to the device in one copy: every copy takes the driver's lock, and 24
-// windows created by 16 threads spent most of 10 ms in 620 of them (7.5 ms so;
-// a page-locked block gave the same).  At most kStageBytes; the holder waits
-// for the copies before the object goes.
-constexpr size_t kStageBytes = size_t(4) << 20;
+// The arrays of a small problem being set up, and those of up to kStageArray of a
+// larger one, gather in a block of host memory and go to the device in one copy:
+// every copy takes the driver's lock, and 24 windows created by 16 threads spent
+// most of 10 ms in 620 of them (7.5 ms so; a page-locked block gave the same).
+// Larger arrays of larger problems go by themselves: gathering them too only
+// copied them once more (100-camera sphere: create, read and close 1.87 ms, 1.71
+// so).  The holder waits for the copies before the object goes.
+constexpr size_t kStageBytes = size_t(4) << 20, kStageLarge = size_t(1) << 20, kStageArray = size_t(256) << 10;
 struct Stage {
   std::unique_ptr<char[]> base;
   char* dev = nullptr;  // the device block that mirrors it, copied up to `sent`
-  size_t used = 0, cap = 0, sent = 0;
+  size_t used = 0, cap = 0, sent = 0, most = 0;  // most: bytes of an array that it takes
   // room for `bytes` (at most cap - used)
   char* room(size_t bytes) {
     char* r = base.get() + used;
@@ -241,7 +243,7 @@ int dev_alloc(sgba_problem* p, T** ptr, size_t count) {
 template <class T, class A>
 int dev_upload(sgba_problem* p, T** ptr, const std::vector<T, A>& h) {
   const size_t bytes = sizeof(T) * h.size();
-  if (Stage* s = p->stage; s && bytes > 0 && bytes <= s->cap - s->used) {
+  if (Stage* s = p->stage; s && bytes > 0 && bytes <= s->most && bytes <= s->cap - s->used) {
     char* room = s->room(bytes);
     std::memcpy(room, h.data(), bytes);
     *ptr = reinterpret_cast<T*>(s->dev + (room - s->base.get()));
@@ -937,14 +939,16 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   for (int k = 0; k < 3; ++k) s.gauge_center[k] = P.gauge_center[k];
   int st;
   {
-    // about what the arrays below take; those that do not fit are copied one by one
+    // about what the arrays below take: all of a small problem, the small arrays
+    // of a larger one
     const size_t want = 24 * static_cast<size_t>(P.no) + 28 * static_cast<size_t>(P.ng) + 64 * static_cast<size_t>(P.np) +
                         128 * static_cast<size_t>(P.nc) + (size_t(64) << 10);
-    const size_t cap = std::min(want & ~size_t(255), kStageBytes);
+    const size_t cap = want <= kStageBytes ? want & ~size_t(255) : kStageLarge;
     p->stage->base.reset(new (std::nothrow) char[cap]);
     if (p->stage->base) {
       if ((st = dev_alloc(p, &p->stage->dev, cap))) return st;
       p->stage->cap = cap;
+      p->stage->most = want <= kStageBytes ? cap : kStageArray;
     }
   }
   // host staging of the copies below: alive until the stream is synchronised
@@ -1205,7 +1209,7 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
   // fx, alpha and beta nearly trade off over a camera's field of view, so
   // their block of S is close to singular and FP32 Jacobian products move the
   // step by ~1e-6 relative (measured on the 10-camera circle and the 4-camera
-  // example); and on the one-CTA solver (systems of at most 144 rows, bound
+  // example); and on the one-CTA solver (systems of at most 234 rows, bound
   // by launch latency, where float-float costs nothing measurable), where the
   // FP32 EUCM Jacobians left 7.6e-7 in the cost of the reference's
   // 10-camera benchmark scene.

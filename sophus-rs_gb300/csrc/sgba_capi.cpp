@@ -1250,6 +1250,8 @@ int upload(sgba_problem* p, const sgba_problem_desc* desc) {
     return st;
   if (s.dense_c == 0 && s.band_c == 0) {
     // multi-launch dense solver
+    if (!s.small_dense && sgba::panel_solver_setup(s.n6) != 0)
+      return set_error(SGBA_ERR_CUDA, "shared memory of the panel solver");
     if ((st = dev_alloc(p, &d.A, n6 * n6))) return st;
     if ((st = dev_alloc(p, &d.dpiv, n6))) return st;
     if ((st = dev_alloc(p, &d.wpanel, n6 * 48))) return st;

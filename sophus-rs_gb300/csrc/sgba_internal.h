@@ -451,6 +451,7 @@ int schur_dd_setup();            // of the float-float Schur pass
 int landmark_setup(int cap);     // of the chunked landmark pass
 int landmark_dd_setup(int cap);  // of its float-float variant
 int backsub_chunks_setup(int cap);  // the chunked back-substitution (0 = ok)
+int panel_solver_setup(int n);      // of the multi-launch dense solver
 int solver_launch_count(const Sizes& s);
 
 // Single-launch cluster solver (sgba_dense.cu): chooses the cluster size for

@@ -273,6 +273,14 @@ __global__ void __launch_bounds__(256) k_residual(int n, const double* __restric
 
 }  // namespace
 
+// k_ldlt_solve holds y, 4 bytes a row, in shared memory: above 48 KB from 12,289 rows on.
+int panel_solver_setup(int n) {
+  return raise_dynamic_smem(reinterpret_cast<const void*>(k_ldlt_solve), sizeof(float) * static_cast<size_t>(n)) ==
+                 cudaSuccess
+             ? 0
+             : -1;
+}
+
 int solver_launch_count(const Sizes& s) {
   const int pcg = s.pcg_mode ? pcg_launch_count(s) : 0;
   if (s.small_dense) return pcg + 1;
